@@ -202,3 +202,39 @@ def test_autotuner_picks_a_measured_kernel(tmp_path, monkeypatch):
     monkeypatch.setattr(autotune, "_mem", {})
     monkeypatch.setattr(autotune, "time_lu", lambda *a, **k: pytest.fail("timed again"))
     assert autotune.tune_lu(129)["kernel"] == rec["kernel"]
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("N,P,pad", [(32, 3, 0), (33, 3, 3), (255, 2, 1), (256, 310, 0), (257, 2, 3), (257, 310, 3),
+                                     (385, 306, 3), (511, 2, 1), (512, 306, 0), (513, 2, 0), (1023, 1, 1), (1025, 1, 3),
+                                     (1400, 1, 0), (1401, 2, 3),
+                                     (2048, 1, 0)])
+def test_lu_solve_block_edges(N, P, pad, dtype):
+    """The substitution at the edges of its row groups, of its kernels' size and batch ranges, and
+    with rows that do (ld a multiple of 4) and do not allow 16-byte loads. Tolerance: the normwise
+    backward error bound c N eps of LU with partial pivoting, c = 2 as for the factorization tests."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    ld = N + pad
+    tdt = torch.float64 if dtype == "f64" else torch.float32
+    g = torch.Generator(device="cuda").manual_seed(N + P)
+    A = torch.randn((P, N, ld), device="cuda", generator=g, dtype=tdt)
+    A[:, :, :N] += 0.1 * torch.eye(N, device="cuda", dtype=tdt)
+    A[:, :, N:] = float("nan")  # what lies between the rows is never used
+    b = torch.randn((P, N), device="cuda", generator=g, dtype=tdt)
+    F, x = A.clone(), b.clone()
+    piv = torch.empty((P, N), dtype=torch.int32, device="cuda")
+    info = torch.empty(P, dtype=torch.int32, device="cuda")
+    code, st = (0 if dtype == "f64" else 1), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    # the one-CTA FP64 factorization ends near N = 1500 (shared memory); the split one does not
+    kernel = 6 if dtype == "f64" and N > 1281 else 0
+    _lib.check(lib.bte_lu_factor_ex(code, P, N, ptr(F), ld, N * ld, ptr(piv), ptr(info), kernel, st), "lu_factor")
+    _lib.check(lib.bte_lu_solve(code, P, N, ptr(F), ld, N * ld, ptr(piv), ptr(x), st), "lu_solve")
+    torch.cuda.synchronize()
+    assert bool((info == 0).all())
+    for i in {0, P // 2, P - 1}:
+        Ad, xd, bd = A[i, :, :N].double(), x[i].double(), b[i].double()
+        berr = torch.linalg.norm(Ad @ xd - bd) / (torch.linalg.matrix_norm(Ad, 2) * torch.linalg.norm(xd) + torch.linalg.norm(bd))
+        assert float(berr) < 2 * N * torch.finfo(tdt).eps, (i, float(berr))
