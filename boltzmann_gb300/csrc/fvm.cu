@@ -2,12 +2,13 @@
 // solver_type "fully_implicit" (bte_1d3v_solver.py:1890-2009), preconditioned by its op-split
 // step (:1745-1870, type XVTVRC).
 //
-// Operator: one fused kernel (k_fvm_mvec, fvm_core.h) reads each value's upwind stencils along
-// x, v_r and v_theta and writes one output, after the ordinate moments m = w^T v
-// (k_fvm_moment) and the gain product G m (FP64 GEMM, Nr x Nr by Nr x Nx). The reference
+// Operator: one fused kernel (k_fvm_mvec, the arithmetic of fvm_core.h's fvm_mvec_at on tabulated
+// coefficients) reads each value's upwind stencils along x, v_r and v_theta and writes one
+// output, after the ordinate moments m = w^T v (k_fvm_moment) and the gain product G m over
+// the few non-zeros of G's rows (k_fvm_gain). The reference
 // multiplies dense (Nr Nvt)^2 collision and advection matrices instead; here the work per
 // value is O(p + Nr), so the operator is one read and one write of v (HBM-bound).
-// Preconditioner: the collision inverse in closed form, (D^-1 (x) I + H (x) 1 w^T) v, then the
+// Preconditioner: the collision inverse in closed form, (D^-1 (x) I + H (x) 1 w^T) v (k_fvm_hmul), then the
 // v_r, v_theta and x sweeps in the natural layout: the v_r and v_theta recurrences run one
 // thread per line with the warp's lanes on consecutive x (coalesced), the x recurrence on rows
 // staged in shared memory; the reference (and the drop-in sweeps of sweeps.cu) swap layouts
@@ -38,6 +39,14 @@ struct bte_fvm {
     bool have_inverse = false;
     double *M = nullptr, *T = nullptr, *aE = nullptr, *axvr = nullptr;   // (Nr, Nx), (Nr, Nx), Nx, Nr
     double *A = nullptr, *Bf = nullptr;                                  // N each
+    // operator coefficients of a step (k_fvm_mvec_coef) and their set-up parts
+    double *bx = nullptr, *arc = nullptr, *lr = nullptr, *vinv = nullptr;  // Nx, Nr Nvt, Nr, Nr
+    int8_t *eflag = nullptr, *cpos = nullptr;                             // Nx: bit 0 E >= 0, bit 1 E < 0; Nvt: cos > 0
+    int32_t *gptr = nullptr, *gcol = nullptr;                             // the gain matrix by rows (exact non-zeros)
+    double* gval = nullptr;
+    uint32_t* hmask = nullptr;   // per 8-row tile of H: which chunks of HC columns hold a non-zero
+    int32_t* bad = nullptr;      // per x: a non-finite ordinate moment (it reaches every row of G m and H m)
+    double* swc = nullptr;       // sweep coefficients (k_fvm_sweep_coef), allocated on first use
     double *B = nullptr, *X = nullptr, *R = nullptr, *W = nullptr, *Z = nullptr, *Tv = nullptr;
     double* Kr = nullptr;
     int kcap = 0;
@@ -72,202 +81,369 @@ FvmView view_of(const bte_fvm* h) {
     return v;
 }
 
-// m[r][x] = sum_j w_j X[r][j][x], one thread per (r, x)
-__global__ void k_fvm_moment(FvmView v, const double* __restrict__ X, double* __restrict__ m) {
+// GB300 runs FP64 at 2 fused multiply-adds per clock and SM: a warp instruction (compares and
+// conversions included) occupies its sub-partition's FP64 pipe for 64 cycles, and 16 bytes from
+// L2 cost less than one. The kernels of this file are bound by that pipe, so what does not depend
+// on the vector is tabulated once per step, divisions above all.
+
+// m[r][x] = sum_j w_j X[r][j][x], one thread per (r, x); bad[x] is set where a moment is not finite
+__global__ void k_fvm_moment(FvmView v, const double* __restrict__ X, double* __restrict__ m, int32_t* bad) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)v.Nr * v.Nx) return;
     const int x = (int)(i % v.Nx), r = (int)(i / v.Nx);
-    m[i] = fvm_moment_at(v, X, r, x);
+    const double s = fvm_moment_at(v, X, r, x);
+    m[i] = s;
+    if ((__double2hiint(s) & 0x7ff00000) == 0x7ff00000) bad[x] = 1;  // Inf or NaN, without an FP64 instruction
 }
 
-// Y = rhs_mvec(X), one thread per value, x fastest
-__global__ void k_fvm_mvec(FvmView v, FvmCoef c, const double* __restrict__ E, const double* __restrict__ G,
-                           const double* __restrict__ X, double* __restrict__ Y) {
+// The operator's coefficients for a step: bx = dt tau cA E, arc = dtx ax v_r cos(theta), lr =
+// dt tau kappa loss, and the sign of E as bits
+__global__ void k_fvm_mvec_coef(FvmView v, FvmCoef c, const double* __restrict__ E, double* __restrict__ bx,
+                                double* __restrict__ arc, double* __restrict__ lr, int8_t* __restrict__ eflag) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < v.Nx) {
+        const double e = E[i];
+        bx[i] = c.dt * c.tau * (e * c.cA);
+        eflag[i] = (int8_t)((e >= 0.0 ? 1 : 0) | (e < 0.0 ? 2 : 0));
+    }
+    if (i < v.Nr) lr[i] = c.dt * c.tau * (c.kappa * v.loss[i]);
+    if (i < v.Nr * v.Nvt) arc[i] = c.dtx * c.ax * v.vr[i / v.Nvt] * v.cos_t[i % v.Nvt];
+}
+
+// T = kt (G m) over the non-zeros of G's rows: at most two per process and row
+__global__ void k_fvm_gain(int Nr, int Nx, double kt, const int32_t* __restrict__ ptr, const int32_t* __restrict__ col,
+                           const double* __restrict__ val, const double* __restrict__ m, const int32_t* __restrict__ bad,
+                           double* __restrict__ T) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= Nr * Nx) return;
+    const int x = i % Nx, r = i / Nx;
+    double s = 0.0;
+    for (int e = ptr[r]; e < ptr[r + 1]; ++e) s += val[e] * m[(size_t)col[e] * Nx + x];
+    T[i] = bad[x] ? __longlong_as_double(0x7ff8000000000000ll) : kt * s;
+}
+
+// Y = rhs_mvec(X) (fvm_mvec_at) with the tabulated coefficients, one thread per value, x fastest:
+// three stencils and seven more FP64 instructions per value; the form that computes them all per
+// value took 33 with a division (976,000 values, 200 x 305 x 16: 61 us -> 29 us; 16 FP64
+// instructions take 26 us). T = dt tau kappa G m.
+__global__ void k_fvm_mvec(FvmView v, const double* __restrict__ bx, const double* __restrict__ arc,
+                           const double* __restrict__ lr, const double* __restrict__ vinv,
+                           const int8_t* __restrict__ eflag, const int8_t* __restrict__ cpos,
+                           const double* __restrict__ T, const double* __restrict__ X, double* __restrict__ Y,
+                           int32_t* bad) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t n = (size_t)v.Nr * v.Nvt * v.Nx;
     if (i >= n) return;
     const int x = (int)(i % v.Nx);
-    const size_t rj = i / v.Nx;
-    const int j = (int)(rj % v.Nvt), r = (int)(rj / v.Nvt);
-    Y[i] = fvm_mvec_at(v, c, E, G, X, r, j, x);
+    const int rj = (int)(i / v.Nx);
+    const int j = rj % v.Nvt, r = rj / v.Nvt;
+    if (rj == 0) bad[x] = 0;  // the moments of the next product start clean
+    const double* line = X + (size_t)rj * v.Nx;
+    const double z = line[x];
+    const bool nx = v.north[j] != 0;
+    const double yx = z + arc[rj] * fvm_band_row(nx ? v.xL : v.xR, v.ndx, v.Nx, x, nx, line, 1);
+    if (fvm_inflow(v, j, x)) {
+        Y[i] = yx;
+        return;
+    }
+    const int e = eflag[x];
+    const bool up_r = ((e & 1) != 0) == (cpos[j] != 0);
+    const double dr = fvm_band_row(up_r ? v.vrR : v.vrL, v.ndr, v.Nr, r, !up_r, X + (size_t)j * v.Nx + x,
+                                   (long long)v.Nvt * v.Nx);
+    const bool lo_t = (e & 2) != 0;
+    const double dth = fvm_band_row(lo_t ? v.vtL : v.vtR, v.ndt, v.Nvt, j, lo_t, X + (size_t)r * v.Nvt * v.Nx + x,
+                                    (long long)v.Nx);
+    const double adv = v.cos_t[j] * dr - vinv[r] * dth;
+    Y[i] = (yx - T[(size_t)r * v.Nx + x]) + lr[r] * z - bx[x] * adv;
+}
+
+// T = H M (Nr x Nr by Nr x Nx) for the collision inverse. One warp per 8 rows x 32 columns and a
+// quarter of the columns of H, the four partial sums added in a fixed order. Chunks of HC columns
+// that hold no non-zero in the 8 rows are passed over: collisions only move electrons down in
+// energy, so most of H below its diagonal is zero. 305 x 305 by 200: 101 us as a general product
+// of 32 x 32 tiles (70 CTAs) -> 38 us; all its FP64 multiply-adds take 31 us.
+constexpr int HR = 8;    // rows per tile
+constexpr int HC = 16;   // columns of H per chunk
+__global__ void __launch_bounds__(128)
+k_fvm_hmul(int Nr, int Nx, int words, const uint32_t* __restrict__ mask, const double* __restrict__ H,
+           const double* __restrict__ M, const int32_t* __restrict__ bad, double* __restrict__ T) {
+    __shared__ double part[3][HR][32];
+    __shared__ __align__(16) double sh[4][HC][HR];  // a warp's chunk of H, transposed
+    const int r0 = blockIdx.y * HR, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int x = blockIdx.x * 32 + lane, xc = min(x, Nx - 1);
+    const uint32_t* mk = mask + (size_t)blockIdx.y * words;
+    double acc[HR];
+#pragma unroll
+    for (int i = 0; i < HR; ++i) acc[i] = 0.0;
+    double mv[HC], hv[HR * HC / 32];
+    // chunk c: HC rows of M, and H's HR x HC block (rows r0 .., lane -> column lane % HC)
+    auto fetch = [&](int c) {
+        const int k0 = c * HC;
+#pragma unroll
+        for (int k = 0; k < HC; ++k) mv[k] = M[(size_t)min(k0 + k, Nr - 1) * Nx + xc];
+        const int k = min(k0 + lane % HC, Nr - 1);
+#pragma unroll
+        for (int q = 0; q < HR * HC / 32; ++q) {
+            const int r = min(r0 + lane / HC + q * (32 / HC), Nr - 1);
+            hv[q] = (k0 + lane % HC < Nr) ? H[(size_t)r * Nr + k] : 0.0;
+        }
+    };
+    int seen = 0;  // the tile's chunks go to the four warps in turn
+    for (int cw = 0; cw < words; ++cw) {
+        uint32_t bits = mk[cw];
+        while (bits) {
+            const int c = 32 * cw + __ffs(bits) - 1;
+            bits &= bits - 1;
+            if ((seen++ & 3) != w) continue;
+            fetch(c);
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < HR * HC / 32; ++q) sh[w][lane % HC][lane / HC + q * (32 / HC)] = hv[q];
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < HC; ++k)
+#pragma unroll
+                for (int i = 0; i < HR; i += 2) {
+                    const double2 h2 = *reinterpret_cast<const double2*>(&sh[w][k][i]);
+                    acc[i] += h2.x * mv[k];
+                    acc[i + 1] += h2.y * mv[k];
+                }
+        }
+    }
+    if (w > 0)
+#pragma unroll
+        for (int i = 0; i < HR; ++i) part[w - 1][i][lane] = acc[i];
+    __syncthreads();
+    if (w > 0 || x >= Nx) return;
+    const bool nan = bad[x] != 0;
+#pragma unroll
+    for (int i = 0; i < HR; ++i)
+        if (r0 + i < Nr)
+            T[(size_t)(r0 + i) * Nx + x] = nan ? __longlong_as_double(0x7ff8000000000000ll)
+                                               : ((acc[i] + part[0][i][lane]) + part[1][i][lane]) + part[2][i][lane];
 }
 
 // out (Nx, Nvt, Nr) = the collision inverse applied to B (Nr, Nvt, Nx), one thread per output
 __global__ void k_fvm_coll_permute(FvmView v, const double* __restrict__ dinv, const double* __restrict__ T,
-                                   const double* __restrict__ B, double* __restrict__ out) {
+                                   const double* __restrict__ B, double* __restrict__ out, int32_t* bad) {
     const size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t n = (size_t)v.Nr * v.Nvt * v.Nx;
     if (o >= n) return;
     const int r = (int)(o % v.Nr);
     const size_t xj = o / v.Nr;
     const int j = (int)(xj % v.Nvt), x = (int)(xj / v.Nvt);
+    if (j == 0 && r == 0) bad[x] = 0;
     out[o] = fvm_coll_apply_at(v, dinv, T, B, r, j, x);
 }
 
-// Y (Nr, Nvt, Nx) = the collision inverse applied to B, same layout
+// Y (Nr, Nvt, Nx) = the collision inverse applied to B, same layout, times sc where given (the
+// diagonal reciprocals of the sweep that follows)
 __global__ void k_fvm_coll_apply(FvmView v, const double* __restrict__ dinv, const double* __restrict__ T,
-                                 const double* __restrict__ B, double* __restrict__ Y) {
+                                 const double* __restrict__ B, const double* __restrict__ sc, double* __restrict__ Y,
+                                 int32_t* bad) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t n = (size_t)v.Nr * v.Nvt * v.Nx;
     if (i >= n) return;
     const int x = (int)(i % v.Nx);
     const size_t rj = i / v.Nx;
-    Y[i] = fvm_coll_apply_at(v, dinv, T, B, (int)(rj / v.Nvt), (int)(rj % v.Nvt), x);
+    if (rj == 0) bad[x] = 0;  // the moments of the next product start clean
+    const double y = fvm_coll_apply_at(v, dinv, T, B, (int)(rj / v.Nvt), (int)(rj % v.Nvt), x);
+    Y[i] = sc ? y * sc[i] : y;
 }
 
-// Y = the semi-Lagrangian advection of V, one thread per value
 // ---- preconditioner sweeps in the natural (Nr, Nvt, Nx) layout --------------------------------
-// One upwind backward-Euler recurrence (I + a h D) o = b per thread along a line of N values
-// spaced `stride` apart, in place. The bands are the sweeps' column-stored ones (lower
-// D[i][i-k] = L[k][i-k], upper D[i][i+k] = R[k][i+k], rawkernel.py:168-375); the last nd - 1
-// outputs of the line stay in registers. Along v_r (stride Nvt Nx) and v_theta (stride Nx)
-// the threads of a warp take consecutive x, so every step is one coalesced 256-byte access:
-// no layout swaps, unlike the reference's sweeps on permuted copies. L and R are the calling
-// CTA's shared-memory copies of the bands (stage_bands), so a step waits on no global load but
-// its right-hand side, which is loaded SW_PF steps ahead.
+// An upwind backward-Euler solve (I + a h D) o = b along a line is the recurrence
+//   o_i = (b_i - a h sum_k D[i][i -/+ k] o_{i -/+ k}) / (1 + a h D[i][i])
+// (bands column-stored: lower D[i][i-k] = L[k][i-k], upper D[i][i+k] = R[k][i+k],
+// rawkernel.py:168-375). The lines are few and long (one warp on an SM sub-partition, 64 cycles
+// per FP64 instruction), so the chain is cut to its nd - 1 multiply-adds: k_fvm_sweep_coef
+// tabulates rho_i = 1 / (1 + a h D[i][i]) and c_k,i = a h D[i][i -/+ k] rho_i once per step, the
+// kernel before each sweep (or its load) multiplies b by rho, and the sweep is
+//   o_i = b_i - sum_k c_k,i o_{i -/+ k}.
+// Along v_r (stride Nvt Nx) and v_theta (stride Nx) the threads of a warp take consecutive x, so
+// every step is one coalesced access; x rows are staged in shared memory, their c_k in
+// line-fastest order. Against recurrences of five FP64 instructions (200 x 305 x 16): v_r 94 ->
+// 30 us, v_theta 35 -> 12 us, x 66 -> 39 us, and no reciprocals per application (37 us).
 constexpr int SW_NDMAX = 4;
-constexpr int SW_PF = 8;   // right-hand sides loaded ahead of the recurrence
-__device__ inline void stage_bands(const double* __restrict__ L, const double* __restrict__ R, int nd, int N,
-                                   double* sL, double* sR) {
-    for (int e = threadIdx.x; e < nd * N; e += blockDim.x) {
-        sL[e] = L[e];
-        sR[e] = R[e];
+constexpr int SW_U = 16;  // steps of a long line whose loads are in flight ahead of the chain
+constexpr int SW_US = 8;  // of the short v_theta lines, where more resident warps pay instead
+
+// a of the three sweeps' lines and the direction: 0 v_r (a = -aE cos, rawkernel.py:168-230),
+// 1 v_theta (a = aE / v_r, sweeping left to right when -a >= 0, :232-296), 2 x (a = ax v_r cos, :298-375)
+struct FvmSweep {
+    const double *L, *R;
+    int nd, N;
+};
+__device__ inline void sweep_coef(const FvmSweep& d, double ad, bool ltr, int i, double* rho, double c[SW_NDMAX - 1]) {
+    const double* B = ltr ? d.L : d.R;
+    const double q = 1.0 / (1.0 + ad * B[i]);
+    *rho = q;
+#pragma unroll
+    for (int k = 1; k < SW_NDMAX; ++k) {
+        const int o = ltr ? i - k : i + k;
+        c[k - 1] = (k < d.nd && o >= 0 && o < d.N) ? ad * B[(size_t)k * d.N + o] * q : 0.0;
     }
 }
-// With rc (the reciprocals of the line's diagonal 1 + ad D[i][i], at the same positions as v,
-// k_fvm_diag_rcp) a step is five FP64 operations instead of a division's dozen: the few long
-// v_r and x lines run one warp per SM, each bound by its SM sub-partition's FP64 issue rate.
-template <bool RC>
-__device__ inline void fvm_sweep_line(const double* L, const double* R, int nd, int N,
-                                      double ad, bool ltr, double* __restrict__ v, long long stride,
-                                      const double* __restrict__ rc = nullptr) {
-    double prev[SW_NDMAX - 1];
+
+// Layout of the table (arrays of N values): v_r rho, c_1 .., v_theta rho, c_1 .., x rho, all in the
+// natural layout, then the x sweep's c_1 .. at [x][line], line = r Nvt + j. One CTA per (line
+// block of 32, x block of 32).
+__global__ void __launch_bounds__(256)
+k_fvm_sweep_coef(FvmView v, const double* __restrict__ aE, const double* __restrict__ axvr, double h,
+                 double* __restrict__ tab) {
+    __shared__ double tile[SW_NDMAX - 1][32][33];
+    const int nlines = v.Nr * v.Nvt;
+    const size_t n = (size_t)nlines * v.Nx;
+    const int l0 = blockIdx.y * 32, x0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    double* tr = tab;
+    double* tt = tr + (size_t)v.ndr * n;
+    double* xr = tt + (size_t)v.ndt * n;
+    double* xc = xr + n;
+    double rho, c[SW_NDMAX - 1];
+    for (int l = ty; l < 32; l += 8) {
+        const int line = l0 + l, x = x0 + tx;
 #pragma unroll
-    for (int k = 0; k < SW_NDMAX - 1; ++k) prev[k] = 0.0;
-    const double* B = ltr ? L : R;
-    // the loads of b (and of the reciprocals) do not depend on the recurrence: keep SW_PF of
-    // them in flight
-    double pf[SW_PF], pr[SW_PF];
-#pragma unroll
-    for (int q = 0; q < SW_PF; ++q) {
-        const long long o = (long long)(ltr ? q : N - 1 - q) * stride;
-        pf[q] = (q < N) ? v[o] : 0.0;
-        if (RC) pr[q] = (q < N) ? rc[o] : 0.0;
-    }
-    for (int step = 0; step < N; ++step) {
-        const int i = ltr ? step : N - 1 - step;
-        const double bi = pf[0];
-        const double ri = RC ? pr[0] : 0.0;
-#pragma unroll
-        for (int q = 0; q < SW_PF - 1; ++q) {
-            pf[q] = pf[q + 1];
-            if (RC) pr[q] = pr[q + 1];
+        for (int k = 0; k < SW_NDMAX - 1; ++k) c[k] = 0.0;
+        if (line < nlines && x < v.Nx) {
+            const int j = line % v.Nvt, r = line / v.Nvt;
+            const size_t o = (size_t)line * v.Nx + x;
+            double a = -aE[x] * v.cos_t[j];
+            sweep_coef(FvmSweep{v.vrL, v.vrR, v.ndr, v.Nr}, a * h, a >= 0.0, r, &rho, c);
+            tr[o] = rho;
+            for (int k = 1; k < v.ndr; ++k) tr[k * n + o] = c[k - 1];
+            a = aE[x] / v.vr[r];
+            sweep_coef(FvmSweep{v.vtL, v.vtR, v.ndt, v.Nvt}, a * h, -a >= 0.0, j, &rho, c);
+            tt[o] = rho;
+            for (int k = 1; k < v.ndt; ++k) tt[k * n + o] = c[k - 1];
+            a = axvr[r] * v.cos_t[j];
+            sweep_coef(FvmSweep{v.xL, v.xR, v.ndx, v.Nx}, a * h, a >= 0.0, x, &rho, c);
+            xr[o] = rho;
         }
-        const int nxt = step + SW_PF;
-        const long long on = (long long)(ltr ? nxt : N - 1 - nxt) * stride;
-        pf[SW_PF - 1] = (nxt < N) ? v[on] : 0.0;
-        if (RC) pr[SW_PF - 1] = (nxt < N) ? rc[on] : 0.0;
-        double sacc = 0.0;
 #pragma unroll
-        for (int k = 1; k < SW_NDMAX; ++k)
-            if (k < nd && step >= k) sacc += B[(size_t)k * N + (ltr ? i - k : i + k)] * prev[k - 1];
-        const double o = RC ? (bi - ad * sacc) * ri : (bi - ad * sacc) / (1.0 + ad * B[i]);
-#pragma unroll
-        for (int k = SW_NDMAX - 2; k > 0; --k) prev[k] = prev[k - 1];
-        prev[0] = o;
-        v[(long long)i * stride] = o;
+        for (int k = 0; k < SW_NDMAX - 1; ++k) tile[k][l][tx] = c[k];
     }
-}
-
-// Rc = 1 / (1 + a h D[i][i]) at every position of the natural layout, for the v_r sweep
-// (which = 0: a and the band as k_fvm_sweep_vr takes them, i = r) or the x sweep (which = 2:
-// as k_fvm_sweep_x, i = x); all SMs share the divisions the recurrences would serialise
-__global__ void k_fvm_diag_rcp(FvmView v, int which, const double* __restrict__ aE,
-                               const double* __restrict__ axvr, double h, double* __restrict__ Rc) {
-    const size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t n = (size_t)v.Nr * v.Nvt * v.Nx;
-    if (o >= n) return;
-    const int x = (int)(o % v.Nx);
-    const size_t rj = o / v.Nx;
-    const int j = (int)(rj % v.Nvt), r = (int)(rj / v.Nvt);
-    double a, d;
-    if (which == 0) {
-        a = -aE[x] * v.cos_t[j];
-        d = (a >= 0.0 ? v.vrL : v.vrR)[r];
-    } else {
-        a = axvr[r] * v.cos_t[j];
-        d = (a >= 0.0 ? v.xL : v.xR)[x];
-    }
-    const double ad = a * h;
-    Rc[o] = 1.0 / (1.0 + ad * d);
-}
-
-// v_r sweep: line (j, x), a = -aE[x] cos(theta_j), left to right when a >= 0 (rawkernel.py:168-230)
-__global__ void k_fvm_sweep_vr(FvmView v, const double* __restrict__ aE, double h, double* __restrict__ V,
-                               const double* __restrict__ Rc) {
-    extern __shared__ double sband[];  // [2][ndr][Nr]
-    double *sL = sband, *sR = sband + (size_t)v.ndr * v.Nr;
-    stage_bands(v.vrL, v.vrR, v.ndr, v.Nr, sL, sR);
     __syncthreads();
+    for (int x = ty; x < 32; x += 8)
+        if (x0 + x < v.Nx && l0 + tx < nlines)
+            for (int k = 1; k < v.ndx; ++k)
+                xc[(k - 1) * n + (size_t)(x0 + x) * nlines + l0 + tx] = tile[k - 1][tx][x];
+}
+
+// The recurrence along one line of N values spaced `stride`: v in and out (v already times rho
+// unless rho is given), c_k at c + k cstep with spacing cstride
+template <int ND, int U, bool RHO>
+__device__ inline void sweep_line(int N, bool ltr, double* v, long long stride, const double* __restrict__ c,
+                                  size_t cstep, long long cstride, const double* __restrict__ rho) {
+    double prev[ND > 1 ? ND - 1 : 1];
+#pragma unroll
+    for (int k = 0; k < ND - 1; ++k) prev[k] = 0.0;
+    double nb[U], nc[ND > 1 ? ND - 1 : 1][U], nr[U];
+    auto fetch = [&](int s0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int st = min(s0 + u, N - 1);
+            const int i = ltr ? st : N - 1 - st;
+            nb[u] = v[i * stride];
+            if (RHO) nr[u] = rho[i * stride];
+#pragma unroll
+            for (int k = 0; k < ND - 1; ++k) nc[k][u] = c[k * cstep + i * cstride];
+        }
+    };
+    fetch(0);
+    for (int s0 = 0; s0 < N; s0 += U) {
+        double b[U], cc[ND > 1 ? ND - 1 : 1][U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            b[u] = RHO ? nb[u] * nr[u] : nb[u];
+#pragma unroll
+            for (int k = 0; k < ND - 1; ++k) cc[k][u] = nc[k][u];
+        }
+        if (s0 + U < N) fetch(s0 + U);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (s0 + u >= N) break;
+            const int i = ltr ? s0 + u : N - 1 - s0 - u;
+            double o = b[u];
+            // the oldest value first: only the last multiply-add waits for the step before
+#pragma unroll
+            for (int k = ND - 2; k >= 0; --k) o -= cc[k][u] * prev[k];
+#pragma unroll
+            for (int k = ND - 2; k > 0; --k) prev[k] = prev[k - 1];
+            if (ND > 1) prev[0] = o;
+            v[i * stride] = o;
+        }
+    }
+}
+template <int U, bool RHO>
+__device__ inline void sweep_line_nd(int nd, int N, bool ltr, double* v, long long stride, const double* c, size_t cstep,
+                                     long long cstride, const double* rho) {
+    if (nd == 1) sweep_line<1, U, RHO>(N, ltr, v, stride, c, cstep, cstride, rho);
+    else if (nd == 2) sweep_line<2, U, RHO>(N, ltr, v, stride, c, cstep, cstride, rho);
+    else if (nd == 3) sweep_line<3, U, RHO>(N, ltr, v, stride, c, cstep, cstride, rho);
+    else sweep_line<4, U, RHO>(N, ltr, v, stride, c, cstep, cstride, rho);
+}
+
+// v_r sweep of V (times rho already): line (j, x), one thread each
+__global__ void k_fvm_sweep_vr(FvmView v, const double* __restrict__ aE, double* __restrict__ V,
+                               const double* __restrict__ c) {
     const int line = blockIdx.x * blockDim.x + threadIdx.x;
     if (line >= v.Nvt * v.Nx) return;
     const int j = line / v.Nx, x = line % v.Nx;
+    const long long st = (long long)v.Nvt * v.Nx;
     const double a = -aE[x] * v.cos_t[j];
-    fvm_sweep_line<true>(sL, sR, v.ndr, v.Nr, a * h, a >= 0.0, V + (size_t)j * v.Nx + x, (long long)v.Nvt * v.Nx,
-                         Rc + (size_t)j * v.Nx + x);
+    sweep_line_nd<SW_U, false>(v.ndr, v.Nr, a >= 0.0, V + line, st, c + line, (size_t)v.Nr * st, st, nullptr);
 }
 
-// v_theta sweep: line (r, x), a = aE[x] / v_r, left to right when -a >= 0 (rawkernel.py:232-296)
-__global__ void k_fvm_sweep_vt(FvmView v, const double* __restrict__ aE, double h, double* __restrict__ V) {
-    extern __shared__ double sband[];  // [2][ndt][Nvt]
-    double *sL = sband, *sR = sband + (size_t)v.ndt * v.Nvt;
-    stage_bands(v.vtL, v.vtR, v.ndt, v.Nvt, sL, sR);
-    __syncthreads();
+// v_theta sweep: line (r, x), one thread each
+__global__ void k_fvm_sweep_vt(FvmView v, const double* __restrict__ aE, double* __restrict__ V,
+                               const double* __restrict__ rho, const double* __restrict__ c) {
     const int line = blockIdx.x * blockDim.x + threadIdx.x;
     if (line >= v.Nr * v.Nx) return;
     const int r = line / v.Nx, x = line % v.Nx;
-    const double a = aE[x] / v.vr[r];
-    fvm_sweep_line<false>(sL, sR, v.ndt, v.Nvt, a * h, -a >= 0.0, V + (size_t)r * v.Nvt * v.Nx + x, (long long)v.Nx);
+    const size_t o = (size_t)r * v.Nvt * v.Nx + x;
+    // the direction -aE / v_r >= 0 without the division (v_r > 0; a quotient that underflows to 0
+    // leaves the line as it is in either direction)
+    sweep_line_nd<SW_US, true>(v.ndt, v.Nvt, aE[x] <= 0.0, V + o, (long long)v.Nx, c + o, (size_t)v.Nr * v.Nvt * v.Nx,
+                        (long long)v.Nx, rho + o);
 }
 
-// x sweep with the inflow values zeroed first: line (r, j) is a contiguous row of Nx values;
-// a CTA stages XT_L consecutive rows (one contiguous block) in shared memory with coalesced
-// loads, sweeps each row in shared memory (row pitch Nx + 1 against bank conflicts) and
-// writes the block back coalesced. a = ax v_r cos(theta_j), left to right when a >= 0
-// (rawkernel.py:298-375).
-constexpr int XT_L = 32;       // rows per CTA
-constexpr int XT_T = 256;      // threads per CTA: all load and store, the first XT_L sweep
-__global__ void __launch_bounds__(XT_T) k_fvm_sweep_x(FvmView v, const double* __restrict__ axvr, double h,
+// x sweep with the inflow values zeroed first: line (r, j) is a contiguous row of Nx values; a CTA
+// stages `rows` consecutive rows times rho in shared memory with coalesced loads, one thread
+// sweeps each row there (row pitch Nx + 1 against bank conflicts), and the block is written back
+// coalesced
+constexpr int XT_L = 32;       // most rows per CTA
+constexpr int XT_T = 128;      // threads per CTA: all load and store, the first `rows` sweep (registers of two CTAs per SM)
+__global__ void __launch_bounds__(XT_T, 2) k_fvm_sweep_x(FvmView v, int rows, const double* __restrict__ axvr,
                                                       const double* __restrict__ B, double* __restrict__ Y,
-                                                      const double* __restrict__ Rc) {
-    extern __shared__ double rows[];  // [XT_L][Nx + 1], then the bands [2][ndx][Nx]
+                                                      const double* __restrict__ rho, const double* __restrict__ c) {
+    extern __shared__ double buf[];  // [rows][Nx + 1]
     const int Nx = v.Nx, pitch = Nx + 1;
-    double* sL = rows + (size_t)XT_L * pitch;
-    double* sR = sL + (size_t)v.ndx * Nx;
-    stage_bands(v.xL, v.xR, v.ndx, Nx, sL, sR);
     const int nlines = v.Nr * v.Nvt;
-    const int l0 = blockIdx.x * XT_L;
-    const int nl = min(XT_L, nlines - l0);
+    const int l0 = blockIdx.x * rows;
+    const int nl = min(rows, nlines - l0);
     const double* src = B + (size_t)l0 * Nx;
+    const double* rs = rho + (size_t)l0 * Nx;
+#pragma unroll 4
     for (int e = threadIdx.x; e < nl * Nx; e += blockDim.x) {
         const int l = e / Nx, x = e % Nx;
         const int j = (l0 + l) % v.Nvt;
         const bool inflow = v.north[j] ? (x == 0) : (x == Nx - 1);
-        rows[l * pitch + x] = inflow ? 0.0 : src[e];
+        const double y = src[e] * rs[e];
+        buf[l * pitch + x] = inflow ? 0.0 : y;
     }
     __syncthreads();
     if (threadIdx.x < nl) {
         const int line = l0 + threadIdx.x;
-        const int r = line / v.Nvt, j = line % v.Nvt;
-        const double a = axvr[r] * v.cos_t[j];
-        fvm_sweep_line<true>(sL, sR, v.ndx, Nx, a * h, a >= 0.0, rows + threadIdx.x * pitch, 1,
-                             Rc + (size_t)line * Nx);
+        const double a = axvr[line / v.Nvt] * v.cos_t[line % v.Nvt];
+        sweep_line_nd<SW_U, false>(v.ndx, Nx, a >= 0.0, buf + threadIdx.x * pitch, 1, c + line, (size_t)nlines * Nx,
+                             (long long)nlines, nullptr);
     }
     __syncthreads();
     double* dst = Y + (size_t)l0 * Nx;
-    for (int e = threadIdx.x; e < nl * Nx; e += blockDim.x) dst[e] = rows[(e / Nx) * pitch + e % Nx];
+    for (int e = threadIdx.x; e < nl * Nx; e += blockDim.x) dst[e] = buf[(e / Nx) * pitch + e % Nx];
 }
 
+// Y = the semi-Lagrangian advection of V, one thread per value
 __global__ void k_fvm_sl(FvmSl sl, const double* __restrict__ E, const double* __restrict__ V, double* __restrict__ Y) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t n = (size_t)sl.Nr * sl.Nvt * sl.Nx;
@@ -351,34 +527,77 @@ int sweep_rc(int rc, const char* what) {
     return fvm_fail(BTE_ERR_CUDA, std::string(what) + ": " + bte_sweep_last_error());
 }
 
-// Y = rhs_mvec(X) on stream s
-int fvm_mvec(bte_fvm* h, const FvmCoef& c, const double* E, const double* X, double* Y, cudaStream_t s) {
+// the coefficients of rhs_mvec for a step at field E
+int fvm_mvec_coef(bte_fvm* h, const FvmCoef& c, const double* E, cudaStream_t s) {
+    const size_t m = std::max((size_t)h->Nr * h->Nvt, (size_t)h->Nx);
+    k_fvm_mvec_coef<<<fblocks(m), FT, 0, s>>>(view_of(h), c, E, h->bx, h->arc, h->lr, h->eflag);
+    ++h->launches;
+    return launched("k_fvm_mvec_coef");
+}
+
+// Y = rhs_mvec(X) on stream s (fvm_mvec_coef done)
+int fvm_mvec(bte_fvm* h, const FvmCoef& c, const double* X, double* Y, cudaStream_t s) {
     const FvmView v = view_of(h);
     const size_t nrx = (size_t)h->Nr * h->Nx;
-    k_fvm_moment<<<fblocks(nrx), FT, 0, s>>>(v, X, h->M);
+    k_fvm_moment<<<fblocks(nrx), FT, 0, s>>>(v, X, h->M, h->bad);
     if (int rc = launched("k_fvm_moment")) return rc;
-    if (int rc = sweep_rc(bte_dgemm_nn(h->Nr, h->Nx, h->Nr, h->gain, h->Nr, h->M, h->Nx, h->T, h->Nx, s), "gain product"))
-        return rc;
-    k_fvm_mvec<<<fblocks(h->N), FT, 0, s>>>(v, c, E, h->T, X, Y);
+    k_fvm_gain<<<fblocks(nrx), FT, 0, s>>>(h->Nr, h->Nx, c.dt * c.tau * c.kappa, h->gptr, h->gcol, h->gval, h->M, h->bad,
+                                           h->T);
+    if (int rc = launched("k_fvm_gain")) return rc;
+    k_fvm_mvec<<<fblocks(h->N), FT, 0, s>>>(v, h->bx, h->arc, h->lr, h->vinv, h->eflag, h->cpos, h->T, X, Y, h->bad);
     h->launches += 3;
     return launched("k_fvm_mvec");
 }
 
-// Y = the op-split step applied to X (aE = cE E must already be in h->aE, ax v_r in h->axvr)
+// T = H (moments of X)
+int fvm_hmul(bte_fvm* h, const double* X, cudaStream_t s) {
+    const int Nr = h->Nr, Nx = h->Nx;
+    k_fvm_moment<<<fblocks((size_t)Nr * Nx), FT, 0, s>>>(view_of(h), X, h->M, h->bad);
+    if (int rc = launched("k_fvm_moment")) return rc;
+    const int words = ((Nr + HC - 1) / HC + 31) / 32;
+    k_fvm_hmul<<<dim3((unsigned)((Nx + 31) / 32), (unsigned)((Nr + HR - 1) / HR)), 128, 0, s>>>(Nr, Nx, words, h->hmask,
+                                                                                            h->H, h->M, h->bad, h->T);
+    h->launches += 2;
+    return launched("k_fvm_hmul");
+}
+
+// rows per CTA of the x sweep: two CTAs per SM where the lines allow it, as many rows as fit in
+// 200 KB; 0 when not even four do
+int sweep_x_rows(const bte_fvm* h) {
+    const int lines = h->Nr * h->Nvt;
+    const int fit = (int)(200 * 1024 / ((size_t)(h->Nx + 1) * sizeof(double)));
+    const int want = std::max(4, (lines + 2 * 152 - 1) / (2 * 152));
+    const int rows = std::min(std::min(XT_L, fit), want);
+    return rows >= 4 ? rows : 0;
+}
+
+// the sweeps that run on the natural layout: stencils up to SW_NDMAX points, x rows that fit
+bool natural_sweeps(const bte_fvm* h) {
+    return h->ndr <= SW_NDMAX && h->ndt <= SW_NDMAX && h->ndx <= SW_NDMAX && sweep_x_rows(h) > 0;
+}
+
+// the sweep coefficients for step h at the coefficients in h->aE, h->axvr
+int fvm_sweep_coef(bte_fvm* h, double hstep, cudaStream_t s) {
+    if (!natural_sweeps(h)) return BTE_OK;
+    const size_t arrays = (size_t)h->ndr + h->ndt + h->ndx;
+    if (!h->swc)
+        if (int rc = fvm_alloc(h, (void**)&h->swc, arrays * h->N * sizeof(double))) return rc;
+    const dim3 grid((unsigned)((h->Nx + 31) / 32), (unsigned)((h->Nr * h->Nvt + 31) / 32));
+    k_fvm_sweep_coef<<<grid, 256, 0, s>>>(view_of(h), h->aE, h->axvr, hstep, h->swc);
+    ++h->launches;
+    return launched("k_fvm_sweep_coef");
+}
+
+// Y = the op-split step applied to X (aE = cE E must already be in h->aE, ax v_r in h->axvr, and
+// the sweep coefficients of hstep tabulated)
 int fvm_precond(bte_fvm* h, double hstep, const double* X, double* Y, cudaStream_t s) {
     const FvmView v = view_of(h);
     const int Nr = h->Nr, Nvt = h->Nvt, Nx = h->Nx;
-    const size_t nrx = (size_t)Nr * Nx;
-    k_fvm_moment<<<fblocks(nrx), FT, 0, s>>>(v, X, h->M);
-    if (int rc = launched("k_fvm_moment")) return rc;
-    if (int rc = sweep_rc(bte_dgemm_nn(Nr, Nx, Nr, h->H, Nr, h->M, Nx, h->T, Nx, s), "collision inverse")) return rc;
-    const size_t xsm = ((size_t)XT_L * (Nx + 1) + 2 * (size_t)h->ndx * Nx) * sizeof(double);
-    const size_t rsm = 2 * (size_t)h->ndr * Nr * sizeof(double), tsm = 2 * (size_t)h->ndt * Nvt * sizeof(double);
-    if (h->ndr > SW_NDMAX || h->ndt > SW_NDMAX || h->ndx > SW_NDMAX || xsm > 200 * 1024 || rsm > 200 * 1024 ||
-        tsm > 200 * 1024) {
+    if (int rc = fvm_hmul(h, X, s)) return rc;
+    if (!natural_sweeps(h)) {
         // stencils wider than the register recurrence or x lines longer than the staged rows:
         // the drop-in sweeps on permuted copies
-        k_fvm_coll_permute<<<fblocks(h->N), FT, 0, s>>>(v, h->dinv, h->T, X, h->A);   // (Nx, Nvt, Nr)
+        k_fvm_coll_permute<<<fblocks(h->N), FT, 0, s>>>(v, h->dinv, h->T, X, h->A, h->bad);   // (Nx, Nvt, Nr)
         if (int rc = launched("k_fvm_coll_permute")) return rc;
         int rc = sweep_rc(bte_adv_be_sweep(0, h->vrL, h->vrR, h->aE, h->cos_t, hstep, h->A, h->Bf, h->ndr, Nr, Nvt, Nx, s),
                           "v_r sweep");
@@ -391,28 +610,26 @@ int fvm_precond(bte_fvm* h, double hstep, const double* X, double* Y, cudaStream
         if (!rc)
             rc = sweep_rc(bte_adv_be_sweep(2, h->xL, h->xR, h->axvr, h->cos_t, hstep, h->A, Y, h->ndx, Nr, Nvt, Nx, s),
                           "x sweep");
-        h->launches += 10;
+        h->launches += 8;
         return rc;
     }
-    k_fvm_coll_apply<<<fblocks(h->N), FT, 0, s>>>(v, h->dinv, h->T, X, h->A);   // natural layout
+    const size_t n = h->N;
+    const double* tr = h->swc;
+    const double* tt = tr + (size_t)h->ndr * n;
+    const double* xr = tt + (size_t)h->ndt * n;
+    k_fvm_coll_apply<<<fblocks(n), FT, 0, s>>>(v, h->dinv, h->T, X, tr, h->A, h->bad);
     if (int rc = launched("k_fvm_coll_apply")) return rc;
-    // the three sweeps in place on the natural layout, coalesced (no layout swaps)
-    // the v_r lines are few (Nvt Nx) and long: small CTAs spread them over the SMs
-    if (bte_raise_smem_limit((const void*)k_fvm_sweep_vr, rsm) != cudaSuccess ||
-        bte_raise_smem_limit((const void*)k_fvm_sweep_vt, tsm) != cudaSuccess ||
-        bte_raise_smem_limit((const void*)k_fvm_sweep_x, xsm) != cudaSuccess)
-        return fvm_fail(BTE_ERR_ARG, "sweep lines too long for the shared-memory sweeps");
-    // h->Bf (the drop-in path's scratch) holds the diagonal reciprocals of the v_r, then the x sweep
-    k_fvm_diag_rcp<<<fblocks(h->N), FT, 0, s>>>(v, 0, h->aE, h->axvr, hstep, h->Bf);
-    if (int rc = launched("k_fvm_diag_rcp")) return rc;
-    k_fvm_sweep_vr<<<(unsigned)(((size_t)Nvt * Nx + 31) / 32), 32, rsm, s>>>(v, h->aE, hstep, h->A, h->Bf);
+    // the v_r lines are few (Nvt Nx) and long: CTAs of one warp spread them over the SMs
+    k_fvm_sweep_vr<<<(unsigned)(((size_t)Nvt * Nx + 31) / 32), 32, 0, s>>>(v, h->aE, h->A, tr + n);
     if (int rc = launched("k_fvm_sweep_vr")) return rc;
-    k_fvm_sweep_vt<<<fblocks((size_t)Nr * Nx), FT, tsm, s>>>(v, h->aE, hstep, h->A);
+    k_fvm_sweep_vt<<<(unsigned)(((size_t)Nr * Nx + 127) / 128), 128, 0, s>>>(v, h->aE, h->A, tt, tt + n);
     if (int rc = launched("k_fvm_sweep_vt")) return rc;
-    k_fvm_diag_rcp<<<fblocks(h->N), FT, 0, s>>>(v, 2, h->aE, h->axvr, hstep, h->Bf);
-    if (int rc = launched("k_fvm_diag_rcp")) return rc;
-    k_fvm_sweep_x<<<(unsigned)((Nr * Nvt + XT_L - 1) / XT_L), XT_T, xsm, s>>>(v, h->axvr, hstep, h->A, Y, h->Bf);
-    h->launches += 8;
+    const int rows = sweep_x_rows(h);
+    const size_t xsm = (size_t)rows * (Nx + 1) * sizeof(double);
+    if (bte_raise_smem_limit((const void*)k_fvm_sweep_x, xsm) != cudaSuccess)
+        return fvm_fail(BTE_ERR_CUDA, "x sweep: shared-memory limit");
+    k_fvm_sweep_x<<<(unsigned)((Nr * Nvt + rows - 1) / rows), XT_T, xsm, s>>>(v, rows, h->axvr, h->A, Y, xr, xr + n);
+    h->launches += 4;
     return launched("k_fvm_sweep_x");
 }
 
@@ -443,14 +660,9 @@ int fvm_sl(bte_fvm* h, const FvmCoef& c, const double* E, const double* V, doubl
 
 // Y = (I - c C)^-1 B in the natural layout (Y must not alias B)
 int fvm_coll_solve(bte_fvm* h, const double* B, double* Y, cudaStream_t s) {
-    const FvmView v = view_of(h);
-    const size_t nrx = (size_t)h->Nr * h->Nx;
-    k_fvm_moment<<<fblocks(nrx), FT, 0, s>>>(v, B, h->M);
-    if (int rc = launched("k_fvm_moment")) return rc;
-    if (int rc = sweep_rc(bte_dgemm_nn(h->Nr, h->Nx, h->Nr, h->H, h->Nr, h->M, h->Nx, h->T, h->Nx, s), "collision inverse"))
-        return rc;
-    k_fvm_coll_apply<<<fblocks(h->N), FT, 0, s>>>(v, h->dinv, h->T, B, Y);
-    h->launches += 3;
+    if (int rc = fvm_hmul(h, B, s)) return rc;
+    k_fvm_coll_apply<<<fblocks(h->N), FT, 0, s>>>(view_of(h), h->dinv, h->T, B, nullptr, Y, h->bad);
+    ++h->launches;
     return launched("k_fvm_coll_apply");
 }
 
@@ -458,13 +670,12 @@ struct DeviceOps {
     bte_fvm* h;
     cudaStream_t s;
     FvmCoef c;
-    const double* E;
     double hstep;
     size_t N;
     double *B, *X, *R, *W, *Z, *T, *Kr;
     bool identity;   // pc_type "none": no preconditioner
 
-    int matvec(const double* x, double* y) { return fvm_mvec(h, c, E, x, y, s); }
+    int matvec(const double* x, double* y) { return fvm_mvec(h, c, x, y, s); }
     int precond(const double* x, double* y) {
         if (!identity) return fvm_precond(h, hstep, x, y, s);
         if (cudaMemcpyAsync(y, x, N * 8, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
@@ -556,6 +767,23 @@ int bte_fvm_create(int device, int Nr, int Nvt, int Nx, int ndr, int ndt, int nd
     A(&h->vtR, (size_t)ndt * Nvt); A(&h->xL, (size_t)ndx * Nx); A(&h->xR, (size_t)ndx * Nx);
     A(&h->dinv, Nr); A(&h->H, (size_t)Nr * Nr);
     A(&h->M, (size_t)Nr * Nx); A(&h->T, (size_t)Nr * Nx); A(&h->aE, Nx); A(&h->axvr, Nr);
+    A(&h->bx, Nx); A(&h->arc, (size_t)Nr * Nvt); A(&h->lr, Nr); A(&h->vinv, Nr);
+    // the gain matrix by rows; the scattered entries of at most two per process and row
+    std::vector<int32_t> gptr(1, 0), gcol;
+    std::vector<double> gval;
+    for (int r = 0; r < Nr; ++r) {
+        for (int k = 0; k < Nr; ++k)
+            if (gain[(size_t)r * Nr + k] != 0.0) {
+                gcol.push_back(k);
+                gval.push_back(gain[(size_t)r * Nr + k]);
+            }
+        gptr.push_back((int32_t)gcol.size());
+    }
+    const size_t hwords = (size_t)((Nr + HR - 1) / HR) * (((Nr + HC - 1) / HC + 31) / 32);
+    auto Ab = [&](void** p, size_t bytes) { if (rc == BTE_OK) rc = fvm_alloc(h, p, bytes); };
+    Ab((void**)&h->eflag, Nx); Ab((void**)&h->cpos, Nvt); Ab((void**)&h->gptr, gptr.size() * 4);
+    Ab((void**)&h->gcol, gcol.size() * 4); Ab((void**)&h->gval, gval.size() * 8);
+    Ab((void**)&h->hmask, hwords * 4); Ab((void**)&h->bad, (size_t)Nx * 4);
     A(&h->A, N); A(&h->Bf, N); A(&h->B, N); A(&h->X, N); A(&h->R, N); A(&h->W, N); A(&h->Z, N); A(&h->Tv, N);
     if (rc == BTE_OK) rc = fvm_alloc(h, (void**)&h->north, Nvt);
     if (rc != BTE_OK) {
@@ -564,11 +792,15 @@ int bte_fvm_create(int device, int Nr, int Nvt, int Nx, int ndr, int ndt, int nd
         return rc;
     }
     std::vector<double> cth(Nvt);
-    std::vector<int8_t> north(Nvt);
+    std::vector<int8_t> north(Nvt), cpos(Nvt);
+    std::vector<double> vinv(Nr);
+    std::vector<int32_t> zero((size_t)Nx, 0);
+    for (int r = 0; r < Nr; ++r) vinv[r] = 1.0 / vr[r];
     const double half_pi = 0.5 * 3.14159265358979323846;
     for (int j = 0; j < Nvt; ++j) {
         cth[j] = std::cos(vt[j]);
         north[j] = vt[j] <= half_pi ? 1 : 0;
+        cpos[j] = cth[j] > 0.0 ? 1 : 0;
     }
     struct Cp { void* d; const void* s; size_t b; };
     const Cp cps[] = {{h->vr, vr, (size_t)Nr * 8}, {h->vt, vt, (size_t)Nvt * 8}, {h->cos_t, cth.data(), (size_t)Nvt * 8},
@@ -576,9 +808,12 @@ int bte_fvm_create(int device, int Nr, int Nvt, int Nx, int ndr, int ndt, int nd
                       {h->vrL, vr_l2r, (size_t)ndr * Nr * 8}, {h->vrR, vr_r2l, (size_t)ndr * Nr * 8},
                       {h->vtL, vt_l2r, (size_t)ndt * Nvt * 8}, {h->vtR, vt_r2l, (size_t)ndt * Nvt * 8},
                       {h->xL, x_l2r, (size_t)ndx * Nx * 8}, {h->xR, x_r2l, (size_t)ndx * Nx * 8},
-                      {h->north, north.data(), (size_t)Nvt}};
+                      {h->north, north.data(), (size_t)Nvt}, {h->cpos, cpos.data(), (size_t)Nvt},
+                      {h->vinv, vinv.data(), (size_t)Nr * 8}, {h->gptr, gptr.data(), gptr.size() * 4},
+                      {h->gcol, gcol.data(), gcol.size() * 4}, {h->gval, gval.data(), gval.size() * 8},
+                      {h->bad, zero.data(), (size_t)Nx * 4}};
     for (const Cp& c : cps)
-        if (cudaMemcpy(c.d, c.s, c.b, cudaMemcpyHostToDevice) != cudaSuccess) {
+        if (c.b && cudaMemcpy(c.d, c.s, c.b, cudaMemcpyHostToDevice) != cudaSuccess) {
             fvm_free(h);
             delete h;
             return fvm_fail(BTE_ERR_CUDA, "bte_fvm_create: copy of the set-up failed");
@@ -603,8 +838,14 @@ long long bte_fvm_launches(const bte_fvm* h) { return h ? h->launches : 0; }
 int bte_fvm_set_collision_inverse(bte_fvm* h, const double* dinv, const double* H) {
     if (!h || !dinv || !H) return fvm_fail(BTE_ERR_ARG, "bte_fvm_set_collision_inverse: null argument");
     cudaSetDevice(h->device);
+    const int Nr = h->Nr, words = ((Nr + HC - 1) / HC + 31) / 32;
+    std::vector<uint32_t> mask((size_t)((Nr + HR - 1) / HR) * words, 0u);
+    for (int r = 0; r < Nr; ++r)
+        for (int k = 0; k < Nr; ++k)
+            if (H[(size_t)r * Nr + k] != 0.0) mask[(size_t)(r / HR) * words + k / HC / 32] |= 1u << (k / HC % 32);
     if (cudaMemcpy(h->dinv, dinv, (size_t)h->Nr * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(h->H, H, (size_t)h->Nr * h->Nr * 8, cudaMemcpyHostToDevice) != cudaSuccess)
+        cudaMemcpy(h->H, H, (size_t)h->Nr * h->Nr * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(h->hmask, mask.data(), mask.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess)
         return fvm_fail(BTE_ERR_CUDA, "bte_fvm_set_collision_inverse: copy failed");
     h->have_inverse = true;
     return BTE_OK;
@@ -615,7 +856,8 @@ int bte_fvm_mvec(bte_fvm* h, const bte_fvm_coef* c, const double* E, const doubl
     if (!coef_ok(c)) return fvm_fail(BTE_ERR_ARG, "bte_fvm_mvec: coefficients missing or not finite");
     if (X == Y) return fvm_fail(BTE_ERR_ARG, "bte_fvm_mvec: Y must not alias X");
     cudaSetDevice(h->device);
-    return fvm_mvec(h, coef_of(c), E, X, Y, (cudaStream_t)stream);
+    if (int rc = fvm_mvec_coef(h, coef_of(c), E, (cudaStream_t)stream)) return rc;
+    return fvm_mvec(h, coef_of(c), X, Y, (cudaStream_t)stream);
 }
 
 int bte_fvm_precond(bte_fvm* h, double cE, double ax, double hstep, const double* E, const double* X, double* Y,
@@ -626,6 +868,7 @@ int bte_fvm_precond(bte_fvm* h, double cE, double ax, double hstep, const double
     cudaSetDevice(h->device);
     cudaStream_t s = (cudaStream_t)stream;
     if (int rc = fvm_coefficients(h, cE, ax, E, s)) return rc;
+    if (int rc = fvm_sweep_coef(h, hstep, s)) return rc;
     return fvm_precond(h, hstep, X, Y, s);
 }
 
@@ -722,11 +965,14 @@ int bte_fvm_step(bte_fvm* h, const bte_fvm_coef* c, double alpha, int pc_mode, c
     }
     const FvmCoef fc = coef_of(c);
     if (int rc = fvm_coefficients(h, fc.tau * fc.cA, fc.ax, E, s)) return rc;
+    if (int rc = fvm_mvec_coef(h, fc, E, s)) return rc;
+    if (pc_mode != 2)
+        if (int rc = fvm_sweep_coef(h, alpha * fc.dt, s)) return rc;
     // right-hand side: V with its inflow values zeroed (bte_1d3v_solver.py:1907-1911)
     if (cudaMemcpyAsync(h->B, V, N * 8, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
         return fvm_fail(BTE_ERR_CUDA, "bte_fvm_step: copy of the state failed");
     if (int rc = sweep_rc(bte_fvm_inflow_zero(h->Nr, h->Nvt, h->Nx, h->vt, h->B, s), "inflow")) return rc;
-    DeviceOps op{h, s, fc, E, alpha * fc.dt, N, h->B, h->X, h->R, h->W, h->Z, h->Tv, h->Kr, pc_mode == 2};
+    DeviceOps op{h, s, fc, alpha * fc.dt, N, h->B, h->X, h->R, h->W, h->Z, h->Tv, h->Kr, pc_mode == 2};
     FvmGmresInfo info{};
     if (int rc = pc_mode == 1 ? fvm_gmres_left(op, restart, rtol, atol, max_iter, &info)
                               : fvm_gmres(op, restart, rtol, atol, max_iter, &info))
