@@ -18,8 +18,9 @@
 //               column) and written once. No read-modify-write of a trailing matrix.
 //   k_lu_right  (any N)     right-looking by panels (trailing matrix in global memory),
 //               for the largest systems.
-// (k_lu_tc in lu_tc.cu is the FP32 tensor-core kernel; k_lus_* below split one FP64
-// factorization over many CTAs.)
+// (k_lu_tc in lu_tc.cu is the FP32 tensor-core kernel; k_lu_cluster in lu_cluster.cu keeps one
+// matrix in the shared memory of a thread-block cluster; k_lus_* below split one FP64
+// factorization over many CTAs by launches.)
 #include <cstdint>
 #include <algorithm>
 #include <type_traits>
@@ -99,7 +100,7 @@ __device__ inline void warp_argmax(double& best, int& bi) {
     }
 }
 __device__ inline float recip(float d) { return __frcp_rn(d); }
-__device__ inline double recip(double d) { return 1.0 / d; }
+__device__ inline double recip(double d) { return bte_recip(d); }
 
 // Unblocked partial-pivoting factorization of a panel in shared memory, column-major
 // P[c * ldp + r], rows 0..mrows-1 (pivot positions base..base+mrows-1), pivots on the
@@ -536,12 +537,20 @@ k_lus_update(int N, int NC, int k0, int nrb, int ncb, T* __restrict__ A, int ld,
         Us[k][c] = (k < kb && cl < ncol) ? a[(size_t)pk[k] * ld + c0g + cl] : T(0);
     }
     __syncthreads();
+    // each element takes its products in the order of k, one multiply-add each, as in the cluster
+    // kernel: a matrix has the same factors whichever kernel its batch size selects
     const int tx = tid & 15, ty = tid >> 4;
     T acc[4][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i) {
+        const int pr = prow[ty + 16 * i];
+        const T* row = a + (size_t)max(pr, 0) * ld + c0g + cb * SP_T;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = T(0);
+        for (int j = 0; j < 4; ++j) {
+            const int c = tx + 16 * j;
+            acc[i][j] = (pr >= 0 && cb * SP_T + c < ncol) ? row[c] : T(0);
+        }
+    }
 #pragma unroll 8
     for (int k = 0; k < NB; ++k) {
         T av[4], bv[4];
@@ -552,7 +561,7 @@ k_lus_update(int N, int NC, int k0, int nrb, int ncb, T* __restrict__ A, int ld,
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] += av[i] * bv[j];
+            for (int j = 0; j < 4; ++j) acc[i][j] -= av[i] * bv[j];
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -562,7 +571,7 @@ k_lus_update(int N, int NC, int k0, int nrb, int ncb, T* __restrict__ A, int ld,
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int c = tx + 16 * j;
-            if (cb * SP_T + c < ncol) row[c] -= acc[i][j];
+            if (cb * SP_T + c < ncol) row[c] = acc[i][j];
         }
     }
 }
@@ -912,20 +921,29 @@ cudaError_t factor_right(int P, int N, int NC, T* A, int ld, long long stride, i
 }  // namespace
 
 int bte_lu_tc_max_n();
+int bte_lu_cluster_size(int P, int N, int NC);
+cudaError_t bte_lu_factor_cluster(int P, int N, int NC, double* A, int ld, long long stride, int32_t* piv, int32_t* info,
+                                  cudaStream_t s, int C);
 cudaError_t bte_lu_factor_tc(int P, int N, int NC, float* A, int ld, long long stride, int32_t* piv, int32_t* info,
                              cudaStream_t s, int variant);
 
 // Factor P matrices in place; piv[P][N] receives perm (position -> stored row).
-// kernel: 0 = automatic (FP32, N <= 512: tensor cores; FP32 above: right-looking; FP64:
-// right-looking), 1 = right-looking, 2 = FP32 with the trailing updates on the tensor cores
+// kernel: 0 = automatic (FP32, N <= 512: tensor cores; else a cluster per matrix where
+// bte_lu_cluster_size says so, or right-looking), 1 = right-looking, 2 = FP32 with the trailing updates on the tensor cores
 // (lu_tc.cu; N <= 512; 256 threads, two CTAs per SM), 3 = left-looking SIMT (N <= 512), 4 = as
 // 2 with one CTA per SM, 5 = as 2 with 128 threads per CTA, 6 = FP64 split over many CTAs per
-// matrix (panel, triangular solve and 64 x 64 trailing tiles as separate launches).
+// matrix (a cluster, or panel, triangular solve and 64 x 64 trailing tiles as separate launches).
 template <typename T>
 cudaError_t bte_lu_factor_t(int P, int N, int NC, T* A, int ld, long long stride, int32_t* piv, int32_t* info,
                             cudaStream_t s, int kernel) {
     if (P <= 0) return cudaSuccess;
     if (N < 1 || N > LU_MAX_N || NC < N || NC > N + 1 || ld < NC) return cudaErrorInvalidValue;
+    // FP64, the automatic choice and split over many CTAs: one cluster per matrix where that is
+    // faster, with the same factors
+    if constexpr (sizeof(T) == 8)
+        if (kernel == 0 || kernel == 6)
+            if (const int C = bte_lu_cluster_size(P, N, NC))
+                return bte_lu_factor_cluster(P, N, NC, A, ld, stride, piv, info, s, C);
     // FP64: the right-looking kernel (the left-looking one serialises FP64 substitutions)
     if (sizeof(T) == 8 && kernel == 0) kernel = 1;
     if (kernel == 6) {

@@ -238,3 +238,42 @@ def test_lu_solve_block_edges(N, P, pad, dtype):
         Ad, xd, bd = A[i, :, :N].double(), x[i].double(), b[i].double()
         berr = torch.linalg.norm(Ad @ xd - bd) / (torch.linalg.matrix_norm(Ad, 2) * torch.linalg.norm(xd) + torch.linalg.norm(bd))
         assert float(berr) < 2 * N * torch.finfo(tdt).eps, (i, float(berr))
+
+
+@pytest.mark.parametrize("N", [1, 8, 9, 64, 127, 128, 129, 193, 256, 257, 385, 449, 512, 513])
+def test_lu_fp64_factors_do_not_depend_on_the_batch(N):
+    """The FP64 factorization of a matrix is the same bit by bit in a batch of one, of a few and of many
+    (one cluster per matrix of several sizes, or launches split over many CTAs), with ties, a negative
+    zero and rows that must be exchanged; its backward error is within 2 N eps."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    ld = N + 3
+    g = torch.Generator(device="cuda").manual_seed(N)
+    M = torch.randn((3, N, ld), device="cuda", generator=g, dtype=torch.float64)
+    M[1] = torch.round(M[1] * 2)             # many equal candidates in a column
+    M[1, :, :N] += 5 * torch.eye(N, dtype=torch.float64, device="cuda").flip(0)
+    if N > 2:
+        M[2, 0, 0] = -0.0
+    got = []
+    for P in (3, 24, 66 if N > 400 else 402):
+        A = M.repeat(P // 3, 1, 1).contiguous()
+        piv = torch.empty((P, N), dtype=torch.int32, device="cuda")
+        info = torch.empty(P, dtype=torch.int32, device="cuda")
+        st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        _lib.check(lib.bte_lu_factor_ex(0, P, N, C.c_void_p(A.data_ptr()), ld, N * ld, C.c_void_p(piv.data_ptr()),
+                                        C.c_void_p(info.data_ptr()), 6, st), "lu_factor")
+        torch.cuda.synchronize()
+        assert bool((info == info[:3].repeat(P // 3)).all())
+        got.append((A[-3:, :, :N].clone(), piv[-3:].clone(), info[:3].clone()))
+    for A, piv, info in got[1:]:
+        assert torch.equal(piv, got[0][1]) and torch.equal(info, got[0][2])
+        assert torch.equal(A, got[0][0])
+    A, piv, info = got[0]
+    for i in range(3):
+        LU = A[i][piv[i].long()]
+        L = torch.tril(LU, -1) + torch.eye(N, dtype=torch.float64, device="cuda")
+        R = L @ torch.triu(LU) - M[i, :, :N][piv[i].long()]
+        scale = torch.linalg.matrix_norm(L, 2) * torch.linalg.matrix_norm(torch.triu(LU), 2)
+        assert float(torch.linalg.matrix_norm(R, 2)) <= 2 * N * 2.3e-16 * float(scale)
+        assert float(L.abs().max()) <= 1.0 + 1e-15  # partial pivoting
