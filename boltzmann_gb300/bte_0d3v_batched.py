@@ -530,7 +530,7 @@ class bte_0d3v_batched:
         if k or self._precision() != _lib.PREC_MIXED or not int(getattr(self._args, "autotune", 1)):
             return k
         N = self._grid_info[grid_idx]["n"] + 1
-        if N > 512:  # one candidate kernel for the tuner: the library chooses by size and points
+        if N > 512:  # above the tuner's candidates the library has one choice
             return 0
         from . import autotune
         return autotune.lu_kernel_for(N, device=self._dev_id)

@@ -921,6 +921,8 @@ cudaError_t factor_right(int P, int N, int NC, T* A, int ld, long long stride, i
 }  // namespace
 
 int bte_lu_tc_max_n();
+cudaError_t bte_lu_factor_tcs(int P, int N, int NC, float* A, int ld, long long stride, int32_t* piv, int32_t* info,
+                              cudaStream_t s);
 int bte_lu_cluster_size(int P, int N, int NC);
 cudaError_t bte_lu_factor_cluster(int P, int N, int NC, double* A, int ld, long long stride, int32_t* piv, int32_t* info,
                                   cudaStream_t s, int C);
@@ -928,8 +930,8 @@ cudaError_t bte_lu_factor_tc(int P, int N, int NC, float* A, int ld, long long s
                              cudaStream_t s, int variant);
 
 // Factor P matrices in place; piv[P][N] receives perm (position -> stored row).
-// kernel: 0 = automatic (FP32, N <= 512: tensor cores; else a cluster per matrix where
-// bte_lu_cluster_size says so, or right-looking), 1 = right-looking, 2 = FP32 with the trailing updates on the tensor cores
+// kernel: 0 = automatic (FP32: tensor cores, one CTA per matrix up to N = 512 and split over many
+// CTAs above; FP64: a cluster per matrix where bte_lu_cluster_size says so, or right-looking), 1 = right-looking, 2 = FP32 with the trailing updates on the tensor cores
 // (lu_tc.cu; N <= 512; 256 threads, two CTAs per SM), 3 = left-looking SIMT (N <= 512), 4 = as
 // 2 with one CTA per SM, 5 = as 2 with 128 threads per CTA, 6 = FP64 split over many CTAs per
 // matrix (a cluster, or panel, triangular solve and 64 x 64 trailing tiles as separate launches).
@@ -966,6 +968,8 @@ cudaError_t bte_lu_factor_t(int P, int N, int NC, T* A, int ld, long long stride
         // 1.3x at N = 129 and 257, 1.7x at N = 512)
         return bte_lu_factor_tc(P, N, NC, reinterpret_cast<float*>(A), ld, stride, piv, info, s, 0);
     }
+    if constexpr (sizeof(T) == 4)
+        if (kernel == 0) return bte_lu_factor_tcs(P, N, NC, A, ld, stride, piv, info, s);
     if (kernel == 3) kernel = 0;
     if (kernel == 0 && N <= 128) return launch_left<T, 4>(P, N, NC, A, ld, stride, piv, info, s);
     if (kernel == 0 && N <= 256) return launch_left<T, 8>(P, N, NC, A, ld, stride, piv, info, s);

@@ -23,6 +23,7 @@
 //      The epilogue reads it back with tcgen05.ld (lane = column, so a warp's 32 lanes are
 //      32 consecutive columns of one row: coalesced) and updates A22 in global memory,
 //      which stays L2-resident while the CTA works on it.
+// Above N = 512 (k_tcs_*) the same steps are separate launches over many CTAs per matrix.
 // The split: hi = tf32(x) (round to nearest), lo = x - hi (exact in FP32); hi*hi is exact
 // in the FP32 accumulator, the dropped lo*lo term is below 2^-22 |x y|.
 #include <cstdint>
@@ -441,6 +442,273 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
     if (wid == 0) tmem_dealloc(tbase, TC_TMEM_COLS);
 }
 
+// ---------------------------------------------------------------------------------
+// N > 512: one factorization split over many CTAs, two launches per panel of NB columns:
+//   k_tcs_panel   one CTA per matrix: pivoting of the panel with the rows in registers (rows stay
+//                 with their threads, only their positions change; one barrier per column), then
+//                 U12 = L11^-1 A12, one thread per column;
+//   k_tcs_update  one CTA per 128 x 128 tile of the trailing matrix: A22 -= L21 U12 as in k_lu_tc.
+// A matrix of N = 769 keeps one CTA busy for 5.5 ms (k_lu_right), with half the SMs idle for 75 of them;
+// split, the trailing updates spread over the GPU and the chain is the panels' columns.
+// Bound by that chain for few matrices and by the trailing matrices' reads and writes for many.
+// The result does not depend on the number of matrices. Measured (us, k_lu_right -> these):
+// N = 513: 2090 -> 540 (1 matrix), 2380 -> 1049 (150); N = 769: 5521 -> 879 (1), 6118 -> 1705 (75),
+// 19415 -> 6858 (400); N = 1281: 41980 -> 4992 (48); N = 2048: 247724 -> 3558 (2).
+// ---------------------------------------------------------------------------------
+constexpr int TS_NT = 512;             // threads of the panel kernel
+constexpr int TS_NW = TS_NT / 32;
+constexpr int TS_LD = TC_NB + 4;       // a published row, 16-byte aligned
+
+template <int NB, int ROWS>
+__global__ void __launch_bounds__(TS_NT, 1)
+k_tcs_panel(int N, int NC, int k0, float* __restrict__ A, int ld, long long stride, int32_t* __restrict__ perm_g,
+            int32_t* __restrict__ info, int vec4) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ __align__(16) float cand[2][TS_NW][TS_LD];  // a warp's best row of the column
+    __shared__ uint2 ckey[2][TS_NW];                       // its |a| as bits, its position
+    __shared__ __align__(16) float L11[NB][NB + 4];        // transposed: L11[column][row]
+    int* pos2row = reinterpret_cast<int*>(smraw);          // stored row at position k0 + i
+    const int mrows = N - k0, kb = min(NB, mrows), ncol = min(NB, NC - k0);
+    const int mat = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    float* a = A + (size_t)mat * stride;
+    int32_t* pg = perm_g + (size_t)mat * N;
+    float pr[ROWS][NB];
+    int pos[ROWS], row[ROWS];  // position relative to k0 (-1: no row), stored row
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        const int s = tid + i * TS_NT;
+        pos[i] = (s < mrows) ? s : -1;
+        row[i] = (s < mrows) ? (k0 == 0 ? s : pg[k0 + s]) : 0;
+        const float* src = a + (size_t)row[i] * ld + k0;
+        if (vec4 && ncol == NB) {
+#pragma unroll
+            for (int c = 0; c < NB; c += 4) {
+                const float4 v = (s < mrows) ? *reinterpret_cast<const float4*>(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                pr[i][c] = v.x; pr[i][c + 1] = v.y; pr[i][c + 2] = v.z; pr[i][c + 3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < NB; ++c) pr[i][c] = (s < mrows && c < ncol) ? src[c] : 0.f;
+        }
+    }
+    int inf = 0;
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+        if (j >= kb) break;
+        // the thread's, the warp's and the CTA's candidate: largest |a| (NaN counts as 0), first position
+        uint32_t key = 0, at = 0xffffffffu;
+        int bi = 0;
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i)
+            if (pos[i] >= j) {
+                const float v = fabsf(pr[i][j]);
+                const uint32_t k = (v == v) ? __float_as_uint(v) : 0u;
+                if (at == 0xffffffffu || k > key || (k == key && (uint32_t)pos[i] < at)) { key = k; at = pos[i]; bi = i; }
+            }
+        const uint32_t wk = __reduce_max_sync(0xffffffffu, key);
+        const uint32_t wa = __reduce_min_sync(0xffffffffu, key == wk ? at : 0xffffffffu);
+        if (wa == 0xffffffffu ? lane == 0 : at == wa) {
+            float* my = cand[j & 1][wid];
+            ckey[j & 1][wid] = make_uint2(wk, wa);
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i)
+                if (i == bi) {
+#pragma unroll
+                    for (int c = (j & ~3); c < NB; c += 4)
+                        *reinterpret_cast<float4*>(my + c) = make_float4(pr[i][c], pr[i][c + 1], pr[i][c + 2], pr[i][c + 3]);
+                }
+        }
+        __syncthreads();
+        const uint2 o = (lane < TS_NW) ? ckey[j & 1][lane] : make_uint2(0u, 0xffffffffu);
+        const uint32_t bk = __reduce_max_sync(0xffffffffu, o.y == 0xffffffffu ? 0u : o.x);
+        const uint32_t S = __reduce_min_sync(0xffffffffu, o.x == bk ? o.y : 0xffffffffu);
+        const int W = __ffs(__ballot_sync(0xffffffffu, o.x == bk && o.y == S)) - 1;
+        const float* prow = cand[j & 1][W];
+        float pv[NB];
+#pragma unroll
+        for (int c = (j & ~3); c < NB; c += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(prow + c);
+            pv[c] = v.x; pv[c + 1] = v.y; pv[c + 2] = v.z; pv[c + 3] = v.w;
+        }
+        const float d = pv[j];
+        if (!(d != 0.f) && inf == 0) inf = k0 + j + 1;
+        const float inv = (d != 0.f) ? __frcp_rn(d) : 0.f;
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            if (pos[i] == (int)S) pos[i] = j;
+            else if (pos[i] == j) pos[i] = (int)S;
+            if (pos[i] > j) {
+                const float l = pr[i][j] * inv;
+                pr[i][j] = l;
+#pragma unroll
+                for (int c = j + 1; c < NB; ++c) pr[i][c] -= l * pv[c];
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+        if (pos[i] >= 0) {
+            float* dst = a + (size_t)row[i] * ld + k0;
+            if (vec4 && ncol == NB) {
+#pragma unroll
+                for (int c = 0; c < NB; c += 4)
+                    *reinterpret_cast<float4*>(dst + c) = make_float4(pr[i][c], pr[i][c + 1], pr[i][c + 2], pr[i][c + 3]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < NB; ++c)
+                    if (c < ncol) dst[c] = pr[i][c];
+            }
+            pos2row[pos[i]] = row[i];
+            if (pos[i] < NB)
+#pragma unroll
+                for (int c = 0; c < NB; ++c) L11[c][pos[i]] = pr[i][c];
+        }
+    __syncthreads();
+    for (int r = tid; r < mrows; r += TS_NT) pg[k0 + r] = pos2row[r];
+    if (tid == 0) {
+        const int cur = (k0 == 0) ? 0 : info[mat];
+        info[mat] = cur != 0 ? cur : inf;
+    }
+    if (kb < NB) return;  // the last panel: nothing to its right but columns it holds
+    // U12 = L11^-1 A12, one thread per column
+    for (int c = k0 + NB + tid; c < NC; c += TS_NT) {
+        float x[NB];
+#pragma unroll
+        for (int j = 0; j < NB; ++j) x[j] = a[(size_t)pos2row[j] * ld + c];
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            asm volatile("" ::: "memory");  // keeps the compiler from hoisting all multipliers into registers
+            float lc[NB];
+#pragma unroll
+            for (int j = ((i + 1) & ~3); j < NB; j += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(&L11[i][j]);
+                lc[j] = v.x; lc[j + 1] = v.y; lc[j + 2] = v.z; lc[j + 3] = v.w;
+            }
+#pragma unroll
+            for (int j = i + 1; j < NB; ++j) x[j] -= lc[j] * x[i];
+        }
+#pragma unroll
+        for (int j = 0; j < NB; ++j) a[(size_t)pos2row[j] * ld + c] = x[j];
+    }
+}
+
+// one 128 x 128 tile of A22 -= L21 U12 (kb = 16 or 32 panel columns at k0)
+__global__ void __launch_bounds__(256, 3)
+k_tcs_update(int N, int NC, int k0, int kb, int nct, int nrt, float* __restrict__ A, int ld, long long stride,
+             const int32_t* __restrict__ perm_g, int32_t* __restrict__ info, int vec4) {
+    extern __shared__ unsigned char smraw[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_fault;
+    __shared__ int rows[TC_TR], piv[TC_NB];
+    unsigned char* sm = smraw + ((1024 - (smem_u32(smraw) & 1023)) & 1023);
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int per = nct * nrt, mat = blockIdx.x / per, t = blockIdx.x % per;
+    const int c0 = k0 + kb + (t % nct) * TC_TM, r0 = k0 + kb + (t / nct) * TC_TR;
+    const int ncols = min(TC_TM, NC - c0), nrows = min(TC_TR, N - r0);
+    float* a = A + (size_t)mat * stride;
+    const int32_t* pg = perm_g + (size_t)mat * N;
+    const uint32_t mb = smem_u32(&mbar);
+    if (tid < TC_TR) rows[tid] = (tid < nrows) ? pg[r0 + tid] * ld : -1;  // N ld < 2^31
+    if (tid >= 128 && tid < 128 + kb) piv[tid - 128] = pg[k0 + tid - 128] * ld;
+    if (tid == 0) {
+        mbar_init(mb, 1);
+        s_fault = 0;
+    }
+    if (wid == 0) tmem_alloc(smem_u32(&tmem_slot), TC_TMEM_COLS);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tbase = tmem_slot;
+    const int k4 = kb / 4;
+    // B operand: rows of L21; A operand: U12^T (row m = column c0 + m)
+    for (int e = tid; e < TC_TR * k4; e += 256) {
+        const int r = e / k4, k = (e % k4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (rows[r] >= 0) {
+            const float* src = a + rows[r] + k0 + k;
+            if (vec4) v = *reinterpret_cast<const float4*>(src);
+            else v = make_float4(src[0], src[1], src[2], src[3]);
+        }
+        put_split4(sm + SM_B_HI, r, k, v.x, v.y, v.z, v.w);
+    }
+    for (int e = tid; e < TC_TM * k4; e += 256) {
+        const int m = e & (TC_TM - 1), k = (e >> 7) * 4;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (m < ncols)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = a[piv[k + q] + c0 + m];
+        put_split4(sm + SM_A_HI, m, k, v[0], v[1], v[2], v[3]);
+    }
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+        tc_fence_after();
+        const uint32_t ahi = smem_u32(sm + SM_A_HI), alo = smem_u32(sm + SM_A_LO);
+        const uint32_t bhi = smem_u32(sm + SM_B_HI), blo = smem_u32(sm + SM_B_LO);
+        constexpr uint32_t idesc = idesc_tf32(TC_TM, TC_TR);
+        for (int ks = 0; ks < kb / 8; ++ks) {
+            const uint32_t o = ks * 256;
+            mma_tf32(tbase, op_desc(alo + o), op_desc(bhi + o), idesc, ks > 0 ? 1u : 0u);
+            mma_tf32(tbase, op_desc(ahi + o), op_desc(blo + o), idesc, 1u);
+            mma_tf32(tbase, op_desc(ahi + o), op_desc(bhi + o), idesc, 1u);
+        }
+        mma_commit(mb);
+    }
+    // the tile's first values while the products run: warp w reads TMEM lanes 32 (w % 4) .. (columns)
+    // and 64 (w / 4) .. of the TMEM columns (rows)
+    const int q = wid & 3, h = wid >> 2, m = 32 * q + lane;
+    const bool colok = m < ncols;
+    float* colp = a + c0 + m;
+    float old[16];
+    auto fetch = [&](int rr) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) old[i] = (colok && rows[rr + i] >= 0) ? colp[rows[rr + i]] : 0.f;
+    };
+    fetch(64 * h);
+    if (tid == 0) {
+        uint32_t it = 0;
+        while (!mbar_try_wait(mb, 0))
+            if (++it > TC_WAIT_LIMIT) { s_fault = 1; break; }
+    }
+    __syncthreads();
+    tc_fence_after();
+    if (!s_fault) {
+#pragma unroll 1
+        for (int rr = 64 * h; rr < 64 * h + 64; rr += 16) {
+            if (rr >= nrows) break;  // warp-uniform
+            float dv[16];
+            tmem_ld16(tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)rr, dv);
+            float out[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) out[i] = old[i] - dv[i];
+            if (rr + 16 < 64 * h + 64) fetch(rr + 16);
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (colok && rows[rr + i] >= 0) colp[rows[rr + i]] = out[i];
+        }
+    } else {
+        // an MMA commit never arrived: wait once more (bounded) before giving TMEM back
+        if (tid == 0) {
+            uint32_t it = 0;
+            while (!mbar_try_wait(mb, 0) && ++it < TC_WAIT_LIMIT) {}
+            info[mat] = -1;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (wid == 0) tmem_dealloc(tbase, TC_TMEM_COLS);
+}
+
+template <int NB, int ROWS>
+cudaError_t launch_tcs_panel(int P, int N, int NC, int k0, float* A, int ld, long long stride, int32_t* piv, int32_t* info,
+                             cudaStream_t s, int vec4) {
+    k_tcs_panel<NB, ROWS><<<P, TS_NT, (size_t)(N - k0) * 4, s>>>(N, NC, k0, A, ld, stride, piv, info, vec4);
+    return cudaGetLastError();
+}
+
 template <int ROWS, int OCC, int NT>
 cudaError_t launch_tc(int P, int N, int NC, float* A, int ld, long long stride, int32_t* piv, int32_t* info,
                       cudaStream_t s) {
@@ -453,6 +721,34 @@ cudaError_t launch_tc(int P, int N, int NC, float* A, int ld, long long stride, 
 }
 
 }  // namespace
+
+// FP32 factorization of P matrices with N > 512 (any N up to 2048) by panels: 32 columns while two
+// rows per thread hold them (up to 1024 rows), 16 above
+cudaError_t bte_lu_factor_tcs(int P, int N, int NC, float* A, int ld, long long stride, int32_t* piv, int32_t* info,
+                              cudaStream_t s) {
+    if (P <= 0) return cudaSuccess;
+    if (N < 1 || N > 4 * TS_NT || NC < N || NC > N + 1 || ld < NC) return cudaErrorInvalidValue;
+    if ((long long)N * ld >= (1ll << 31)) return cudaErrorInvalidValue;  // row offsets are 32-bit
+    const int vec4 = (ld % 4 == 0 && stride % 4 == 0 && ((uintptr_t)A & 15) == 0) ? 1 : 0;
+    const size_t usm = (size_t)SM_L11 + 1024;
+    cudaError_t e = bte_raise_smem_limit((const void*)k_tcs_update, usm);
+    if (e != cudaSuccess) return e;
+    for (int k0 = 0; k0 < N;) {
+        const int mrows = N - k0, nb = mrows > 2 * TS_NT ? 16 : 32;
+        if (mrows > 2 * TS_NT) e = launch_tcs_panel<16, 4>(P, N, NC, k0, A, ld, stride, piv, info, s, vec4);
+        else if (mrows > TS_NT) e = launch_tcs_panel<32, 2>(P, N, NC, k0, A, ld, stride, piv, info, s, vec4);
+        else e = launch_tcs_panel<32, 1>(P, N, NC, k0, A, ld, stride, piv, info, s, vec4);
+        if (e != cudaSuccess) return e;
+        const int nr = mrows - nb, ncol = NC - k0 - nb;
+        if (nr > 0 && ncol > 0) {
+            const int nct = (ncol + TC_TM - 1) / TC_TM, nrt = (nr + TC_TR - 1) / TC_TR;
+            k_tcs_update<<<(unsigned)P * nct * nrt, 256, usm, s>>>(N, NC, k0, nb, nct, nrt, A, ld, stride, piv, info, vec4);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
+        k0 += nb;
+    }
+    return cudaSuccess;
+}
 
 // largest N the tensor-core kernel takes (its panel is two 32-column rows per thread)
 int bte_lu_tc_max_n() { return 2 * TC_NT; }

@@ -86,7 +86,9 @@ typedef struct {
                                      choice                                                   */
     int lu64_kernel;              /* FP64 factorizations (the plain form, and the mixed form's
                                      FP64 lane): 0: the library's choice (6); 1: one CTA per
-                                     system; 6: each system split over many CTAs            */
+                                     system; 6: each system split over many CTAs
+                                     (a thread-block cluster or launches, by size and number:
+                                     the same factors either way)                         */
     int reserved[2];
 } bte_solve_opts;
 
@@ -208,14 +210,16 @@ int bte_qoi(const bte_grid* g, int P, const double* f, const double* n0, const d
 int bte_lu_factor(int dtype, int P, int N, void* A, int ld, long long stride, int32_t* piv, int32_t* info,
                   void* stream);
 
-/* As bte_lu_factor with an explicit kernel: 0 = automatic (FP32: tensor-core kernel for
- * N <= 512, right-looking above; FP64: right-looking),
+/* As bte_lu_factor with an explicit kernel: 0 = automatic (FP32: tensor-core kernels, one CTA
+ * per matrix for N <= 512, split over many above; FP64: a thread-block cluster per matrix for
+ * the sizes and numbers where that is the fastest, else right-looking),
  * 1 = right-looking for every N, 2 = FP32 only, N <= 512: trailing updates on the tcgen05
  * tensor cores in split TF32 (FP32-accurate factors), 3 = left-looking (N <= 512),
  * 4 = as 2 with one CTA per SM instead of two (fewer matrices in flight, kept in L2),
  * 5 = as 2 with 128 threads per CTA (less pivot-search work per matrix),
- * 6 = FP64 only: each factorization split over many CTAs (per panel: pivoting, triangular
- *     solve, 64 x 64 trailing tiles as separate launches), for few large FP64 systems.
+ * 6 = FP64 only: each factorization split over many CTAs (a cluster as for 0, or per panel:
+ *     pivoting, triangular solve, 64 x 64 trailing tiles as separate launches); the factors
+ *     do not depend on which, nor on P.
  * No counterpart in the reference; used to cross-check the factorizations. */
 int bte_lu_factor_ex(int dtype, int P, int N, void* A, int ld, long long stride, int32_t* piv, int32_t* info,
                      int kernel, void* stream);

@@ -277,3 +277,40 @@ def test_lu_fp64_factors_do_not_depend_on_the_batch(N):
         scale = torch.linalg.matrix_norm(L, 2) * torch.linalg.matrix_norm(torch.triu(LU), 2)
         assert float(torch.linalg.matrix_norm(R, 2)) <= 2 * N * 2.3e-16 * float(scale)
         assert float(L.abs().max()) <= 1.0 + 1e-15  # partial pivoting
+
+
+@pytest.mark.parametrize("N,pad", [(513, 3), (544, 0), (545, 1), (640, 0), (769, 3), (1024, 0), (1025, 3), (1056, 1),
+                                   (1537, 0), (2048, 0)])
+def test_lu_fp32_above_512(N, pad):
+    """The FP32 factorization split over many CTAs (N > 512): sizes around its panels and tiles, the
+    appended right-hand side left alone, rows that do and do not allow 16-byte loads, a zero pivot
+    reported and the same factors in a batch of 1 and of 5. Backward error as for the other kernels."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    ld = N + pad
+    g = torch.Generator(device="cuda").manual_seed(N)
+    A0 = torch.randn((5, N, ld), device="cuda", generator=g, dtype=torch.float32)
+    A0[:, :, :N] += 0.1 * torch.eye(N, device="cuda")
+    b0 = torch.randn((5, N), device="cuda", generator=g, dtype=torch.float32)
+    ptr, st = (lambda t: C.c_void_p(t.data_ptr())), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    got = []
+    for P in (1, 5):
+        A, x = A0[:P].clone(), b0[:P].clone()
+        piv = torch.empty((P, N), dtype=torch.int32, device="cuda")
+        info = torch.empty(P, dtype=torch.int32, device="cuda")
+        _lib.check(lib.bte_lu_factor_ex(1, P, N, ptr(A), ld, N * ld, ptr(piv), ptr(info), 0, st), "lu_factor")
+        _lib.check(lib.bte_lu_solve(1, P, N, ptr(A), ld, N * ld, ptr(piv), ptr(x), st), "lu_solve")
+        torch.cuda.synchronize()
+        assert bool((info == 0).all()) and torch.equal(A[:, :, N:], A0[:P, :, N:])
+        for i in range(P):
+            Ad, xd, bd = A0[i, :, :N].double(), x[i].double(), b0[i].double()
+            berr = torch.linalg.norm(Ad @ xd - bd) / (torch.linalg.matrix_norm(Ad, 2) * torch.linalg.norm(xd) + torch.linalg.norm(bd))
+            assert float(berr) < 2 * N * 1.2e-7, (i, float(berr))
+        got.append((A[0].clone(), piv[0].clone()))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    Z = torch.eye(N, device="cuda").reshape(1, N, N).contiguous()
+    Z[0, N - 3, N - 3] = 0.0
+    _lib.check(lib.bte_lu_factor_ex(1, 1, N, ptr(Z), N, N * N, ptr(piv), ptr(info), 0, st), "lu_factor")
+    torch.cuda.synchronize()
+    assert int(info[0].item()) == N - 2
