@@ -29,6 +29,7 @@
 #include <algorithm>
 #include "bte_common.cuh"
 #include "bte_grid.h"
+#include "dgemm_warp.cuh"
 #include "../../include/bte1d_gb300.h"
 
 template <typename T>
@@ -43,25 +44,26 @@ namespace {
 constexpr int RED_BLOCKS = 120;   // partial-sum blocks of the reductions (deterministic order)
 
 // out[i][c] = sum_k Qm[i][k] in[k][c], i, k < Nr, c < C (C = Nvt * Nx): the radial basis change
-__global__ void k_radial_mix(int Nr, int C, const double* __restrict__ Qm, const double* __restrict__ in,
-                             double* __restrict__ out) {
-    extern __shared__ double sq[];
-    for (int e = threadIdx.x; e < Nr * Nr; e += blockDim.x) sq[e] = Qm[e];
-    __syncthreads();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y;
-    if (c >= C) return;
-    double s = 0.0;
-    for (int k = 0; k < Nr; ++k) s += sq[i * Nr + k] * in[(size_t)k * C + c];
-    out[(size_t)i * C + c] = s;
+// (TA: Qm stored transposed). The form with a CTA per row and 128 columns staged Qm in every CTA;
+// 64 x 64 by 3200: 41 -> 29 us (its FP64 multiply-adds take 22).
+template <int R, bool TA>
+__global__ void __launch_bounds__(DGW_WARPS * 32)
+k_radial_mix(int Nr, int C, const double* __restrict__ Qm, const double* __restrict__ in, double* __restrict__ out) {
+    int i0, col;
+    if (!dgw_place(Nr, C, R, &i0, &col)) return;
+    double acc[R];
+    dgw_product<R, TA>(Nr, Nr, Qm, Nr, in, C, i0, min(col, C - 1), acc, dgw_buffer<R>());
+    if (col >= C) return;
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+        if (i0 + i < Nr) out[(size_t)(i0 + i) * C + col] = acc[i];
 }
-
-// inflow boundary values: x = 0 (x = -1) for ordinates moving right, x = Nx - 1 for the others
-__global__ void k_zero_inflow(int Nr, int Nvt, int Nx, const int8_t* __restrict__ right, double* V) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= Nr * Nvt) return;
-    const int j = e % Nvt;
-    V[(size_t)e * Nx + (right[j] ? 0 : Nx - 1)] = 0.0;
+template <bool TA>
+void launch_radial_mix(int Nr, int C, const double* Qm, const double* in, double* out, cudaStream_t s) {
+    const int R = dgw_rows(Nr, C);
+    dgw_dispatch(R, [&](auto rc) {
+        k_radial_mix<decltype(rc)::value, TA><<<dgw_grid(Nr, C, R), DGW_WARPS * 32, 0, s>>>(Nr, C, Qm, in, out);
+    });
 }
 
 // A[(r * Nvt + j)] = I + h d_r cos(theta_j) D_X, D_L = D with row 0 zeroed (right-moving
@@ -94,32 +96,39 @@ __global__ void k_store_invcol(int P, int Nx, int c, const double* __restrict__ 
     const size_t m = e / Nx, i = e % Nx;
     XT[(m * Nx + c) * Nx + i] = B[e];
 }
-// out[m][i] = sum_k A^-1[m][i][k] in[m][k] with the transposed inverse XT[m][k][i]: one CTA
-// per system, threads along i (coalesced rows of XT), in[m][:] staged in shared memory
-__global__ void __launch_bounds__(256) k_xstep_apply(int Nx, const double* __restrict__ XT,
-                                                     const double* __restrict__ in, double* __restrict__ out) {
+// out[m][i] = sum_k A^-1[m][i][k] in[m][k] with the transposed inverse XT[m][k][i] and the inflow
+// values of in (x = 0 for ordinates moving right, x = Nx - 1 otherwise) taken as 0: one CTA per
+// system, threads along i (coalesced rows of XT, read once: no reuse to keep), in[m][:] in shared
+// memory. 1024 systems of 200: 90 us for 328 MB (48 us) and 7 warps x 200 FP64 multiply-adds per
+// system (75 us). Outputs laid end to end over the warps (no idle lanes) took 102.
+__global__ void __launch_bounds__(256) k_xstep_apply(int Nvt, int Nx, const int8_t* __restrict__ right,
+                                                     const double* __restrict__ XT, const double* __restrict__ in,
+                                                     double* __restrict__ out) {
     extern __shared__ double sv[];
     const int m = blockIdx.x;
     const double* A = XT + (size_t)m * Nx * Nx;
-    for (int k = threadIdx.x; k < Nx; k += blockDim.x) sv[k] = in[(size_t)m * Nx + k];
+    const int zero = right[m % Nvt] ? 0 : Nx - 1;
+    for (int k = threadIdx.x; k < Nx; k += blockDim.x) sv[k] = (k == zero) ? 0.0 : in[(size_t)m * Nx + k];
     __syncthreads();
     for (int i = threadIdx.x; i < Nx; i += blockDim.x) {
         double acc = 0.0;
-#pragma unroll 4
-        for (int k = 0; k < Nx; ++k) acc += A[(size_t)k * Nx + i] * sv[k];
+#pragma unroll 8
+        for (int k = 0; k < Nx; ++k) acc += __ldcs(A + (size_t)k * Nx + i) * sv[k];
         out[(size_t)m * Nx + i] = acc;
     }
 }
 
-// ordinates -> spherical harmonics, into the x-major layout: U[x][r nsh + l] = sum_j Ps[l][j] V[r][j][x]
+// ordinates -> spherical harmonics, into the x-major layout: U[x][r nsh + l] = sum_j Ps[l][j] V[r][j][x],
+// and rounded to FP32 where Uf is given (the preconditioner's right-hand side)
 __global__ void k_ords_to_lm(int Nr, int Nvt, int nsh, int Nx, const double* __restrict__ Ps,
-                             const double* __restrict__ V, double* __restrict__ U) {
+                             const double* __restrict__ V, double* __restrict__ U, float* __restrict__ Uf) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= Nr * nsh * Nx) return;
     const int x = e % Nx, a = e / Nx, r = a / nsh, l = a % nsh;
     double s = 0.0;
     for (int j = 0; j < Nvt; ++j) s += Ps[l * Nvt + j] * V[((size_t)r * Nvt + j) * Nx + x];
     U[(size_t)x * (Nr * nsh) + a] = s;
+    if (Uf) Uf[(size_t)x * (Nr * nsh) + a] = (float)s;
 }
 
 // spherical harmonics -> ordinates: V[r][j][x] = sum_l Po[j][l] U[x][r nsh + l]
@@ -133,35 +142,84 @@ __global__ void k_lm_to_ords(int Nr, int Nvt, int nsh, int Nx, const double* __r
     V[e] = s;
 }
 
-// Lmat_mvec (bte_1d3v_solver.py:1051-1055) in the x-major layout:
-//   Y[x][a] = X[x][a] - dt (sum_b Cv[a][b] X[x][b] + E[x] sum_b Av[a][b] X[x][b])
-// CvT / AvT are stored transposed so that the threads of a CTA (one per a) read along a.
-constexpr int MV_X = 8;
-__global__ void __launch_bounds__(256)
+// The v-space operator L = Cv + E_x Av applied per x point, X x-major (X[x * n + b]):
+//   Lmat_mvec (bte_1d3v_solver.py:1051-1055): Y[x][a] = X[x][a] - dt (L X)[x][a]   (SUB)
+//   or Y[x][a] = (L X)[x][a]
+// with CvT / AvT stored transposed. A warp takes 32 a's of R points; a CTA per 8 points ran on 13 SMs
+// for 101 points (n = 96: 73 -> 9 us).
+template <int R, bool SUB>
+__global__ void __launch_bounds__(DGW_WARPS * 32)
 k_lmat(int n, int Nx, double dt, const double* __restrict__ CvT, const double* __restrict__ AvT,
        const double* __restrict__ E, const double* __restrict__ X, double* __restrict__ Y) {
-    extern __shared__ double sx[];  // [MV_X][n]
-    const int x0 = blockIdx.x * MV_X;
-    const int nx = min(MV_X, Nx - x0);
-    for (int e = threadIdx.x; e < nx * n; e += blockDim.x) sx[e] = X[(size_t)x0 * n + e];
-    __syncthreads();
-    for (int a = threadIdx.x; a < n; a += blockDim.x) {
-        double c[MV_X], v[MV_X];
+    int x0, a;
+    if (!dgw_place(Nx, n, R, &x0, &a)) return;
+    const int ac = min(a, n - 1), lane = threadIdx.x & 31;
+    constexpr int U = 8;
+    double* sX = dgw_buffer<R>();  // 32 b's of the R points, a lane per b
+    double c[R], v[R], xn[R], nc[U], na[U];
+    const double* xr[R];
 #pragma unroll
-        for (int t = 0; t < MV_X; ++t) { c[t] = 0.0; v[t] = 0.0; }
-        for (int b = 0; b < n; ++b) {
-            const double cb = CvT[(size_t)b * n + a], ab = AvT[(size_t)b * n + a];
-#pragma unroll
-            for (int t = 0; t < MV_X; ++t) {
-                const double xb = (t < nx) ? sx[t * n + b] : 0.0;
-                c[t] += cb * xb;
-                v[t] += ab * xb;
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < MV_X; ++t)
-            if (t < nx) Y[(size_t)(x0 + t) * n + a] = sx[t * n + a] - dt * (c[t] + E[x0 + t] * v[t]);
+    for (int t = 0; t < R; ++t) {
+        c[t] = v[t] = 0.0;
+        xr[t] = X + (size_t)min(x0 + t, Nx - 1) * n;
     }
+    auto fetch_x = [&](int b0) {
+#pragma unroll
+        for (int t = 0; t < R; ++t) xn[t] = xr[t][min(b0 + lane, n - 1)];
+    };
+    auto fetch_op = [&](int b0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const size_t o = (size_t)min(b0 + u, n - 1) * n + ac;
+            nc[u] = CvT[o];
+            na[u] = AvT[o];
+        }
+    };
+    fetch_x(0);
+    fetch_op(0);
+    for (int b0 = 0; b0 < n; b0 += 32) {
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < R; ++t) sX[lane * R + t] = xn[t];
+        __syncwarp();
+        if (b0 + 32 < n) fetch_x(b0 + 32);
+#pragma unroll
+        for (int q = 0; q < 32; q += U) {
+            if (b0 + q >= n) break;
+            double cb[U], ab[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                cb[u] = nc[u];
+                ab[u] = na[u];
+            }
+            if (b0 + q + U < n) fetch_op(b0 + q + U);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (b0 + q + u < n)
+#pragma unroll
+                    for (int t = 0; t < R; ++t) {
+                        const double xb = sX[(q + u) * R + t];
+                        c[t] += cb[u] * xb;
+                        v[t] += ab[u] * xb;
+                    }
+        }
+    }
+    if (a >= n) return;
+#pragma unroll
+    for (int t = 0; t < R; ++t)
+        if (x0 + t < Nx) {
+            const double l = c[t] + E[x0 + t] * v[t];
+            Y[(size_t)(x0 + t) * n + a] = SUB ? xr[t][a] - dt * l : l;
+        }
+}
+template <bool SUB>
+void launch_lmat(int n, int Nx, double dt, const double* CvT, const double* AvT, const double* E, const double* X, double* Y,
+                 cudaStream_t s) {
+    const int R = std::min(6, dgw_rows(Nx, n));
+    dgw_dispatch(R, [&](auto rc) {
+        constexpr int R6 = decltype(rc)::value > 6 ? 6 : decltype(rc)::value;  // two sums per element
+        k_lmat<R6, SUB><<<dgw_grid(Nx, n, R), DGW_WARPS * 32, 0, s>>>(n, Nx, dt, CvT, AvT, E, X, Y);
+    });
 }
 
 // the per-point blocks I - dt (Cv + E_x Av), FP32, row-major with leading dimension ld
@@ -244,109 +302,52 @@ inline unsigned nb(size_t m, int b) { return (unsigned)((m + b - 1) / b); }
 // ---- fully implicit spectral step ------------------------------------------------------------
 // T[m][x] = sum_k D[x][k] V[m][k] for each (r, j) line m = r * Nvt + j, with the inflow row of
 // the upwinded derivative zeroed (row 0 for ordinates moving right, D_L; row Nx - 1 otherwise,
-// D_R: bte_1d3v_solver.py:792-800). DT = D transposed, so that the threads (one per output x)
-// read consecutive entries; each entry feeds FD_L lines staged in shared memory.
-constexpr int FD_L = 8;
-__global__ void __launch_bounds__(256)
+// D_R: bte_1d3v_solver.py:792-800). DT = D transposed (lanes along x). 1024 lines of 200: 109 us
+// with a CTA per 8 lines (128 CTAs of 6.25 busy warps) -> 93 us; the FP64 multiply-adds take 67.
+template <int R>
+__global__ void __launch_bounds__(DGW_WARPS * 32)
 k_fim_dx(int Nlines, int Nvt, int Nx, const double* __restrict__ DT, const int8_t* __restrict__ right,
          const double* __restrict__ V, double* __restrict__ T) {
-    extern __shared__ double sv[];  // [FD_L][Nx]
-    const int l0 = blockIdx.x * FD_L;
-    const int nl = min(FD_L, Nlines - l0);
-    for (int e = threadIdx.x; e < nl * Nx; e += blockDim.x) sv[e] = V[(size_t)l0 * Nx + e];
-    __syncthreads();
-    for (int x = threadIdx.x; x < Nx; x += blockDim.x) {
-        double acc[FD_L];
+    int l0, x;
+    if (!dgw_place(Nlines, Nx, R, &l0, &x)) return;
+    double acc[R];
+    dgw_product<R, false>(Nlines, Nx, V, Nx, DT, Nx, l0, min(x, Nx - 1), acc, dgw_buffer<R>());
+    if (x >= Nx) return;
 #pragma unroll
-        for (int t = 0; t < FD_L; ++t) acc[t] = 0.0;
-        for (int k = 0; k < Nx; ++k) {
-            const double dk = DT[(size_t)k * Nx + x];
-#pragma unroll
-            for (int t = 0; t < FD_L; ++t) acc[t] += dk * sv[(t < nl ? t : 0) * Nx + k];
-        }
-#pragma unroll
-        for (int t = 0; t < FD_L; ++t) {
-            if (t >= nl) break;
-            const int j = (l0 + t) % Nvt;
+    for (int i = 0; i < R; ++i)
+        if (l0 + i < Nlines) {
+            const int j = (l0 + i) % Nvt;
             const bool inflow_row = right[j] ? (x == 0) : (x == Nx - 1);
-            T[(size_t)(l0 + t) * Nx + x] = inflow_row ? 0.0 : acc[t];
+            T[(size_t)(l0 + i) * Nx + x] = inflow_row ? 0.0 : acc[i];
         }
-    }
 }
 
-// The backward-Euler operator of the fully implicit step on ordinates, per x point:
-//   Y = V - dt (P_sh2o (Cv + E_x Av) P_o2sh V - cos(theta_j) adv_x T)
+// The backward-Euler operator of the fully implicit step on ordinates, from its products:
+//   Y = V - dt (P_sh2o W - cos(theta_j) G), W = (Cv + E_x Av) P_o2sh V (k_lmat, x-major), G = adv_x T
 // (T = the x-derivative lines of k_fim_dx; Cv, Av carry tau), with identity rows on the inflow
-// boundary. One CTA per FC_X consecutive x points; V, T, adv_x staged in shared memory.
-constexpr int FC_X = 1;   // one x point per CTA: Nx CTAs (the radial mixing dominates)
-__global__ void __launch_bounds__(256)
-k_fim_combine(int Nr, int Nvt, int nsh, int Nx, double dt, const double* __restrict__ Ps,
-              const double* __restrict__ Po, const double* __restrict__ CvT, const double* __restrict__ AvT,
-              const double* __restrict__ AxT, const double* __restrict__ cth, const int8_t* __restrict__ right,
-              const double* __restrict__ E, const double* __restrict__ V, const double* __restrict__ T,
-              double* __restrict__ Y) {
-    extern __shared__ double sm[];
-    const int M = Nr * Nvt, n = Nr * nsh;
-    double* sV = sm;                 // [FC_X][M]
-    double* sT = sV + FC_X * M;      // [FC_X][M]
-    double* sU = sT + FC_X * M;      // [FC_X][n]  harmonics
-    double* sW = sU + FC_X * n;      // [FC_X][n]  (Cv + E Av) harmonics
-    double* sA = sW + FC_X * n;      // [Nr][Nr]   adv_x transposed
-    const int x0 = blockIdx.x * FC_X;
-    const int nx = min(FC_X, Nx - x0);
-    for (int e = threadIdx.x; e < M * FC_X; e += blockDim.x) {
-        const int m = e / FC_X, t = e % FC_X;
-        const bool ok = t < nx;
-        sV[t * M + m] = ok ? V[(size_t)m * Nx + x0 + t] : 0.0;
-        sT[t * M + m] = ok ? T[(size_t)m * Nx + x0 + t] : 0.0;
+// boundary. One thread per value. One kernel with a CTA per x point did all products but T's in 85 us
+// (two rounds of CTAs); k_lmat, the radial mix and this take 65 with the harmonics.
+__global__ void k_fim_combine(int Nr, int Nvt, int nsh, int Nx, double dt, const double* __restrict__ Po,
+                              const double* __restrict__ cth, const int8_t* __restrict__ right,
+                              const double* __restrict__ W, const double* __restrict__ G, const double* __restrict__ V,
+                              double* __restrict__ Y) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= Nr * Nvt * Nx) return;
+    const int x = e % Nx, rj = e / Nx, r = rj / Nvt, j = rj % Nvt;
+    const double vx = V[e];
+    if (right[j] ? (x == 0) : (x == Nx - 1)) {
+        Y[e] = vx;
+        return;
     }
-    for (int e = threadIdx.x; e < Nr * Nr; e += blockDim.x) sA[e] = AxT[e];
-    __syncthreads();
-    for (int e = threadIdx.x; e < n * FC_X; e += blockDim.x) {
-        const int a = e % n, t = e / n, r = a / nsh, l = a % nsh;
-        double u = 0.0;
-        for (int j = 0; j < Nvt; ++j) u += Ps[l * Nvt + j] * sV[t * M + r * Nvt + j];
-        sU[t * n + a] = u;
-    }
-    __syncthreads();
-    for (int a = threadIdx.x; a < n; a += blockDim.x) {
-        double c[FC_X], v[FC_X];
-#pragma unroll
-        for (int t = 0; t < FC_X; ++t) { c[t] = 0.0; v[t] = 0.0; }
-        for (int b = 0; b < n; ++b) {
-            const double cb = CvT[(size_t)b * n + a], ab = AvT[(size_t)b * n + a];
-#pragma unroll
-            for (int t = 0; t < FC_X; ++t) {
-                c[t] += cb * sU[t * n + b];
-                v[t] += ab * sU[t * n + b];
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < FC_X; ++t) sW[t * n + a] = c[t] + ((t < nx) ? E[x0 + t] : 0.0) * v[t];
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < M * FC_X; e += blockDim.x) {
-        const int t = e / M, m = e % M, r = m / Nvt, j = m % Nvt;
-        if (t >= nx) continue;
-        const int x = x0 + t;
-        const double vx = sV[t * M + m];
-        const bool inflow_row = right[j] ? (x == 0) : (x == Nx - 1);
-        double y = vx;
-        if (!inflow_row) {
-            double yv = 0.0;
-            for (int l = 0; l < nsh; ++l) yv += Po[j * nsh + l] * sW[t * n + r * nsh + l];
-            double yx = 0.0;
-            for (int k = 0; k < Nr; ++k) yx += sA[k * Nr + r] * sT[t * M + k * Nvt + j];
-            y = vx - dt * (yv - cth[j] * yx);
-        }
-        Y[(size_t)m * Nx + x] = y;
-    }
+    double yv = 0.0;
+    for (int l = 0; l < nsh; ++l) yv += Po[j * nsh + l] * W[(size_t)x * (Nr * nsh) + r * nsh + l];
+    Y[e] = vx - dt * (yv - cth[j] * G[e]);
 }
 
 // out = in + P_sh2o (Z - U): the exact inverse of I - dt P_sh2o L_v P_o2sh on ordinates from the
-// per-point inverse Z = (I - dt L_v)^-1 U of the harmonics U = P_o2sh in (P_o2sh P_sh2o = I)
+// per-point inverse Z = (I - dt L_v)^-1 U (FP32) of the harmonics U = P_o2sh in (P_o2sh P_sh2o = I)
 __global__ void k_lm_correct(int Nr, int Nvt, int nsh, int Nx, const double* __restrict__ Po,
-                             const double* __restrict__ in, const double* __restrict__ Z,
+                             const double* __restrict__ in, const float* __restrict__ Z,
                              const double* __restrict__ U, double* __restrict__ out) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= Nr * Nvt * Nx) return;
@@ -354,7 +355,7 @@ __global__ void k_lm_correct(int Nr, int Nvt, int nsh, int Nx, const double* __r
     double s = in[e];
     for (int l = 0; l < nsh; ++l) {
         const size_t a = (size_t)x * (Nr * nsh) + r * nsh + l;
-        s += Po[j * nsh + l] * (Z[a] - U[a]);
+        s += Po[j * nsh + l] * ((double)Z[a] - U[a]);
     }
     out[e] = s;
 }
@@ -398,7 +399,8 @@ struct Bte1d {
     // fully implicit step: adv_x transposed, D transposed, and the ordinates-space GMRES buffers
     // (allocated on first use)
     double *AxT = nullptr, *DT = nullptr;
-    double *Fk = nullptr, *Fr = nullptr, *Fw = nullptr, *Fz = nullptr, *Fx = nullptr, *Fb = nullptr, *Ft = nullptr;
+    double *Fk = nullptr, *Fr = nullptr, *Fw = nullptr, *Fz = nullptr, *Fx = nullptr, *Fb = nullptr, *Ft = nullptr,
+           *Fg = nullptr;
     double *Fpart = nullptr;
     int fcap = 0;
     std::vector<void*> allocs;
@@ -557,15 +559,13 @@ int bte1d_step_x(Bte1d* h, double hstep, double* V, void* stream) {
         h->hx = hstep;
         h->launches += 2 + 3 * (long long)Nx;
     }
-    const size_t smem = (size_t)Nr * Nr * 8;
-    CK1(bte_raise_smem_limit((const void*)k_radial_mix, smem));
-    k_radial_mix<<<dim3(nb(C, 128), Nr), 128, smem, s>>>(Nr, C, h->Qinv, V, h->Vt);
-    k_zero_inflow<<<nb((size_t)Nr * Nvt, 256), 256, 0, s>>>(Nr, Nvt, Nx, h->right, h->Vt);
+    launch_radial_mix<false>(Nr, C, h->Qinv, V, h->Vt, s);
     CK1(cudaGetLastError());
-    k_xstep_apply<<<Nr * Nvt, 256, (size_t)Nx * 8, s>>>(Nx, h->XI, h->Vt, h->Vt2);
-    k_radial_mix<<<dim3(nb(C, 128), Nr), 128, smem, s>>>(Nr, C, h->Q, h->Vt2, V);
+    k_xstep_apply<<<Nr * Nvt, 256, (size_t)Nx * 8, s>>>(Nvt, Nx, h->right, h->XI, h->Vt, h->Vt2);
     CK1(cudaGetLastError());
-    h->launches += 4;
+    launch_radial_mix<false>(Nr, C, h->Q, h->Vt2, V, s);
+    CK1(cudaGetLastError());
+    h->launches += 3;
     return BTE_OK;
 }
 
@@ -573,8 +573,7 @@ int bte1d_step_x(Bte1d* h, double hstep, double* V, void* stream) {
 int bte1d_lmat(Bte1d* h, double dt, const double* E, const double* X, double* Y, void* stream) {
     if (!h || !E || !X || !Y) { g_err1d = "null argument"; return BTE_ERR_ARG; }
     cudaSetDevice(h->device);
-    const size_t smem = (size_t)MV_X * h->n * 8;
-    k_lmat<<<nb(h->Nx, MV_X), 128, smem, (cudaStream_t)stream>>>(h->n, h->Nx, dt, h->CvT, h->AvT, E, X, Y);
+    launch_lmat<true>(h->n, h->Nx, dt, h->CvT, h->AvT, E, X, Y, (cudaStream_t)stream);
     CK1(cudaGetLastError());
     h->launches += 1;
     return BTE_OK;
@@ -592,7 +591,7 @@ int bte1d_step_v(Bte1d* h, double dt, const double* E, double* V, double rtol, d
     const long long vs = (long long)n * h->vld;
     long long L = 0;
     auto lmat = [&](const double* x, double* y) {
-        k_lmat<<<nb(Nx, MV_X), 128, (size_t)MV_X * n * 8, s>>>(n, Nx, dt, h->CvT, h->AvT, E, x, y);
+        launch_lmat<true>(n, Nx, dt, h->CvT, h->AvT, E, x, y, s);
         ++L;
     };
     auto precond = [&](const double* x, double* y) -> cudaError_t {  // y = M^-1 x (per-x FP32 block LU)
@@ -611,7 +610,7 @@ int bte1d_step_v(Bte1d* h, double dt, const double* E, double* V, double rtol, d
         return cudaStreamSynchronize(s);
     };
     // right-hand side U = P_o2sh V, and the per-point FP32 block factors
-    k_ords_to_lm<<<nb(N, 256), 256, 0, s>>>(h->Nr, h->Nvt, h->nsh, Nx, h->Ps, V, h->U);
+    k_ords_to_lm<<<nb(N, 256), 256, 0, s>>>(h->Nr, h->Nvt, h->nsh, Nx, h->Ps, V, h->U, nullptr);
     k_build_vblocks<<<dim3(std::min<unsigned>(nb((size_t)n * n, 256), 32), Nx), 256, 0, s>>>(n, Nx, dt, h->CvT, h->AvT, E,
                                                                                         h->VB, h->vld, vs);
     CK1(cudaGetLastError());
@@ -726,7 +725,8 @@ int bte1d_block_solve(Bte1d* h, double dt, const double* E, const double* X, dou
 int bte1d_ords_to_lm(Bte1d* h, const double* V, double* U, void* stream) {
     if (!h || !V || !U) { g_err1d = "null argument"; return BTE_ERR_ARG; }
     cudaSetDevice(h->device);
-    k_ords_to_lm<<<nb((size_t)h->n * h->Nx, 256), 256, 0, (cudaStream_t)stream>>>(h->Nr, h->Nvt, h->nsh, h->Nx, h->Ps, V, U);
+    k_ords_to_lm<<<nb((size_t)h->n * h->Nx, 256), 256, 0, (cudaStream_t)stream>>>(h->Nr, h->Nvt, h->nsh, h->Nx, h->Ps, V, U,
+                                                                                        nullptr);
     CK1(cudaGetLastError());
     return BTE_OK;
 }
@@ -743,15 +743,23 @@ int bte1d_lm_to_ords(Bte1d* h, const double* U, double* V, void* stream) {
 static int fim_matvec(Bte1d* h, double dt, const double* E, const double* V, double* Y, cudaStream_t s) {
     const int Nr = h->Nr, Nvt = h->Nvt, Nx = h->Nx, M = Nr * Nvt;
     if (!h->Ft && alloc1d(h, (void**)&h->Ft, (size_t)M * Nx * 8) != BTE_OK) return BTE_ERR_ALLOC;
-    const size_t sdx = (size_t)FD_L * Nx * 8;
-    const size_t scb = ((size_t)2 * FC_X * M + 2 * FC_X * h->n + (size_t)Nr * Nr) * 8;
-    CK1(bte_raise_smem_limit((const void*)k_fim_dx, sdx));
-    CK1(bte_raise_smem_limit((const void*)k_fim_combine, scb));
-    k_fim_dx<<<nb(M, FD_L), 256, sdx, s>>>(M, Nvt, Nx, h->DT, h->right, V, h->Ft);
-    k_fim_combine<<<nb(Nx, FC_X), 256, scb, s>>>(Nr, Nvt, h->nsh, Nx, dt, h->Ps, h->Po, h->CvT, h->AvT, h->AxT,
-                                                 h->cth, h->right, E, V, h->Ft, Y);
+    if (!h->Fg && alloc1d(h, (void**)&h->Fg, (size_t)M * Nx * 8) != BTE_OK) return BTE_ERR_ALLOC;
+    const int n = h->n, R = dgw_rows(M, Nx);
+    const size_t N = (size_t)M * Nx;
+    // h->R and h->W hold the harmonics and their operator (the v-step's vectors, free here)
+    k_ords_to_lm<<<nb((size_t)n * Nx, 256), 256, 0, s>>>(Nr, Nvt, h->nsh, Nx, h->Ps, V, h->R, nullptr);
     CK1(cudaGetLastError());
-    h->launches += 2;
+    launch_lmat<false>(n, Nx, dt, h->CvT, h->AvT, E, h->R, h->W, s);
+    CK1(cudaGetLastError());
+    dgw_dispatch(R, [&](auto rc) {
+        k_fim_dx<decltype(rc)::value><<<dgw_grid(M, Nx, R), DGW_WARPS * 32, 0, s>>>(M, Nvt, Nx, h->DT, h->right, V, h->Ft);
+    });
+    CK1(cudaGetLastError());
+    launch_radial_mix<true>(Nr, Nvt * Nx, h->AxT, h->Ft, h->Fg, s);
+    CK1(cudaGetLastError());
+    k_fim_combine<<<nb(N, 256), 256, 0, s>>>(Nr, Nvt, h->nsh, Nx, dt, h->Po, h->cth, h->right, h->W, h->Fg, V, Y);
+    CK1(cudaGetLastError());
+    h->launches += 5;
     return BTE_OK;
 }
 
@@ -790,13 +798,11 @@ int bte1d_step_fim(Bte1d* h, double dt, const double* E, double* V, double rtol,
     if (int rc = check_blocks(h, s)) return rc;
     auto precond = [&](const double* x, double* y) -> int {
         // v part: y = x + P_sh2o ((I - dt L_v)^-1 - I) P_o2sh x, per point, FP32 factors
-        k_ords_to_lm<<<nb(Nu, 256), 256, 0, s>>>(Nr, Nvt, h->nsh, Nx, h->Ps, x, h->U);
-        k_to_f32<<<nb(Nu, 256), 256, 0, s>>>(Nu, h->U, h->Zf);
+        k_ords_to_lm<<<nb(Nu, 256), 256, 0, s>>>(Nr, Nvt, h->nsh, Nx, h->Ps, x, h->U, h->Zf);
         CK1(bte_lu_solve_t<float>(Nx, n, h->VB, h->vld, vs, h->Vpiv, h->Zf, 0, s));
-        k_to_f64<<<nb(Nu, 256), 256, 0, s>>>(Nu, h->Zf, h->Z);
-        k_lm_correct<<<nb(N, 256), 256, 0, s>>>(Nr, Nvt, h->nsh, Nx, h->Po, x, h->Z, h->U, y);
+        k_lm_correct<<<nb(N, 256), 256, 0, s>>>(Nr, Nvt, h->nsh, Nx, h->Po, x, h->Zf, h->U, y);
         CK1(cudaGetLastError());
-        L += 5;
+        L += 3;
         // x part (pc 0): the backward-Euler x-advection over dt
         if (pc == 0) {
             int rc = bte1d_step_x(h, dt, y, s);

@@ -46,7 +46,7 @@ struct bte_fvm {
     double* gval = nullptr;
     uint32_t* hmask = nullptr;   // per 8-row tile of H: which chunks of HC columns hold a non-zero
     int32_t* bad = nullptr;      // per x: a non-finite ordinate moment (it reaches every row of G m and H m)
-    double* swc = nullptr;       // sweep coefficients (k_fvm_sweep_coef), allocated on first use
+    double* swc = nullptr;       // sweep coefficients (k_fvm_sweep_coef), allocated with the collision inverse
     double *B = nullptr, *X = nullptr, *R = nullptr, *W = nullptr, *Z = nullptr, *Tv = nullptr;
     double* Kr = nullptr;
     int kcap = 0;
@@ -579,9 +579,6 @@ bool natural_sweeps(const bte_fvm* h) {
 // the sweep coefficients for step h at the coefficients in h->aE, h->axvr
 int fvm_sweep_coef(bte_fvm* h, double hstep, cudaStream_t s) {
     if (!natural_sweeps(h)) return BTE_OK;
-    const size_t arrays = (size_t)h->ndr + h->ndt + h->ndx;
-    if (!h->swc)
-        if (int rc = fvm_alloc(h, (void**)&h->swc, arrays * h->N * sizeof(double))) return rc;
     const dim3 grid((unsigned)((h->Nx + 31) / 32), (unsigned)((h->Nr * h->Nvt + 31) / 32));
     k_fvm_sweep_coef<<<grid, 256, 0, s>>>(view_of(h), h->aE, h->axvr, hstep, h->swc);
     ++h->launches;
@@ -838,6 +835,8 @@ long long bte_fvm_launches(const bte_fvm* h) { return h ? h->launches : 0; }
 int bte_fvm_set_collision_inverse(bte_fvm* h, const double* dinv, const double* H) {
     if (!h || !dinv || !H) return fvm_fail(BTE_ERR_ARG, "bte_fvm_set_collision_inverse: null argument");
     cudaSetDevice(h->device);
+    if (!h->swc && natural_sweeps(h))
+        if (int rc = fvm_alloc(h, (void**)&h->swc, (size_t)(h->ndr + h->ndt + h->ndx) * h->N * sizeof(double))) return rc;
     const int Nr = h->Nr, words = ((Nr + HC - 1) / HC + 31) / 32;
     std::vector<uint32_t> mask((size_t)((Nr + HR - 1) / HR) * words, 0u);
     for (int r = 0; r < Nr; ++r)

@@ -16,6 +16,7 @@
 #include <string>
 
 #include "bte_common.cuh"
+#include "dgemm_warp.cuh"
 
 namespace {
 
@@ -181,38 +182,20 @@ __global__ void k_bsr_upper_unit(int nbr, int bs, int nrhs, const double* __rest
     }
 }
 
-// C = A B (row-major; A M x K, B K x N), FP64, 32 x 32 output tiles through shared memory:
-// the op-split step's collision solve PmatC v (bte_1d3v_solver.py:1797).
-constexpr int GT = 32;
-__global__ void __launch_bounds__(GT * 8)
+// C = A B (row-major; A M x K, B K x N), FP64 (dgemm_warp.cuh): the op-split step's collision solve
+// PmatC v (bte_1d3v_solver.py:1797) and the QoI functionals.
+template <int R>
+__global__ void __launch_bounds__(DGW_WARPS * 32)
 k_dgemm_nn(int M, int N, int K, const double* __restrict__ A, int lda, const double* __restrict__ B, int ldb,
            double* __restrict__ C, int ldc) {
-    __shared__ double As[GT][GT + 1];
-    __shared__ double Bs[GT][GT + 1];
-    const int tx = threadIdx.x % GT, ty = threadIdx.x / GT;  // 32 x 8 threads, 4 rows each
-    const int row0 = blockIdx.y * GT, col = blockIdx.x * GT + tx;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int k0 = 0; k0 < K; k0 += GT) {
-        for (int r = ty; r < GT; r += 8) {
-            const int ar = row0 + r, ak = k0 + tx;
-            As[r][tx] = (ar < M && ak < K) ? A[(size_t)ar * lda + ak] : 0.0;
-            const int bk = k0 + r;
-            Bs[r][tx] = (bk < K && col < N) ? B[(size_t)bk * ldb + col] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int kk = 0; kk < GT; ++kk) {
-            const double b = Bs[kk][tx];
+    int i0, col;
+    if (!dgw_place(M, N, R, &i0, &col)) return;
+    double acc[R];
+    dgw_product<R, false>(M, K, A, lda, B, ldb, i0, min(col, N - 1), acc, dgw_buffer<R>());
+    if (col >= N) return;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) acc[i] += As[ty + 8 * i][kk] * b;
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = row0 + ty + 8 * i;
-        if (r < M && col < N) C[(size_t)r * ldc + col] = acc[i];
-    }
+    for (int i = 0; i < R; ++i)
+        if (i0 + i < M) C[(size_t)(i0 + i) * ldc + col] = acc[i];
 }
 
 // out = in with its three axes reordered: in has dims (d0, d1, d2); output axis a is input
@@ -321,8 +304,11 @@ int bte_dgemm_nn(int M, int N, int K, const double* A, int lda, const double* B,
     if (M == 0 || N == 0) return 0;
     if (!A || !B || !C) return sw_fail("bte_dgemm_nn: null pointer");
     if (C == A || C == B) return sw_fail("bte_dgemm_nn: C must not alias A or B");
-    dim3 grid((unsigned)((N + GT - 1) / GT), (unsigned)((M + GT - 1) / GT));
-    k_dgemm_nn<<<grid, GT * 8, 0, (cudaStream_t)stream>>>(M, N, K, A, lda, B, ldb, C, ldc);
+    const int R = dgw_rows(M, N);
+    dgw_dispatch(R, [&](auto rc) {
+        k_dgemm_nn<decltype(rc)::value><<<dgw_grid(M, N, R), DGW_WARPS * 32, 0, (cudaStream_t)stream>>>(M, N, K, A, lda, B,
+                                                                                                   ldb, C, ldc);
+    });
     return sw_launched("bte_dgemm_nn");
 }
 
