@@ -438,6 +438,38 @@ __global__ void k_to_float(const double* __restrict__ in, float* out, size_t n) 
     if (i < n) out[i] = (float)in[i];
 }
 
+// out[m][c][r] = in[m][r][c]: nm matrices of nr rows and nc columns
+__global__ void k_transpose_op(int nm, int nr, int nc, const double* __restrict__ in, double* __restrict__ out) {
+    const size_t n = (size_t)nm * nr * nc;
+    for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x) {
+        const int r = (int)(o % nr), c = (int)(o / nr % nc);
+        out[o] = in[(o / nr / nc * nr + r) * nc + c];
+    }
+}
+// the 37 pairs (dk, dr), |dk - dr| <= 3, of each (triple, p) in order, p fastest (the others are zero:
+// splines k and r do not overlap)
+__global__ void k_coulomb_pairs(int ntri, int nsp, const double* __restrict__ in, double* __restrict__ out) {
+    const size_t n = (size_t)ntri * nsp;
+    for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x) {
+        const int p = (int)(o % nsp), t = (int)(o / nsp);
+        int e = 0;
+        for (int dk = 0; dk < BTE_NB; ++dk)
+            for (int dr = max(0, dk - BTE_BAND); dr <= min(BTE_NB - 1, dk + BTE_BAND); ++dr, ++e)
+                out[((size_t)t * BTE_PAIRS + e) * nsp + p] = in[(((size_t)t * nsp + p) * BTE_NB + dk) * BTE_NB + dr];
+    }
+}
+// coupling of mode q to q + 1 (w = 0) and q - 1 (w = 1), zero where there is no such mode
+__global__ void k_adv_bands(int nsp, int nsh, const double* __restrict__ mm1, const double* __restrict__ mm2,
+                            const double* __restrict__ coef, double* __restrict__ out) {
+    const int n = nsh * 2 * BTE_NB * nsp;
+    for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < n; o += gridDim.x * blockDim.x) {
+        const int p = o % nsp, d = o / nsp % BTE_NB, w = o / nsp / BTE_NB % 2, q = o / nsp / BTE_NB / 2;
+        const bool on = w == 0 ? q + 1 < nsh : q >= 1;
+        const int bi = p * BTE_NB + d;
+        out[o] = on ? mm1[bi] * coef[q * 4 + 2 * w] + coef[q * 4 + 2 * w + 1] * mm2[bi] : 0.0;
+    }
+}
+
 __global__ void k_absmax(const double* __restrict__ in, size_t n, double* out) {
     __shared__ double red[32];
     double m = 0.0;
@@ -755,6 +787,27 @@ int bte_assemble(BteGrid* g, cudaStream_t s) {
         size_t csz = (size_t)g->ntri * nsp * BTE_NB * BTE_NB;
         if (tof(g->d_CA, g->f_CA, csz)) return BTE_ERR_CUDA;
         if (tof(g->d_CB, g->f_CB, csz)) return BTE_ERR_CUDA;
+    }
+    // tables with the spline index fastest
+    auto transposed = [&](const double* src, double*& dst, int nm, int nr, int nc) -> int {
+        GALLOC(dst, (size_t)nm * nr * nc);
+        k_transpose_op<<<256, 256, 0, s>>>(nm, nr, nc, src, dst);
+        return cudaGetLastError() == cudaSuccess ? BTE_OK : BTE_ERR_CUDA;
+    };
+    if (transposed(g->d_q0, g->t_q0, g->nspecies, nsp, nsp) || transposed(g->d_q1, g->t_q1, g->nspecies, nsp, BTE_NB) ||
+        transposed(g->d_Mr, g->t_Mr, 1, nsp, BTE_NB) || transposed(g->d_cgT, g->t_cgT, 1, nsp, BTE_NB))
+        return BTE_ERR_CUDA;
+    GALLOC(g->t_adv, (size_t)nsh * 2 * BTE_NB * nsp);
+    k_adv_bands<<<64, 256, 0, s>>>(nsp, nsh, g->d_mm1, g->d_mm2, g->d_adv_coef, g->t_adv);
+    CK(cudaGetLastError());
+    if (g->ee) {
+        if (transposed(g->d_HL, g->t_HL, nsh, nsp, nsp) || transposed(g->d_GL, g->t_GL, nsh, nsp, nsp)) return BTE_ERR_CUDA;
+        const size_t pairs = (size_t)g->ntri * BTE_PAIRS * nsp;
+        GALLOC(g->t_CA, pairs);
+        GALLOC(g->t_CB, pairs);
+        k_coulomb_pairs<<<128, 256, 0, s>>>(g->ntri, nsp, g->d_CA, g->t_CA);
+        k_coulomb_pairs<<<128, 256, 0, s>>>(g->ntri, nsp, g->d_CB, g->t_CB);
+        CK(cudaGetLastError());
     }
     // magnitudes for scaling the bordered system
     {

@@ -11,6 +11,7 @@
 #define BTE_SP_ORDER 3          // cubic B-splines only (the reference's driver default)
 #define BTE_BAND 3              // |p - k| <= 3 for overlapping cubic supports
 #define BTE_NB (2 * BTE_BAND + 1)
+#define BTE_PAIRS 37            // (dk, dr) in a band with |dk - dr| <= BTE_BAND
 
 // Physical constants (CODATA 2018, identical doubles to scipy.constants 1.18).
 #define BTE_QE 1.602176634e-19

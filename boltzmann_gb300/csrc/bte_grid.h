@@ -79,6 +79,15 @@ struct BteGrid {
     float* f_mm1 = nullptr; float* f_mm2 = nullptr; float* f_Mr = nullptr;
     float* f_HL = nullptr; float* f_GL = nullptr; float* f_CA = nullptr; float* f_CB = nullptr;
 
+    // the same operators with the spline index p fastest, for kernels whose lanes are consecutive p:
+    // dense [..][column][p], bands [7][p], the Coulomb tensors' 37 pairs |dk - dr| <= 3 [triple][pair][p]
+    double* t_HL = nullptr; double* t_GL = nullptr;   // nsh x nsp x nsp
+    double* t_q0 = nullptr;                           // nspecies x nsp x nsp
+    double* t_q1 = nullptr;                           // nspecies x 7 x nsp
+    double* t_Mr = nullptr; double* t_cgT = nullptr;  // 7 x nsp
+    double* t_adv = nullptr;  // nsh x 2 x 7 x nsp: the advection's coupling of mode q to q + 1 and q - 1
+    double* t_CA = nullptr; double* t_CB = nullptr;   // ntri x 37 x nsp
+
     std::vector<void*> allocations;
     struct BteWork* work = nullptr;      // solver workspace, grown on demand
 };

@@ -20,6 +20,7 @@
 #include <vector>
 #include <algorithm>
 #include <cmath>
+#include <cooperative_groups.h>
 #include "bte_common.cuh"
 #include "bte_grid.h"
 #include "dd_arith.h"
@@ -30,6 +31,8 @@ cudaError_t bte_lu_factor_t(int P, int N, int NC, T* A, int ld, long long stride
 template <typename T>
 cudaError_t bte_lu_solve_t(int P, int N, const T* A, int ld, long long stride, const int32_t* piv, T* b, int mode,
                            cudaStream_t s, const int32_t* mats = nullptr);
+
+namespace cg = cooperative_groups;
 
 // device view of a grid (passed by value to kernels)
 struct GridView {
@@ -42,6 +45,7 @@ struct GridView {
     const double *HL, *GL, *CA, *CB;
     const int* tri;
     const float *fq0, *fq1, *fcgT, *fmm1, *fmm2, *fMr, *fHL, *fGL, *fCA, *fCB;
+    const double *tHL, *tGL, *tq0, *tq1, *tMr, *tcgT, *tadv, *tCA, *tCB;  // spline index fastest
 };
 
 struct PointParams {
@@ -53,279 +57,371 @@ struct PointParams {
 // per-point scalar slots
 enum { SC_GAMMA = 0, SC_MU, SC_T0, SC_M0, SC_NE, SC_COUNT = 8 };
 
-// Double-double accumulation (the residual of a point at its FP64 rounding floor): an exact
-// product (fma) and a compensated sum per term, rounded once at the end of a row (dd_arith.h).
+// ---------------------------------------------------------------------------------
+// Residual F_raw(h) of one point per cluster of S CTAs, plus the merit.
+// If dh != nullptr it is taken at h + alpha * dh and that state is written to hout.
+// aux (if non-null) receives hh = HL h, gg = GL h, U = C_ee(h, h) raw, Mh = M h.
+//
+// GB300's FP64 pipe bounds it (64 cycles per warp instruction and sub-partition), ten-fold so for
+// a point in double-double (an exact product and a compensated sum per term: dd_arith.h). So the
+// work is laid out for full warps of equal instructions: tasks of one row of a potential, one
+// row's terms linear in h, or one e-e triple of one row, with the lanes along consecutive splines
+// (all operator tables are stored that way: a 256-byte access per warp where row-major operators
+// took 32 lines), the triples' 12 of 49 pairs of splines that do not overlap left out, and the
+// advection's coefficients tabulated. For few points the splines are split over the CTAs of a
+// cluster; a row's value does not depend on the split, nor on the number of points. Measured:
+// 4096 points of 384 unknowns with e-e 1000 -> 624 us, 75 points of 768 815 -> 218 us.
+// ---------------------------------------------------------------------------------
+constexpr int RES_T = 256;
 
-// One row (mode q, spline p) of F_raw in double-double: the terms of k_residual's FP64 rows
-// (electron-heavy collisions, gas temperature, advection, growth, e-e) with the Rosenbluth
-// products shh/sgg given as hi + lo. Returns the row and its U and M h parts, rounded.
-__device__ void residual_row_dd(const GridView& g, const PointParams& pp, int pt, int ee, int q, int p,
-                                const double* sh, const double* shh, const double* shl, const double* sgg,
-                                const double* sgl, double n0, double Tg, double cadv, double mu, double negam,
-                                double& y, double& Uo, double& mho) {
-    const int nsh = g.nsh, nsp = g.nsp;
-    double yh = 0.0, yl = 0.0;
+// (hi, lo) += (bh, bl)
+__device__ inline void dd_sum(double& hi, double& lo, double bh, double bl) {
+    const double sm = hi + bh, v = sm - hi;
+    lo += ((hi - (sm - v)) + (bh - v)) + bl;
+    hi = sm;
+}
+
+// The sums of four values over RES_T threads, in two rounds of shuffles that carry all four
+// (6 additions per warp where four separate sums take 20; 64 cycles each on this FP64 pipe).
+// red: 36 doubles.
+__device__ inline void block_sum4(double (&v)[4], double* red) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const bool hi = (lane & 16) != 0, mid = (lane & 8) != 0;
+    double a = hi ? v[2] : v[0], b = hi ? v[3] : v[1];
+    a += __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
+    b += __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 16);
+    double x = mid ? b : a;
+    x += __shfl_xor_sync(0xffffffffu, mid ? a : b, 8);
+    for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if ((lane & 7) == 0) red[wid * 4 + (lane >> 3)] = x;
+    __syncthreads();
+    if (wid < 4) {
+        double y = lane < RES_T / 32 ? red[lane * 4 + wid] : 0.0;
+        for (int o = RES_T / 64; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+        if (lane == 0) red[32 + wid] = y;
+    }
+    __syncthreads();
+    for (int i = 0; i < 4; ++i) v[i] = red[32 + i];
+}
+
+// the terms of row (q, p) that are linear in h (mode-major: sh[l nsp + p]) in FP64 or double-double:
+// electron-heavy collisions, gas temperature, advection, growth; and (M h) of the row
+template <bool DD>
+__device__ inline void residual_linear(const GridView& g, const double* sns, int q, int p, const double* sh, double n0Tg,
+                                       double cadv, double mu, double& yh, double& yl, double& mho) {
+    const int nsp = g.nsp;
+    const double* hq = sh + q * nsp;
+    yh = yl = 0.0;
     for (int s = 0; s < g.nspecies; ++s) {
-        const double ns = n0 * pp.ns[(size_t)s * pp.P + pt];
         double ah = 0.0, al = 0.0;
         if (q == 0) {
-            const double* row = g.q0 + ((size_t)s * nsp + p) * nsp;
-            for (int k = 0; k < nsp; ++k) dd_acc(ah, al, row[k], sh[k * nsh]);
+            const double* col = g.tq0 + (size_t)s * nsp * nsp + p;
+#pragma unroll (DD ? 4 : 16)
+            for (int k = 0; k < nsp; ++k) {
+                if (DD) dd_acc(ah, al, col[(size_t)k * nsp], sh[k]);
+                else ah += col[(size_t)k * nsp] * sh[k];
+            }
         } else {
-            const double* row = g.q1 + ((size_t)s * nsp + p) * BTE_NB;
-            for (int dk = -BTE_BAND; dk <= BTE_BAND; ++dk) {
-                const int k = p + dk;
-                if (k >= 0 && k < nsp) dd_acc(ah, al, row[dk + BTE_BAND], sh[k * nsh + q]);
+            const double* col = g.tq1 + (size_t)s * BTE_NB * nsp + p;
+            for (int d = 0; d < BTE_NB; ++d) {
+                const int k = p + d - BTE_BAND;
+                if (k < 0 || k >= nsp) continue;
+                if (DD) dd_acc(ah, al, col[d * nsp], hq[k]);
+                else ah += col[d * nsp] * hq[k];
             }
         }
-        dd_acc2(yh, yl, ah, al, ns);
+        if (DD) dd_acc2(yh, yl, ah, al, sns[s]);
+        else yh += sns[s] * ah;
     }
     double gh = 0.0, gl = 0.0, vh = 0.0, vl = 0.0, mh = 0.0, ml = 0.0;
-    for (int dk = -BTE_BAND; dk <= BTE_BAND; ++dk) {
-        const int k = p + dk;
+    const double* up = g.tadv + (size_t)q * 2 * BTE_NB * nsp + p;
+    const double* dn = up + BTE_NB * nsp;
+    for (int d = 0; d < BTE_NB; ++d) {
+        const int k = p + d - BTE_BAND;
         if (k < 0 || k >= nsp) continue;
-        const int bi = p * BTE_NB + dk + BTE_BAND;
-        if (q == 0) dd_acc(gh, gl, g.cgT[bi], sh[k * nsh]);
-        if (q + 1 <= g.lmax) {
-            const double a = g.mm1[bi] * g.adv_coef[q * 4 + 0] + g.adv_coef[q * 4 + 1] * g.mm2[bi];
-            dd_acc(vh, vl, a, sh[k * nsh + q + 1]);
+        const int o = d * nsp + p;
+        if (DD) {
+            if (q == 0) dd_acc(gh, gl, g.tcgT[o], sh[k]);
+            if (q + 1 <= g.lmax) dd_acc(vh, vl, up[d * nsp], hq[nsp + k]);
+            if (q >= 1) dd_acc(vh, vl, dn[d * nsp], hq[k - nsp]);
+            dd_acc(mh, ml, g.tMr[o], hq[k]);
+        } else {
+            if (q == 0) gh += g.tcgT[o] * sh[k];
+            if (q + 1 <= g.lmax) vh += up[d * nsp] * hq[nsp + k];
+            if (q >= 1) vh += dn[d * nsp] * hq[k - nsp];
+            mh += g.tMr[o] * hq[k];
         }
-        if (q >= 1) {
-            const double a = g.mm1[bi] * g.adv_coef[q * 4 + 2] + g.adv_coef[q * 4 + 3] * g.mm2[bi];
-            dd_acc(vh, vl, a, sh[k * nsh + q - 1]);
-        }
-        dd_acc(mh, ml, g.Mr[bi], sh[k * nsh + q]);
     }
-    dd_acc2(yh, yl, gh, gl, n0 * Tg);
-    dd_acc2(yh, yl, vh, vl, cadv);
-    dd_acc2(yh, yl, mh, ml, -mu);
-    double Uh = 0.0, Ul = 0.0;
-    if (ee) {
-        for (int t = 0; t < g.ntri; ++t) {
-            if (g.tri[3 * t] != q) continue;
-            const int l = g.tri[3 * t + 1], s = g.tri[3 * t + 2];
-            const double* ca = g.CA + ((size_t)t * nsp + p) * BTE_NB * BTE_NB;
-            const double* cb = g.CB + ((size_t)t * nsp + p) * BTE_NB * BTE_NB;
-            for (int dk = -BTE_BAND; dk <= BTE_BAND; ++dk) {
-                const int k = p + dk;
-                if (k < 0 || k >= nsp) continue;
-                double ih = 0.0, il = 0.0;
-                for (int dr = -BTE_BAND; dr <= BTE_BAND; ++dr) {
-                    const int rr = p + dr;
-                    if (rr < 0 || rr >= nsp) continue;
-                    const int o = (dk + BTE_BAND) * BTE_NB + dr + BTE_BAND;
-                    dd_acc2(ih, il, shh[rr * nsh + s], shl[rr * nsh + s], ca[o]);
-                    dd_acc2(ih, il, sgg[rr * nsh + s], sgl[rr * nsh + s], cb[o]);
-                }
-                dd_acc2(Uh, Ul, ih, il, sh[k * nsh + l]);
-            }
-        }
-        dd_acc2(yh, yl, Uh, Ul, negam);
+    if (DD) {
+        dd_acc2(yh, yl, gh, gl, n0Tg);
+        dd_acc2(yh, yl, vh, vl, cadv);
+        dd_acc2(yh, yl, mh, ml, -mu);
+    } else {
+        yh += n0Tg * gh + cadv * vh - mu * mh;
     }
-    y = yh + yl;
-    Uo = Uh + Ul;
     mho = mh + ml;
 }
 
-// ---------------------------------------------------------------------------------
-// Residual F_raw(h) for one point per CTA, plus ||(I - p p^T) M^-1 F_raw||.
-// If dh != nullptr the CTA evaluates at h + alpha * dh and writes that state to hout.
-// aux (if non-null) receives hh = HL h, gg = GL h, U = C_ee(h, h) raw, Mh = M h.
-// ---------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
+// triple t = (q, l, s) of row p: sum_dk h[p + dk, l] sum_dr (CA HLh + CB GLh)[p + dr, s]
+template <bool DD>
+__device__ inline void residual_triple(const GridView& g, int t, int p, const double* hl, const double* hh, const double* hhl,
+                                       const double* gg, const double* ggl, double& Uh, double& Ul) {
+    const int nsp = g.nsp;
+    const double* ca = g.tCA + (size_t)t * BTE_PAIRS * nsp + p;
+    const double* cb = g.tCB + (size_t)t * BTE_PAIRS * nsp + p;
+    Uh = Ul = 0.0;
+    // the neighbours' potentials; outside the grid the coefficients are zero
+    double vh[BTE_NB], vg[BTE_NB];
+    if (!DD)
+#pragma unroll
+        for (int d = 0; d < BTE_NB; ++d) {
+            const int r = min(max(p + d - BTE_BAND, 0), nsp - 1);
+            vh[d] = hh[r];
+            vg[d] = gg[r];
+        }
+    int e = 0;
+#pragma unroll
+    for (int dk = 0; dk < BTE_NB; ++dk) {
+        const double hv = hl[min(max(p + dk - BTE_BAND, 0), nsp - 1)];
+        double ih = 0.0, il = 0.0;
+#pragma unroll
+        for (int dr = (dk > BTE_BAND ? dk - BTE_BAND : 0); dr <= (dk < BTE_BAND ? dk + BTE_BAND : BTE_NB - 1); ++dr, ++e) {
+            const double a = ca[(size_t)e * nsp], b = cb[(size_t)e * nsp];
+            if (DD) {
+                const int r = min(max(p + dr - BTE_BAND, 0), nsp - 1);
+                dd_acc2(ih, il, hh[r], hhl[r], a);
+                dd_acc2(ih, il, gg[r], ggl[r], b);
+            } else {
+                ih += a * vh[dr] + b * vg[dr];
+            }
+        }
+        if (DD) dd_acc2(Uh, Ul, ih, il, hv);
+        else Uh += ih * hv;
+    }
+}
+
+// doubles of shared memory: h, the potentials and their low parts (n each), per row of the CTA the
+// linear terms, their low parts, M h, U and its low part, and the triples' partial sums (two per triple
+// and spline, tc triples at a time), and the species' densities
+static size_t res_doubles(const GridView& g, int npl, int tc) {
+    return (size_t)5 * g.n + (size_t)5 * g.nsh * npl + (size_t)2 * tc * npl + g.nspecies;
+}
+
+__global__ void __launch_bounds__(RES_T, 3)
 k_residual(GridView g, PointParams pp, int ee, const int* __restrict__ act, int nact,
            const double* __restrict__ h, const double* __restrict__ dh, int ldd, const double* __restrict__ alpha,
            const int* __restrict__ need, double* hout, double* F, double* aux, double* scal, double* rnorm,
-           double* srel, const int* __restrict__ ddm) {
+           double* srel, const int* __restrict__ ddm, int npl, int tc) {
     extern __shared__ double sm[];
-    const int slot = blockIdx.x;
+    __shared__ double red[36];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int slot = blockIdx.x / S;
     if (slot >= nact) return;
     const int pt = act[slot];
     if (pp.eept) ee = pp.eept[pt];
     if (need && !need[pt]) return;
-    // a point at its FP64 rounding floor is evaluated in double-double (smem 7 n instead of 5 n)
+    // a point at its FP64 rounding floor is evaluated in double-double
     const bool dd = ddm != nullptr && ddm[pt] != 0;
     const int n = g.n, nsh = g.nsh, nsp = g.nsp, tid = threadIdx.x, nt = blockDim.x;
-    double* sh = sm;           // h
-    double* shh = sm + n;      // HL h
-    double* sgg = sm + 2 * n;  // GL h
-    double* sF = sm + 3 * n;   // F_raw, later M^-1 F
-    double* sR = sm + 4 * n;
-    double* shl = sm + 5 * n;  // low parts of HL h and GL h (double-double points)
-    double* sgl = sm + 6 * n;
-    __shared__ double red[32];
+    const int p0 = min(nsp, rank * npl), p1 = min(nsp, p0 + npl), np = p1 - p0;  // my splines
+    double* sh = sm;                // h, mode-major
+    double* shh = sm + n;           // HL h
+    double* sgg = sm + 2 * n;       // GL h
+    double* shl = sm + 3 * n;       // their low parts (double-double points)
+    double* sgl = sm + 4 * n;
+    double* ylin = sm + 5 * n;      // [q][p - p0]: linear terms, low parts, M h, U, its low part
+    double* ylow = ylin + nsh * npl;
+    double* ymh = ylow + nsh * npl;
+    double* uhi = ymh + nsh * npl;
+    double* ulo = uhi + nsh * npl;
+    double* part = ulo + nsh * npl;  // [triple of the chunk][p - p0], then the low parts
+    double* parl = part + (size_t)tc * npl;
+    double* ns = parl + (size_t)tc * npl;  // n0 ns per species
 
     const double* hp = h + (size_t)pt * n;
     const double a = alpha ? alpha[pt] : 0.0;
-    double sd = 0.0, shn = 0.0;
+    const double n0 = pp.n0[pt], Tg = pp.Tg[pt], E = pp.E[pt], ne = pp.ne[pt];
+    for (int s = tid; s < g.nspecies; s += nt) ns[s] = n0 * pp.ns[(size_t)s * pp.P + pt];
+    __syncthreads();
+    double shn = 0.0, sums[4] = {0.0, 0.0, 0.0, 0.0};  // mass, temperature, growth; |dh|^2
     for (int i = tid; i < n; i += nt) {
         double v = hp[i];
         if (dh) {
             double d = dh[(size_t)pt * ldd + i];
-            sd += d * d;
+            sums[3] += d * d;
             shn += v * v;
             v += a * d;
         }
-        sh[i] = v;
-        if (hout) hout[(size_t)pt * n + i] = v;
-    }
-    __syncthreads();
-    if (srel) {
-        sd = block_sum(sd, red);
-        shn = block_sum(shn, red);
-        if (tid == 0) srel[pt] = sqrt(sd / fmax(shn, 1e-300));
-    }
-    const double n0 = pp.n0[pt], Tg = pp.Tg[pt], E = pp.E[pt], ne = pp.ne[pt];
-    double m0 = 0, t0 = 0, mu = 0;
-    for (int i = tid; i < n; i += nt) {
-        double v = sh[i];
-        m0 += g.mass[i] * v;
-        t0 += g.temp[i] * v;
+        sh[(i % nsh) * nsp + i / nsh] = v;
+        if (hout && rank == 0) hout[(size_t)pt * n + i] = v;
+        sums[0] += g.mass[i] * v;
+        sums[1] += g.temp[i] * v;
         double ws = 0;
-        for (int s = 0; s < g.nspecies; ++s) ws += n0 * pp.ns[(size_t)s * pp.P + pt] * g.W[(size_t)s * n + i];
-        mu += ws * v;
+        for (int s = 0; s < g.nspecies; ++s) ws += ns[s] * g.W[(size_t)s * n + i];
+        sums[2] += ws * v;
     }
-    m0 = block_sum(m0, red);
-    t0 = block_sum(t0, red);
-    mu = block_sum(mu, red);
-    double gam = 0.0;
+    block_sum4(sums, red);
+    const double m0 = sums[0], t0 = sums[1], mu = sums[2];
+    if (srel && rank == 0) {
+        shn = block_sum(shn, red);
+        if (tid == 0) srel[pt] = sqrt(sums[3] / fmax(shn, 1e-300));
+    }
     if (ee) {
-        for (int r = tid; r < n; r += nt) {
-            int p = r / nsh, l = r % nsh;
-            const double* HLr = g.HL + ((size_t)l * nsp + p) * nsp;
-            const double* GLr = g.GL + ((size_t)l * nsp + p) * nsp;
+        // potentials of my splines and their neighbours
+        const int h0 = max(0, p0 - BTE_BAND), nh = min(nsp, p1 + BTE_BAND) - h0;
+        const int rows = np > 0 ? nsh * nh : 0;
+        for (int e = tid; e < 2 * rows; e += nt) {
+            const int l = (e % rows) / nh, p = h0 + e % nh;
+            const double* col = (e < rows ? g.tHL : g.tGL) + (size_t)l * nsp * nsp + p;
+            const double* hl = sh + l * nsp;
+            double s1 = 0.0, l1 = 0.0;
             if (dd) {
-                double h1 = 0, l1 = 0, h2 = 0, l2 = 0;
-                for (int c = 0; c < nsp; ++c) {
-                    const double hv = sh[c * nsh + l];
-                    dd_acc(h1, l1, HLr[c], hv);
-                    dd_acc(h2, l2, GLr[c], hv);
-                }
-                shh[r] = h1;
-                shl[r] = l1;
-                sgg[r] = h2;
-                sgl[r] = l2;
-                continue;
+#pragma unroll 4
+                for (int c = 0; c < nsp; ++c) dd_acc(s1, l1, col[(size_t)c * nsp], hl[c]);
+            } else {
+#pragma unroll 8
+                for (int c = 0; c < nsp; ++c) s1 += col[(size_t)c * nsp] * hl[c];
             }
-            double s1 = 0, s2 = 0;
-            for (int c = 0; c < nsp; ++c) {
-                double hv = sh[c * nsh + l];
-                s1 += HLr[c] * hv;
-                s2 += GLr[c] * hv;
-            }
-            shh[r] = s1;
-            sgg[r] = s2;
+            const int o = l * nsp + p;
+            (e < rows ? shh : sgg)[o] = s1;
+            if (dd) (e < rows ? shl : sgl)[o] = l1;
         }
-        // Coulomb logarithm (bte_0d3v_batched.py:652-661)
-        double mm0 = g.mw0 * m0 * g.vth * g.vth * g.vth;
-        double kT = fabs(g.mw0 * ((t0 * g.k1ev) / mm0) * pow(g.vth, 5.0) * BTE_KB);
-        double cl = (12.0 * BTE_PI * pow(BTE_EPS0 * kT, 1.5)) / (BTE_QE * BTE_QE * BTE_QE * sqrt(ne));
-        gam = log(cl) * g.gam_c;
+        if (tid >= nt - 32) {
+            // Coulomb logarithm (bte_0d3v_batched.py:652-661), by one warp: in each of eight its
+            // powers and logarithm held the FP64 pipe as long as the rest of a small point
+            double mm0 = g.mw0 * m0 * g.vth * g.vth * g.vth;
+            double kT = fabs(g.mw0 * ((t0 * g.k1ev) / mm0) * pow(g.vth, 5.0) * BTE_KB);
+            double cl = (12.0 * BTE_PI * pow(BTE_EPS0 * kT, 1.5)) / (BTE_QE * BTE_QE * BTE_QE * sqrt(ne));
+            if (tid == nt - 1) red[0] = log(cl) * g.gam_c;
+        }
         __syncthreads();
     }
+    const double gam = ee ? red[0] : 0.0;
     const double cadv = E * g.c_adv;
-    // rows mode-major: the lanes of a warp share the mode, so the dense l = 0 row and the
-    // e-e triples of that mode run without divergence
-    for (int rm = tid; rm < n; rm += nt) {
-        const int q = rm / nsp, p = rm % nsp;
-        const int r = p * nsh + q;
-        if (dd) {
-            double y, U, mh;
-            residual_row_dd(g, pp, pt, ee, q, p, sh, shh, shl, sgg, sgl, n0, Tg, cadv, mu, ne * gam, y, U, mh);
-            sF[r] = y;
-            F[(size_t)pt * n + r] = y;
-            if (aux) {
-                double* ax = aux + (size_t)pt * 4 * n;
-                ax[r] = shh[r] + shl[r];
-                ax[n + r] = sgg[r] + sgl[r];
-                ax[2 * n + r] = U;
-                ax[3 * n + r] = mh;
-            }
-            continue;
-        }
-        double y = 0.0;
-        // electron-heavy collisions
-        for (int s = 0; s < g.nspecies; ++s) {
-            double ns = n0 * pp.ns[(size_t)s * pp.P + pt];
-            double acc = 0.0;
-            if (q == 0) {
-                const double* row = g.q0 + ((size_t)s * nsp + p) * nsp;
-                for (int k = 0; k < nsp; ++k) acc += row[k] * sh[k * nsh];
+    const int rows = nsh * np;
+    // tasks: the linear terms of my rows (with the first chunk), and the e-e triples of my splines
+    for (int t0c = 0; t0c == 0 || (ee && t0c < g.ntri); t0c += tc) {
+        const int lin = t0c == 0 ? rows : 0, nt3 = ee ? min(tc, g.ntri - t0c) * np : 0;
+        for (int e = tid; e < lin + nt3; e += nt) {
+            if (e < lin) {
+                const int q = e / np, i = e % np;
+                double yh, yl, mh;
+                if (dd) residual_linear<true>(g, ns, q, p0 + i, sh, n0 * Tg, cadv, mu, yh, yl, mh);
+                else residual_linear<false>(g, ns, q, p0 + i, sh, n0 * Tg, cadv, mu, yh, yl, mh);
+                ylin[q * npl + i] = yh;
+                ylow[q * npl + i] = yl;
+                ymh[q * npl + i] = mh;
             } else {
-                const double* row = g.q1 + ((size_t)s * nsp + p) * BTE_NB;
-                for (int dk = -BTE_BAND; dk <= BTE_BAND; ++dk) {
-                    int k = p + dk;
-                    if (k >= 0 && k < nsp) acc += row[dk + BTE_BAND] * sh[k * nsh + q];
-                }
-            }
-            y += ns * acc;
-        }
-        double gt = 0.0, adv = 0.0, mh = 0.0;
-        for (int dk = -BTE_BAND; dk <= BTE_BAND; ++dk) {
-            int k = p + dk;
-            if (k < 0 || k >= nsp) continue;
-            int bi = p * BTE_NB + dk + BTE_BAND;
-            if (q == 0) gt += g.cgT[bi] * sh[k * nsh];
-            if (q + 1 <= g.lmax)
-                adv += (g.mm1[bi] * g.adv_coef[q * 4 + 0] + g.adv_coef[q * 4 + 1] * g.mm2[bi]) * sh[k * nsh + q + 1];
-            if (q >= 1)
-                adv += (g.mm1[bi] * g.adv_coef[q * 4 + 2] + g.adv_coef[q * 4 + 3] * g.mm2[bi]) * sh[k * nsh + q - 1];
-            mh += g.Mr[bi] * sh[k * nsh + q];
-        }
-        y += n0 * Tg * gt + cadv * adv - mu * mh;
-        double U = 0.0;
-        if (ee) {
-            for (int t = 0; t < g.ntri; ++t) {
-                if (g.tri[3 * t] != q) continue;
+                const int j = (e - lin) / np, i = (e - lin) % np, t = t0c + j;
                 const int l = g.tri[3 * t + 1], s = g.tri[3 * t + 2];
-                const double* ca = g.CA + ((size_t)t * nsp + p) * BTE_NB * BTE_NB;
-                const double* cb = g.CB + ((size_t)t * nsp + p) * BTE_NB * BTE_NB;
-                for (int dk = -BTE_BAND; dk <= BTE_BAND; ++dk) {
-                    int k = p + dk;
-                    if (k < 0 || k >= nsp) continue;
-                    double inner = 0.0;
-                    for (int dr = -BTE_BAND; dr <= BTE_BAND; ++dr) {
-                        int rr = p + dr;
-                        if (rr < 0 || rr >= nsp) continue;
-                        int o = (dk + BTE_BAND) * BTE_NB + dr + BTE_BAND;
-                        inner += ca[o] * shh[rr * nsh + s] + cb[o] * sgg[rr * nsh + s];
-                    }
-                    U += inner * sh[k * nsh + l];
-                }
+                double Uh, Ul;
+                if (dd) residual_triple<true>(g, t, p0 + i, sh + l * nsp, shh + s * nsp, shl + s * nsp, sgg + s * nsp,
+                                              sgl + s * nsp, Uh, Ul);
+                else residual_triple<false>(g, t, p0 + i, sh + l * nsp, shh + s * nsp, nullptr, sgg + s * nsp, nullptr, Uh, Ul);
+                part[j * npl + i] = Uh;
+                parl[j * npl + i] = Ul;
             }
-            y += ne * gam * U;
         }
-        sF[r] = y;
+        __syncthreads();
+        for (int e = tid; e < rows; e += nt) {  // U += the chunk's triples of the row's mode, in order
+            const int q = e / np, i = e % np, o = q * npl + i;
+            double Uh = t0c == 0 ? 0.0 : uhi[o], Ul = t0c == 0 ? 0.0 : ulo[o];
+            const int m = ee ? min(tc, g.ntri - t0c) : 0;
+            for (int j = 0; j < m; ++j) {
+                if (g.tri[3 * (t0c + j)] != q) continue;
+                if (dd) dd_sum(Uh, Ul, part[j * npl + i], parl[j * npl + i]);
+                else Uh += part[j * npl + i];
+            }
+            uhi[o] = Uh;
+            ulo[o] = Ul;
+        }
+        __syncthreads();
+    }
+    for (int e = tid; e < rows; e += nt) {
+        const int q = e / np, i = e % np, o = q * npl + i, r = (p0 + i) * nsh + q;
+        double y, U;
+        if (dd) {
+            double yh = ylin[o], yl = ylow[o];
+            if (ee) dd_acc2(yh, yl, uhi[o], ulo[o], ne * gam);
+            y = yh + yl;
+            U = uhi[o] + ulo[o];
+        } else {
+            U = uhi[o];
+            y = ylin[o];
+            if (ee) y += ne * gam * U;
+        }
         F[(size_t)pt * n + r] = y;
         if (aux) {
             double* ax = aux + (size_t)pt * 4 * n;
-            ax[r] = shh[r];
-            ax[n + r] = sgg[r];
+            const int m = q * nsp + p0 + i;
+            ax[r] = ee ? (dd ? shh[m] + shl[m] : shh[m]) : 0.0;
+            ax[n + r] = ee ? (dd ? sgg[m] + sgl[m] : sgg[m]) : 0.0;
             ax[2 * n + r] = U;
-            ax[3 * n + r] = mh;
+            ax[3 * n + r] = ymh[o];
         }
     }
+    if (S > 1) cluster.sync();
+    else __syncthreads();
+    if (rank != 0) return;
     if (scal && tid == 0) {
         double* sc = scal + (size_t)pt * SC_COUNT;
         sc[SC_GAMMA] = gam; sc[SC_MU] = mu; sc[SC_T0] = t0; sc[SC_M0] = m0; sc[SC_NE] = ne;
     }
-    __syncthreads();
     // merit ||P_v D F||, D = diag(M)^-1, v = D M p / |D M p|: zero exactly at the reference's
     // roots (Q^T M^-1 F = 0 <=> F || M p) without the round-off amplification of a dense M^-1
     double pr = 0.0;
     for (int r = tid; r < n; r += nt) {
-        double d = sF[r] * g.invMd[r];
-        sR[r] = d;
+        double d = __ldcg(F + (size_t)pt * n + r) * g.invMd[r];
+        sh[r] = d;
         pr += g.vD[r] * d;
     }
     pr = block_sum(pr, red);
     double nn = 0.0;
     for (int r = tid; r < n; r += nt) {
-        double v = sR[r] - g.vD[r] * pr;
+        double v = sh[r] - g.vD[r] * pr;
         nn += v * v;
     }
     nn = block_sum(nn, red);
     if (tid == 0) rnorm[pt] = sqrt(nn);
+}
+
+// CTAs per point for few points (a cluster, at least 12 splines each), so that about one SM each works
+static int point_split(int nact, int nsp) {
+    int S = 1;
+    while (S < 8 && nact * 2 * S <= 160 && nsp / (2 * S) >= 12) S *= 2;
+    return S;
+}
+
+template <class K, class... A>
+static cudaError_t launch_points(K kernel, int nact, int S, size_t smem, cudaStream_t s, A... args) {
+    cudaError_t e = bte_raise_smem_limit((const void*)kernel, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)nact * S);
+    cfg.blockDim = dim3(RES_T);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)S;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// triples whose partial sums are kept at once: all where two CTAs fit an SM, else as many as one CTA holds
+template <class... A>
+static cudaError_t run_residual(const GridView& g, int nact, cudaStream_t s, A... args) {
+    const int S = point_split(nact, g.nsp), npl = (g.nsp + S - 1) / S;
+    int tc = std::max(1, g.ntri);
+    if (res_doubles(g, npl, tc) * 8 > 110 * 1024) {
+        const long long room = 200 * 1024 / 8 - (long long)res_doubles(g, npl, 0);
+        tc = (int)std::max<long long>(1, std::min<long long>(tc, room / (2 * npl)));
+    }
+    return launch_points(k_residual, nact, S, res_doubles(g, npl, tc) * sizeof(double), s, g, args..., npl, tc);
 }
 
 // The reference's merit ||(I - p p^T) M^-1 F|| = ||Q^T M^-1 F|| (bte_0d3v_batched.py:920-926)
@@ -373,106 +469,117 @@ __host__ __device__ inline int kc_row(int nsh) { return 3 * BTE_NB * nsh; }
 // The residual is scaled by its max-norm sigma and stored in FP32 (slot-major) for the
 // FP32 substitution; sigma[slot] is kept to undo the scaling.
 // ---------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
+// Laid out as k_residual: lanes along consecutive splines of one mode on tables stored that way,
+// the splines split over a cluster's CTAs for few points (the scaling's maximum is exchanged
+// through distributed shared memory and does not depend on the split). Measured: 4096 points of 384 unknowns with e-e 350 -> 214 us, 75 points of 768 197 -> 49 us.
+__global__ void __launch_bounds__(RES_T, 3)
 k_refine_residual(GridView g, PointParams pp, int ee, const int* __restrict__ act, int nact,
                   const double* __restrict__ h, const double* __restrict__ F, const double* __restrict__ aux,
                   const double* __restrict__ scal, const double* __restrict__ x, int ldd, double beta_scale,
                   const double* __restrict__ rowscale, float* __restrict__ rs, double* __restrict__ sigma,
                   const int* __restrict__ done, const double* __restrict__ kc, const int* __restrict__ slots,
-                  int matvec, const double* __restrict__ xlist, int ldx, double* __restrict__ out64) {
-    // slots (optional): CTA i works on slot slots[i]; xlist (optional): x of CTA i at
+                  int matvec, const double* __restrict__ xlist, int ldx, double* __restrict__ out64, int npl) {
+    // slots (optional): point i is slot slots[i]; xlist (optional): x of point i at
     // xlist + i * ldx instead of x[pt * ldd]; matvec: D (J x) instead of D (b - J x);
-    // out64 (optional): the FP64 result of CTA i at out64 + i * (n + 1), and no FP32 output
+    // out64 (optional): the FP64 result of point i at out64 + i * (n + 1), and no FP32 output
     extern __shared__ double sm[];
-    if ((int)blockIdx.x >= nact) return;
-    const int slot = slots ? slots[blockIdx.x] : (int)blockIdx.x;
+    __shared__ double red[36];
+    __shared__ double smax;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int idx = blockIdx.x / S;
+    if (idx >= nact) return;
+    const int slot = slots ? slots[idx] : idx;
     const int pt = act[slot];
     if (pp.eept) ee = pp.eept[pt];
     const int n = g.n, nsh = g.nsh, nsp = g.nsp, N = n + 1, tid = threadIdx.x, nt = blockDim.x;
     if (done && done[pt]) {  // refinement finished for this point: a zero correction
-        for (int i = tid; i < N; i += nt) rs[(size_t)slot * N + i] = 0.0f;
-        if (tid == 0) sigma[slot] = 0.0;
+        if (rank == 0) {
+            for (int i = tid; i < N; i += nt) rs[(size_t)slot * N + i] = 0.0f;
+            if (tid == 0) sigma[slot] = 0.0;
+        }
         return;
     }
-    double* sx = sm;            // x (n + 1)
-    double* sh = sm + N;        // h
-    double* sxh = sh + n;       // HL x
+    const int p0 = min(nsp, rank * npl), p1 = min(nsp, p0 + npl), np = p1 - p0;  // my splines
+    double* sx = sm;            // x, mode-major
+    double* sxh = sx + n;       // HL x
     double* sxg = sxh + n;      // GL x
-    double* sr = sxg + n;       // r
-    __shared__ double red[32];
+    double* sr = sxg + n;       // my rows of the result [q][p - p0], then the constraint row
     const double* hp = h + (size_t)pt * n;
     const double* ax = aux + (size_t)pt * 4 * n;
     const double* sc = scal + (size_t)pt * SC_COUNT;
-    for (int i = tid; i < N; i += nt) sx[i] = xlist ? xlist[(size_t)blockIdx.x * ldx + i] : x[(size_t)pt * ldd + i];
-    for (int i = tid; i < n; i += nt) sh[i] = hp[i];
-    __syncthreads();
+    const double* xp = xlist ? xlist + (size_t)idx * ldx : x + (size_t)pt * ldd;
+    for (int i = tid; i < n; i += nt) sx[(i % nsh) * nsp + i / nsh] = xp[i];
+    const double xn = xp[n];
     const double n0 = pp.n0[pt], Tg = pp.Tg[pt], E = pp.E[pt], ne = sc[SC_NE];
     const double gam = sc[SC_GAMMA], mu = sc[SC_MU], t0 = sc[SC_T0], m0 = sc[SC_M0];
     const double beta = beta_scale * n0;
+    const double it0 = ee ? 1.0 / t0 : 0.0, im0 = ee ? 1.0 / m0 : 0.0;
     double wx = 0, dgx = 0, ux = 0, uh = 0;
     for (int i = tid; i < n; i += nt) {
+        const double xi = xp[i];
         double ws = 0;
         for (int s = 0; s < g.nspecies; ++s) ws += n0 * pp.ns[(size_t)s * pp.P + pt] * g.W[(size_t)s * n + i];
-        wx += ws * sx[i];
-        dgx += (g.temp[i] / t0 - g.mass[i] / m0) * sx[i];
-        ux += g.u[i] * sx[i];
-        uh += g.u[i] * sh[i];
+        wx += ws * xi;
+        if (ee) dgx += (g.temp[i] * it0 - g.mass[i] * im0) * xi;
+        ux += g.u[i] * xi;
+        uh += g.u[i] * hp[i];
     }
-    wx = block_sum(wx, red);
-    dgx = block_sum(dgx, red) * g.gam_c * 1.5;
-    ux = block_sum(ux, red);
-    uh = block_sum(uh, red);
-    if (ee) {
-        // HL x and GL x; rows taken mode-major so that a warp shares the mode
-        for (int rm = tid; rm < n; rm += nt) {
-            const int l = rm / nsp, p = rm % nsp;
-            const double* HLr = g.HL + (size_t)rm * nsp;
-            const double* GLr = g.GL + (size_t)rm * nsp;
-            double s1 = 0, s2 = 0;
-            for (int c = 0; c < nsp; ++c) {
-                double v = sx[c * nsh + l];
-                s1 += HLr[c] * v;
-                s2 += GLr[c] * v;
-            }
-            sxh[p * nsh + l] = s1;
-            sxg[p * nsh + l] = s2;
+    double sums[4] = {wx, dgx, ux, uh};
+    block_sum4(sums, red);
+    wx = sums[0];
+    dgx = sums[1] * g.gam_c * 1.5;
+    ux = sums[2];
+    uh = sums[3];
+    if (ee) {  // HL x and GL x of my splines and their neighbours
+        const int h0 = max(0, p0 - BTE_BAND), nh = min(nsp, p1 + BTE_BAND) - h0;
+        const int rows = np > 0 ? nsh * nh : 0;
+        for (int e = tid; e < 2 * rows; e += nt) {
+            const int l = (e % rows) / nh, p = h0 + e % nh;
+            const double* col = (e < rows ? g.tHL : g.tGL) + (size_t)l * nsp * nsp + p;
+            const double* xl = sx + l * nsp;
+            double s1 = 0.0;
+#pragma unroll 8
+            for (int c = 0; c < nsp; ++c) s1 += col[(size_t)c * nsp] * xl[c];
+            (e < rows ? sxh : sxg)[l * nsp + p] = s1;
         }
         __syncthreads();
     }
     const double cadv = E * g.c_adv;
-    const int kcn = kc_row(nsh);
+    const int kcn = kc_row(nsh), rows = nsh * np;
     double amax = 0.0;
-    // rows mode-major: the lanes of a warp take the same branch (dense l = 0 row or band)
-    for (int rm = tid; rm < n; rm += nt) {
-        const int q = rm / nsp, p = rm % nsp;
+    for (int e = tid; e < rows; e += nt) {
+        const int q = e / np, p = p0 + e % np;
         const int r = p * nsh + q;
+        const double* xq = sx + q * nsp;
         double y = 0.0;
         for (int s = 0; s < g.nspecies; ++s) {
             double ns = n0 * pp.ns[(size_t)s * pp.P + pt];
             double acc = 0.0;
             if (q == 0) {
-                const double* row = g.q0 + ((size_t)s * nsp + p) * nsp;
-                for (int k = 0; k < nsp; ++k) acc += row[k] * sx[k * nsh];
+                const double* col = g.tq0 + (size_t)s * nsp * nsp + p;
+#pragma unroll 16
+                for (int k = 0; k < nsp; ++k) acc += col[(size_t)k * nsp] * sx[k];
             } else {
-                const double* row = g.q1 + ((size_t)s * nsp + p) * BTE_NB;
-                for (int dk = -BTE_BAND; dk <= BTE_BAND; ++dk) {
-                    int k = p + dk;
-                    if (k >= 0 && k < nsp) acc += row[dk + BTE_BAND] * sx[k * nsh + q];
+                const double* col = g.tq1 + (size_t)s * BTE_NB * nsp + p;
+                for (int d = 0; d < BTE_NB; ++d) {
+                    const int k = p + d - BTE_BAND;
+                    if (k >= 0 && k < nsp) acc += col[d * nsp] * xq[k];
                 }
             }
             y += ns * acc;
         }
         double gt = 0.0, adv = 0.0, mx = 0.0;
-        for (int dk = -BTE_BAND; dk <= BTE_BAND; ++dk) {
-            int k = p + dk;
+        const double* up = g.tadv + (size_t)q * 2 * BTE_NB * nsp + p;
+        const double* dn = up + BTE_NB * nsp;
+        for (int d = 0; d < BTE_NB; ++d) {
+            const int k = p + d - BTE_BAND;
             if (k < 0 || k >= nsp) continue;
-            int bi = p * BTE_NB + dk + BTE_BAND;
-            if (q == 0) gt += g.cgT[bi] * sx[k * nsh];
-            if (q + 1 <= g.lmax)
-                adv += (g.mm1[bi] * g.adv_coef[q * 4 + 0] + g.adv_coef[q * 4 + 1] * g.mm2[bi]) * sx[k * nsh + q + 1];
-            if (q >= 1)
-                adv += (g.mm1[bi] * g.adv_coef[q * 4 + 2] + g.adv_coef[q * 4 + 3] * g.mm2[bi]) * sx[k * nsh + q - 1];
-            mx += g.Mr[bi] * sx[k * nsh + q];
+            const int o = d * nsp + p;
+            if (q == 0) gt += g.tcgT[o] * sx[k];
+            if (q + 1 <= g.lmax) adv += up[d * nsp] * xq[nsp + k];
+            if (q >= 1) adv += dn[d * nsp] * xq[k - nsp];
+            mx += g.tMr[o] * xq[k];
         }
         y += n0 * Tg * gt + cadv * adv - mu * mx - ax[3 * n + r] * wx;
         if (ee && kc) {
@@ -480,47 +587,63 @@ k_refine_residual(GridView g, PointParams pp, int ee, const int* __restrict__ ac
             // Jacobian of this Newton step wrote: K1 . x over the band, K2a . (HL x) + K2b . (GL x)
             const double* kr = kc + ((size_t)slot * n + r) * kcn;
             double c1 = 0.0;
-            for (int e = 0; e < BTE_NB * nsh; ++e) {
-                const int k = p + e / nsh - BTE_BAND;
-                if (k >= 0 && k < nsp) c1 += kr[e] * sx[k * nsh + e % nsh];
+            for (int w = 0; w < BTE_NB * nsh; ++w) {
+                const int k = p + w / nsh - BTE_BAND;
+                if (k >= 0 && k < nsp) c1 += kr[w] * sx[(w % nsh) * nsp + k];
             }
-            for (int e = 0; e < BTE_NB * nsh; ++e) {
-                const int rr = p + e % BTE_NB - BTE_BAND;
+            for (int w = 0; w < BTE_NB * nsh; ++w) {
+                const int rr = p + w % BTE_NB - BTE_BAND;
                 if (rr < 0 || rr >= nsp) continue;
-                const int o = rr * nsh + e / BTE_NB;
-                c1 += kr[BTE_NB * nsh + e] * sxh[o] + kr[2 * BTE_NB * nsh + e] * sxg[o];
+                const int o = (w / BTE_NB) * nsp + rr;
+                c1 += kr[BTE_NB * nsh + w] * sxh[o] + kr[2 * BTE_NB * nsh + w] * sxg[o];
             }
             y += ne * gam * c1 + ne * ax[2 * n + r] * dgx;
         }
-        y += -beta * g.Mp[r] * sx[n];
+        y += -beta * g.Mp[r] * xn;
         double rv = (matvec ? y : (-F[(size_t)pt * n + r] - y)) * rowscale[(size_t)slot * N + r];
-        sr[r] = rv;
+        sr[e] = rv;
         amax = fmax(amax, fabs(rv));
     }
-    if (tid == 0) {
+    if (tid == 0 && rank == 0) {
         double rv = (matvec ? beta * ux : (beta * (1.0 - uh) - beta * ux)) * rowscale[(size_t)slot * N + n];
-        sr[n] = rv;
+        sr[rows] = rv;
         amax = fmax(amax, fabs(rv));
     }
+    __syncthreads();
     if (out64) {
-        __syncthreads();
-        for (int i = tid; i < N; i += nt) out64[(size_t)blockIdx.x * N + i] = sr[i];
+        for (int e = tid; e < rows; e += nt) out64[(size_t)idx * N + (p0 + e % np) * nsh + e / np] = sr[e];
+        if (tid == 0 && rank == 0) out64[(size_t)idx * N + n] = sr[rows];
         return;
     }
     // max-norm for the FP32 scaling
     for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    __syncthreads();
     if ((tid & 31) == 0) red[tid >> 5] = amax;
     __syncthreads();
     if (tid == 0) {
         double m = 0.0;
         for (int w = 0; w < (nt + 31) / 32; ++w) m = fmax(m, red[w]);
-        red[0] = (m > 0.0) ? m : 1.0;
-        sigma[slot] = red[0];
+        smax = m;
     }
-    __syncthreads();
-    const double inv = 1.0 / red[0];
-    for (int i = tid; i < N; i += nt) rs[(size_t)slot * N + i] = (float)(sr[i] * inv);
+    if (S > 1) cluster.sync();
+    else __syncthreads();
+    double m = smax;
+    if (S > 1) {
+        m = 0.0;
+        for (int c = 0; c < S; ++c) m = fmax(m, *cluster.map_shared_rank(&smax, c));
+    }
+    if (!(m > 0.0)) m = 1.0;
+    if (tid == 0 && rank == 0) sigma[slot] = m;
+    const double inv = 1.0 / m;
+    for (int e = tid; e < rows; e += nt) rs[(size_t)slot * N + (p0 + e % np) * nsh + e / np] = (float)(sr[e] * inv);
+    if (tid == 0 && rank == 0) rs[(size_t)slot * N + n] = (float)(sr[rows] * inv);
+    if (S > 1) cluster.sync();  // no CTA leaves while its maximum is read
+}
+
+template <class... A>
+static cudaError_t run_refine_residual(const GridView& g, int nact, cudaStream_t s, A... args) {
+    const int S = point_split(nact, g.nsp), npl = (g.nsp + S - 1) / S;
+    const size_t smem = ((size_t)3 * g.n + (size_t)g.nsh * npl + 1) * sizeof(double);
+    return launch_points(k_refine_residual, nact, S, smem, s, g, args..., npl);
 }
 
 // x[pt] += sigma * y[slot]; corr[pt] = ||sigma * y|| / ||x|| of this pass
@@ -1361,6 +1484,8 @@ static GridView view_of(const BteGrid* g) {
     v.cgT = g->d_cgT; v.adv_coef = g->d_adv_coef; v.mass = g->d_mass; v.temp = g->d_temp; v.u = g->d_u; v.p = g->d_p;
     v.Mp = g->d_Mp; v.W = g->d_W; v.invMd = g->d_invMd; v.vD = g->d_vD; v.HL = g->d_HL; v.GL = g->d_GL; v.CA = g->d_CA; v.CB = g->d_CB; v.tri = g->d_tri;
     v.fq0 = g->f_q0; v.fq1 = g->f_q1; v.fcgT = g->f_cgT; v.fmm1 = g->f_mm1; v.fmm2 = g->f_mm2; v.fMr = g->f_Mr;
+    v.tHL = g->t_HL; v.tGL = g->t_GL; v.tq0 = g->t_q0; v.tq1 = g->t_q1; v.tMr = g->t_Mr; v.tcgT = g->t_cgT;
+    v.tadv = g->t_adv; v.tCA = g->t_CA; v.tCB = g->t_CB;
     v.fHL = g->f_HL; v.fGL = g->f_GL; v.fCA = g->f_CA; v.fCB = g->f_CB;
     return v;
 }
@@ -1627,7 +1752,6 @@ struct SolveCtx {
     int P, n, N, ld, ldd, ee;
     long long jstride;
     double beta_scale;
-    size_t res_smem, ref_smem;
     const bte_solve_opts* o;
     int32_t* status;
     int32_t* iters;
@@ -1677,7 +1801,7 @@ static cudaError_t gmres_refine(SolveCtx& c, Lane& L, int nact, bool all) {
         GMCK(pf.run(PF_REFINE, s, 0, 0, 2, [&] {
             // r0 = D b (d = 0): the first preconditioned vector is still zero
             cudaMemsetAsync(w->gm_Z, 0, zb, s);
-            k_refine_residual<<<ng, 256, c.ref_smem, s>>>(c.gv, c.pp, ee, L.act, ng, w->h, w->F, w->aux, w->scal, w->dh,
+            run_refine_residual(c.gv, ng, s, c.pp, ee, L.act, ng, w->h, w->F, w->aux, w->scal, w->dh,
                                                           ldd, c.beta_scale, L.rowscale, nullptr, nullptr, nullptr,
                                                           L.kc, w->gm_list, 0, w->gm_Z, GM_M * N, w->gm_W);
             k_gm_start<<<ng, 256, 0, s>>>(ng, N, w->gm_W, w->gm_V, w->gm_g, w->gm_bn, w->gm_on);
@@ -1690,7 +1814,7 @@ static cudaError_t gmres_refine(SolveCtx& c, Lane& L, int nact, bool all) {
                 k_gm_pre<<<ng, 256, 0, s>>>(ng, N, k, w->gm_V, w->gm_on, w->gm_xf, w->gm_sig);
                 le = bte_lu_solve_t<float>(ng, N, (const float*)L.J, ld, c.jstride, L.piv, w->gm_xf, 0, s, w->gm_list);
                 k_gm_post<<<ng, 256, 0, s>>>(ng, N, k, w->gm_xf, w->gm_sig, w->gm_on, w->gm_Z);
-                k_refine_residual<<<ng, 256, c.ref_smem, s>>>(c.gv, c.pp, ee, L.act, ng, w->h, w->F, w->aux, w->scal,
+                run_refine_residual(c.gv, ng, s, c.pp, ee, L.act, ng, w->h, w->F, w->aux, w->scal,
                                                               w->dh, ldd, c.beta_scale, L.rowscale, nullptr, nullptr,
                                                               nullptr, L.kc, w->gm_list, 1, w->gm_Z + (size_t)k * N,
                                                               GM_M * N, w->gm_W);
@@ -1734,7 +1858,6 @@ static int newton_iteration(SolveCtx& c, Lane& L, int nact, int prec) {
     const int n = c.n, N = c.N, ld = c.ld, ldd = c.ldd, ee = c.ee, P = c.P;
     const long long jstride = c.jstride;
     const double beta_scale = c.beta_scale;
-    const size_t res_smem = c.res_smem, ref_smem = c.ref_smem;
     const bte_solve_opts* o = c.o;
     GridView& gv = c.gv;
     PointParams& pp = c.pp;
@@ -1749,7 +1872,7 @@ static int newton_iteration(SolveCtx& c, Lane& L, int nact, int prec) {
     auto other = [&](auto&& fn) { return pf.run(PF_OTHER, s, 0, 0, 1, fn); };
     // points that switched to the double-double residual: their state's F, aux and merit again
     CKR(pf.run(PF_RESIDUAL, s, 0, 0, 2, [&] {
-        k_residual<<<nact, 256, res_smem, s>>>(gv, pp, ee, L.act, nact, w->h, nullptr, 0, nullptr, w->ddpend, nullptr,
+        run_residual(gv, nact, s, pp, ee, L.act, nact, w->h, nullptr, 0, nullptr, w->ddpend, nullptr,
                                                w->F, w->aux, w->scal, w->r, nullptr, w->ddm);
         k_set_list<<<nblk(nact, 256), 256, 0, s>>>(nact, L.act, w->ddpend, 0);
     }));
@@ -1786,7 +1909,7 @@ static int newton_iteration(SolveCtx& c, Lane& L, int nact, int prec) {
                 double* ccur = (rf & 1) ? w->corr1 : w->corr0;
                 CKR(pf.run(PF_REFINE, s, nact * (res_flops_pt(g, ee) + 2.0 * (double)N * N),
                            nact * (res_bytes_pt(g, true) + 0.5 * N * (N + 1) * wsz), 3, [&] {
-                    k_refine_residual<<<nact, 256, ref_smem, s>>>(gv, pp, ee, L.act, nact, w->h, w->F, w->aux,
+                    run_refine_residual(gv, nact, s, pp, ee, L.act, nact, w->h, w->F, w->aux,
                                                                   w->scal, w->dh, ldd, beta_scale, L.rowscale, xs,
                                                                   L.sigma, w->refdone, L.kc, nullptr, 0, nullptr, 0,
                                                                   nullptr);
@@ -1832,7 +1955,7 @@ static int newton_iteration(SolveCtx& c, Lane& L, int nact, int prec) {
         int nsearch = nact;
         for (int ls = 0; ls < 200; ++ls) {
             CKR(pf.run(PF_RESIDUAL, s, nsearch * res_flops_pt(g, ee), nsearch * res_bytes_pt(g, true), 1, [&] {
-                k_residual<<<nact, 256, res_smem, s>>>(gv, pp, ee, L.act, nact, w->h, w->dh, ldd, w->alpha,
+                run_residual(gv, nact, s, pp, ee, L.act, nact, w->h, w->dh, ldd, w->alpha,
                                                        w->searching, w->ht, w->Ft, w->auxt, w->scalt, w->rt, w->srel,
                                                        w->ddm);
             }));
@@ -1886,18 +2009,14 @@ int bte_solve_impl(BteGrid* g, int P, const double* n0, const double* ne, const 
     c.jstride = (long long)c.N * c.ld;
     // border scale: typical magnitude of the raw collision operator per unit n0
     c.beta_scale = g->q0max / (g->umax > 0 ? g->umax : 1.0);
-    c.res_smem = (size_t)7 * c.n * sizeof(double);
-    c.ref_smem = (size_t)(5 * c.n + 2) * sizeof(double);  // x, r: n + 1 each; h, HL x, GL x: n each
     c.o = o; c.status = status; c.iters = iters; c.s = s;
     const int n = c.n;
-    CKR(bte_raise_smem_limit((const void*)k_residual, c.res_smem));
-    CKR(bte_raise_smem_limit((const void*)k_refine_residual, c.ref_smem));
     Profiler& pf = g_prof;
     Lane L{w->act, w->act2, w->J, w->piv, w->info, w->xs, w->rowscale, w->sigma, w->kc};
     auto other = [&](auto&& fn) { return pf.run(PF_OTHER, s, 0, 0, 1, fn); };
     auto residual_all = [&](int nact) {
         return pf.run(PF_RESIDUAL, s, nact * res_flops_pt(g, c.ee), nact * res_bytes_pt(g, false), 1, [&] {
-            k_residual<<<nact, 256, c.res_smem, s>>>(c.gv, c.pp, c.ee, L.act, nact, w->h, nullptr, 0, nullptr,
+            run_residual(c.gv, nact, s, c.pp, c.ee, L.act, nact, w->h, nullptr, 0, nullptr,
                                                      nullptr, nullptr, w->F, w->aux, w->scal, w->r, nullptr, w->ddm);
         });
     };
@@ -2121,8 +2240,6 @@ static SolveCtx engine_ctx(BteEngine* e, cudaStream_t s) {
     c.ee = g->ee ? 1 : 0;  // per point: the slot's phase
     c.jstride = (long long)c.N * c.ld;
     c.beta_scale = g->q0max / (g->umax > 0 ? g->umax : 1.0);
-    c.res_smem = (size_t)7 * c.n * sizeof(double);
-    c.ref_smem = (size_t)(5 * c.n + 2) * sizeof(double);  // x, r: n + 1 each; h, HL x, GL x: n each
     c.o = &e->opts; c.status = e->status; c.iters = e->iters; c.s = s;
     return c;
 }
@@ -2163,8 +2280,6 @@ int bte_engine_create_impl(BteGrid* g, int cap, int fcap, const bte_solve_opts* 
     e->free_slots.resize(cap);
     for (int i = 0; i < cap; ++i) e->free_slots[i] = cap - 1 - i;  // pop_back hands out 0, 1, 2, ...
     SolveCtx c = engine_ctx(e, 0);
-    if (bte_raise_smem_limit((const void*)k_residual, c.res_smem) != cudaSuccess) { engine_free(e); delete e; return BTE_ERR_CUDA; }
-    if (bte_raise_smem_limit((const void*)k_refine_residual, c.ref_smem) != cudaSuccess) { engine_free(e); delete e; return BTE_ERR_CUDA; }
     const size_t rm_smem = (size_t)2 * n * sizeof(double);
     if (bte_raise_smem_limit((const void*)k_ref_merit, rm_smem) != cudaSuccess) { engine_free(e); delete e; return BTE_ERR_CUDA; }
     *out = e;
@@ -2192,7 +2307,7 @@ static int engine_start_phase(BteEngine* e, SolveCtx& c, const int* list, int m,
     const int n = g->n;
     Profiler& pf = g_prof;
     CKR(pf.run(PF_RESIDUAL, s, m * res_flops_pt(g, c.ee), m * res_bytes_pt(g, false), 1, [&] {
-        k_residual<<<m, 256, c.res_smem, s>>>(c.gv, c.pp, c.ee, list, m, w->h, nullptr, 0, nullptr, nullptr, nullptr,
+        run_residual(c.gv, m, s, c.pp, c.ee, list, m, w->h, nullptr, 0, nullptr, nullptr, nullptr,
                                               w->F, w->aux, w->scal, w->r, nullptr, nullptr);
     }));
     CKR(pf.run(PF_OTHER, s, 0, 0, 4, [&] {
@@ -2250,7 +2365,7 @@ int bte_engine_step_impl(BteEngine* e, int* n_done, int32_t* done_out, cudaStrea
         }));
         CKR(pf.run(PF_RESIDUAL, s, k * res_flops_pt(g, c.ee), k * res_bytes_pt(g, false), 1, [&] {
             k_set_list<<<nblk(k, 256), 256, 0, s>>>(k, e->l_in, w->ddm, 0);
-            k_residual<<<k, 256, c.res_smem, s>>>(c.gv, c.pp, c.ee, e->l_in, k, w->h, nullptr, 0, nullptr, nullptr,
+            run_residual(c.gv, k, s, c.pp, c.ee, e->l_in, k, w->h, nullptr, 0, nullptr, nullptr,
                                                   nullptr, w->F, w->aux, w->scal, w->r, nullptr, nullptr);
         }));
         CKR(cudaMemcpyAsync(e->f64.act + e->nf64, e->l_in, k * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
@@ -2460,9 +2575,7 @@ int bte_transient_impl(BteGrid* g, int P, const double* n0, const double* ne, co
     c.ee = (o->ee && g->ee) ? 1 : 0;
     c.jstride = (long long)N * c.ld;
     c.beta_scale = g->q0max / (g->umax > 0 ? g->umax : 1.0);
-    c.res_smem = (size_t)7 * n * sizeof(double);
     c.o = &so; c.status = status; c.iters = iters; c.s = s;
-    CKR(bte_raise_smem_limit((const void*)k_residual, c.res_smem));
     const size_t rm_smem = (size_t)2 * n * sizeof(double);
     CKR(bte_raise_smem_limit((const void*)k_ref_merit, rm_smem));
     Profiler& pf = g_prof;
@@ -2500,7 +2613,7 @@ int bte_transient_impl(BteGrid* g, int P, const double* n0, const double* ne, co
         CKR(other([&] { k_set_efield<<<nblk(P, 256), 256, 0, s>>>(P, eRe, eIm, t + o->dt, E, harmonic, Et); }));
         // the step's Jacobian at the current state, factored once
         CKR(pf.run(PF_RESIDUAL, s, 0, 0, 1, [&] {
-            k_residual<<<P, 256, c.res_smem, s>>>(c.gv, c.pp, c.ee, all, P, w->h, nullptr, 0, nullptr, nullptr, nullptr,
+            run_residual(c.gv, P, s, c.pp, c.ee, all, P, w->h, nullptr, 0, nullptr, nullptr, nullptr,
                                                   w->F, w->aux, w->scal, w->r, nullptr, nullptr);
         }));
         dim3 gj(nblk(N, JAC_WARPS), P);
@@ -2533,7 +2646,7 @@ int bte_transient_impl(BteGrid* g, int P, const double* n0, const double* ne, co
         int nact = P;
         for (int it = 0;; ++it) {
             CKR(pf.run(PF_RESIDUAL, s, 0, 0, 1, [&] {
-                k_residual<<<nact, 256, c.res_smem, s>>>(c.gv, c.pp, c.ee, w->act, nact, w->h, w->dh, ldd, w->alpha,
+                run_residual(c.gv, nact, s, c.pp, c.ee, w->act, nact, w->h, w->dh, ldd, w->alpha,
                                                          nullptr, w->ht, w->Ft, w->auxt, w->scalt, w->rt, nullptr,
                                                          nullptr);
             }));
