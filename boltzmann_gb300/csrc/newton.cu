@@ -585,17 +585,17 @@ k_refine_residual(GridView g, PointParams pp, int ee, const int* __restrict__ ac
         if (ee && kc) {
             // C(x; HL h, GL h) + C(h; HL x, GL x) through the row's coefficients, which the
             // Jacobian of this Newton step wrote: K1 . x over the band, K2a . (HL x) + K2b . (GL x)
-            const double* kr = kc + ((size_t)slot * n + r) * kcn;
+            const double* kr = kc + (size_t)(slot * nsh + q) * kcn * nsp + p;
             double c1 = 0.0;
             for (int w = 0; w < BTE_NB * nsh; ++w) {
                 const int k = p + w / nsh - BTE_BAND;
-                if (k >= 0 && k < nsp) c1 += kr[w] * sx[(w % nsh) * nsp + k];
+                if (k >= 0 && k < nsp) c1 += kr[(size_t)w * nsp] * sx[(w % nsh) * nsp + k];
             }
             for (int w = 0; w < BTE_NB * nsh; ++w) {
                 const int rr = p + w % BTE_NB - BTE_BAND;
                 if (rr < 0 || rr >= nsp) continue;
                 const int o = (w / BTE_NB) * nsp + rr;
-                c1 += kr[BTE_NB * nsh + w] * sxh[o] + kr[2 * BTE_NB * nsh + w] * sxg[o];
+                c1 += kr[(size_t)(BTE_NB * nsh + w) * nsp] * sxh[o] + kr[(size_t)(2 * BTE_NB * nsh + w) * nsp] * sxg[o];
             }
             y += ne * gam * c1 + ne * ax[2 * n + r] * dgx;
         }
@@ -939,283 +939,442 @@ struct OpsT<float> {
 constexpr int JAC_WARPS = 8;
 constexpr int MIXED_HANDOVER_ITER = 30;  // mixed-form iterations before a running point moves to FP64
 
-// Row equilibration of one bordered row (matrix part [0, N) and the RHS column N): the
-// row is divided by its largest |entry| so that the factorization sees rows of unit
-// size (the l = 0 energy-exchange rows are ~m/M smaller than the l >= 1 rows). The
-// applied factor is returned for the FP64 refinement.
+constexpr int JAC_TRI_MAX = 48;  // e-e triples of one mode (42 in all at l_max = 4)
+
+// Row equilibration: each row of the bordered matrix (matrix part [0, N) and the RHS column N)
+// is divided by its largest |entry| so that the factorization sees rows of unit size (the l = 0
+// energy-exchange rows are ~m/M smaller than the l >= 1 rows). The factor is returned for the
+// FP64 refinement.
 template <typename T>
-__device__ inline void equilibrate_row(T* Jr, int N, int lane, double* scale_out) {
+__device__ inline void put_row(const T* row, T* Jr, int N, int lane, double* scale_out) {
     T m = T(0);
-    for (int j = lane; j < N; j += 32) m = fmax(m, fabs(Jr[j]));
+    for (int j = lane; j < N; j += 32) m = fmax(m, fabs(row[j]));
     for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
     const T sc = (m > T(0)) ? T(1) / m : T(1);
-    for (int j = lane; j < N + 1; j += 32) Jr[j] *= sc;
+    for (int j = lane; j < N + 1; j += 32) Jr[j] = row[j] * sc;
     if (lane == 0 && scale_out) *scale_out = (double)sc;
 }
 
-// Byte offset of the staged HL / GL rows in k_jacobian's dynamic shared memory: before them
-// sit the per-point column vectors of the l = 0 columns (FP64 W sums, their T copy, T copies
-// of the temperature and mass rows) and the per-species scalars n0 * ns.
-template <typename T>
-__host__ __device__ inline size_t jac_col_bytes(int nsp, int nspecies) {
-    return (((size_t)nsp + nspecies) * sizeof(double) + (size_t)3 * nsp * sizeof(T) + 15) & ~(size_t)15;
-}
-// then the per-warp partial sums of the e-e coefficients: tqmax triples x 7 offsets x
-// (K2a, K2b, K1) in FP64
-constexpr int JAC_TRI_MAX = 48;  // e-e triples of one mode (42 in all at l_max = 4)
-__host__ __device__ inline size_t jac_part_bytes(int tqmax) {
-    return (size_t)JAC_WARPS * tqmax * BTE_NB * 3 * sizeof(double);
+// ---------------------------------------------------------------------------------
+// e-e coefficients of the rows, in FP64 (the linearization of C(h; HL h, GL h)):
+//   K2a[s][dr] = sum_{t = (q, l, s)} sum_dk CA[t][p][dk][dr] h[(p + dk, l)]   (K2b: CB)
+//   K1[dk][s]  = sum_{t = (q, s, s')} sum_dr (CA[t][p][dk][dr] HLh[(p + dr, s')] + CB .. GLh)
+// kc[((slot nsh + q) kc_row + e) nsp + p]: K1 at e = dk nsh + s, then K2a, K2b at s 7 + dr.
+// Read by the FP32 Jacobian and by the refinement.
+//
+// The FP64 pipe bounds it: 148 multiply-adds per triple and spline, each warp with 32 splines of
+// one mode and one s (K1: one l), of G points together where a point's splines do not fill a
+// warp. One warp per row of the Jacobian with a lane per (triple, offset) spent three times
+// these instructions, half of them on idle lanes and on summing the lanes' parts.
+// ---------------------------------------------------------------------------------
+constexpr int EEC_T = 256;
+__global__ void __launch_bounds__(EEC_T, 2)
+k_ee_coef(GridView g, PointParams pp, int ee, const int* __restrict__ act, int nact, int G, const double* __restrict__ h,
+          const double* __restrict__ aux, double* __restrict__ kc) {
+    extern __shared__ double sm[];  // per point: h, HL h, GL h, mode-major
+    const int n = g.n, nsh = g.nsh, nsp = g.nsp;
+    const int slot0 = blockIdx.x * G, m = min(G, nact - slot0);
+    for (int i = threadIdx.x; i < m * n; i += EEC_T) {
+        const int k = i / n, r = i % n, pt = act[slot0 + k];
+        double* d = sm + (size_t)k * 3 * n + (r % nsh) * nsp + r / nsh;
+        d[0] = h[(size_t)pt * n + r];
+        d[n] = aux[(size_t)pt * 4 * n + r];
+        d[2 * n] = aux[(size_t)pt * 4 * n + n + r];
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, nw = EEC_T / 32 * gridDim.y;
+    const int blocks = (m * nsp + 31) / 32, kcn = kc_row(nsh);
+    for (int task = (int)(threadIdx.x >> 5) * gridDim.y + blockIdx.y; task < 2 * nsh * nsh * blocks; task += nw) {
+        const int i = task % blocks * 32 + lane, u = task / blocks % (2 * nsh), q = task / blocks / (2 * nsh);
+        if (i >= m * nsp) continue;
+        const int k = i / nsp, p = i % nsp;
+        if (pp.eept ? !pp.eept[act[slot0 + k]] : !ee) continue;
+        const double* hk = sm + (size_t)k * 3 * n;
+        double* out = kc + (size_t)((slot0 + k) * nsh + q) * kcn * nsp + p;
+        if (u < nsh) {  // K2 of s = u
+            double xa[BTE_NB] = {}, xb[BTE_NB] = {};
+            for (int t = 0; t < g.ntri; ++t) {
+                if (g.tri[3 * t] != q || g.tri[3 * t + 2] != u) continue;
+                const double* ca = g.tCA + (size_t)t * BTE_PAIRS * nsp + p;
+                const double* cb = g.tCB + (size_t)t * BTE_PAIRS * nsp + p;
+                const double* hl = hk + g.tri[3 * t + 1] * nsp;
+                int e = 0;
+#pragma unroll
+                for (int dk = 0; dk < BTE_NB; ++dk) {
+                    const double hv = hl[min(max(p + dk - BTE_BAND, 0), nsp - 1)];
+#pragma unroll
+                    for (int dr = (dk > BTE_BAND ? dk - BTE_BAND : 0);
+                         dr <= (dk < BTE_BAND ? dk + BTE_BAND : BTE_NB - 1); ++dr, ++e) {
+                        xa[dr] += ca[(size_t)e * nsp] * hv;
+                        xb[dr] += cb[(size_t)e * nsp] * hv;
+                    }
+                }
+            }
+#pragma unroll
+            for (int dr = 0; dr < BTE_NB; ++dr) {
+                out[(size_t)(BTE_NB * (nsh + u) + dr) * nsp] = xa[dr];
+                out[(size_t)(BTE_NB * (2 * nsh + u) + dr) * nsp] = xb[dr];
+            }
+        } else {  // K1 of l = u - nsh
+            double x[BTE_NB] = {};
+            for (int t = 0; t < g.ntri; ++t) {
+                if (g.tri[3 * t] != q || g.tri[3 * t + 1] != u - nsh) continue;
+                const double* ca = g.tCA + (size_t)t * BTE_PAIRS * nsp + p;
+                const double* cb = g.tCB + (size_t)t * BTE_PAIRS * nsp + p;
+                const double* hh = hk + n + g.tri[3 * t + 2] * nsp;
+                double vh[BTE_NB], vg[BTE_NB];
+#pragma unroll
+                for (int d = 0; d < BTE_NB; ++d) {
+                    const int r = min(max(p + d - BTE_BAND, 0), nsp - 1);
+                    vh[d] = hh[r];
+                    vg[d] = hh[n + r];
+                }
+                int e = 0;
+#pragma unroll
+                for (int dk = 0; dk < BTE_NB; ++dk)
+#pragma unroll
+                    for (int dr = (dk > BTE_BAND ? dk - BTE_BAND : 0);
+                         dr <= (dk < BTE_BAND ? dk + BTE_BAND : BTE_NB - 1); ++dr, ++e)
+                        x[dk] += ca[(size_t)e * nsp] * vh[dr] + cb[(size_t)e * nsp] * vg[dr];
+            }
+#pragma unroll
+            for (int dk = 0; dk < BTE_NB; ++dk) out[(size_t)(dk * nsh + u - nsh) * nsp] = x[dk];
+        }
+    }
 }
 
-// One bordered Jacobian row per warp. The row's entries fall in three groups, each
-// handled by its own pass so that the lanes of a warp do the same work (an FP64
-// instruction costs a full FP64-pipe slot however few lanes are active):
-//   (1) l > 0 columns off the band: the dense Coulomb product only, T arithmetic;
-//   (2) l = 0 columns off the band: rank-1 terms, plus the inelastic l = 0 block on
-//       l = 0 rows, summed in FP64 there (they cancel nearly equal terms at low E/N);
-//   (3) the band (p - 3 .. p + 3 splines x all modes): every term summed in FP64.
+// Points per CTA (while a point's splines leave lanes idle and there are points enough to fill
+// the chip), and CTAs per group of points (for few points). A coefficient depends on neither.
+static cudaError_t run_ee_coef(const GridView& g, int nact, cudaStream_t s, const PointParams& pp, int ee, const int* act,
+                               const double* h, const double* aux, double* kc) {
+    int G = 1;
+    while (G < 4 && nact >= 608 * G && (g.nsp * G) % 32 != 0 && (size_t)6 * G * g.n * 8 <= 48 * 1024) G *= 2;
+    const int groups = (nact + G - 1) / G, tasks = 2 * g.nsh * g.nsh * ((g.nsp * G + 31) / 32);
+    const int split = std::max(1, std::min((tasks + 7) / 8, 304 / groups));
+    const size_t smem = (size_t)3 * G * g.n * sizeof(double);
+    cudaError_t e = bte_raise_smem_limit((const void*)k_ee_coef, smem);
+    if (e != cudaSuccess) return e;
+    k_ee_coef<<<dim3(groups, split), EEC_T, smem, s>>>(g, pp, ee, act, nact, G, h, aux, kc);
+    return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------------
+// Jacobian rows, one warp per spline p (its nsh rows), a CTA's warps on consecutive splines.
+// It is bound by the FP64 pipe (64 cycles per warp instruction and sub-partition, conversions
+// included) and by shared memory and L1 bandwidth, so
+//  - the rows of one spline share the HL / GL values of the Coulomb product (they differ in the
+//    seven K2 coefficients only), read straight from L1 by lanes of consecutive columns, and
+//    the product of an entry in the band is taken there too;
+//  - the FP64 terms are few: the per-point column vectors come summed (growth, and the Coulomb
+//    logarithm's derivative), the e-e coefficients from k_ee_coef (KC), the divisions are taken
+//    once per CTA, the band's nsh x 7 nsh entries fill the lanes over all rows;
+//  - a row is put together in shared memory, equilibrated there and written once, coalesced.
+// A warp per row with its own coefficients, partial sums and divisions, equilibrating in global
+// memory, took 6.75 ms per Newton iteration of a solve of 4096 points of 384 unknowns; now 3.1 ms
+// with k_ee_coef (0.8 ms where e-e is on).
+// Without KC (the FP64 and transient forms keep no coefficient buffer, which would cost a third
+// of their matrices' memory) a warp forms its rows' coefficients from the triples.
+// ---------------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(JAC_WARPS * 32)
+struct JacShape {
+    // offsets in bytes: the CTA's W (FP64, T), D (FP64, T), species; then per warp
+    __host__ __device__ static size_t up(size_t x) { return (x + 15) & ~(size_t)15; }
+    __host__ __device__ static size_t cols(int nsp, int nspecies) {
+        return up(((size_t)2 * nsp + nspecies) * sizeof(double) + (size_t)2 * nsp * sizeof(T));
+    }
+    // M h and U of the rows and their T copies, K1, K2 (a and b of a (q, s) at 0..6 and 8..14 of 16), partial sums, rows
+    __host__ __device__ static size_t k1(int nsh) { return up((size_t)2 * nsh * (sizeof(double) + sizeof(T))); }
+    __host__ __device__ static size_t k2(int nsh, int ee) { return k1(nsh) + (ee ? up((size_t)nsh * nsh * BTE_NB * sizeof(double)) : 0); }
+    __host__ __device__ static size_t part(int nsh, int ee) { return k2(nsh, ee) + (ee ? (size_t)nsh * nsh * 16 * sizeof(T) : 0); }
+    __host__ __device__ static size_t rows(int nsh, int ee, int tqmax) {
+        return part(nsh, ee) + up((size_t)tqmax * BTE_NB * 3 * sizeof(double));
+    }
+    __host__ __device__ static size_t warp(int nsh, int ee, int tqmax, int N) {
+        return rows(nsh, ee, tqmax) + up((size_t)nsh * (N + 1) * sizeof(T));
+    }
+};
+
+template <typename T, bool KC>
+__global__ void __launch_bounds__(JAC_WARPS * 32, sizeof(T) == 4 ? 3 : 2)
 k_jacobian(GridView g, PointParams pp, int ee, const int* __restrict__ act, int nact, const double* __restrict__ h,
            const double* __restrict__ F, const double* __restrict__ aux, const double* __restrict__ scal,
            T* __restrict__ J, int ld, long long stride, double beta_scale, double* __restrict__ rowscale,
-           int stage_hl, double jscale, double jshift, double* __restrict__ kc) {
+           double jscale, double jshift, const double* __restrict__ kc, int sized_ee) {
+    // sized_ee: the shared memory holds the e-e parts (ee of the launch; a point may have it off)
+    using L = JacShape<T>;
     extern __shared__ __align__(16) unsigned char jsm[];
+    __shared__ double sdg[2];
     const int slot = blockIdx.y;
     if (slot >= nact) return;
     const int pt = act[slot];
     if (pp.eept) ee = pp.eept[pt];
     const int n = g.n, nsh = g.nsh, nsp = g.nsp, N = n + 1, nspc = g.nspecies;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int a = blockIdx.x * JAC_WARPS + wid;  // row
-    const double n0 = pp.n0[pt], Tg = pp.Tg[pt], E = pp.E[pt];
-    // per-point column vectors of the l = 0 columns and the species scalars
-    double* sWd = reinterpret_cast<double*>(jsm);
-    double* sNs = sWd + nsp;
-    T* sWt = reinterpret_cast<T*>(sNs + nspc);
-    T* sTt = sWt + nsp;
-    T* sMt = sTt + nsp;
-    for (int sp = threadIdx.x; sp < nspc; sp += blockDim.x) sNs[sp] = n0 * pp.ns[(size_t)sp * pp.P + pt];
-    for (int c = threadIdx.x; c < nsp; c += blockDim.x) {
-        double w = 0.0;
-        for (int sp = 0; sp < nspc; ++sp) w += n0 * pp.ns[(size_t)sp * pp.P + pt] * g.W[(size_t)sp * n + c * nsh];
-        sWd[c] = w;
-        sWt[c] = (T)w;
-        sTt[c] = (T)g.temp[c * nsh];
-        sMt[c] = (T)g.mass[c * nsh];
-    }
-    // rows of HL / GL this CTA's rows touch (p - 3 .. p + 3), staged in shared memory
-    const int a0 = blockIdx.x * JAC_WARPS;
-    const int prow0 = max(0, min(a0, n - 1) / nsh - BTE_BAND);
-    const int prow1 = min(nsp - 1, min(a0 + JAC_WARPS - 1, n - 1) / nsh + BTE_BAND);
-    const int nr = prow1 - prow0 + 1;
-    double* part = reinterpret_cast<double*>(jsm + jac_col_bytes<T>(nsp, nspc)) + (size_t)wid * g.tqmax * BTE_NB * 3;
-    T* sHL = reinterpret_cast<T*>(jsm + jac_col_bytes<T>(nsp, nspc) + jac_part_bytes(g.tqmax));
-    T* sGL = sHL + (size_t)nr * nsh * nsp;
-    if (stage_hl && ee) {
-        const T* HLg = OpsT<T>::HL(g);
-        const T* GLg = OpsT<T>::GL(g);
-        for (int e = threadIdx.x; e < nr * nsh * nsp; e += blockDim.x) {
-            const int sidx = e / (nr * nsp), rem = e % (nr * nsp);
-            const size_t src = ((size_t)sidx * nsp + prow0 + rem / nsp) * nsp + rem % nsp;
-            sHL[e] = HLg[src];
-            sGL[e] = GLg[src];
-        }
-    }
-    __syncthreads();
-    if (a > n) return;
-    T* Jr = J + (size_t)slot * stride + (size_t)a * ld;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int tqmax = KC ? 0 : (sized_ee ? g.tqmax : 0);
     const double* hp = h + (size_t)pt * n;
     const double* ax = aux + (size_t)pt * 4 * n;
     const double* sc = scal + (size_t)pt * SC_COUNT;
+    const double n0 = pp.n0[pt], Tg = pp.Tg[pt], E = pp.E[pt];
+    const double ne = sc[SC_NE], gam = sc[SC_GAMMA], mu = sc[SC_MU];
+    double* sWd = reinterpret_cast<double*>(jsm);
+    double* sDd = sWd + nsp;
+    double* sNs = sDd + nsp;
+    T* sWt = reinterpret_cast<T*>(sNs + nspc);
+    T* sDt = sWt + nsp;
+    for (int sp = threadIdx.x; sp < nspc; sp += blockDim.x) sNs[sp] = n0 * pp.ns[(size_t)sp * pp.P + pt];
+    // dgamma/dh = gam_c * 1.5 * (Top / (Top.h) - Mop / (Mop.h)), Top = temp * K_1eV
+    if (ee && wid == nw - 1) {
+        const double d = ne * g.gam_c * 1.5 / (lane & 1 ? sc[SC_M0] : sc[SC_T0]);
+        if (lane < 2) sdg[lane] = d;
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < nsp; c += blockDim.x) {
+        double w = 0.0;
+        for (int sp = 0; sp < nspc; ++sp) w += sNs[sp] * g.W[(size_t)sp * n + c * nsh];
+        const double d = ee ? sdg[0] * g.temp[c * nsh] - sdg[1] * g.mass[c * nsh] : 0.0;
+        sWd[c] = w;
+        sWt[c] = (T)w;
+        sDd[c] = d;
+        sDt[c] = (T)d;
+    }
+    __syncthreads();
+    const int p = blockIdx.x * nw + wid;
+    if (p > nsp) return;
+    unsigned char* wsm = jsm + L::cols(nsp, nspc) + wid * L::warp(nsh, sized_ee, tqmax, N);
+    double* smh = reinterpret_cast<double*>(wsm);
+    double* sU = smh + nsh;
+    T* smt = reinterpret_cast<T*>(sU + nsh);
+    T* sUt = smt + nsh;
+    double* k1 = reinterpret_cast<double*>(wsm + L::k1(nsh));
+    T* k2 = reinterpret_cast<T*>(wsm + L::k2(nsh, sized_ee));
+    double* part = reinterpret_cast<double*>(wsm + L::part(nsh, sized_ee));
+    T* row = reinterpret_cast<T*>(wsm + L::rows(nsh, sized_ee, tqmax));
+    const int ldr = N + 1;
     const bool be = (jshift != 0.0);
     // border scale: per unit n0 for the steady Jacobian (it matches the collision operator);
     // absolute for the backward-Euler matrix (it matches the mass matrix)
     const double beta = be ? beta_scale : beta_scale * n0;
-    if (a == n) {  // constraint row
+    if (p == nsp) {  // constraint row
         double uh = 0.0;
         for (int j = lane; j < n; j += 32) {
-            Jr[j] = (T)(beta * g.u[j]);
+            row[j] = (T)(beta * g.u[j]);
             uh += g.u[j] * hp[j];
         }
         uh = warp_sum(uh);
         if (lane == 0) {
-            Jr[n] = T(0);
-            Jr[n + 1] = (T)(beta * (1.0 - uh));
+            row[n] = T(0);
+            row[n + 1] = (T)(beta * (1.0 - uh));
         }
         __syncwarp();
-        equilibrate_row(Jr, N, lane, rowscale ? rowscale + (size_t)slot * N + a : nullptr);
+        put_row(row, J + (size_t)slot * stride + (size_t)n * ld, N, lane, rowscale ? rowscale + (size_t)slot * N + n : nullptr);
         return;
     }
-    const int p = a / nsh, q = a % nsh;
-    const double ne = sc[SC_NE], gam = sc[SC_GAMMA], mu = sc[SC_MU], t0 = sc[SC_T0], m0 = sc[SC_M0];
-    const double mh = ax[3 * n + a];
-    const double Ua = ax[2 * n + a];
-    const double negam = ee ? ne * gam : 0.0;
-    // dgamma/dh = gam_c * 1.5 * (Top / (Top.h) - Mop / (Mop.h)), Top = temp * K_1eV
-    const double dg_t = ee ? ne * Ua * g.gam_c * 1.5 / t0 : 0.0;
-    const double dg_m = ee ? ne * Ua * g.gam_c * 1.5 / m0 : 0.0;
-    // e-e coefficients of this row, in FP64 (the linearization of C(h; HL h, GL h)):
-    //   K2a[s][dr] = sum_{t = (q, l, s)} sum_dk CA[t][p][dk][dr] h[(p + dk, l)]   (K2b: CB)
-    //   K1[dk][s]  = sum_{t = (q, s, s')} sum_dr (CA[t][p][dk][dr] HLh[(p + dr, s')] + CB .. GLh)
-    // One lane per (triple of mode q, offset) computes both partial sums, so that every lane
-    // is busy; the partials are then summed over the triples in triple order. K2 is kept in
-    // shared memory as T for the dense Coulomb product, K1 in FP64 for the band.
-    __shared__ T k2s[JAC_WARPS][2][BTE_NB * 5];
-    __shared__ double k1s[JAC_WARPS][BTE_NB * 5];
-    __shared__ int tqs[JAC_WARPS][JAC_TRI_MAX];
-    T* k2a = k2s[wid][0];
-    T* k2b = k2s[wid][1];
-    double* k1r = k1s[wid];
-    int* tq = tqs[wid];
-    double* kcr = (ee && kc) ? kc + ((size_t)slot * n + a) * kc_row(nsh) : nullptr;
-    if (ee) {
-        int ntq = 0;
-        for (int t0 = 0; t0 < g.ntri; t0 += 32) {
-            const int t = t0 + lane;
-            const bool m = t < g.ntri && g.tri[3 * t] == q;
-            const unsigned bal = __ballot_sync(0xffffffffu, m);
-            const int at = ntq + __popc(bal & ((1u << lane) - 1u));
-            if (m && at < JAC_TRI_MAX) tq[at] = t;
-            ntq += __popc(bal);
+    for (int q = lane; q < nsh; q += 32) {
+        const int a = p * nsh + q;
+        smh[q] = ax[3 * n + a];
+        sU[q] = ax[2 * n + a];
+        smt[q] = (T)smh[q];
+        sUt[q] = (T)sU[q];
+        row[q * ldr + n] = (T)(-beta * g.Mp[a]);
+        row[q * ldr + n + 1] = (T)(-F[(size_t)pt * n + a]);
+    }
+    const int nk = nsh * BTE_NB;  // K1, K2a and K2b entries of one row
+    if (ee && KC) {
+        const double* src = kc + (size_t)slot * nsh * 3 * nk * nsp + p;
+        for (int e = lane; e < nsh * nk; e += 32) {
+            const int q = e / nk, w = e % nk;
+            const double* s3 = src + (size_t)(q * 3 * nk + w) * nsp;
+            k1[e] = s3[0];
+            T* kk = k2 + (q * nsh + w / BTE_NB) * 16 + w % BTE_NB;
+            kk[0] = (T)s3[(size_t)nk * nsp];
+            kk[8] = (T)s3[(size_t)2 * nk * nsp];
         }
-        ntq = min(ntq, g.tqmax);
-        __syncwarp();
-        for (int e = lane; e < ntq * BTE_NB; e += 32) {
-            const int t = tq[e / BTE_NB], o = e % BTE_NB;
-            const int l = g.tri[3 * t + 1], s2 = g.tri[3 * t + 2];
-            const double* ca = g.CA + ((size_t)t * nsp + p) * BTE_NB * BTE_NB;
-            const double* cb = g.CB + ((size_t)t * nsp + p) * BTE_NB * BTE_NB;
-            double pa = 0.0, pb = 0.0, p1 = 0.0;
-            for (int dk = -BTE_BAND; dk <= BTE_BAND; ++dk) {  // K2 partial, o = dr
-                const int k = p + dk;
-                if (k < 0 || k >= nsp) continue;
-                const double hv = hp[k * nsh + l];
-                pa += ca[(dk + BTE_BAND) * BTE_NB + o] * hv;
-                pb += cb[(dk + BTE_BAND) * BTE_NB + o] * hv;
+    }
+    if (ee && !KC) {
+        // one lane per (triple of mode q, offset) computes its partial sums; the partials are
+        // then summed over the triples in triple order
+        __shared__ int tqs[JAC_WARPS][JAC_TRI_MAX];
+        int* tq = tqs[wid];
+        for (int q = 0; q < nsh; ++q) {
+            int ntq = 0;
+            for (int t0 = 0; t0 < g.ntri; t0 += 32) {
+                const int t = t0 + lane;
+                const bool m = t < g.ntri && g.tri[3 * t] == q;
+                const unsigned bal = __ballot_sync(0xffffffffu, m);
+                const int at = ntq + __popc(bal & ((1u << lane) - 1u));
+                if (m && at < JAC_TRI_MAX) tq[at] = t;
+                ntq += __popc(bal);
             }
-            const int c = p + o - BTE_BAND;  // K1 partial, o = dk + 3
-            if (c >= 0 && c < nsp) {
-                for (int dr = -BTE_BAND; dr <= BTE_BAND; ++dr) {
-                    const int rr = p + dr;
-                    if (rr < 0 || rr >= nsp) continue;
-                    p1 += ca[o * BTE_NB + dr + BTE_BAND] * ax[rr * nsh + s2] +
-                          cb[o * BTE_NB + dr + BTE_BAND] * ax[n + rr * nsh + s2];
+            ntq = min(ntq, g.tqmax);
+            __syncwarp();
+            for (int e = lane; e < ntq * BTE_NB; e += 32) {
+                const int t = tq[e / BTE_NB], o = e % BTE_NB;
+                const int l = g.tri[3 * t + 1], s2 = g.tri[3 * t + 2];
+                const double* ca = g.CA + ((size_t)t * nsp + p) * BTE_NB * BTE_NB;
+                const double* cb = g.CB + ((size_t)t * nsp + p) * BTE_NB * BTE_NB;
+                double pa = 0.0, pb = 0.0, p1 = 0.0;
+                for (int dk = -BTE_BAND; dk <= BTE_BAND; ++dk) {  // K2 partial, o = dr
+                    const int k = p + dk;
+                    if (k < 0 || k >= nsp) continue;
+                    const double hv = hp[k * nsh + l];
+                    pa += ca[(dk + BTE_BAND) * BTE_NB + o] * hv;
+                    pb += cb[(dk + BTE_BAND) * BTE_NB + o] * hv;
                 }
-            }
-            part[3 * e + 0] = pa;
-            part[3 * e + 1] = pb;
-            part[3 * e + 2] = p1;
-        }
-        __syncwarp();
-        for (int e = lane; e < nsh * BTE_NB; e += 32) {
-            const int s = e / BTE_NB, dr = e % BTE_NB;     // K2[s][dr]
-            const int dk3 = e / nsh, s1 = e % nsh;          // K1 at e = (dk + 3) nsh + s1
-            double acc_a = 0.0, acc_b = 0.0, k1 = 0.0;
-            for (int i = 0; i < ntq; ++i) {
-                const int t = tq[i];
-                if (g.tri[3 * t + 2] == s) {
-                    acc_a += part[3 * (i * BTE_NB + dr) + 0];
-                    acc_b += part[3 * (i * BTE_NB + dr) + 1];
+                const int c = p + o - BTE_BAND;  // K1 partial, o = dk + 3
+                if (c >= 0 && c < nsp) {
+                    for (int dr = -BTE_BAND; dr <= BTE_BAND; ++dr) {
+                        const int rr = p + dr;
+                        if (rr < 0 || rr >= nsp) continue;
+                        p1 += ca[o * BTE_NB + dr + BTE_BAND] * ax[rr * nsh + s2] +
+                              cb[o * BTE_NB + dr + BTE_BAND] * ax[n + rr * nsh + s2];
+                    }
                 }
-                if (g.tri[3 * t + 1] == s1) k1 += part[3 * (i * BTE_NB + dk3) + 2];
+                part[3 * e + 0] = pa;
+                part[3 * e + 1] = pb;
+                part[3 * e + 2] = p1;
             }
-            k2a[e] = (T)acc_a;
-            k2b[e] = (T)acc_b;
-            k1r[e] = k1;
-            if (kcr) {
-                kcr[e] = k1;
-                kcr[BTE_NB * nsh + e] = acc_a;
-                kcr[2 * BTE_NB * nsh + e] = acc_b;
+            __syncwarp();
+            for (int e = lane; e < nk; e += 32) {
+                const int s = e / BTE_NB, dr = e % BTE_NB;  // K2[s][dr]
+                const int dk = e / nsh, s1 = e % nsh;       // K1 at e = dk nsh + s1
+                double acc_a = 0.0, acc_b = 0.0, a1 = 0.0;
+                for (int i = 0; i < ntq; ++i) {
+                    const int t = tq[i];
+                    if (g.tri[3 * t + 2] == s) {
+                        acc_a += part[3 * (i * BTE_NB + dr) + 0];
+                        acc_b += part[3 * (i * BTE_NB + dr) + 1];
+                    }
+                    if (g.tri[3 * t + 1] == s1) a1 += part[3 * (i * BTE_NB + dk) + 2];
+                }
+                k1[q * nk + e] = a1;
+                k2[(q * nsh + s) * 16 + dr] = (T)acc_a;
+                k2[(q * nsh + s) * 16 + 8 + dr] = (T)acc_b;
             }
+            __syncwarp();
         }
-        __syncwarp();
-    }
-    const T* HL = OpsT<T>::HL(g);
-    const T* GL = OpsT<T>::GL(g);
-    // dense Coulomb product of column (c, s) in T: sum_dr K2[s][dr] HL/GL[s][p + dr - 3][c]
-    auto coulomb = [&](int c, int s) -> T {
-        const T* hl = stage_hl ? sHL + ((ptrdiff_t)s * nr - prow0) * nsp + c : HL + (size_t)s * nsp * nsp + c;
-        const T* gl = stage_hl ? sGL + ((ptrdiff_t)s * nr - prow0) * nsp + c : GL + (size_t)s * nsp * nsp + c;
-        T acc = T(0);
-#pragma unroll
-        for (int dr = 0; dr < BTE_NB; ++dr) {
-            int r = p + dr - BTE_BAND;
-            if (r < 0 || r >= nsp) continue;
-            acc += k2a[s * BTE_NB + dr] * hl[(size_t)r * nsp] + k2b[s * BTE_NB + dr] * gl[(size_t)r * nsp];
-        }
-        return acc;
-    };
-    const double cadv = E * g.c_adv;
-    const T mh_t = (T)mh, negam_t = (T)negam, dgt_t = (T)dg_t, dgm_t = (T)dg_m, jscale_t = (T)jscale;
-    if (lane == 0) {
-        Jr[n] = (T)(-beta * g.Mp[a]);
-        Jr[n + 1] = (T)(-F[(size_t)pt * n + a]);
-    }
-    // (1) l > 0 columns off the band
-    const int nh = nsh - 1;
-    for (int e = lane; e < nsp * nh; e += 32) {
-        const int c = e / nh, s = 1 + e % nh;
-        if (c >= p - BTE_BAND && c <= p + BTE_BAND) continue;
-        T v = ee ? negam_t * coulomb(c, s) : T(0);
-        Jr[c * nsh + s] = be ? v * jscale_t : v;
-    }
-    // (2) l = 0 columns off the band
-    for (int c = lane; c < nsp; c += 32) {
-        if (c >= p - BTE_BAND && c <= p + BTE_BAND) continue;
-        const int j = c * nsh;
-        const T acc = ee ? coulomb(c, 0) : T(0);
-        if (q == 0) {
-            double v = -mh * sWd[c];
-            if (ee) {
-                v += dg_t * g.temp[j] - dg_m * g.mass[j];
-                v += negam * (double)acc;
-            }
-            const double* q0 = g.q0 + (size_t)p * nsp + c;
-            for (int sp = 0; sp < nspc; ++sp) v += sNs[sp] * q0[(size_t)sp * nsp * nsp];
-            if (be) v *= jscale;
-            Jr[j] = (T)v;
-        } else {
-            T v = negam_t * acc;
-            v += -mh_t * sWt[c];
-            if (ee) v += dgt_t * sTt[c] - dgm_t * sMt[c];
-            Jr[j] = be ? v * jscale_t : v;
-        }
-    }
-    // (3) the band
-    for (int e = lane; e < BTE_NB * nsh; e += 32) {
-        const int dk = e / nsh - BTE_BAND, s = e % nsh;
-        const int c = p + dk;
-        if (c < 0 || c >= nsp) continue;
-        const int j = c * nsh + s;
-        const int bi = p * BTE_NB + dk + BTE_BAND;
-        double v = 0.0;
-        if (s == 0) {
-            v = -mh * sWd[c];
-            if (ee) v += dg_t * g.temp[j] - dg_m * g.mass[j];
-        }
-        if (ee) v += negam * (double)coulomb(c, s);
-        if (s == q) {
-            if (q == 0) {
-                const double* q0 = g.q0 + (size_t)p * nsp + c;
-                for (int sp = 0; sp < nspc; ++sp) v += sNs[sp] * q0[(size_t)sp * nsp * nsp];
-                v += (n0 * Tg) * g.cgT[bi];
-            } else {
-                for (int sp = 0; sp < nspc; ++sp) v += sNs[sp] * g.q1[((size_t)sp * nsp + p) * BTE_NB + dk + BTE_BAND];
-            }
-            v -= mu * g.Mr[bi];
-        }
-        if (s == q + 1) v += cadv * (g.mm1[bi] * g.adv_coef[q * 4 + 0] + g.adv_coef[q * 4 + 1] * g.mm2[bi]);
-        if (s == q - 1) v += cadv * (g.mm1[bi] * g.adv_coef[q * 4 + 2] + g.adv_coef[q * 4 + 3] * g.mm2[bi]);
-        if (ee) v += negam * k1r[e];
-        if (be) {  // backward-Euler form only: the steady kernel spends no FP64 op here
-            v *= jscale;
-            if (s == q) v += jshift * g.Mr[bi];
-        }
-        Jr[j] = (T)v;
     }
     __syncwarp();
-    equilibrate_row(Jr, N, lane, rowscale ? rowscale + (size_t)slot * N + a : nullptr);
+    const double negam = ee ? ne * gam : 0.0;
+    const T negam_t = (T)negam, jscale_t = (T)jscale;
+    // (1) the Coulomb product of every column, and the entries off the band
+    constexpr int CB = sizeof(T) == 4 ? 2 : 1;  // columns per lane at once
+    const T* HL = OpsT<T>::HL(g);
+    const T* GL = OpsT<T>::GL(g);
+    for (int s = 0; s < nsh; ++s) {
+        for (int c0 = lane; c0 < nsp; c0 += 32 * CB) {
+            T hv[CB][BTE_NB], gv[CB][BTE_NB];
+            if (ee) {
+#pragma unroll
+                for (int b = 0; b < CB; ++b) {
+                    const size_t o = (size_t)s * nsp * nsp + min(c0 + 32 * b, nsp - 1);
+#pragma unroll
+                    for (int dr = 0; dr < BTE_NB; ++dr) {
+                        // outside the grid the coefficient is zero
+                        const size_t r = (size_t)min(max(p + dr - BTE_BAND, 0), nsp - 1) * nsp;
+                        hv[b][dr] = HL[o + r];
+                        gv[b][dr] = GL[o + r];
+                    }
+                }
+            }
+            for (int q = 0; q < nsh; ++q) {
+                T acc[CB];
+#pragma unroll
+                for (int b = 0; b < CB; ++b) acc[b] = T(0);
+                if (ee) {
+                    const T* kk = k2 + (q * nsh + s) * 16;
+#pragma unroll
+                    for (int dr = 0; dr < BTE_NB; ++dr)
+#pragma unroll
+                        for (int b = 0; b < CB; ++b) acc[b] += kk[dr] * hv[b][dr] + kk[8 + dr] * gv[b][dr];
+                }
+#pragma unroll
+                for (int b = 0; b < CB; ++b) {
+                    const int c = c0 + 32 * b;
+                    if (c >= nsp) continue;
+                    T v = acc[b];
+                    if (c < p - BTE_BAND || c > p + BTE_BAND) {
+                        if (s > 0) {
+                            v *= negam_t;
+                            if (be) v *= jscale_t;
+                        } else if (q > 0) {
+                            v = negam_t * v - smt[q] * sWt[c] + sUt[q] * sDt[c];
+                            if (be) v *= jscale_t;
+                        } else {
+                            double d = -smh[0] * sWd[c];
+                            if (ee) d += sU[0] * sDd[c] + negam * (double)v;
+                            const double* q0 = g.q0 + (size_t)p * nsp + c;
+                            for (int sp = 0; sp < nspc; ++sp) d += sNs[sp] * q0[(size_t)sp * nsp * nsp];
+                            if (be) d *= jscale;
+                            v = (T)d;
+                        }
+                    }
+                    row[q * ldr + c * nsh + s] = v;
+                }
+            }
+        }
+    }
+    __syncwarp();
+    // (2) the band of all the rows
+    const double cadv = E * g.c_adv, n0Tg = n0 * Tg;
+    for (int e = lane; e < nsh * nk; e += 32) {
+        const int q = e / nk, dk = e % nk / nsh, s = e % nsh;
+        const int c = p + dk - BTE_BAND;
+        if (c < 0 || c >= nsp) continue;
+        T* at = row + q * ldr + c * nsh + s;
+        const int bi = dk * nsp + p;
+        double v = 0.0;
+        if (s == 0) {
+            v = -smh[q] * sWd[c];
+            if (ee) v += sU[q] * sDd[c];
+        }
+        if (ee) v += negam * ((double)*at + k1[e]);
+        if (s == q) {
+            const double* op = q == 0 ? g.tq0 + (size_t)c * nsp + p : g.tq1 + bi;
+            const size_t ops = q == 0 ? (size_t)nsp * nsp : (size_t)BTE_NB * nsp;
+            for (int sp = 0; sp < nspc; ++sp) v += sNs[sp] * op[sp * ops];
+            if (q == 0) v += n0Tg * g.tcgT[bi];
+            v -= mu * g.tMr[bi];
+        }
+        if (s == q + 1 || s == q - 1) v += cadv * g.tadv[(size_t)(q * 2 + (s < q)) * BTE_NB * nsp + bi];
+        if (be) {  // backward-Euler form only: the steady kernel spends no FP64 op here
+            v *= jscale;
+            if (s == q) v += jshift * g.tMr[bi];
+        }
+        *at = (T)v;
+    }
+    __syncwarp();
+    for (int q = 0; q < nsh; ++q) {
+        const size_t a = (size_t)p * nsh + q;
+        put_row(row + q * ldr, J + (size_t)slot * stride + a * ld, N, lane, rowscale ? rowscale + (size_t)slot * N + a : nullptr);
+    }
+}
+
+// Warps per CTA: as many as keep three CTAs on an SM, fewer where a few points leave SMs idle.
+// A row does not depend on it.
+template <typename T, bool KC, class... A>
+static cudaError_t launch_jacobian(const GridView& g, int nact, cudaStream_t s, const PointParams& pp, int ee, A... args) {
+    using L = JacShape<T>;
+    const size_t per = L::warp(g.nsh, ee, KC || !ee ? 0 : g.tqmax, g.n + 1), cols = L::cols(g.nsp, g.nspecies);
+    int nw = JAC_WARPS;
+    while (nw > 1 && cols + nw * per > 72 * 1024) nw /= 2;
+    while (nw > 2 && nact * ((g.nsp + nw) / nw) < 304) nw /= 2;
+    const size_t smem = cols + nw * per;
+    cudaError_t e = bte_raise_smem_limit((const void*)k_jacobian<T, KC>, smem);
+    if (e != cudaSuccess) return e;
+    k_jacobian<T, KC><<<dim3((g.nsp + nw) / nw, nact), nw * 32, smem, s>>>(g, pp, ee, args..., ee);
+    return cudaGetLastError();
+}
+// kc (optional): the rows' e-e coefficients, as k_ee_coef wrote them
+template <typename T>
+static cudaError_t run_jacobian(const GridView& g, int nact, cudaStream_t s, const PointParams& pp, int ee, const int* act,
+                                const double* h, const double* F, const double* aux, const double* scal, T* J, int ld,
+                                long long stride, double beta_scale, double* rowscale, double jscale, double jshift,
+                                const double* kc) {
+    if (sizeof(T) == 4 && kc && ee)
+        return launch_jacobian<T, sizeof(T) == 4>(g, nact, s, pp, ee, act, nact, h, F, aux, scal, J, ld, stride, beta_scale,
+                                                  rowscale, jscale, jshift, kc);
+    return launch_jacobian<T, false>(g, nact, s, pp, ee, act, nact, h, F, aux, scal, J, ld, stride, beta_scale, rowscale,
+                                     jscale, jshift, kc);
 }
 
 // h <- f / (u . f) (bte_0d3v_batched.py:903-911)
@@ -1445,7 +1604,7 @@ struct BteWork {
     int32_t* nit = nullptr;                      // Newton iterations of each point in its current solve
     void* J = nullptr;
     // e-e coefficients of the Jacobian rows in FP64 by slot (mixed form with e-e only):
-    // P x n x kc_row(nsh), written by k_jacobian and applied by the refinement
+    // P x nsh x kc_row(nsh) x nsp, written by k_ee_coef, read by the FP32 Jacobian and the refinement
     double* kc = nullptr;
     size_t kcbytes = 0;
     // GMRES refinement of stalled points (mixed form), gm_cap points at a time
@@ -1547,33 +1706,6 @@ static int ensure_work(BteWork* w, const BteGrid* g, int P, int prec, int krylov
 }
 
 static inline unsigned nblk(int n, int b) { return (unsigned)((n + b - 1) / b); }
-
-// Dynamic shared memory of k_jacobian: the per-point column vectors, and (with e-e on) the
-// HL / GL rows of the CTA's splines when they fit in 96 KB (else they are read from HBM).
-struct JacSmem {
-    size_t bytes;
-    int stage;
-};
-template <typename T>
-static JacSmem jac_smem(const BteGrid* g, int ee) {
-    int tqmax = 0;
-    for (int q = 0; q < g->nsh; ++q) {
-        int c = 0;
-        for (int t = 0; t < g->ntri; ++t) c += (g->tri[3 * t] == q);
-        tqmax = std::max(tqmax, c);
-    }
-    JacSmem r{jac_col_bytes<T>(g->nsp, g->nspecies) + jac_part_bytes(tqmax), 0};
-    const int rows = (JAC_WARPS + g->nsh - 1) / g->nsh + 1 + 2 * BTE_BAND;
-    const size_t hl = (size_t)2 * rows * g->nsh * g->nsp * sizeof(T);
-    if (ee && r.bytes + hl <= 96 * 1024) {
-        r.bytes += hl;
-        r.stage = 1;
-    }
-    // above the default 48 KB the kernel's limit is raised (never lowered); a failure shows
-    // at the launch
-    bte_raise_smem_limit((const void*)k_jacobian<T>, r.bytes);
-    return r;
-}
 
 BteWork* bte_work_get(BteGrid* g) {
     if (!g->work) g->work = new BteWork();
@@ -1878,19 +2010,19 @@ static int newton_iteration(SolveCtx& c, Lane& L, int nact, int prec) {
     }));
     {
         // Jacobian straight into the factorization buffer, then LU of [J | -F] and back substitution
-        dim3 gj(nblk(N, JAC_WARPS), nact);
         const double jb = (double)nact * N * (N + 1) * wsz;
         const double lub = 2.0 * (double)nact * N * (N + 1) * wsz;
         const double lsb = (double)nact * (0.5 * N * (N + 1) * wsz + N * wsz);
         cudaError_t le = cudaSuccess;
         if (prec == BTE_PREC_MIXED) {
             float* xs = reinterpret_cast<float*>(L.xs);
-            CKR(pf.run(PF_JACOBIAN, s, nact * jac_flops_pt(g, ee), jb, 1, [&] {
-                const JacSmem jm = jac_smem<float>(g, ee);
-                k_jacobian<float><<<gj, JAC_WARPS * 32, jm.bytes, s>>>(gv, pp, ee, L.act, nact, w->h, w->F, w->aux, w->scal,
-                                                                 (float*)L.J, ld, jstride, beta_scale, L.rowscale,
-                                                                 jm.stage, 1.0, 0.0, L.kc);
+            CKR(pf.run(PF_JACOBIAN, s, nact * jac_flops_pt(g, ee), jb, L.kc && ee ? 2 : 1, [&] {
+                if (L.kc && ee) le = run_ee_coef(gv, nact, s, pp, ee, L.act, w->h, w->aux, L.kc);
+                if (le == cudaSuccess)
+                    le = run_jacobian<float>(gv, nact, s, pp, ee, L.act, w->h, w->F, w->aux, w->scal, (float*)L.J, ld,
+                                          jstride, beta_scale, L.rowscale, 1.0, 0.0, L.kc);
             }));
+            CKR(le);
             CKR(pf.run(PF_LU, s, nact * lu_flops(N), lub, 1, [&] {
                 le = bte_lu_factor_t<float>(nact, N, N + 1, (float*)L.J, ld, jstride, L.piv, L.info, s,
                                             lu_kernel_for(o->lu_kernel, N));
@@ -1932,11 +2064,10 @@ static int newton_iteration(SolveCtx& c, Lane& L, int nact, int prec) {
         } else {
             double* xs = L.xs;
             CKR(pf.run(PF_JACOBIAN, s, nact * jac_flops_pt(g, ee), jb, 1, [&] {
-                const JacSmem jm = jac_smem<double>(g, ee);
-                k_jacobian<double><<<gj, JAC_WARPS * 32, jm.bytes, s>>>(gv, pp, ee, L.act, nact, w->h, w->F, w->aux, w->scal,
-                                                                  (double*)L.J, ld, jstride, beta_scale, L.rowscale,
-                                                                  jm.stage, 1.0, 0.0, nullptr);
+                le = run_jacobian<double>(gv, nact, s, pp, ee, L.act, w->h, w->F, w->aux, w->scal, (double*)L.J, ld,
+                                          jstride, beta_scale, L.rowscale, 1.0, 0.0, nullptr);
             }));
+            CKR(le);
             CKR(pf.run(PF_LU64, s, nact * lu_flops(N), lub, 1, [&] {
                 le = bte_lu_factor_t<double>(nact, N, N + 1, (double*)L.J, ld, jstride, L.piv, L.info, s,
                                              lu64_kernel_for(o->lu64_kernel));
@@ -2616,25 +2747,22 @@ int bte_transient_impl(BteGrid* g, int P, const double* n0, const double* ne, co
             run_residual(c.gv, P, s, c.pp, c.ee, all, P, w->h, nullptr, 0, nullptr, nullptr, nullptr,
                                                   w->F, w->aux, w->scal, w->r, nullptr, nullptr);
         }));
-        dim3 gj(nblk(N, JAC_WARPS), P);
         cudaError_t le = cudaSuccess;
         if (prec == BTE_PREC_MIXED) {
             CKR(pf.run(PF_JACOBIAN, s, 0, 0, 1, [&] {
-                const JacSmem jm = jac_smem<float>(g, c.ee);
-                k_jacobian<float><<<gj, JAC_WARPS * 32, jm.bytes, s>>>(
-                    c.gv, c.pp, c.ee, all, P, w->h, w->F, w->aux, w->scal, (float*)w->J, ld, js, beta, w->rowscale,
-                    jm.stage, -cdt, 1.0, nullptr);
+                le = run_jacobian<float>(c.gv, P, s, c.pp, c.ee, all, w->h, w->F, w->aux, w->scal, (float*)w->J, ld,
+                                          js, beta, w->rowscale, -cdt, 1.0, nullptr);
             }));
+            CKR(le);
             CKR(pf.run(PF_LU, s, P * lu_flops(N), 0, 1, [&] {
                 le = bte_lu_factor_t<float>(P, N, N, (float*)w->J, ld, js, w->piv, w->info, s, 0);
             }));
         } else {
             CKR(pf.run(PF_JACOBIAN, s, 0, 0, 1, [&] {
-                const JacSmem jm = jac_smem<double>(g, c.ee);
-                k_jacobian<double><<<gj, JAC_WARPS * 32, jm.bytes, s>>>(
-                    c.gv, c.pp, c.ee, all, P, w->h, w->F, w->aux, w->scal, (double*)w->J, ld, js, beta, w->rowscale,
-                    jm.stage, -cdt, 1.0, nullptr);
+                le = run_jacobian<double>(c.gv, P, s, c.pp, c.ee, all, w->h, w->F, w->aux, w->scal, (double*)w->J, ld,
+                                          js, beta, w->rowscale, -cdt, 1.0, nullptr);
             }));
+            CKR(le);
             CKR(pf.run(PF_LU, s, P * lu_flops(N), 0, 1, [&] {
                 le = bte_lu_factor_t<double>(P, N, N, (double*)w->J, ld, js, w->piv, w->info, s, 0);
             }));
