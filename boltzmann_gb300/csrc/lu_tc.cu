@@ -9,20 +9,24 @@
 // memory, perm[position] = stored row, info = first zero pivot (1-based), 0 if none.
 //
 // One CTA per matrix, right-looking by 32-column panels:
-//   1. panel: the 32 columns of positions k0..N-1 are held in registers (thread t owns
-//      positions k0 + t + i * 256); each column costs one barrier: every warp publishes its
-//      best candidate row in shared memory, all threads pick the same winner (largest |a|,
-//      lowest position on ties, as LAPACK's i?amax), swap it with position j by registers
-//      and apply the rank-one update;
+//   1. panel: the 32 columns of positions k0..N-1 are held in registers; each column costs one
+//      barrier: every warp publishes its best candidate row in shared memory, every warp picks
+//      the same winner from them (one candidate per lane; largest |a|, lowest position on ties,
+//      as LAPACK's i?amax) and applies the rank-one update. A row stays with its thread: only
+//      its position changes;
 //   2. U12 = L11^-1 A12 for the 32 pivot rows, one thread per column;
-//   3. A22 -= L21 U12 in tiles of 128 columns x 128 rows: U12^T (M = 128 columns) and L21
-//      (N = 128 rows) are staged in shared memory in the canonical K-major layout (8 x 16 B
-//      core matrices, no swizzle), split into a TF32 high part and an FP32 remainder, and
-//      one thread issues 4 k-steps x 3 products (hi*hi + hi*lo + lo*hi) of
-//      tcgen05.mma.cta_group::1.kind::tf32 into a 128-lane x 128-column TMEM accumulator.
-//      The epilogue reads it back with tcgen05.ld (lane = column, so a warp's 32 lanes are
-//      32 consecutive columns of one row: coalesced) and updates A22 in global memory,
-//      which stays L2-resident while the CTA works on it.
+//   3. A22 -= L21 U12 in tiles of 128 columns x up to 192 rows (as even as multiples of 32
+//      allow): U12^T (M = 128 columns) and L21 (N = rows) are staged in shared memory in the
+//      canonical K-major layout (8 x 16 B core matrices, no swizzle), split into a TF32 high
+//      part and an FP32 remainder, and one thread issues 4 k-steps x 3 products (hi*hi +
+//      hi*lo + lo*hi) of tcgen05.mma.cta_group::1.kind::tf32 into a TMEM accumulator of 128
+//      lanes. The warps read their part of A22 (lane = column: 32 consecutive columns of one
+//      row, coalesced) before the product is issued and subtract the accumulator
+//      (tcgen05.ld) from it after.
+// Bound by latency: the panel's chain of columns and the tiles' reads, writes and barriers; two CTAs
+// share an SM. Reading A22 only after the product, in groups of 16 rows, with tiles of 128 x 128 and
+// rows exchanged between threads, one matrix of N = 385 took 708 us and 4096 took 14.2 ms; now
+// @TC1@ us and @TC4@ ms.
 // Above N = 512 (k_tcs_*) the same steps are separate launches over many CTAs per matrix.
 // The split: hi = tf32(x) (round to nearest), lo = x - hi (exact in FP32); hi*hi is exact
 // in the FP32 accumulator, the dropped lo*lo term is below 2^-22 |x y|.
@@ -38,6 +42,9 @@ constexpr int TC_NB = 32;          // panel width = K of one block step
 constexpr int TC_TM = 128;         // trailing columns per tile: MMA M, TMEM lanes
 constexpr int TC_TR = 128;         // trailing rows per tile: MMA N, TMEM columns
 constexpr uint32_t TC_TMEM_COLS = 128;
+constexpr int TC_TRX = 192;        // tallest tile of k_lu_tc (its tiles are as even as 32 rows allow)
+constexpr uint32_t TC_TMEM_COLS_X = 256;
+constexpr int TC_PRE = 4;          // groups of 16 rows of a tile read ahead of its product
 constexpr int TC_TILE_BYTES = TC_TM * TC_NB * 4;   // one operand part: 16 KB (TM == TR)
 constexpr int TC_L11_LD = TC_NB + 4;        // L11 stored transposed, 16-byte rows
 constexpr int TC_CAND_LD = TC_NB + 4;              // a candidate row + key + slot, 16-byte rows
@@ -47,11 +54,11 @@ constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;       // bounded wait for an MMA co
 constexpr int SM_A_HI = 0;
 constexpr int SM_A_LO = SM_A_HI + TC_TILE_BYTES;
 constexpr int SM_B_HI = SM_A_LO + TC_TILE_BYTES;
-constexpr int SM_B_LO = SM_B_HI + TC_TILE_BYTES;
-constexpr int SM_L11 = SM_B_LO + TC_TILE_BYTES;
+constexpr int TC_TILEX_BYTES = TC_TRX * TC_NB * 4;
+constexpr int SM_B_LO = SM_B_HI + TC_TILEX_BYTES;
+constexpr int SM_L11 = SM_B_LO + TC_TILEX_BYTES;
 constexpr int SM_CAND = SM_L11 + ((TC_NB * TC_L11_LD * 4 + 15) & ~15);
-constexpr int SM_JBUF = SM_CAND + 2 * TC_NW * TC_CAND_LD * 4;
-constexpr int SM_PERM = SM_JBUF + 2 * TC_NB * 4;
+constexpr int SM_PERM = SM_CAND + 2 * TC_NW * TC_CAND_LD * 4;
 __host__ __device__ inline size_t tc_smem_bytes(int N) { return (size_t)SM_PERM + (size_t)N * 4 + 1024; }
 
 // byte offset of element (row m, k) in a [rows x 32] TF32 tile, K-major, no swizzle:
@@ -70,7 +77,7 @@ __device__ inline uint64_t op_desc(uint32_t saddr) {
 
 // instruction descriptor of kind::tf32: D F32 (bits 4-5 = 1), A and B TF32 (bits 7-9, 10-12
 // = 2), both K-major (bits 15, 16 = 0), N >> 3 at bit 17, M >> 4 at bit 24
-constexpr uint32_t idesc_tf32(int M, int N) {
+__host__ __device__ constexpr uint32_t idesc_tf32(int M, int N) {
     return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
@@ -134,12 +141,13 @@ __device__ inline float tf32_rn(float x) {
 }
 
 // four values of one operand row (m, k..k+3) as high and low parts
-__device__ inline void put_split4(unsigned char* sm, int m, int k, float a, float b, float c, float d) {
+__device__ inline void put_split4(unsigned char* sm, int m, int k, float a, float b, float c, float d,
+                                  int lo_off = TC_TILE_BYTES) {
     float4 hi = make_float4(tf32_rn(a), tf32_rn(b), tf32_rn(c), tf32_rn(d));
     float4 lo = make_float4(a - hi.x, b - hi.y, c - hi.z, d - hi.w);
     const int o = op_off(m, k);
     *reinterpret_cast<float4*>(sm + o) = hi;
-    *reinterpret_cast<float4*>(sm + TC_TILE_BYTES + o) = lo;
+    *reinterpret_cast<float4*>(sm + lo_off + o) = lo;
 }
 
 template <int ROWS, int OCC, int NT>
@@ -154,7 +162,6 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
     unsigned char* sm = smraw + ((1024 - (smem_u32(smraw) & 1023)) & 1023);
     float* L11 = reinterpret_cast<float*>(sm + SM_L11);
     float* cand = reinterpret_cast<float*>(sm + SM_CAND);
-    float* jbuf = reinterpret_cast<float*>(sm + SM_JBUF);
     int* perm = reinterpret_cast<int*>(sm + SM_PERM);
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -165,7 +172,7 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
         mbar_init(mb, 1);
         s_fault = 0;
     }
-    if (wid == 0) tmem_alloc(smem_u32(&tmem_slot), TC_TMEM_COLS);
+    if (wid == 0) tmem_alloc(smem_u32(&tmem_slot), TC_TMEM_COLS_X);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -177,74 +184,62 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
         const int mrows = N - k0;
         const int kb = min(TC_NB, mrows);
         const int ncol = min(TC_NB, NC - k0);
-        // ---- 1. panel: positions k0.., columns k0..k0+31 in registers
+        // ---- 1. panel: positions k0.., columns k0..k0+31 in registers. A row stays with its thread
+        // and only its position changes; the warps' candidates are compared by one lane each.
         float pr[ROWS][TC_NB];
+        int pos[ROWS], row[ROWS];  // position relative to k0 (-1: no row), stored row
 #pragma unroll
         for (int i = 0; i < ROWS; ++i) {
             const int s = tid + i * NT;
-            const float* row = a + (size_t)perm[k0 + min(s, mrows - 1)] * ld + k0;
+            pos[i] = (s < mrows) ? s : -1;
+            row[i] = perm[k0 + min(s, mrows - 1)];
+            const float* src = a + (size_t)row[i] * ld + k0;
             if (vec4 && ncol == TC_NB) {
 #pragma unroll
                 for (int c = 0; c < TC_NB; c += 4) {
-                    float4 v = (s < mrows) ? *reinterpret_cast<const float4*>(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    float4 v = (s < mrows) ? *reinterpret_cast<const float4*>(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
                     pr[i][c] = v.x; pr[i][c + 1] = v.y; pr[i][c + 2] = v.z; pr[i][c + 3] = v.w;
                 }
             } else {
 #pragma unroll
-                for (int c = 0; c < TC_NB; ++c) pr[i][c] = (s < mrows && c < ncol) ? row[c] : 0.f;
+                for (int c = 0; c < TC_NB; ++c) pr[i][c] = (s < mrows && c < ncol) ? src[c] : 0.f;
             }
         }
 #pragma unroll
         for (int j = 0; j < TC_NB; ++j) {
             if (j >= kb) break;
-            const int par = j & 1;
-            float* cb = cand + par * TC_NW * TC_CAND_LD;
-            float* jb = jbuf + par * TC_NB;
-            if (tid == j) {
+            float* cb = cand + (j & 1) * TC_NW * TC_CAND_LD;
+            // the thread's and the warp's candidate among positions >= j: largest |a| (NaN counts
+            // as 0), first position
+            uint32_t key = 0, at = 0xffffffffu;
+            int bi = 0;
 #pragma unroll
-                for (int c = 0; c < TC_NB; c += 4)
-                    *reinterpret_cast<float4*>(jb + c) = make_float4(pr[0][c], pr[0][c + 1], pr[0][c + 2], pr[0][c + 3]);
-            }
-            // the thread's best candidate among positions >= j: largest |a| (NaN counts as 0)
-            uint32_t bkey = 0;
-            int bs = INT_MAX;
-#pragma unroll
-            for (int i = 0; i < ROWS; ++i) {
-                const int s = tid + i * NT;
-                if (s >= j && s < mrows) {
+            for (int i = 0; i < ROWS; ++i)
+                if (pos[i] >= j) {
                     const float v = fabsf(pr[i][j]);
-                    const uint32_t key = (v == v) ? __float_as_uint(v) : 0u;
-                    if (bs == INT_MAX || key > bkey) { bkey = key; bs = s; }
+                    const uint32_t k = (v == v) ? __float_as_uint(v) : 0u;
+                    if (at == 0xffffffffu || k > key || (k == key && (uint32_t)pos[i] < at)) { key = k; at = pos[i]; bi = i; }
                 }
-            }
-            const uint32_t kmax = __reduce_max_sync(0xffffffffu, bkey);
-            const uint32_t smin =
-                __reduce_min_sync(0xffffffffu, (bs != INT_MAX && bkey == kmax) ? (uint32_t)bs : 0xffffffffu);
-            float* myc = cb + wid * TC_CAND_LD;
-            if (smin != 0xffffffffu && (uint32_t)bs == smin) {
+            const uint32_t wk = __reduce_max_sync(0xffffffffu, key);
+            const uint32_t wa = __reduce_min_sync(0xffffffffu, key == wk ? at : 0xffffffffu);
+            if (wa == 0xffffffffu ? lane == 0 : at == wa) {
+                float* my = cb + wid * TC_CAND_LD;
+                *reinterpret_cast<uint2*>(my + TC_NB) = make_uint2(wk, wa);
 #pragma unroll
                 for (int i = 0; i < ROWS; ++i)
-                    if (tid + i * NT == bs) {
+                    if (i == bi) {
 #pragma unroll
-                        for (int c = 0; c < TC_NB; c += 4)
-                            *reinterpret_cast<float4*>(myc + c) =
-                                make_float4(pr[i][c], pr[i][c + 1], pr[i][c + 2], pr[i][c + 3]);
+                        for (int c = (j & ~3); c < TC_NB; c += 4)
+                            *reinterpret_cast<float4*>(my + c) = make_float4(pr[i][c], pr[i][c + 1], pr[i][c + 2], pr[i][c + 3]);
                     }
-                reinterpret_cast<uint32_t*>(myc)[TC_NB] = kmax;
-                reinterpret_cast<int*>(myc)[TC_NB + 1] = bs;
-            } else if (smin == 0xffffffffu && lane == 0) {
-                reinterpret_cast<int*>(myc)[TC_NB + 1] = INT_MAX;
             }
             __syncthreads();
-            // the same winner in every thread: (key, slot) pairs read 8 bytes at a time
-            uint32_t K = 0;
-            int S = INT_MAX, W = 0;
-#pragma unroll
-            for (int w2 = 0; w2 < NT / 32; ++w2) {
-                const uint2 ks = *reinterpret_cast<const uint2*>(cb + w2 * TC_CAND_LD + TC_NB);
-                const int s2 = (int)ks.y;
-                if (s2 != INT_MAX && (S == INT_MAX || ks.x > K || (ks.x == K && s2 < S))) { K = ks.x; S = s2; W = w2; }
-            }
+            // the same winner in every thread
+            const uint2 o = (lane < NT / 32) ? *reinterpret_cast<const uint2*>(cb + lane * TC_CAND_LD + TC_NB)
+                                             : make_uint2(0u, 0xffffffffu);
+            const uint32_t bk = __reduce_max_sync(0xffffffffu, o.y == 0xffffffffu ? 0u : o.x);
+            const uint32_t S = __reduce_min_sync(0xffffffffu, o.x == bk ? o.y : 0xffffffffu);
+            const int W = __ffs(__ballot_sync(0xffffffffu, o.x == bk && o.y == S)) - 1;
             const float* prow = cb + W * TC_CAND_LD;
             // the pivot row's columns j.. in registers (16-byte loads from the 4-aligned start)
             float pv[TC_NB];
@@ -253,36 +248,14 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
                 const float4 v = *reinterpret_cast<const float4*>(prow + c);
                 pv[c] = v.x; pv[c + 1] = v.y; pv[c + 2] = v.z; pv[c + 3] = v.w;
             }
-            if (S != j && S != INT_MAX) {
-                if (tid == j) {
-#pragma unroll
-                    for (int c = 0; c < TC_NB; c += 4) {
-                        const float4 v = *reinterpret_cast<const float4*>(prow + c);
-                        pr[0][c] = v.x; pr[0][c + 1] = v.y; pr[0][c + 2] = v.z; pr[0][c + 3] = v.w;
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < ROWS; ++i)
-                    if (tid + i * NT == S) {
-#pragma unroll
-                        for (int c = 0; c < TC_NB; c += 4) {
-                            const float4 v = *reinterpret_cast<const float4*>(jb + c);
-                            pr[i][c] = v.x; pr[i][c + 1] = v.y; pr[i][c + 2] = v.z; pr[i][c + 3] = v.w;
-                        }
-                    }
-                if (tid == 0) {
-                    const int t = perm[k0 + j];
-                    perm[k0 + j] = perm[k0 + S];
-                    perm[k0 + S] = t;
-                }
-            }
             const float d = pv[j];
-            if (tid == 0 && !(d != 0.f) && inf == 0) inf = k0 + j + 1;
+            if (!(d != 0.f) && inf == 0) inf = k0 + j + 1;
             const float inv = (d != 0.f) ? __frcp_rn(d) : 0.f;
 #pragma unroll
             for (int i = 0; i < ROWS; ++i) {
-                const int s = tid + i * NT;
-                if (s > j && s < mrows) {
+                if (pos[i] == (int)S) pos[i] = j;
+                else if (pos[i] == j) pos[i] = (int)S;
+                if (pos[i] > j) {
                     const float l = pr[i][j] * inv;
                     pr[i][j] = l;
 #pragma unroll
@@ -290,32 +263,31 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
                 }
             }
         }
-        __syncthreads();  // perm of this panel final
-        // write the panel back (each position's data returns to its own stored row) and L11
+        // write the panel back (each position's data returns to its own stored row), the positions
+        // and L11
 #pragma unroll
         for (int i = 0; i < ROWS; ++i) {
-            const int s = tid + i * NT;
-            if (s < mrows) {
-                float* row = a + (size_t)perm[k0 + s] * ld + k0;
-                if (vec4 && ncol == TC_NB) {
+            if (pos[i] < 0) continue;
+            float* dst = a + (size_t)row[i] * ld + k0;
+            if (vec4 && ncol == TC_NB) {
 #pragma unroll
-                    for (int c = 0; c < TC_NB; c += 4)
-                        *reinterpret_cast<float4*>(row + c) = make_float4(pr[i][c], pr[i][c + 1], pr[i][c + 2], pr[i][c + 3]);
-                } else {
+                for (int c = 0; c < TC_NB; c += 4)
+                    *reinterpret_cast<float4*>(dst + c) = make_float4(pr[i][c], pr[i][c + 1], pr[i][c + 2], pr[i][c + 3]);
+            } else {
 #pragma unroll
-                    for (int c = 0; c < TC_NB; ++c)
-                        if (c < ncol) row[c] = pr[i][c];
-                }
-                if (i == 0 && s < TC_NB) {
+                for (int c = 0; c < TC_NB; ++c)
+                    if (c < ncol) dst[c] = pr[i][c];
+            }
+            perm[k0 + pos[i]] = row[i];
+            if (pos[i] < TC_NB) {
 #pragma unroll
-                    for (int c = 0; c < TC_NB; ++c) L11[c * TC_L11_LD + s] = pr[0][c];
-                }
+                for (int c = 0; c < TC_NB; ++c) L11[c * TC_L11_LD + pos[i]] = pr[i][c];
             }
         }
         const int ncols = NC - k0 - TC_NB;   // columns right of the panel (> 0 implies kb == 32)
         const int nrows = N - k0 - TC_NB;    // trailing rows
+        __syncthreads();  // the panel's positions and L11
         if (ncols <= 0) break;
-        __syncthreads();
         // ---- 2. U12 = L11^-1 A12, one thread per column
         for (int c = tid; c < ncols; c += NT) {
             float x[TC_NB];
@@ -340,9 +312,12 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
         if (nrows <= 0) break;  // last panel
         __syncthreads();
         // ---- 3. A22 -= L21 U12 on the tensor cores
-        for (int g0 = 0; g0 < nrows; g0 += TC_TR) {
+        const int nrt = (nrows + TC_TRX - 1) / TC_TRX;              // row tiles
+        const int th = ((nrows + nrt - 1) / nrt + 31) & ~31;        // rows of each, a multiple of 32
+        const uint32_t idesc = idesc_tf32(TC_TM, th);
+        for (int g0 = 0; g0 < nrows; g0 += th) {
             // B operand: L21 rows g0.., K = the panel's 32 columns
-            for (int e = tid; e < TC_TR * (TC_NB / 4); e += NT) {
+            for (int e = tid; e < th * (TC_NB / 4); e += NT) {
                 const int r = e >> 3, k = (e & 7) * 4;
                 float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
                 if (g0 + r < nrows) {
@@ -354,9 +329,23 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
                         v0 = row[0]; v1 = row[1]; v2 = row[2]; v3 = row[3];
                     }
                 }
-                put_split4(sm + SM_B_HI, r, k, v0, v1, v2, v3);
+                put_split4(sm + SM_B_HI, r, k, v0, v1, v2, v3, TC_TILEX_BYTES);
             }
             for (int c0 = 0; c0 < ncols; c0 += TC_TM) {
+                // warp w updates the columns of TMEM lanes 32 (w % 4).. in its share of the rows:
+                // all of the tile's with 4 warps, half with 8. Its first 16 TC_PRE rows are read
+                // here, ahead of the product.
+                const int wq = wid & 3, rh = th / (NT / 128), rw = g0 + rh * (wid >> 2);
+                const bool colok = (c0 + 32 * wq + lane) < ncols;
+                float* colp = a + k0 + TC_NB + c0 + 32 * wq + lane;
+                const int* rperm = perm + k0 + TC_NB + rw;
+                const int nr = min(rh, nrows - rw);  // rows of this warp (none if <= 0)
+                float old[TC_PRE][16];
+#pragma unroll
+                for (int u = 0; u < TC_PRE; ++u)
+#pragma unroll
+                    for (int t = 0; t < 16; ++t)
+                        old[u][t] = (colok && u * 16 + t < nr) ? colp[(size_t)rperm[u * 16 + t] * ld] : 0.f;
                 // A operand: U12^T, row m = column c0 + m of U12, k = pivot row
                 for (int e = tid; e < TC_TM * (TC_NB / 4); e += NT) {
                     const int m = e & (TC_TM - 1), k = (e >> 7) * 4;
@@ -374,7 +363,6 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
                     tc_fence_after();
                     const uint32_t ahi = smem_u32(sm + SM_A_HI), alo = smem_u32(sm + SM_A_LO);
                     const uint32_t bhi = smem_u32(sm + SM_B_HI), blo = smem_u32(sm + SM_B_LO);
-                    constexpr uint32_t idesc = idesc_tf32(TC_TM, TC_TR);
 #pragma unroll
                     for (int ks = 0; ks < TC_NB / 8; ++ks) {
                         const uint32_t o = ks * 256;
@@ -391,31 +379,32 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
                 __syncthreads();
                 tc_fence_after();
                 if (s_fault) break;
-                // epilogue: warp w reads TMEM lanes 32 (w % 4).. (columns) and its share of
-                // the TMEM columns (rows): all 128 with 4 warps, 64 (w / 4).. with 8
-                {
-                    constexpr int RH = TC_TR / (NT / 128);
-                    const int q = wid & 3, h = wid >> 2;
-                    const int m = 32 * q + lane;
-                    const bool colok = (c0 + m) < ncols;
-                    float* colp = a + k0 + TC_NB + c0 + m;
+                const uint32_t trow = tbase + ((uint32_t)(32 * wq) << 16) + (uint32_t)(rw - g0);
+#pragma unroll
+                for (int u = 0; u < TC_PRE; ++u) {
+                    if (u * 16 >= nr) break;  // warp-uniform
+                    float dv[16];
+                    tmem_ld16(trow + u * 16, dv);
+#pragma unroll
+                    for (int t = 0; t < 16; ++t)
+                        if (colok && u * 16 + t < nr) colp[(size_t)rperm[u * 16 + t] * ld] = old[u][t] - dv[t];
+                }
 #pragma unroll 1
-                    for (int r0 = RH * h; r0 < RH * h + RH; r0 += 16) {
-                        if (g0 + r0 >= nrows) break;  // warp-uniform
-                        float dv[16];
-                        tmem_ld16(tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)r0, dv);
-                        float old[16];
-                        int rowoff[16];
+                for (int r0 = TC_PRE * 16; r0 < nr; r0 += 32) {
+                    float ov[2][16];
 #pragma unroll
-                        for (int t = 0; t < 16; ++t) {
-                            const int r = g0 + r0 + t;
-                            rowoff[t] = (r < nrows) ? perm[k0 + TC_NB + r] * ld : -1;
-                        }
-#pragma unroll
-                        for (int t = 0; t < 16; ++t) old[t] = (colok && rowoff[t] >= 0) ? colp[rowoff[t]] : 0.f;
+                    for (int u = 0; u < 2; ++u)
 #pragma unroll
                         for (int t = 0; t < 16; ++t)
-                            if (colok && rowoff[t] >= 0) colp[rowoff[t]] = old[t] - dv[t];
+                            ov[u][t] = (colok && r0 + u * 16 + t < nr) ? colp[(size_t)rperm[r0 + u * 16 + t] * ld] : 0.f;
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        if (r0 + u * 16 >= nr) break;
+                        float dv[16];
+                        tmem_ld16(trow + r0 + u * 16, dv);
+#pragma unroll
+                        for (int t = 0; t < 16; ++t)
+                            if (colok && r0 + u * 16 + t < nr) colp[(size_t)rperm[r0 + u * 16 + t] * ld] = ov[u][t] - dv[t];
                     }
                 }
                 tc_fence_before();
@@ -439,7 +428,7 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (wid == 0) tmem_dealloc(tbase, TC_TMEM_COLS);
+    if (wid == 0) tmem_dealloc(tbase, TC_TMEM_COLS_X);
 }
 
 // ---------------------------------------------------------------------------------
@@ -646,7 +635,7 @@ k_tcs_update(int N, int NC, int k0, int kb, int nct, int nrt, float* __restrict_
     if (tid == 0) {
         tc_fence_after();
         const uint32_t ahi = smem_u32(sm + SM_A_HI), alo = smem_u32(sm + SM_A_LO);
-        const uint32_t bhi = smem_u32(sm + SM_B_HI), blo = smem_u32(sm + SM_B_LO);
+        const uint32_t bhi = smem_u32(sm + SM_B_HI), blo = bhi + TC_TILE_BYTES;
         constexpr uint32_t idesc = idesc_tf32(TC_TM, TC_TR);
         for (int ks = 0; ks < kb / 8; ++ks) {
             const uint32_t o = ks * 256;
@@ -730,7 +719,7 @@ cudaError_t bte_lu_factor_tcs(int P, int N, int NC, float* A, int ld, long long 
     if (N < 1 || N > 4 * TS_NT || NC < N || NC > N + 1 || ld < NC) return cudaErrorInvalidValue;
     if ((long long)N * ld >= (1ll << 31)) return cudaErrorInvalidValue;  // row offsets are 32-bit
     const int vec4 = (ld % 4 == 0 && stride % 4 == 0 && ((uintptr_t)A & 15) == 0) ? 1 : 0;
-    const size_t usm = (size_t)SM_L11 + 1024;
+    const size_t usm = (size_t)4 * TC_TILE_BYTES + 1024;
     cudaError_t e = bte_raise_smem_limit((const void*)k_tcs_update, usm);
     if (e != cudaSuccess) return e;
     for (int k0 = 0; k0 < N;) {

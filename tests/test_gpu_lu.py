@@ -314,3 +314,33 @@ def test_lu_fp32_above_512(N, pad):
     _lib.check(lib.bte_lu_factor_ex(1, 1, N, ptr(Z), N, N * N, ptr(piv), ptr(info), 0, st), "lu_factor")
     torch.cuda.synchronize()
     assert int(info[0].item()) == N - 2
+
+
+@pytest.mark.parametrize("kernel", [2, 4, 5], ids=["tc", "tc1", "tc128"])
+@pytest.mark.parametrize("N,pad", [(2, 0), (33, 3), (64, 0), (96, 1), (97, 3), (224, 0), (225, 3), (226, 2), (257, 0),
+                                   (289, 3), (416, 0), (417, 3), (449, 1), (512, 0)])
+def test_lu_tc_tile_edges(N, pad, kernel):
+    """The tensor-core factorization at sizes where its trailing matrix is one row more than one or
+    two tiles of 192, a multiple of a panel, or smaller than a tile; rows with and without 16-byte
+    loads. Backward error as for the other kernels."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    P, ld = 3, N + pad
+    g = torch.Generator(device="cuda").manual_seed(N)
+    A0 = torch.randn((P, N, ld), device="cuda", generator=g, dtype=torch.float32)
+    A0[:, :, :N] += 0.1 * torch.eye(N, device="cuda")
+    b0 = torch.randn((P, N), device="cuda", generator=g, dtype=torch.float32)
+    ptr, st = (lambda t: C.c_void_p(t.data_ptr())), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    A, x = A0.clone(), b0.clone()
+    piv = torch.empty((P, N), dtype=torch.int32, device="cuda")
+    info = torch.empty(P, dtype=torch.int32, device="cuda")
+    _lib.check(lib.bte_lu_factor_ex(1, P, N, ptr(A), ld, N * ld, ptr(piv), ptr(info), kernel, st), "lu_factor")
+    _lib.check(lib.bte_lu_solve(1, P, N, ptr(A), ld, N * ld, ptr(piv), ptr(x), st), "lu_solve")
+    torch.cuda.synchronize()
+    assert bool((info == 0).all()) and torch.equal(A[:, :, N:], A0[:, :, N:])
+    assert torch.equal(torch.sort(piv, dim=1).values.long(), torch.arange(N, device="cuda").expand(P, N))
+    for i in range(P):
+        Ad, xd, bd = A0[i, :, :N].double(), x[i].double(), b0[i].double()
+        berr = torch.linalg.norm(Ad @ xd - bd) / (torch.linalg.matrix_norm(Ad, 2) * torch.linalg.norm(xd) + torch.linalg.norm(bd))
+        assert float(berr) < 2 * N * 1.2e-7, (i, float(berr))
