@@ -25,8 +25,8 @@
 //      (tcgen05.ld) from it after.
 // Bound by latency: the panel's chain of columns and the tiles' reads, writes and barriers; two CTAs
 // share an SM. Reading A22 only after the product, in groups of 16 rows, with tiles of 128 x 128 and
-// rows exchanged between threads, one matrix of N = 385 took 708 us and 4096 took 14.2 ms; now
-// @TC1@ us and @TC4@ ms.
+// rows exchanged between threads under branches, one matrix of N = 385 took 708 us and 4096 took
+// 14.4 ms; now // 352 us and 7.0 ms.
 // Above N = 512 (k_tcs_*) the same steps are separate launches over many CTAs per matrix.
 // The split: hi = tf32(x) (round to nearest), lo = x - hi (exact in FP32); hi*hi is exact
 // in the FP32 accumulator, the dropped lo*lo term is below 2^-22 |x y|.
@@ -59,7 +59,8 @@ constexpr int SM_B_LO = SM_B_HI + TC_TILEX_BYTES;
 constexpr int SM_L11 = SM_B_LO + TC_TILEX_BYTES;
 constexpr int SM_CAND = SM_L11 + ((TC_NB * TC_L11_LD * 4 + 15) & ~15);
 constexpr int SM_PERM = SM_CAND + 2 * TC_NW * TC_CAND_LD * 4;
-__host__ __device__ inline size_t tc_smem_bytes(int N) { return (size_t)SM_PERM + (size_t)N * 4 + 1024; }
+constexpr int TC_OFF_PAD = TC_TRX + 4;  // offsets past the last row, read but not used
+__host__ __device__ inline size_t tc_smem_bytes(int N) { return (size_t)SM_PERM + (size_t)(2 * N + 4 + TC_OFF_PAD) * 4 + 1024; }
 
 // byte offset of element (row m, k) in a [rows x 32] TF32 tile, K-major, no swizzle:
 // core matrix (m / 8, k / 4) at (m / 8) * 1024 + (k / 4) * 128, rows of a core matrix 16 B apart
@@ -150,6 +151,27 @@ __device__ inline void put_split4(unsigned char* sm, int m, int k, float a, floa
     *reinterpret_cast<float4*>(sm + lo_off + o) = lo;
 }
 
+// Predicated stores and a reciprocal without branches, for the panels' chain of columns: a branch that
+// may diverge costs about 50 cycles there, whether taken or not.
+__device__ inline void put_if(bool on, uint32_t addr, float x, float y, float z, float w) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %0, 0;\n\t@p st.shared.v4.f32 [%1], {%2, %3, %4, %5};\n\t}\n" ::"r"(
+                     (uint32_t)on),
+                 "r"(addr), "f"(x), "f"(y), "f"(z), "f"(w)
+                 : "memory");
+}
+__device__ inline void put_if(bool on, uint32_t addr, uint32_t x, uint32_t y) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %0, 0;\n\t@p st.shared.v2.b32 [%1], {%2, %3};\n\t}\n" ::"r"((uint32_t)on),
+                 "r"(addr), "r"(x), "r"(y)
+                 : "memory");
+}
+// 1 / d to within an ulp, 0 for d = 0: the hardware's approximation and one Newton step where that is finite
+__device__ inline float recip_or_0(float d) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;\n" : "=f"(r) : "f"(d));
+    const float c = fmaf(r, fmaf(-d, r, 1.f), r);
+    return (d != 0.f) ? (fabsf(c) <= 3.402823466e38f ? c : r) : 0.f;
+}
+
 template <int ROWS, int OCC, int NT>
 __global__ void __launch_bounds__(NT, OCC)
 k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t* __restrict__ perm_out,
@@ -162,11 +184,13 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
     unsigned char* sm = smraw + ((1024 - (smem_u32(smraw) & 1023)) & 1023);
     float* L11 = reinterpret_cast<float*>(sm + SM_L11);
     float* cand = reinterpret_cast<float*>(sm + SM_CAND);
-    int* perm = reinterpret_cast<int*>(sm + SM_PERM);
+    int* perm = reinterpret_cast<int*>(sm + SM_PERM);  // stored row of a position
+    int* roff = perm + ((N + 3) & ~3);                 // its offset in elements, 0 past the last
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     float* a = A + (size_t)blockIdx.x * stride;
     for (int r = tid; r < N; r += NT) perm[r] = r;
+    for (int r = tid; r < N + TC_OFF_PAD; r += NT) roff[r] = (r < N) ? r * ld : 0;
     const uint32_t mb = smem_u32(&mbar);
     if (tid == 0) {
         mbar_init(mb, 1);
@@ -215,24 +239,24 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
             int bi = 0;
 #pragma unroll
             for (int i = 0; i < ROWS; ++i)
-                if (pos[i] >= j) {
+                {
                     const float v = fabsf(pr[i][j]);
                     const uint32_t k = (v == v) ? __float_as_uint(v) : 0u;
-                    if (at == 0xffffffffu || k > key || (k == key && (uint32_t)pos[i] < at)) { key = k; at = pos[i]; bi = i; }
+                    const bool better = pos[i] >= j && (at == 0xffffffffu || k > key || (k == key && (uint32_t)pos[i] < at));
+                    key = better ? k : key;
+                    at = better ? (uint32_t)pos[i] : at;
+                    bi = better ? i : bi;
                 }
             const uint32_t wk = __reduce_max_sync(0xffffffffu, key);
             const uint32_t wa = __reduce_min_sync(0xffffffffu, key == wk ? at : 0xffffffffu);
-            if (wa == 0xffffffffu ? lane == 0 : at == wa) {
-                float* my = cb + wid * TC_CAND_LD;
-                *reinterpret_cast<uint2*>(my + TC_NB) = make_uint2(wk, wa);
+            const bool mine = wa == 0xffffffffu ? lane == 0 : at == wa;
+            const uint32_t my = smem_u32(cb + wid * TC_CAND_LD);
+            put_if(mine, my + TC_NB * 4, wk, wa);
 #pragma unroll
-                for (int i = 0; i < ROWS; ++i)
-                    if (i == bi) {
+            for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-                        for (int c = (j & ~3); c < TC_NB; c += 4)
-                            *reinterpret_cast<float4*>(my + c) = make_float4(pr[i][c], pr[i][c + 1], pr[i][c + 2], pr[i][c + 3]);
-                    }
-            }
+                for (int c = (j & ~3); c < TC_NB; c += 4)
+                    put_if(mine && i == bi, my + c * 4, pr[i][c], pr[i][c + 1], pr[i][c + 2], pr[i][c + 3]);
             __syncthreads();
             // the same winner in every thread
             const uint2 o = (lane < NT / 32) ? *reinterpret_cast<const uint2*>(cb + lane * TC_CAND_LD + TC_NB)
@@ -249,18 +273,15 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
                 pv[c] = v.x; pv[c + 1] = v.y; pv[c + 2] = v.z; pv[c + 3] = v.w;
             }
             const float d = pv[j];
-            if (!(d != 0.f) && inf == 0) inf = k0 + j + 1;
-            const float inv = (d != 0.f) ? __frcp_rn(d) : 0.f;
+            inf = (!(d != 0.f) && inf == 0) ? k0 + j + 1 : inf;
+            const float inv = recip_or_0(d);
 #pragma unroll
             for (int i = 0; i < ROWS; ++i) {
-                if (pos[i] == (int)S) pos[i] = j;
-                else if (pos[i] == j) pos[i] = (int)S;
-                if (pos[i] > j) {
-                    const float l = pr[i][j] * inv;
-                    pr[i][j] = l;
+                pos[i] = pos[i] == (int)S ? j : (pos[i] == j ? (int)S : pos[i]);
+                const float l = pos[i] > j ? pr[i][j] * inv : 0.f;
+                pr[i][j] = pos[i] > j ? l : pr[i][j];
 #pragma unroll
-                    for (int c = j + 1; c < TC_NB; ++c) pr[i][c] -= l * pv[c];
-                }
+                for (int c = j + 1; c < TC_NB; ++c) pr[i][c] -= l * pv[c];
             }
         }
         // write the panel back (each position's data returns to its own stored row), the positions
@@ -279,6 +300,7 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
                     if (c < ncol) dst[c] = pr[i][c];
             }
             perm[k0 + pos[i]] = row[i];
+            roff[k0 + pos[i]] = row[i] * ld;
             if (pos[i] < TC_NB) {
 #pragma unroll
                 for (int c = 0; c < TC_NB; ++c) L11[c * TC_L11_LD + pos[i]] = pr[i][c];
@@ -292,7 +314,7 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
         for (int c = tid; c < ncols; c += NT) {
             float x[TC_NB];
 #pragma unroll
-            for (int j = 0; j < TC_NB; ++j) x[j] = a[(size_t)perm[k0 + j] * ld + k0 + TC_NB + c];
+            for (int j = 0; j < TC_NB; ++j) x[j] = a[roff[k0 + j] + k0 + TC_NB + c];
 #pragma unroll
             for (int i = 0; i < TC_NB; ++i) {
                 // keeps the compiler from hoisting all 496 multipliers into registers
@@ -307,7 +329,7 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
                 for (int j = i + 1; j < TC_NB; ++j) x[j] -= lc[j] * x[i];
             }
 #pragma unroll
-            for (int j = 0; j < TC_NB; ++j) a[(size_t)perm[k0 + j] * ld + k0 + TC_NB + c] = x[j];
+            for (int j = 0; j < TC_NB; ++j) a[roff[k0 + j] + k0 + TC_NB + c] = x[j];
         }
         if (nrows <= 0) break;  // last panel
         __syncthreads();
@@ -317,44 +339,63 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
         const uint32_t idesc = idesc_tf32(TC_TM, th);
         for (int g0 = 0; g0 < nrows; g0 += th) {
             // B operand: L21 rows g0.., K = the panel's 32 columns
-            for (int e = tid; e < th * (TC_NB / 4); e += NT) {
-                const int r = e >> 3, k = (e & 7) * 4;
-                float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
-                if (g0 + r < nrows) {
-                    const float* row = a + (size_t)perm[k0 + TC_NB + g0 + r] * ld + k0 + k;
-                    if (vec4) {
-                        float4 v = *reinterpret_cast<const float4*>(row);
-                        v0 = v.x; v1 = v.y; v2 = v.z; v3 = v.w;
-                    } else {
-                        v0 = row[0]; v1 = row[1]; v2 = row[2]; v3 = row[3];
+            // Groups of rows are loaded together, 8 lanes on consecutive rows: their 16-byte stores
+            // fill one core matrix.
+            const int br = (tid & 7) + (tid >> 6) * 8, bk = ((tid >> 3) & 7) * 4;
+#pragma unroll 1
+            for (int rb = br; rb < th; rb += 3 * (NT / 8)) {
+                float4 bv[3];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const int r = rb + i * (NT / 8);
+                    bv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (r < th && g0 + r < nrows) {
+                        const float* src = a + roff[k0 + TC_NB + g0 + r] + k0 + bk;
+                        if (vec4) bv[i] = *reinterpret_cast<const float4*>(src);
+                        else bv[i] = make_float4(src[0], src[1], src[2], src[3]);
                     }
                 }
-                put_split4(sm + SM_B_HI, r, k, v0, v1, v2, v3, TC_TILEX_BYTES);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const int r = rb + i * (NT / 8);
+                    if (r < th) put_split4(sm + SM_B_HI, r, bk, bv[i].x, bv[i].y, bv[i].z, bv[i].w, TC_TILEX_BYTES);
+                }
             }
             for (int c0 = 0; c0 < ncols; c0 += TC_TM) {
-                // warp w updates the columns of TMEM lanes 32 (w % 4).. in its share of the rows:
-                // all of the tile's with 4 warps, half with 8. Its first 16 TC_PRE rows are read
-                // here, ahead of the product.
+                // A operand: U12^T, row m = column c0 + m of U12, k = pivot row; and the warp's first
+                // 16 TC_PRE rows of A22, read ahead of the product. Warp w updates the columns of
+                // TMEM lanes 32 (w % 4).. in its share of the rows: all of the tile's with 4
+                // warps, half with 8.
+                constexpr int AI = TC_TM * (TC_NB / 4) / NT;
+                const int am = tid & (TC_TM - 1);
+                const float* ap = a + k0 + TC_NB + min(c0 + am, ncols - 1);
+                float av[AI][4];
+#pragma unroll
+                for (int i = 0; i < AI; ++i) {
+                    const int4 ro = *reinterpret_cast<const int4*>(roff + k0 + ((tid >> 7) + i * (NT / TC_TM)) * 4);
+                    av[i][0] = ap[ro.x]; av[i][1] = ap[ro.y]; av[i][2] = ap[ro.z]; av[i][3] = ap[ro.w];
+                }
                 const int wq = wid & 3, rh = th / (NT / 128), rw = g0 + rh * (wid >> 2);
                 const bool colok = (c0 + 32 * wq + lane) < ncols;
-                float* colp = a + k0 + TC_NB + c0 + 32 * wq + lane;
-                const int* rperm = perm + k0 + TC_NB + rw;
+                float* colp = a + k0 + TC_NB + min(c0 + 32 * wq + lane, ncols - 1);
+                const int* ro = roff + k0 + TC_NB + rw;
                 const int nr = min(rh, nrows - rw);  // rows of this warp (none if <= 0)
-                float old[TC_PRE][16];
+                float old[TC_PRE][16] = {};
+                auto ahead = [&](int u, float (&x)[16]) {  // 16 rows of A22 (row 0 past the last one)
+#pragma unroll
+                    for (int t = 0; t < 16; t += 4) {
+                        const int4 r4 = *reinterpret_cast<const int4*>(ro + u * 16 + t);
+                        x[t] = colp[r4.x]; x[t + 1] = colp[r4.y]; x[t + 2] = colp[r4.z]; x[t + 3] = colp[r4.w];
+                    }
+                };
 #pragma unroll
                 for (int u = 0; u < TC_PRE; ++u)
+                    if (u * 16 < nr) ahead(u, old[u]);
 #pragma unroll
-                    for (int t = 0; t < 16; ++t)
-                        old[u][t] = (colok && u * 16 + t < nr) ? colp[(size_t)rperm[u * 16 + t] * ld] : 0.f;
-                // A operand: U12^T, row m = column c0 + m of U12, k = pivot row
-                for (int e = tid; e < TC_TM * (TC_NB / 4); e += NT) {
-                    const int m = e & (TC_TM - 1), k = (e >> 7) * 4;
-                    float v[4] = {0.f, 0.f, 0.f, 0.f};
-                    if (c0 + m < ncols) {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) v[q] = a[(size_t)perm[k0 + k + q] * ld + k0 + TC_NB + c0 + m];
-                    }
-                    put_split4(sm + SM_A_HI, m, k, v[0], v[1], v[2], v[3]);
+                for (int i = 0; i < AI; ++i) {
+                    const int k = ((tid >> 7) + i * (NT / TC_TM)) * 4;
+                    if (c0 + am < ncols) put_split4(sm + SM_A_HI, am, k, av[i][0], av[i][1], av[i][2], av[i][3]);
+                    else put_split4(sm + SM_A_HI, am, k, 0.f, 0.f, 0.f, 0.f);
                 }
                 fence_async_smem();
                 tc_fence_before();
@@ -380,31 +421,24 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
                 tc_fence_after();
                 if (s_fault) break;
                 const uint32_t trow = tbase + ((uint32_t)(32 * wq) << 16) + (uint32_t)(rw - g0);
-#pragma unroll
-                for (int u = 0; u < TC_PRE; ++u) {
-                    if (u * 16 >= nr) break;  // warp-uniform
-                    float dv[16];
-                    tmem_ld16(trow + u * 16, dv);
-#pragma unroll
-                    for (int t = 0; t < 16; ++t)
-                        if (colok && u * 16 + t < nr) colp[(size_t)rperm[u * 16 + t] * ld] = old[u][t] - dv[t];
-                }
 #pragma unroll 1
-                for (int r0 = TC_PRE * 16; r0 < nr; r0 += 32) {
-                    float ov[2][16];
+                for (int u0 = 0; u0 * 16 < nr; u0 += TC_PRE) {
 #pragma unroll
-                    for (int u = 0; u < 2; ++u)
-#pragma unroll
-                        for (int t = 0; t < 16; ++t)
-                            ov[u][t] = (colok && r0 + u * 16 + t < nr) ? colp[(size_t)rperm[r0 + u * 16 + t] * ld] : 0.f;
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        if (r0 + u * 16 >= nr) break;
+                    for (int v = 0; v < TC_PRE; ++v) {
+                        const int u = u0 + v;
+                        if (u * 16 >= nr) break;  // warp-uniform
                         float dv[16];
-                        tmem_ld16(trow + r0 + u * 16, dv);
+                        tmem_ld16(trow + u * 16, dv);
 #pragma unroll
-                        for (int t = 0; t < 16; ++t)
-                            if (colok && r0 + u * 16 + t < nr) colp[(size_t)rperm[r0 + u * 16 + t] * ld] = ov[u][t] - dv[t];
+                        for (int t = 0; t < 16; t += 4) {
+                            const int4 r4 = *reinterpret_cast<const int4*>(ro + u * 16 + t);
+                            const int n4 = colok ? nr - u * 16 - t : 0;
+                            if (n4 > 0) colp[r4.x] = old[v][t] - dv[t];
+                            if (n4 > 1) colp[r4.y] = old[v][t + 1] - dv[t + 1];
+                            if (n4 > 2) colp[r4.z] = old[v][t + 2] - dv[t + 2];
+                            if (n4 > 3) colp[r4.w] = old[v][t + 3] - dv[t + 3];
+                        }
+                        if ((u + TC_PRE) * 16 < nr) ahead(u + TC_PRE, old[v]);
                     }
                 }
                 tc_fence_before();
