@@ -1975,8 +1975,8 @@ static int lu_kernel_for(int requested, int N) {
     return (requested >= 0 && requested <= 5) ? requested : 0;
 }
 
-// FP64 factorization kernel (bte_solve_opts.lu64_kernel): the split kernel unless the one-CTA
-// kernel is asked for. A point's arithmetic does not depend on how many points share a launch
+// FP64 factorization kernel (bte_solve_opts.lu64_kernel): a matrix per cluster or split over many CTAs
+// (the same operations in the same order) unless the one-CTA kernel is asked for. A point's arithmetic does not depend on how many points share a launch
 // with either kernel.
 static int lu64_kernel_for(int requested) { return requested == 1 ? 1 : 6; }
 
