@@ -394,6 +394,7 @@ struct Bte1d {
     double* Kr = nullptr;  // Krylov basis, (restart + 1) vectors
     int kcap = 0;
     double *part = nullptr, *hd = nullptr;
+    double* hp = nullptr;  // pinned: what the reductions gave
     double* Vt = nullptr;  // ordinates scratch
     double* Vt2 = nullptr;
     // fully implicit step: adv_x transposed, D transposed, and the ordinates-space GMRES buffers
@@ -435,6 +436,8 @@ static int alloc1d(Bte1d* h, void** p, size_t bytes) {
 static void free1d(Bte1d* h) {
     for (void* p : h->allocs) cudaFree(p);
     h->allocs.clear();
+    cudaFreeHost(h->hp);
+    h->hp = nullptr;
 }
 
 extern "C" {
@@ -476,6 +479,10 @@ int bte1d_create(int device, int Nr, int nsh, int Nvt, int Nx, const double* Q, 
     A((void**)&h->Xs, nu * 8); A((void**)&h->T, nu * 8); A((void**)&h->Zf, nu * 4);
     A((void**)&h->Kr, (size_t)(restart + 1) * nu * 8);
     A((void**)&h->part, (size_t)(restart + 1) * RED_BLOCKS * 8); A((void**)&h->hd, (size_t)(restart + 1) * 8);
+    if (rc == BTE_OK && cudaMallocHost((void**)&h->hp, (size_t)(2 * (restart + 1) + 1) * 8) != cudaSuccess) {
+        g_err1d = "host allocation failed";
+        rc = BTE_ERR_ALLOC;
+    }
     A((void**)&h->Vt, nv * 8);
     A((void**)&h->Vt2, nv * 8);
     A((void**)&h->AxT, (size_t)Nr * Nr * 8); A((void**)&h->DT, (size_t)Nx * Nx * 8);
@@ -601,13 +608,18 @@ int bte1d_step_v(Bte1d* h, double dt, const double* E, double* V, double rtol, d
         L += 3;
         return e;
     };
-    auto dots = [&](int k, const double* Vb, const double* w, double* host_out) -> cudaError_t {
+    // k products into hd, and from there to pinned memory
+    auto queue_dots = [&](int k, const double* Vb, const double* w, double* pinned) -> cudaError_t {
         k_dots_partial<<<dim3(RED_BLOCKS, k), 256, 0, s>>>(N, k, Vb, N, w, h->part);
         k_dots_final<<<k, 256, 0, s>>>(k, RED_BLOCKS, h->part, h->hd);
         L += 2;
-        cudaError_t e = cudaMemcpyAsync(host_out, h->hd, k * 8, cudaMemcpyDeviceToHost, s);
-        if (e != cudaSuccess) return e;
-        return cudaStreamSynchronize(s);
+        return cudaMemcpyAsync(pinned, h->hd, k * 8, cudaMemcpyDeviceToHost, s);
+    };
+    auto dots = [&](int k, const double* Vb, const double* w, double* host_out) -> cudaError_t {
+        cudaError_t e = queue_dots(k, Vb, w, h->hp);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) std::copy(h->hp, h->hp + k, host_out);
+        return e;
     };
     // right-hand side U = P_o2sh V, and the per-point FP32 block factors
     k_ords_to_lm<<<nb(N, 256), 256, 0, s>>>(h->Nr, h->Nvt, h->nsh, Nx, h->Ps, V, h->U, nullptr);
@@ -626,7 +638,7 @@ int bte1d_step_v(Bte1d* h, double dt, const double* E, double* V, double rtol, d
     int it = 0;
     double rnorm = 0.0;
     bool conv = false;
-    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), hh(m + 1), y(m);
+    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m);
     while (true) {
         lmat(h->Xs, h->W);
         k_sub<<<nb(N, 256), 256, 0, s>>>(N, h->U, h->W, h->R);
@@ -645,17 +657,20 @@ int bte1d_step_v(Bte1d* h, double dt, const double* E, double* V, double rtol, d
             double* vk1 = h->Kr + (size_t)(k + 1) * N;
             CK1(precond(vk, h->Z));
             lmat(h->Z, vk1);
-            // classical Gram-Schmidt, applied twice
+            // classical Gram-Schmidt, applied twice: the combinations take their coefficients from hd,
+            // where the products left them, and the host waits once (it waited for each of the
+            // three reductions and sent the coefficients back)
+            double* hp1 = h->hp + m + 1;
+            double* hp2 = hp1 + m + 1;
             for (int pass = 0; pass < 2; ++pass) {
-                CK1(dots(k + 1, h->Kr, vk1, hh.data()));
-                CK1(cudaMemcpyAsync(h->hd, hh.data(), (k + 1) * 8, cudaMemcpyHostToDevice, s));
+                CK1(queue_dots(k + 1, h->Kr, vk1, pass == 0 ? h->hp : hp1));
                 k_sub_combo<<<nb(N, 256), 256, 0, s>>>(N, k + 1, h->Kr, N, h->hd, vk1);
                 ++L;
-                for (int j = 0; j <= k; ++j) H[(size_t)j * m + k] = (pass == 0 ? 0.0 : H[(size_t)j * m + k]) + hh[j];
             }
-            double nn = 0.0;
-            CK1(dots(1, vk1, vk1, &nn));
-            nn = std::sqrt(nn);
+            CK1(queue_dots(1, vk1, vk1, hp2));
+            CK1(cudaStreamSynchronize(s));
+            for (int j = 0; j <= k; ++j) H[(size_t)j * m + k] = h->hp[j] + hp1[j];
+            const double nn = std::sqrt(*hp2);
             H[(size_t)(k + 1) * m + k] = nn;
             if (nn > 0) { k_scale<<<nb(N, 256), 256, 0, s>>>(N, 1.0 / nn, vk1, vk1); ++L; }
             // Givens rotations on column k
@@ -810,13 +825,18 @@ int bte1d_step_fim(Bte1d* h, double dt, const double* E, double* V, double rtol,
         }
         return BTE_OK;
     };
-    auto dots = [&](int k, const double* Vb, const double* w, double* host_out) -> cudaError_t {
+    // k products into hd, and from there to pinned memory
+    auto queue_dots = [&](int k, const double* Vb, const double* w, double* pinned) -> cudaError_t {
         k_dots_partial<<<dim3(RED_BLOCKS, k), 256, 0, s>>>(N, k, Vb, N, w, h->Fpart);
         k_dots_final<<<k, 256, 0, s>>>(k, RED_BLOCKS, h->Fpart, h->hd);
         L += 2;
-        cudaError_t e = cudaMemcpyAsync(host_out, h->hd, k * 8, cudaMemcpyDeviceToHost, s);
-        if (e != cudaSuccess) return e;
-        return cudaStreamSynchronize(s);
+        return cudaMemcpyAsync(pinned, h->hd, k * 8, cudaMemcpyDeviceToHost, s);
+    };
+    auto dots = [&](int k, const double* Vb, const double* w, double* host_out) -> cudaError_t {
+        cudaError_t e = queue_dots(k, Vb, w, h->hp);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) std::copy(h->hp, h->hp + k, host_out);
+        return e;
     };
     // b = V with the inflow values set to 0 (the boundary condition); x0 = P^-1 b
     k_copy_zero_inflow<<<nb(N, 256), 256, 0, s>>>(Nr, Nvt, Nx, h->right, V, h->Fb);
@@ -829,7 +849,7 @@ int bte1d_step_fim(Bte1d* h, double dt, const double* E, double* V, double rtol,
     int it = 0;
     double rnorm = 0.0;
     bool conv = false;
-    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), hh(m + 1), y(m);
+    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m);
     while (true) {
         if (int rc = fim_matvec(h, dt, E, h->Fx, h->Fw, s)) return rc;
         k_sub<<<nb(N, 256), 256, 0, s>>>(N, h->Fb, h->Fw, h->Fr);
@@ -848,16 +868,20 @@ int bte1d_step_fim(Bte1d* h, double dt, const double* E, double* V, double rtol,
             double* vk1 = h->Fk + (size_t)(k + 1) * N;
             if (int rc = precond(vk, h->Fz)) return rc;
             if (int rc = fim_matvec(h, dt, E, h->Fz, vk1, s)) return rc;
-            for (int pass = 0; pass < 2; ++pass) {  // classical Gram-Schmidt, applied twice
-                CK1(dots(k + 1, h->Fk, vk1, hh.data()));
-                CK1(cudaMemcpyAsync(h->hd, hh.data(), (k + 1) * 8, cudaMemcpyHostToDevice, s));
+            // classical Gram-Schmidt, applied twice: the combinations take their coefficients from hd,
+            // where the products left them, and the host waits once (it waited for each of the
+            // three reductions and sent the coefficients back)
+            double* hp1 = h->hp + m + 1;
+            double* hp2 = hp1 + m + 1;
+            for (int pass = 0; pass < 2; ++pass) {
+                CK1(queue_dots(k + 1, h->Fk, vk1, pass == 0 ? h->hp : hp1));
                 k_sub_combo<<<nb(N, 256), 256, 0, s>>>(N, k + 1, h->Fk, N, h->hd, vk1);
                 ++L;
-                for (int j = 0; j <= k; ++j) H[(size_t)j * m + k] = (pass == 0 ? 0.0 : H[(size_t)j * m + k]) + hh[j];
             }
-            double nn = 0.0;
-            CK1(dots(1, vk1, vk1, &nn));
-            nn = std::sqrt(nn);
+            CK1(queue_dots(1, vk1, vk1, hp2));
+            CK1(cudaStreamSynchronize(s));
+            for (int j = 0; j <= k; ++j) H[(size_t)j * m + k] = h->hp[j] + hp1[j];
+            const double nn = std::sqrt(*hp2);
             H[(size_t)(k + 1) * m + k] = nn;
             if (nn > 0) { k_scale<<<nb(N, 256), 256, 0, s>>>(N, 1.0 / nn, vk1, vk1); ++L; }
             for (int j = 0; j < k; ++j) {  // Givens rotations on column k

@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <cmath>
 #include <string>
 #include <vector>
@@ -51,6 +52,7 @@ struct bte_fvm {
     double* Kr = nullptr;
     int kcap = 0;
     double *part = nullptr, *hd = nullptr;
+    double* hp = nullptr;  // pinned: what the reductions gave
     double *xg = nullptr, *vrp = nullptr, *vta = nullptr;   // semi-Lagrangian grids (set once)
     double sl_vmin = 0.0;
     bool have_sl = false;
@@ -679,26 +681,48 @@ struct DeviceOps {
             return fvm_fail(BTE_ERR_CUDA, "copy failed");
         return BTE_OK;
     }
-    int dots(int k, const double* V, const double* w, double* out) {
+    // k products into hd, and from there to pinned memory
+    int queue_dots(int k, const double* V, const double* w, double* pinned) {
         k_fvm_dots_partial<<<dim3(FVM_RED, k), FT, 0, s>>>(N, V, w, h->part);
         k_fvm_dots_final<<<k, FT, 0, s>>>(FVM_RED, h->part, h->hd);
         h->launches += 2;
         if (int rc = launched("dots")) return rc;
-        if (cudaMemcpyAsync(out, h->hd, (size_t)k * 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess)
+        if (cudaMemcpyAsync(pinned, h->hd, (size_t)k * 8, cudaMemcpyDeviceToHost, s) != cudaSuccess)
             return fvm_fail(BTE_ERR_CUDA, "dots: copy to the host failed");
+        return BTE_OK;
+    }
+    int wait() {
+        return cudaStreamSynchronize(s) == cudaSuccess ? BTE_OK : fvm_fail(BTE_ERR_CUDA, "dots: copy to the host failed");
+    }
+    int dots(int k, const double* V, const double* w, double* out) {
+        if (int rc = queue_dots(k, V, w, h->hp)) return rc;
+        if (int rc = wait()) return rc;
+        std::copy(h->hp, h->hp + k, out);
+        return BTE_OK;
+    }
+    // Both passes of Gram-Schmidt and the norm queued at once: the combinations take their
+    // coefficients from hd, where the products left them, and the host waits once (it waited for
+    // each of the three reductions and sent the coefficients back).
+    int orthogonalize(int k, double* w, double* h0, double* h1, double* ww) {
+        double* hp1 = h->hp + h->kcap + 1;
+        double* hp2 = hp1 + h->kcap + 1;
+        for (int pass = 0; pass < 2; ++pass) {
+            if (int rc = queue_dots(k, Kr, w, pass == 0 ? h->hp : hp1)) return rc;
+            k_fvm_sub_combo<<<fblocks(N), FT, 0, s>>>(N, k, Kr, h->hd, w);
+            ++h->launches;
+            if (int rc = launched("sub_combo")) return rc;
+        }
+        if (int rc = queue_dots(1, w, w, hp2)) return rc;
+        if (int rc = wait()) return rc;
+        std::copy(h->hp, h->hp + k, h0);
+        std::copy(hp1, hp1 + k, h1);
+        *ww = *hp2;
         return BTE_OK;
     }
     int to_device(int k, const double* host) {
         if (cudaMemcpyAsync(h->hd, host, (size_t)k * 8, cudaMemcpyHostToDevice, s) != cudaSuccess)
             return fvm_fail(BTE_ERR_CUDA, "coefficient copy failed");
         return BTE_OK;
-    }
-    int sub_combo(int k, const double* V, const double* hh, double* w) {
-        if (int rc = to_device(k, hh)) return rc;
-        k_fvm_sub_combo<<<fblocks(N), FT, 0, s>>>(N, k, V, h->hd, w);
-        ++h->launches;
-        return launched("sub_combo");
     }
     int combo(int k, const double* V, const double* cc, double* y) {
         if (int rc = to_device(k, cc)) return rc;
@@ -825,6 +849,7 @@ int bte_fvm_destroy(bte_fvm* h) {
     cudaFree(h->Kr);   // the GMRES buffers, sized by the largest restart so far
     cudaFree(h->part);
     cudaFree(h->hd);
+    cudaFreeHost(h->hp);
     fvm_free(h);
     delete h;
     return BTE_OK;
@@ -943,23 +968,27 @@ int bte_fvm_step(bte_fvm* h, const bte_fvm_coef* c, double alpha, int pc_mode, c
     cudaStream_t s = (cudaStream_t)stream;
     const size_t N = h->N;
     if (restart > h->kcap) {
-        double *Kr = nullptr, *part = nullptr, *hd = nullptr;
+        double *Kr = nullptr, *part = nullptr, *hd = nullptr, *hp = nullptr;
         if (cudaMalloc((void**)&Kr, (size_t)(restart + 1) * N * 8) != cudaSuccess)
             return fvm_fail(BTE_ERR_ALLOC, "bte_fvm_step: Krylov basis allocation failed");
         if (cudaMalloc((void**)&part, (size_t)(restart + 1) * FVM_RED * 8) != cudaSuccess ||
-            cudaMalloc((void**)&hd, (size_t)(restart + 1) * 8) != cudaSuccess) {
+            cudaMalloc((void**)&hd, (size_t)(restart + 1) * 8) != cudaSuccess ||
+            cudaMallocHost((void**)&hp, (size_t)(2 * (restart + 1) + 1) * 8) != cudaSuccess) {
             cudaFree(Kr);
             cudaFree(part);
+            cudaFree(hd);
             return fvm_fail(BTE_ERR_ALLOC, "bte_fvm_step: reduction buffers allocation failed");
         }
         if (h->Kr) {
             cudaFree(h->Kr);
             cudaFree(h->part);
             cudaFree(h->hd);
+            cudaFreeHost(h->hp);
         }
         h->Kr = Kr;
         h->part = part;
         h->hd = hd;
+        h->hp = hp;
         h->kcap = restart;
     }
     const FvmCoef fc = coef_of(c);

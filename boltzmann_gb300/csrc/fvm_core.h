@@ -195,6 +195,24 @@ struct FvmGmresInfo {
     double rnorm, bnorm;
 };
 
+// Classical Gram-Schmidt of w against the first k vectors of Kr, applied twice: the coefficients
+// of both passes and w . w after them. Ops may supply it as a whole (orthogonalize), to hand the
+// coefficients from the products to the combination without the host in between.
+template <class Ops>
+auto fvm_orthogonalize(Ops& op, int k, double* w, double* h0, double* h1, double* ww, int)
+    -> decltype(op.orthogonalize(k, w, h0, h1, ww)) {
+    return op.orthogonalize(k, w, h0, h1, ww);
+}
+template <class Ops>
+int fvm_orthogonalize(Ops& op, int k, double* w, double* h0, double* h1, double* ww, long) {
+    for (int pass = 0; pass < 2; ++pass) {
+        double* hh = pass == 0 ? h0 : h1;
+        if (int rc = op.dots(k, op.Kr, w, hh)) return rc;
+        if (int rc = op.sub_combo(k, op.Kr, hh, w)) return rc;
+    }
+    return op.dots(1, w, w, ww);
+}
+
 template <class Ops>
 int fvm_gmres(Ops& op, int m, double rtol, double atol, int max_iter, FvmGmresInfo* info) {
     const size_t N = op.N;
@@ -207,7 +225,7 @@ int fvm_gmres(Ops& op, int m, double rtol, double atol, int max_iter, FvmGmresIn
     int it = 0;
     double rnorm = 0.0;
     bool conv = false;
-    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), hh(m + 1), y(m);
+    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), hh(m + 1), hh2(m + 1), y(m);
     while (true) {
         if ((rc = op.matvec(op.X, op.W))) return rc;
         if ((rc = op.sub(op.B, op.W, op.R))) return rc;
@@ -227,13 +245,9 @@ int fvm_gmres(Ops& op, int m, double rtol, double atol, int max_iter, FvmGmresIn
             double* vk1 = vk + N;
             if ((rc = op.precond(vk, op.Z))) return rc;
             if ((rc = op.matvec(op.Z, vk1))) return rc;
-            for (int pass = 0; pass < 2; ++pass) {
-                if ((rc = op.dots(k + 1, op.Kr, vk1, hh.data()))) return rc;
-                if ((rc = op.sub_combo(k + 1, op.Kr, hh.data(), vk1))) return rc;
-                for (int j = 0; j <= k; ++j) H[(size_t)j * m + k] = (pass == 0 ? 0.0 : H[(size_t)j * m + k]) + hh[j];
-            }
             double nn = 0.0;
-            if ((rc = op.dots(1, vk1, vk1, &nn))) return rc;
+            if ((rc = fvm_orthogonalize(op, k + 1, vk1, hh.data(), hh2.data(), &nn, 0))) return rc;
+            for (int j = 0; j <= k; ++j) H[(size_t)j * m + k] = hh[j] + hh2[j];
             nn = sqrt(nn);
             H[(size_t)(k + 1) * m + k] = nn;
             if (nn > 0.0 && (rc = op.scale(1.0 / nn, vk1, vk1))) return rc;
@@ -288,7 +302,7 @@ int fvm_gmres_left(Ops& op, int m, double rtol, double atol, int max_iter, FvmGm
     int it = 0;
     double rnorm = 0.0;
     bool conv = false;
-    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), hh(m + 1), y(m);
+    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), hh(m + 1), hh2(m + 1), y(m);
     auto solve_y = [&](int k) {
         for (int i = k - 1; i >= 0; --i) {
             double acc = g[i];
@@ -321,13 +335,9 @@ int fvm_gmres_left(Ops& op, int m, double rtol, double atol, int max_iter, FvmGm
             double* vk1 = vk + N;
             if ((rc = op.matvec(vk, op.W))) return rc;
             if ((rc = op.precond(op.W, vk1))) return rc;
-            for (int pass = 0; pass < 2; ++pass) {
-                if ((rc = op.dots(k + 1, op.Kr, vk1, hh.data()))) return rc;
-                if ((rc = op.sub_combo(k + 1, op.Kr, hh.data(), vk1))) return rc;
-                for (int j = 0; j <= k; ++j) H[(size_t)j * m + k] = (pass == 0 ? 0.0 : H[(size_t)j * m + k]) + hh[j];
-            }
             double nn = 0.0;
-            if ((rc = op.dots(1, vk1, vk1, &nn))) return rc;
+            if ((rc = fvm_orthogonalize(op, k + 1, vk1, hh.data(), hh2.data(), &nn, 0))) return rc;
+            for (int j = 0; j <= k; ++j) H[(size_t)j * m + k] = hh[j] + hh2[j];
             nn = sqrt(nn);
             H[(size_t)(k + 1) * m + k] = nn;
             if (nn > 0.0 && (rc = op.scale(1.0 / nn, vk1, vk1))) return rc;

@@ -1607,6 +1607,7 @@ struct BteWork {
     // P x nsh x kc_row(nsh) x nsp, written by k_ee_coef, read by the FP32 Jacobian and the refinement
     double* kc = nullptr;
     size_t kcbytes = 0;
+    int32_t* hcnt = nullptr;  // pinned: counters read by the host
     // GMRES refinement of stalled points (mixed form), gm_cap points at a time
     int gm_cap = 0;
     size_t gmbytes = 0;
@@ -1624,6 +1625,7 @@ static void free_work(BteWork* w) {
                     w->gm_sig, w->gm_xf, w->gm_list, w->gm_on, w->gm_cnt, w->piv, w->info, w->act, w->act2, w->cnt, w->searching, w->accepted};
     for (void* p : ptrs)
         if (p) cudaFree(p);
+    cudaFreeHost(w->hcnt);
     *w = BteWork();
 }
 
@@ -1698,7 +1700,8 @@ static int ensure_work(BteWork* w, const BteGrid* g, int P, int prec, int krylov
               A((void**)&w->piv, (size_t)P * N * sizeof(int32_t)) && A((void**)&w->info, P * sizeof(int32_t)) &&
               A((void**)&w->act, P * sizeof(int32_t)) && A((void**)&w->act2, P * sizeof(int32_t)) &&
               A((void**)&w->cnt, 4 * sizeof(int32_t)) && A((void**)&w->searching, P * sizeof(int32_t)) &&
-              A((void**)&w->accepted, P * sizeof(int32_t));
+              A((void**)&w->accepted, P * sizeof(int32_t)) &&
+              cudaMallocHost((void**)&w->hcnt, 4 * sizeof(int32_t)) == cudaSuccess;
     if (!ok) { free_work(w); return BTE_ERR_ALLOC; }
     w->cap = P; w->n = n; w->jbytes = jb; w->kcbytes = kb; w->prec = prec;
     w->gm_cap = gc; w->gmbytes = gmb;
@@ -2099,8 +2102,9 @@ static int newton_iteration(SolveCtx& c, Lane& L, int nact, int prec) {
                                                         w->ddm, w->ddpend);
             }));
             int hc = 0;
-            CKR(cudaMemcpyAsync(&hc, w->cnt, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+            CKR(cudaMemcpyAsync(w->hcnt, w->cnt, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
             CKR(cudaStreamSynchronize(s));
+            hc = w->hcnt[0];
             nsearch = hc;
             if (hc == 0) break;
         }
@@ -2116,8 +2120,9 @@ static int newton_iteration(SolveCtx& c, Lane& L, int nact, int prec) {
                                                       w->cnt, L.info, 0);
         }));
         int hn = 0;
-        CKR(cudaMemcpyAsync(&hn, w->cnt, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        CKR(cudaMemcpyAsync(w->hcnt, w->cnt, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         CKR(cudaStreamSynchronize(s));
+        hn = w->hcnt[0];
         pf.drain(s);
         std::swap(L.act, L.act2);
         nact = hn;
@@ -2174,8 +2179,9 @@ int bte_solve_impl(BteGrid* g, int P, const double* n0, const double* ne, const 
         CKR(cudaMemsetAsync(w->cnt, 0, sizeof(int32_t), s));
         CKR(other([&] { k_collect_failed<<<nblk(P, 256), 256, 0, s>>>(P, status, L.act2, w->cnt, w->reason); }));
         int nf = 0;
-        CKR(cudaMemcpyAsync(&nf, w->cnt, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        CKR(cudaMemcpyAsync(w->hcnt, w->cnt, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         CKR(cudaStreamSynchronize(s));
+        nf = w->hcnt[0];
         // FP64 chunks of as many matrices as the J buffer holds in FP64 (at least one)
         const int chunk = (int)std::min<size_t>((size_t)P, w->jbytes / ((size_t)c.N * c.ld * sizeof(double)));
         if (chunk < 1) return BTE_ERR_STATE;
@@ -2525,8 +2531,9 @@ int bte_engine_step_impl(BteEngine* e, int* n_done, int32_t* done_out, cudaStrea
         }));
     }
     int hc[4] = {0, 0, 0, 0};
-    CKR(cudaMemcpyAsync(hc, e->cnt, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    CKR(cudaMemcpyAsync(e->w.hcnt, e->cnt, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     CKR(cudaStreamSynchronize(s));
+    std::copy(e->w.hcnt, e->w.hcnt + 4, hc);
     const int nd = hc[0], nfb = hc[1], nsw = hc[2];
     if (nfb > 0) {
         std::vector<int32_t> fb(nfb);
@@ -2789,8 +2796,9 @@ int bte_transient_impl(BteGrid* g, int P, const double* n0, const double* ne, co
                                                                  w->refdone, w->act2, w->cnt);
             }));
             int hn = 0;
-            CKR(cudaMemcpyAsync(&hn, w->cnt, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+            CKR(cudaMemcpyAsync(w->hcnt, w->cnt, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
             CKR(cudaStreamSynchronize(s));
+            hn = w->hcnt[0];
             pf.drain(s);
             if (hn == 0) break;
             if (it >= o->max_iter) { failed = 1; break; }
