@@ -1825,20 +1825,25 @@ extern "C" int bte_stats(double* out, int count) {
     return BTE_OK;
 }
 
-// algorithmic work per point of each kernel family (flops; bytes moved to and from HBM)
+// algorithmic work per point of each kernel family (flops of the family's pipe: the mixed form's FP32
+// Coulomb product does not count towards the Jacobian's FP64 work; bytes moved to and from HBM)
 static double res_flops_pt(const BteGrid* g, int ee) {
     double n = g->n, nsp = g->nsp, tri = g->ntri;
     double f = 2.0 * (nsp * nsp * g->nspecies + n * 7 * 4 + n * nsp);  // collisions, bands, M^-1 F
-    if (ee) f += 2.0 * (2 * n * nsp) + 2.0 * 2.0 * nsp * tri * 49.0;   // potentials, trilinear form
+    if (ee) f += 2.0 * (2 * n * nsp) + 2.0 * 2.0 * nsp * tri * BTE_PAIRS;   // potentials, trilinear form
     return f;
 }
 static double res_bytes_pt(const BteGrid* g, bool trial) {
     double n = g->n;
     return 8.0 * n * (1 + 1 + 4) + (trial ? 8.0 * (n + 1) + 8.0 * n : 0.0);  // h, F, aux (+ dh, h_trial)
 }
-static double jac_flops_pt(const BteGrid* g, int ee) {
-    double n = g->n, N = n + 1;
-    return ee ? 2.0 * (14.0 * n * n) + 4.0 * N * N : 4.0 * N * N;
+static double jac_flops_pt(const BteGrid* g, int ee, int prec) {
+    double n = g->n, nsp = g->nsp, nsh = g->nsh, N = n + 1;
+    // the l = 0 block and the band, then the e-e coefficients
+    double f = 2.0 * (nsp * nsp * (g->nspecies + 3.0) + 7.0 * nsh * n * 3.0);
+    if (ee) f += 2.0 * 4.0 * BTE_PAIRS * g->ntri * nsp;
+    if (prec != BTE_PREC_MIXED) f += (ee ? 2.0 * (14.0 * n * n) : 0.0) + 2.0 * N * N;  // Coulomb product, equilibration
+    return f;
 }
 static double lu_flops(int N) { return (2.0 / 3.0) * (double)N * N * N + (double)N * N; }
 
@@ -2019,7 +2024,7 @@ static int newton_iteration(SolveCtx& c, Lane& L, int nact, int prec) {
         cudaError_t le = cudaSuccess;
         if (prec == BTE_PREC_MIXED) {
             float* xs = reinterpret_cast<float*>(L.xs);
-            CKR(pf.run(PF_JACOBIAN, s, nact * jac_flops_pt(g, ee), jb, L.kc && ee ? 2 : 1, [&] {
+            CKR(pf.run(PF_JACOBIAN, s, nact * jac_flops_pt(g, ee, prec), jb, L.kc && ee ? 2 : 1, [&] {
                 if (L.kc && ee) le = run_ee_coef(gv, nact, s, pp, ee, L.act, w->h, w->aux, L.kc);
                 if (le == cudaSuccess)
                     le = run_jacobian<float>(gv, nact, s, pp, ee, L.act, w->h, w->F, w->aux, w->scal, (float*)L.J, ld,
@@ -2066,7 +2071,7 @@ static int newton_iteration(SolveCtx& c, Lane& L, int nact, int prec) {
                 CKR(gmres_refine(c, L, nact, o->krylov == 2));
         } else {
             double* xs = L.xs;
-            CKR(pf.run(PF_JACOBIAN, s, nact * jac_flops_pt(g, ee), jb, 1, [&] {
+            CKR(pf.run(PF_JACOBIAN, s, nact * jac_flops_pt(g, ee, prec), jb, 1, [&] {
                 le = run_jacobian<double>(gv, nact, s, pp, ee, L.act, w->h, w->F, w->aux, w->scal, (double*)L.J, ld,
                                           jstride, beta_scale, L.rowscale, 1.0, 0.0, nullptr);
             }));
