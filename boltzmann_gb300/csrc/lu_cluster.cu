@@ -18,7 +18,7 @@
 //      update. Rows stay with their threads and only their positions change; the block is
 //      written to shared memory at the new positions and to A;
 //   2. every CTA, after the barrier, copies the block from the owner (distributed shared memory),
-//      moves the (at most 16) displaced rows of its own later columns, solves its U rows, writes
+//      moves the (at most 2 CL_NB) displaced rows of its own later columns, solves its U rows, writes
 //      them to A, and updates its columns: a warp takes 32 rows x CL_NB columns, L in registers,
 //      U broadcast. The next block's owner updates that block first and factors it while its
 //      other warps, and the other CTAs, are still updating: a CTA only arrives at the barrier
@@ -35,7 +35,12 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int CL_NB = 8;       // columns per block
+// Columns per block. The owner of the next block updates it alone before it factors it: with 8 columns
+// that and the panel's rank-one updates took 11.5 multiply-adds per row and column of the chain, with 4 they take
+// 5.5, against one more cluster barrier per 8 columns. Measured (us, 8 -> 4): N = 129: 1 matrix 217 -> 191,
+// 1000 matrices 2549 -> 2448; N = 385: 1 matrix 1068 -> 923. Finer blocks also let six CTAs hold N = 385
+// (16 matrices at once: 2072 -> 1425).
+constexpr int CL_NB = 4;
 constexpr int CL_NT = 256;     // threads per CTA
 constexpr int CL_NW = CL_NT / 32;
 constexpr size_t CL_SMEM_MAX = 220 * 1024;
@@ -342,16 +347,16 @@ cudaError_t launch_cluster(int P, int N, int NC, int C, double* A, int ld, long 
 // Model in microseconds, fitted to measured times (N = 33 to 513, 1 to 1200 matrices): a cluster
 // takes 1.4 N for the chain of columns plus its share of the multiply-adds, in waves of as many
 // clusters as the GPU holds at once (the occupancy interface's numbers for one CTA per SM; two
-// fit below 112 KB and then slow each other by 1.4); the split launches take 6.3 N plus 47 us
-// per matrix of N = 385. Measured (us, split / cluster): N = 129: 1 matrix 730 / 208, 1200
-// matrices 5678 / 2920; N = 257: 30 matrices 1855 / 715; N = 385: 15 matrices 2954 / 1133, 60
-// matrices 4753 / 4523, 150 matrices 8348 / 11347 (stays split); N = 513: 7 matrices 3988 / 2523,
-// 14 matrices 4595 / 5041 (stays split).
+// fit below 112 KB and then slow each other by 1.4); the split launches take 6.3 N plus 43 us
+// per matrix of N = 385. Measured (us, split / cluster): N = 129: 1 matrix 730 / 191, 1200 matrices
+// 5678 / 2920; N = 257: 30 matrices 1855 / 754; N = 385: 1 matrix 2600 / 928, 15 matrices 2954 / 1426,
+// 60 matrices 4753 / 4273, 137 matrices 7679 / 8595 (stays split); N = 513: 7 matrices 3988 /
+// 1690, 16 matrices 4586 / 5008 (stays split).
 int bte_lu_cluster_size(int P, int N, int NC) {
     if (N > 1024) return 0;
     const double n3 = (double)N * N * N;
     const double q = 1.0 + (100.0 / N) * (100.0 / N);
-    double best = 6.3 * N + P * q * n3 / 1.2e6;
+    double best = 6.3 * N + P * q * n3 / 1.43e6;
     int size = 0;
     struct Shape { int C, clusters; };
     constexpr Shape shapes[] = {{1, 152}, {2, 76}, {3, 46}, {4, 36}, {5, 28}, {6, 23}, {7, 15}, {8, 15}, {10, 13}, {16, 7}};
@@ -360,7 +365,7 @@ int bte_lu_cluster_size(int P, int N, int NC) {
         if (sm > CL_SMEM_MAX || (h.C - 1) * CL_NB >= N) continue;
         const bool two = sm <= 112 * 1024 && N <= 512;
         const int hold = two ? 2 * h.clusters : h.clusters;
-        double t = (h.C == 1 ? 2.0 : h.C == 16 ? 1.6 : 1.4) * N + n3 / (1.2e4 * h.C);
+        double t = (h.C == 1 ? 2.0 : h.C == 16 ? 1.75 : 1.4) * N + n3 / (1.1e4 * h.C);
         if (two && P > h.clusters) t *= 1.4;
         t *= (P + hold - 1) / hold;
         if (t < best) {
