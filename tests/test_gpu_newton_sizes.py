@@ -32,3 +32,21 @@ def test_point_does_not_depend_on_the_batch(synthetic_xs, n_sp, l_max, precision
         # coarse grids leave some points unconverged: they too end alike
         np.testing.assert_array_equal(st, ref[1][:P], err_msg="%d points" % P)
         np.testing.assert_array_equal(ff, ref[0][:, :P], err_msg="%d points" % P)
+
+
+@pytest.mark.parametrize("n_sp,l_max", [(20, 1), (47, 2)])
+def test_coefficients_of_several_points_per_cta(synthetic_xs, n_sp, l_max):
+    """From 608 points on, the e-e coefficients of two or four points are formed by one CTA (an odd
+    count leaves its last group partly empty): the same bits as for two points."""
+    from boltzmann_gb300.workloads import batch_parameters
+    prm = batch_parameters(2501, 78)
+    out = []
+    for P in (2, 701, 2501):
+        s, args = gpu_solver(synthetic_xs, n_sp, l_max, True, P, "mixed")
+        sub = {k: (v[..., :P] if np.ndim(v) > 1 else v[:P]) for k, v in prm.items() if np.ndim(v)}
+        ff, q = gpu_solution(s, args, sub, True, P)
+        out.append((np.asarray(ff), np.asarray(q["status"])))
+    for ff, st in out[:-1]:
+        np.testing.assert_array_equal(st, out[-1][1][:len(st)])
+        np.testing.assert_array_equal(ff, out[-1][0][:, :ff.shape[1]])
+    assert np.mean(out[-1][1] <= 1) > 0.5
