@@ -26,6 +26,7 @@
 #include <type_traits>
 #include <utility>
 #include "bte_common.cuh"
+#include "lu_solve_form.h"
 
 namespace {
 
@@ -640,8 +641,8 @@ cudaError_t factor_split(int P, int N, int NC, T* A, int ld, long long stride, i
 //    the loads of the next block are issued before its diagonal block is solved;
 //  * products stay as 8 partial sums per lane and are added over the lanes only when their
 //    rows' own diagonal block comes up (a transposing reduction, 7 shuffles for 32 rows);
-//  * the owner of a diagonal block only arrives at the barrier that publishes its x. It can be two
-//    blocks ahead of the other warps (FP64 owns two blocks in a row), hence four barriers in turn.
+//  * the owner of a diagonal block only arrives at the barrier that publishes its x, and can be all
+//    the blocks of its row group ahead of the other warps (lu_solve_form.h: the barriers in turn).
 // Measured (us, the row-oriented kernel with dependent loads and a division per column before ->
 // now): N = 385: FP32 160 -> 43 (137 matrices) and 1235 -> 705 (4096), FP64 333 -> 158
 // (16) and 3469 -> 2822 (4096); N = 769, 75 matrices: FP32 1137 -> 124; N = 129, 24 matrices: FP64
@@ -706,6 +707,7 @@ k_lu_solve(int N, const T* __restrict__ A, int ld, long long stride, const int32
            T* __restrict__ b, int mode, const int32_t* __restrict__ mats) {
     using V = typename SolveT<T, VEC>::V;
     constexpr int BW = 8 * VEC;
+    static_assert(32 / BW < SOLVE_BARRIERS, "an owner's barriers must not repeat before it waits");
     extern __shared__ __align__(16) unsigned char smraw[];
     const int np = (N + 31) & ~31;
     T* xs = reinterpret_cast<T*>(smraw);
@@ -843,17 +845,17 @@ k_lu_solve(int N, const T* __restrict__ A, int ld, long long stride, const int32
         for (int t = 0; t < nblk; ++t) {
             const int bk = upper ? nblk - 1 - t : t;
             const int grp = (bk * BW) / 32;
-            if (w == grp % NW) {
+            if (w == solve_owner(bk, BW, NW)) {
                 T yv = T(0);
                 static_for<ROWS>([&](auto ic) {
                     constexpr int i = decltype(ic)::value;
                     if (i == grp / NW) yv = y[i] - transpose_reduce8(part[i], lane);
                 });
                 diagonal(bk, yv, upper);
-                if (t + 1 < nblk) bar_arrive(1 + (t & 3), nt);
+                if (t + 1 < nblk) bar_arrive(solve_barrier(t), nt);
                 __syncwarp();
             } else if (t + 1 < nblk) {
-                bar_sync(1 + (t & 3), nt);
+                bar_sync(solve_barrier(t), nt);
             }
             if (t + 1 == nblk) break;
             const int bn = upper ? bk - 1 : bk + 1;
@@ -980,11 +982,13 @@ cudaError_t bte_lu_factor_t(int P, int N, int NC, T* A, int ld, long long stride
 }
 
 namespace {
-template <typename T, int VEC, int NTMAX, int OCC, int ROWS, bool PREF>
+template <typename T, int FORM, bool PREF>
 cudaError_t launch_solve(int P, int N, const T* A, int ld, long long stride, const int32_t* piv, T* b, int mode,
                          cudaStream_t s, const int32_t* mats) {
+    constexpr SolveForm F = SOLVE_FORMS[FORM];
+    constexpr int VEC = F.bytes / sizeof(T);
     const size_t sm = solve_smem_bytes<T, VEC>(N);
-    const int nt = 32 * (((N + 31) / 32 + ROWS - 1) / ROWS);  // as many warps as hold all row groups
+    const int nt = 32 * solve_warps(F, N);
     // 16-byte loads need rows that start on 16 bytes; the library's own matrices do
     const bool vec = ld % VEC == 0 && stride % VEC == 0 && ((uintptr_t)A & 15) == 0;
     auto run = [&](auto kernel) {
@@ -993,32 +997,24 @@ cudaError_t launch_solve(int P, int N, const T* A, int ld, long long stride, con
         kernel<<<P, nt, sm, s>>>(N, A, ld, stride, piv, b, mode, mats);
         return cudaGetLastError();
     };
-    return vec ? run(k_lu_solve<T, VEC, NTMAX, OCC, ROWS, PREF, true>)
-               : run(k_lu_solve<T, VEC, NTMAX, OCC, ROWS, PREF, false>);
+    return vec ? run(k_lu_solve<T, VEC, F.nt_max, F.occ, F.rows, PREF, true>)
+               : run(k_lu_solve<T, VEC, F.nt_max, F.occ, F.rows, PREF, false>);
 }
 }  // namespace
 
-// Row groups per warp by N and P. Few matrices (at most two per SM) are bound by the chain of
-// diagonal blocks: one group per warp, the next block's loads in registers (N = 385, 137
-// matrices: 43 us in FP32 against 55 with two groups per warp and loads when used). More
-// matrices than that hide one another's loads, and more resident CTAs pay: two groups per warp
-// without the prefetch registers (N = 385, 4096 matrices: 705 us against 984 in FP32, 2822
-// against 4161 in FP64). Up to N = 256 the prefetching form has one group per warp and two
-// CTAs per SM and is the faster one for any P (N = 129, 4096 matrices: 146 us against 163).
 template <typename T>
 cudaError_t bte_lu_solve_t(int P, int N, const T* A, int ld, long long stride, const int32_t* piv, T* b, int mode,
                            cudaStream_t s, const int32_t* mats) {
     if (P <= 0) return cudaSuccess;
     if ((long long)N * ld >= (1ll << 31)) return cudaErrorInvalidValue;  // row offsets are 32-bit
-    constexpr bool f32 = sizeof(T) == 4;
-    constexpr int VEC = 16 / sizeof(T);
-    if (N <= 256) return launch_solve<T, VEC, 256, 2, 1, true>(P, N, A, ld, stride, piv, b, mode, s, mats);
-    if (N <= 512 && P <= 304) return launch_solve<T, VEC, 512, 1, 1, true>(P, N, A, ld, stride, piv, b, mode, s, mats);
-    if (N <= 512) return launch_solve<T, VEC, 256, 3, 2, false>(P, N, A, ld, stride, piv, b, mode, s, mats);
-    if (N <= 1024) return launch_solve<T, VEC, 512, 1, 2, f32>(P, N, A, ld, stride, piv, b, mode, s, mats);
-    // above N = 1400 the diagonal blocks of 16-byte loads no longer fit in shared memory
-    if (N <= 1400) return launch_solve<T, VEC, 512, 1, 3, false>(P, N, A, ld, stride, piv, b, mode, s, mats);
-    return launch_solve<T, VEC / 2, 512, 1, 4, false>(P, N, A, ld, stride, piv, b, mode, s, mats);
+    switch (solve_form(P, N)) {
+        case 0: return launch_solve<T, 0, true>(P, N, A, ld, stride, piv, b, mode, s, mats);
+        case 1: return launch_solve<T, 1, true>(P, N, A, ld, stride, piv, b, mode, s, mats);
+        case 2: return launch_solve<T, 2, false>(P, N, A, ld, stride, piv, b, mode, s, mats);
+        case 3: return launch_solve<T, 3, sizeof(T) == 4>(P, N, A, ld, stride, piv, b, mode, s, mats);
+        case 4: return launch_solve<T, 4, false>(P, N, A, ld, stride, piv, b, mode, s, mats);
+        default: return launch_solve<T, 5, false>(P, N, A, ld, stride, piv, b, mode, s, mats);
+    }
 }
 
 template cudaError_t bte_lu_factor_t<double>(int, int, int, double*, int, long long, int32_t*, int32_t*, cudaStream_t, int);
