@@ -874,6 +874,76 @@ k_lu_solve(int N, const T* __restrict__ A, int ld, long long stride, const int32
     for (int i = tid; i < N; i += nt) bb[i] = xs[i];
 }
 
+// The same substitution row by row, for what the block form does not take: N above 2048, or rows so far
+// apart that their offsets do not fit 32 bits. Dependent loads and a division per column in one
+// warp: at the sizes that both take it is 2 to 9 times slower.
+template <typename T>
+__global__ void __launch_bounds__(LU_THREADS)
+k_lu_solve_rows(int N, const T* __restrict__ A, int ld, long long stride, const int32_t* __restrict__ perm,
+           T* __restrict__ b, int mode, const int32_t* __restrict__ mats) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    T* x = reinterpret_cast<T*>(smraw);
+    const int mat = mats ? mats[blockIdx.x] : (int)blockIdx.x;
+    const T* a = A + (size_t)mat * stride;
+    const int32_t* pm = perm + (size_t)mat * N;
+    T* bb = b + (size_t)blockIdx.x * N;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
+    if (mode == 1) {
+        for (int i = tid; i < N; i += nt) x[i] = a[(size_t)pm[i] * ld + N];
+        __syncthreads();
+    } else {
+        for (int i = tid; i < N; i += nt) x[i] = bb[pm[i]];
+        __syncthreads();
+        for (int r0 = 0; r0 < N; r0 += 32) {
+            const int rb = min(32, N - r0);
+            for (int i = wid; i < rb; i += nw) {
+                const T* row = a + (size_t)pm[r0 + i] * ld;
+                T s = T(0);
+                for (int c = lane; c < r0; c += 32) s += row[c] * x[c];
+                s = warp_sum(s);
+                if (lane == 0) x[r0 + i] -= s;
+            }
+            __syncthreads();
+            if (wid == 0) {
+                T xi = (lane < rb) ? x[r0 + lane] : T(0);
+                const T* rowl = a + (size_t)pm[r0 + min(lane, rb - 1)] * ld;
+                for (int j = 0; j < rb; ++j) {
+                    T xj = __shfl_sync(0xffffffffu, xi, j);
+                    if (lane > j && lane < rb) xi -= rowl[r0 + j] * xj;
+                }
+                if (lane < rb) x[r0 + lane] = xi;
+            }
+            __syncthreads();
+        }
+    }
+    for (int r1 = N; r1 > 0; r1 -= 32) {
+        const int r0 = max(0, r1 - 32), rb = r1 - r0;
+        for (int i = wid; i < rb; i += nw) {
+            const T* row = a + (size_t)pm[r0 + i] * ld;
+            T s = T(0);
+            for (int c = r1 + lane; c < N; c += 32) s += row[c] * x[c];
+            s = warp_sum(s);
+            if (lane == 0) x[r0 + i] -= s;
+        }
+        __syncthreads();
+        if (wid == 0) {
+            T xi = (lane < rb) ? x[r0 + lane] : T(0);
+            const T* rowl = a + (size_t)pm[r0 + min(lane, rb - 1)] * ld;
+            for (int j = rb - 1; j >= 0; --j) {
+                T d = a[(size_t)pm[r0 + j] * ld + r0 + j];
+                T xj = __shfl_sync(0xffffffffu, xi, j);
+                xj = (d != T(0)) ? xj / d : xj;
+                if (lane == j) xi = xj;
+                if (lane < j) xi -= rowl[r0 + j] * xj;
+            }
+            if (lane < rb) x[r0 + lane] = xi;
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < N; i += nt) bb[i] = x[i];
+}
+
 template <typename T, int RPT>
 cudaError_t launch_left(int P, int N, int NC, T* A, int ld, long long stride, int32_t* piv, int32_t* info,
                         cudaStream_t s) {
@@ -971,7 +1041,11 @@ cudaError_t bte_lu_factor_t(int P, int N, int NC, T* A, int ld, long long stride
         return bte_lu_factor_tc(P, N, NC, reinterpret_cast<float*>(A), ld, stride, piv, info, s, 0);
     }
     if constexpr (sizeof(T) == 4)
-        if (kernel == 0) return bte_lu_factor_tcs(P, N, NC, A, ld, stride, piv, info, s);
+        if (kernel == 0) {
+            // its row offsets are 32-bit; rows further apart than that take the right-looking kernel
+            if ((long long)N * ld < (1ll << 31)) return bte_lu_factor_tcs(P, N, NC, A, ld, stride, piv, info, s);
+            kernel = 1;
+        }
     if (kernel == 3) kernel = 0;
     if (kernel == 0 && N <= 128) return launch_left<T, 4>(P, N, NC, A, ld, stride, piv, info, s);
     if (kernel == 0 && N <= 256) return launch_left<T, 8>(P, N, NC, A, ld, stride, piv, info, s);
@@ -1006,7 +1080,13 @@ template <typename T>
 cudaError_t bte_lu_solve_t(int P, int N, const T* A, int ld, long long stride, const int32_t* piv, T* b, int mode,
                            cudaStream_t s, const int32_t* mats) {
     if (P <= 0) return cudaSuccess;
-    if ((long long)N * ld >= (1ll << 31)) return cudaErrorInvalidValue;  // row offsets are 32-bit
+    if (N > SOLVE_MAX_N || (long long)N * ld >= (1ll << 31)) {  // the block form's row offsets are 32-bit
+        const size_t sm = (size_t)N * sizeof(T);
+        cudaError_t e = bte_raise_smem_limit((const void*)k_lu_solve_rows<T>, sm);
+        if (e != cudaSuccess) return e;
+        k_lu_solve_rows<T><<<P, LU_THREADS, sm, s>>>(N, A, ld, stride, piv, b, mode, mats);
+        return cudaGetLastError();
+    }
     switch (solve_form(P, N)) {
         case 0: return launch_solve<T, 0, true>(P, N, A, ld, stride, piv, b, mode, s, mats);
         case 1: return launch_solve<T, 1, true>(P, N, A, ld, stride, piv, b, mode, s, mats);

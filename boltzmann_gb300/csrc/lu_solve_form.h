@@ -10,9 +10,9 @@ struct SolveForm {
 };
 constexpr SolveForm SOLVE_FORMS[] = {{16, 256, 2, 1}, {16, 512, 1, 1}, {16, 256, 3, 2},
                                      {16, 512, 1, 2}, {16, 512, 1, 3}, {8, 512, 1, 4}};
-constexpr int SOLVE_NFORMS = 6;
+constexpr int SOLVE_MAX_N = 2048;
 
-// The form for P matrices of size N (up to 2048). Few matrices (at most two per SM) are bound by the chain of
+// The form for P matrices of size N (up to SOLVE_MAX_N). Few matrices (at most two per SM) are bound by the chain of
 // diagonal blocks: one group per warp, the next block's loads in registers (N = 385, 137
 // matrices: 43 us in FP32 against 55 with two groups per warp and loads when used). More
 // matrices than that hide one another's loads, and more resident CTAs pay: two groups per warp

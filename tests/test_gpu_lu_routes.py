@@ -1,0 +1,72 @@
+"""The routes of the batched LU entry points: every size, row distance and batch they accept, and what must
+not depend on the route."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _ptr(t):
+    return C.c_void_p(t.data_ptr())
+
+
+def _stream():
+    import torch
+    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _backward_error(A, x, b):
+    import torch
+    A, x, b = A.double(), x.double(), b.double()
+    return float(torch.linalg.norm(A @ x - b)
+                 / (torch.linalg.matrix_norm(A, "fro") * torch.linalg.norm(x) + torch.linalg.norm(b)))
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("N", [2048, 2049, 2600])
+def test_solve_with_factors_above_the_factorization_size(N, dtype):
+    """bte_lu_solve with factors of the caller's own: it takes sizes above those of bte_lu_factor. Tolerance: the
+    bound 2 N eps of the other substitution tests, on the matrix that the factors multiply to."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    tdt = torch.float64 if dtype == "f64" else torch.float32
+    g = torch.Generator(device="cuda").manual_seed(N)
+    P = 2
+    M = torch.randn((P, N, N), device="cuda", generator=g, dtype=torch.float64)
+    LU = torch.linalg.lu_factor(M)[0].to(tdt)
+    perm = torch.stack([torch.randperm(N, device="cuda", generator=g) for _ in range(P)])
+    A = torch.empty((P, N, N), device="cuda", dtype=tdt)
+    for i in range(P):
+        A[i, perm[i]] = LU[i]
+    b = torch.randn((P, N), device="cuda", generator=g, dtype=tdt)
+    x, piv = b.clone(), perm.int().contiguous()
+    _lib.check(lib.bte_lu_solve(0 if dtype == "f64" else 1, P, N, _ptr(A), N, N * N, _ptr(piv), _ptr(x), _stream()),
+               "lu_solve")
+    torch.cuda.synchronize()
+    for i in range(P):
+        L = torch.tril(LU[i].double(), -1) + torch.eye(N, device="cuda", dtype=torch.float64)
+        err = _backward_error(L @ torch.triu(LU[i].double()), x[i], b[i][perm[i]])
+        assert err < 2 * N * torch.finfo(tdt).eps, (i, err)
+
+
+def test_rows_two_to_the_31_values_apart():
+    """FP32 factorization above N = 512 and substitution with N * ld above 2^31, where 32-bit row offsets end."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    N = 520
+    ld = ((1 << 31) // N + 8) & ~3
+    g = torch.Generator(device="cuda").manual_seed(N)
+    A0 = torch.randn((N, N), device="cuda", generator=g, dtype=torch.float32)
+    b = torch.randn(N, device="cuda", generator=g, dtype=torch.float32)
+    A = torch.empty(N * ld, device="cuda", dtype=torch.float32)
+    A.as_strided((N, N), (ld, 1)).copy_(A0)
+    piv, info, x = torch.empty(N, dtype=torch.int32, device="cuda"), torch.empty(1, dtype=torch.int32, device="cuda"), b.clone()
+    _lib.check(lib.bte_lu_factor(1, 1, N, _ptr(A), ld, N * ld, _ptr(piv), _ptr(info), _stream()), "lu_factor")
+    _lib.check(lib.bte_lu_solve(1, 1, N, _ptr(A), ld, N * ld, _ptr(piv), _ptr(x), _stream()), "lu_solve")
+    torch.cuda.synchronize()
+    assert int(info.item()) == 0
+    assert _backward_error(A0, x, b) < 2 * N * torch.finfo(torch.float32).eps
