@@ -21,6 +21,8 @@
 // (k_lu_tc in lu_tc.cu is the FP32 tensor-core kernel; k_lu_cluster in lu_cluster.cu keeps one
 // matrix in the shared memory of a thread-block cluster; k_lus_* below split one FP64
 // factorization over many CTAs by launches.)
+#include <climits>
+#include <cmath>
 #include <cstdint>
 #include <algorithm>
 #include <type_traits>
@@ -690,11 +692,88 @@ __device__ inline void bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// the exponent's bits, in their place
+__device__ inline int exponent_of(float v) { return __float_as_int(v) & 0x7f800000; }
+__device__ inline int exponent_of(double v) { return __double2hiint(v) & 0x7ff00000; }
+
 // x and the reciprocal diagonals padded to whole row groups, the diagonal blocks, perm
 template <typename T, int VEC>
 __host__ __device__ inline size_t solve_smem_bytes(int N) {
     const size_t np = (size_t)((N + 31) & ~31);
     return 2 * np * sizeof(T) + align16(np * (8 * VEC + 1) * sizeof(T)) + (size_t)N * 4;
+}
+
+// The same substitution row by row, with a division per column: x (N values of shared memory) and one matrix.
+template <typename T>
+__device__ __noinline__ void solve_rows(int N, const T* a, int ld, const int32_t* pm, T* bb, int mode, T* x) {
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
+    if (mode == 1) {
+        for (int i = tid; i < N; i += nt) x[i] = a[(size_t)pm[i] * ld + N];
+        __syncthreads();
+    } else {
+        for (int i = tid; i < N; i += nt) x[i] = bb[pm[i]];
+        __syncthreads();
+        for (int r0 = 0; r0 < N; r0 += 32) {
+            const int rb = min(32, N - r0);
+            for (int i = wid; i < rb; i += nw) {
+                const T* row = a + (size_t)pm[r0 + i] * ld;
+                T s = T(0);
+                for (int c = lane; c < r0; c += 32) s += row[c] * x[c];
+                s = warp_sum(s);
+                if (lane == 0) x[r0 + i] -= s;
+            }
+            __syncthreads();
+            if (wid == 0) {
+                T xi = (lane < rb) ? x[r0 + lane] : T(0);
+                const T* rowl = a + (size_t)pm[r0 + min(lane, rb - 1)] * ld;
+                for (int j = 0; j < rb; ++j) {
+                    T xj = __shfl_sync(0xffffffffu, xi, j);
+                    if (lane > j && lane < rb) xi -= rowl[r0 + j] * xj;
+                }
+                if (lane < rb) x[r0 + lane] = xi;
+            }
+            __syncthreads();
+        }
+    }
+    for (int r1 = N; r1 > 0; r1 -= 32) {
+        const int r0 = max(0, r1 - 32), rb = r1 - r0;
+        for (int i = wid; i < rb; i += nw) {
+            const T* row = a + (size_t)pm[r0 + i] * ld;
+            T s = T(0);
+            for (int c = r1 + lane; c < N; c += 32) s += row[c] * x[c];
+            s = warp_sum(s);
+            if (lane == 0) x[r0 + i] -= s;
+        }
+        __syncthreads();
+        if (wid == 0) {
+            T xi = (lane < rb) ? x[r0 + lane] : T(0);
+            const T* rowl = a + (size_t)pm[r0 + min(lane, rb - 1)] * ld;
+            for (int j = rb - 1; j >= 0; --j) {
+                T d = a[(size_t)pm[r0 + j] * ld + r0 + j];
+                T xj = __shfl_sync(0xffffffffu, xi, j);
+                xj = (d != T(0)) ? xj / d : xj;
+                if (lane == j) xi = xj;
+                if (lane < j) xi -= rowl[r0 + j] * xj;
+            }
+            if (lane < rb) x[r0 + lane] = xi;
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < N; i += nt) bb[i] = x[i];
+}
+
+// For what the block form does not take: N above 2048, or rows so far apart that their offsets do not fit 32 bits.
+// Dependent loads and a division per column in one warp: at the sizes that both take it is 2 to 9
+// times slower.
+template <typename T>
+__global__ void __launch_bounds__(LU_THREADS)
+k_lu_solve_rows(int N, const T* __restrict__ A, int ld, long long stride, const int32_t* __restrict__ perm,
+                T* __restrict__ b, int mode, const int32_t* __restrict__ mats) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int mat = mats ? mats[blockIdx.x] : (int)blockIdx.x;
+    solve_rows(N, A + (size_t)mat * stride, ld, perm + (size_t)mat * N, b + (size_t)blockIdx.x * N, mode,
+               reinterpret_cast<T*>(smraw));
 }
 
 // Row groups of 32 rows: group w + i * NW belongs to warp w, i < ROWS (NW warps, runtime).
@@ -769,6 +848,7 @@ k_lu_solve(int N, const T* __restrict__ A, int ld, long long stride, const int32
         return upper ? base < bk * BW : (base + 31 >= (bk + 1) * BW && base < N);
     };
     const int first = mode == 1 ? nblk - 1 : 0;
+    int top = 0;  // the largest exponent of the scaled values and the diagonals, in place
     static_for<ROWS>([&](auto ic) {
         constexpr int i = decltype(ic)::value;
         const int base = 32 * (w + i * NW);
@@ -790,13 +870,18 @@ k_lu_solve(int N, const T* __restrict__ A, int ld, long long stride, const int32
         const T inv = (dd != T(0)) ? T(1) / dd : T(1);
         sinv[r] = inv;
         __syncwarp();
+        top = max(top, exponent_of(inv) == 0 ? INT_MAX : exponent_of(inv));
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int q = base + 4 * k + g;
             const T sc = sinv[q];
 #pragma unroll
             for (int e = 0; e < VEC; ++e)
-                if (VEC * s + e > q % BW) sd[q * (BW + 1) + VEC * s + e] = v[k][e] * sc;
+                if (VEC * s + e > q % BW) {
+                    const T x = v[k][e] * sc;
+                    top = max(top, exponent_of(x));
+                    sd[q * (BW + 1) + VEC * s + e] = x;
+                }
         }
     });
     // triangular solve of block bk by its warp; yv: the right-hand side of the row this lane holds
@@ -804,9 +889,9 @@ k_lu_solve(int N, const T* __restrict__ A, int ld, long long stride, const int32
         const int off = (bk * BW) & 31;
         const int R = rho - off;
         const bool mine = R >= 0 && R < BW;
-        T d[BW];
         const int row = bk * BW + (mine ? R : 0);
         if (!mine || row >= N) yv = T(0);
+        T d[BW];
 #pragma unroll
         for (int j = 0; j < BW; ++j) {
             const T v = sd[row * (BW + 1) + j];
@@ -828,9 +913,15 @@ k_lu_solve(int N, const T* __restrict__ A, int ld, long long stride, const int32
         }
         if (mine) xs[row] = yv;
     };
+    // A scaled value can overflow where the quotient by the diagonal does not, and a reciprocal below
+    // the normal range has lost bits: such a matrix is solved with divisions.
+    if (__syncthreads_or(top >= exponent_of(T(INFINITY)))) {
+        solve_rows(N, a, ld, perm + (size_t)mat * N, bb, mode, xs);
+        return;
+    }
     for (int sweep = (mode == 1) ? 1 : 0; sweep < 2; ++sweep) {
         const bool upper = sweep == 1;
-        __syncthreads();
+        if (upper && mode == 0) __syncthreads();
         static_for<ROWS>([&](auto ic) {
             constexpr int i = decltype(ic)::value;
             if (upper && mode == 0) {  // the forward result is the right-hand side of the backward sweep
@@ -872,76 +963,6 @@ k_lu_solve(int N, const T* __restrict__ A, int ld, long long stride, const int32
     }
     __syncthreads();
     for (int i = tid; i < N; i += nt) bb[i] = xs[i];
-}
-
-// The same substitution row by row, for what the block form does not take: N above 2048, or rows so far
-// apart that their offsets do not fit 32 bits. Dependent loads and a division per column in one
-// warp: at the sizes that both take it is 2 to 9 times slower.
-template <typename T>
-__global__ void __launch_bounds__(LU_THREADS)
-k_lu_solve_rows(int N, const T* __restrict__ A, int ld, long long stride, const int32_t* __restrict__ perm,
-           T* __restrict__ b, int mode, const int32_t* __restrict__ mats) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    T* x = reinterpret_cast<T*>(smraw);
-    const int mat = mats ? mats[blockIdx.x] : (int)blockIdx.x;
-    const T* a = A + (size_t)mat * stride;
-    const int32_t* pm = perm + (size_t)mat * N;
-    T* bb = b + (size_t)blockIdx.x * N;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
-    if (mode == 1) {
-        for (int i = tid; i < N; i += nt) x[i] = a[(size_t)pm[i] * ld + N];
-        __syncthreads();
-    } else {
-        for (int i = tid; i < N; i += nt) x[i] = bb[pm[i]];
-        __syncthreads();
-        for (int r0 = 0; r0 < N; r0 += 32) {
-            const int rb = min(32, N - r0);
-            for (int i = wid; i < rb; i += nw) {
-                const T* row = a + (size_t)pm[r0 + i] * ld;
-                T s = T(0);
-                for (int c = lane; c < r0; c += 32) s += row[c] * x[c];
-                s = warp_sum(s);
-                if (lane == 0) x[r0 + i] -= s;
-            }
-            __syncthreads();
-            if (wid == 0) {
-                T xi = (lane < rb) ? x[r0 + lane] : T(0);
-                const T* rowl = a + (size_t)pm[r0 + min(lane, rb - 1)] * ld;
-                for (int j = 0; j < rb; ++j) {
-                    T xj = __shfl_sync(0xffffffffu, xi, j);
-                    if (lane > j && lane < rb) xi -= rowl[r0 + j] * xj;
-                }
-                if (lane < rb) x[r0 + lane] = xi;
-            }
-            __syncthreads();
-        }
-    }
-    for (int r1 = N; r1 > 0; r1 -= 32) {
-        const int r0 = max(0, r1 - 32), rb = r1 - r0;
-        for (int i = wid; i < rb; i += nw) {
-            const T* row = a + (size_t)pm[r0 + i] * ld;
-            T s = T(0);
-            for (int c = r1 + lane; c < N; c += 32) s += row[c] * x[c];
-            s = warp_sum(s);
-            if (lane == 0) x[r0 + i] -= s;
-        }
-        __syncthreads();
-        if (wid == 0) {
-            T xi = (lane < rb) ? x[r0 + lane] : T(0);
-            const T* rowl = a + (size_t)pm[r0 + min(lane, rb - 1)] * ld;
-            for (int j = rb - 1; j >= 0; --j) {
-                T d = a[(size_t)pm[r0 + j] * ld + r0 + j];
-                T xj = __shfl_sync(0xffffffffu, xi, j);
-                xj = (d != T(0)) ? xj / d : xj;
-                if (lane == j) xi = xj;
-                if (lane < j) xi -= rowl[r0 + j] * xj;
-            }
-            if (lane < rb) x[r0 + lane] = xi;
-        }
-        __syncthreads();
-    }
-    for (int i = tid; i < N; i += nt) bb[i] = x[i];
 }
 
 template <typename T, int RPT>

@@ -70,3 +70,34 @@ def test_rows_two_to_the_31_values_apart():
     torch.cuda.synchronize()
     assert int(info.item()) == 0
     assert _backward_error(A0, x, b) < 2 * N * torch.finfo(torch.float32).eps
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("N,P", [(3, 1), (40, 2), (200, 1), (300, 2), (300, 310), (700, 1), (1300, 1), (1500, 1)])
+def test_solve_with_a_tiny_pivot_beside_large_entries(N, P, dtype):
+    """Rows whose entries over the pivot leave the type's range although the solution does not: the substitution
+    stays finite, with a componentwise backward error of at most 2 N eps in every row, as by division."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    tdt = torch.float64 if dtype == "f64" else torch.float32
+    tiny, large, x1 = (1e-300, 1e150, 1e-170) if dtype == "f64" else (1e-30, 1e15, 1e-30)
+    g = torch.Generator(device="cuda").manual_seed(N)
+    U = torch.triu(torch.randn((N, N), device="cuda", generator=g, dtype=torch.float64) * (0.3 / N), 1)
+    U += torch.diag(1.0 + torch.rand(N, device="cuda", generator=g, dtype=torch.float64))
+    b = torch.randn(N, device="cuda", generator=g, dtype=torch.float64)
+    rows = [0, N // 2, N - 2] if N > 8 else [N - 2]
+    for r in rows:                              # x[r + 1] = x1 or 0, x[r] about -large x1 / tiny
+        U[r], U[r + 1] = 0.0, 0.0
+        U[r, r], U[r, r + 1], U[r + 1, r + 1] = tiny, large, 2.0
+        b[r], b[r + 1] = -large * x1, (2.0 * x1 if r else 0.0)
+    U, b = U.to(tdt), b.to(tdt)
+    A, x = U.repeat(P, 1, 1).contiguous(), b.repeat(P, 1).contiguous()
+    piv = torch.arange(N, dtype=torch.int32, device="cuda").repeat(P, 1).contiguous()
+    _lib.check(lib.bte_lu_solve(0 if dtype == "f64" else 1, P, N, _ptr(A), N, N * N, _ptr(piv), _ptr(x), _stream()),
+               "lu_solve")
+    torch.cuda.synchronize()
+    assert bool(torch.isfinite(x).all()) and torch.equal(x[0], x[P - 1])
+    Ud, xd, bd = U.double(), x[0].double(), b.double()
+    scale = Ud.abs() @ xd.abs() + bd.abs()
+    assert float(((Ud @ xd - bd).abs() / scale.clamp_min(1e-307)).max()) <= 2 * N * torch.finfo(tdt).eps
