@@ -1024,25 +1024,26 @@ cudaError_t bte_lu_factor_tc(int P, int N, int NC, float* A, int ld, long long s
 
 // Factor P matrices in place; piv[P][N] receives perm (position -> stored row).
 // kernel: 0 = automatic (FP32: tensor cores, one CTA per matrix up to N = 512 and split over many
-// CTAs above; FP64: a cluster per matrix where bte_lu_cluster_size says so, or right-looking), 1 = right-looking, 2 = FP32 with the trailing updates on the tensor cores
+// CTAs above; FP64: 6), 1 = right-looking, 2 = FP32 with the trailing updates on the tensor cores
 // (lu_tc.cu; N <= 512; 256 threads, two CTAs per SM), 3 = left-looking SIMT (N <= 512), 4 = as
 // 2 with one CTA per SM, 5 = as 2 with 128 threads per CTA, 6 = FP64 split over many CTAs per
-// matrix (a cluster, or panel, triangular solve and 64 x 64 trailing tiles as separate launches).
+// matrix (a cluster where bte_lu_cluster_size says so, or panel, triangular solve and 64 x 64 trailing
+// tiles as separate launches).
 template <typename T>
 cudaError_t bte_lu_factor_t(int P, int N, int NC, T* A, int ld, long long stride, int32_t* piv, int32_t* info,
                             cudaStream_t s, int kernel) {
     if (P <= 0) return cudaSuccess;
     if (N < 1 || N > LU_MAX_N || NC < N || NC > N + 1 || ld < NC) return cudaErrorInvalidValue;
-    // FP64, the automatic choice and split over many CTAs: one cluster per matrix where that is
-    // faster, with the same factors
-    if constexpr (sizeof(T) == 8)
-        if (kernel == 0 || kernel == 6)
-            if (const int C = bte_lu_cluster_size(P, N, NC))
-                return bte_lu_factor_cluster(P, N, NC, A, ld, stride, piv, info, s, C);
-    // FP64: the right-looking kernel (the left-looking one serialises FP64 substitutions)
-    if (sizeof(T) == 8 && kernel == 0) kernel = 1;
+    // FP64: a cluster per matrix or launches split over many CTAs, whichever is the faster for P, with the same
+    // factors. Kernel 1 is not among them: its products are summed before they are subtracted, so a
+    // matrix's factors would depend on P, and it is faster for next to no size and batch (us, kernel 1 / these:
+    // N = 33: 1024 matrices 1397 / 177; N = 129: 4096 matrices 23045 / 9299; N = 257: 1024 matrices 19918 / 19820;
+    // N = 385: 137 matrices 7485 / 7687, 1024 matrices 52081 / 51748; N = 769: 24 matrices 46597 / 12098).
+    if (sizeof(T) == 8 && kernel == 0) kernel = 6;
     if (kernel == 6) {
         if constexpr (sizeof(T) == 8) {
+            if (const int C = bte_lu_cluster_size(P, N, NC))
+                return bte_lu_factor_cluster(P, N, NC, A, ld, stride, piv, info, s, C);
             return factor_split<T>(P, N, NC, A, ld, stride, piv, info, s);
         } else {
             return cudaErrorInvalidValue;

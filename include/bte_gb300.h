@@ -211,8 +211,7 @@ int bte_lu_factor(int dtype, int P, int N, void* A, int ld, long long stride, in
                   void* stream);
 
 /* As bte_lu_factor with an explicit kernel: 0 = automatic (FP32: tensor-core kernels, one CTA
- * per matrix for N <= 512, split over many above; FP64: a thread-block cluster per matrix for
- * the sizes and numbers where that is the fastest, else right-looking),
+ * per matrix for N <= 512, split over many above; FP64: as 6),
  * 1 = right-looking for every N, 2 = FP32 only, N <= 512: trailing updates on the tcgen05
  * tensor cores in split TF32 (FP32-accurate factors), 3 = left-looking (N <= 512),
  * 4 = as 2 with one CTA per SM instead of two (fewer matrices in flight, kept in L2),

@@ -101,3 +101,45 @@ def test_solve_with_a_tiny_pivot_beside_large_entries(N, P, dtype):
     Ud, xd, bd = U.double(), x[0].double(), b.double()
     scale = Ud.abs() @ xd.abs() + bd.abs()
     assert float(((Ud @ xd - bd).abs() / scale.clamp_min(1e-307)).max()) <= 2 * N * torch.finfo(tdt).eps
+
+
+@pytest.mark.parametrize("N,P", [(33, 4096), (193, 402), (257, 402), (385, 120), (513, 24), (769, 8)])
+def test_fp64_automatic_choice_does_not_depend_on_the_batch(N, P):
+    """bte_lu_factor in FP64 for two matrices alone and among so many that the size rule takes another route:
+    the same factors to the last bit."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(N)
+    M = torch.randn((2, N, N), device="cuda", generator=g, dtype=torch.float64)
+    got = []
+    for n in (2, P):
+        A = M.repeat(n // 2, 1, 1).contiguous()
+        piv, info = torch.empty((n, N), dtype=torch.int32, device="cuda"), torch.empty(n, dtype=torch.int32, device="cuda")
+        _lib.check(lib.bte_lu_factor(0, n, N, _ptr(A), N, N * N, _ptr(piv), _ptr(info), _stream()), "lu_factor")
+        torch.cuda.synchronize()
+        assert int(info.abs().max()) == 0
+        got.append((A[-2:].clone(), piv[-2:].clone()))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_transient_point_does_not_depend_on_the_batch(synthetic_xs, precision):
+    """A point's transient solution alone with two others and among thousands: the same bits."""
+    from boltzmann_gb300.workloads import batch_parameters
+    from helpers import gpu_solver
+    prm = batch_parameters(4096, 5, ebyn_range=(1.0, 2.0), ee=False)
+    out = []
+    for P in (3, 4096):
+        s, args = gpu_solver(synthetic_xs, 16, 1, False, P, precision)
+        args.Efreq, args.dt, args.cycles = 13.56e6, 1.0 / 8, 1.0
+        for k in ("n0", "ne", "ns_by_n0", "Tg", "E"):
+            v = np.asarray(prm[k])
+            s.set_boltzmann_parameter(0, k, v[..., :P])
+        s.set_boltzmann_parameter(0, "eRe", np.asarray(prm["E"])[:P])
+        s.set_boltzmann_parameter(0, "eIm", np.zeros(P))
+        s.host_to_device_setup(0, 0)
+        u, q = s.solve(0, s.initialize(0, P), 1e-30, 1e-10, 200, "transient")
+        out.append(np.asarray(u.cpu() if hasattr(u, "cpu") else u))
+    few, many = (np.moveaxis(o, [i for i, d in enumerate(o.shape) if d in (3, 4096)][0], -1) for o in out)
+    assert np.all(np.isfinite(few)) and np.array_equal(few, many[..., :3])
