@@ -27,7 +27,8 @@
 // share an SM. Reading A22 only after the product, in groups of 16 rows, with tiles of 128 x 128 and
 // rows exchanged between threads under branches, one matrix of N = 385 took 708 us and 4096 took
 // 14.4 ms; now 352 us and 7.0 ms.
-// Above N = 512 (k_tcs_*) the same steps are separate launches over many CTAs per matrix.
+// Above N = 512 (k_tcs_*) the same steps are separate launches over many CTAs per matrix, with the operands
+// split into three BF16 parts.
 // The split: hi = tf32(x) (round to nearest), lo = x - hi (exact in FP32); hi*hi is exact
 // in the FP32 accumulator, the dropped lo*lo term is below 2^-22 |x y|.
 #include <cstdint>
@@ -470,13 +471,21 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
 //   k_tcs_panel   one CTA per matrix: pivoting of the panel with the rows in registers (rows stay
 //                 with their threads, only their positions change; one barrier per column), then
 //                 U12 = L11^-1 A12, one thread per column;
-//   k_tcs_update  one CTA per 128 x 128 tile of the trailing matrix: A22 -= L21 U12 as in k_lu_tc.
+//   k_tcs_update  one CTA per 128 x 128 tile of the trailing matrix: A22 -= L21 U12 with the tile's layout
+//                 of k_lu_tc. These sizes had FP32 multiply-adds before, so the product must not be less
+//                 exact than they: each operand is split into three BF16 parts, whose sum is the FP32
+//                 value, and the six products of parts down to 2^-16 of the largest are taken, the
+//                 smallest first, so that the accumulator (which truncates) is rounded at the size of the
+//                 sum in the last two only. Backward error of the factors (Frobenius, in FP32 units of
+//                 |L| |U|), FP32 multiply-adds / two TF32 parts and three products / this: N = 513 0.050 /
+//                 0.102 / 0.027; N = 769 0.042 / 0.087 / 0.021; three TF32 parts give 0.030 but their 96 KB
+//                 of operands leave two CTAs per SM (75 matrices of N = 769 2024 us against 1631).
 // A matrix of N = 769 keeps one CTA busy for 5.5 ms (k_lu_right), with half the SMs idle for 75 of them;
 // split, the trailing updates spread over the GPU and the chain is the panels' columns.
 // Bound by that chain for few matrices and by the trailing matrices' reads and writes for many.
 // The result does not depend on the number of matrices. Measured (us, k_lu_right -> these):
-// N = 513: 2090 -> 540 (1 matrix), 2380 -> 1049 (150); N = 769: 5521 -> 879 (1), 6118 -> 1705 (75),
-// 19415 -> 6858 (400); N = 1281: 41980 -> 4992 (48); N = 2048: 247724 -> 3558 (2).
+// N = 513: 2090 -> 540 (1 matrix), 2380 -> 986 (150); N = 769: 5521 -> 889 (1), 6118 -> 1631 (75),
+// 19415 -> 6438 (400); N = 1281: 41980 -> 4699 (48); N = 2048: 247724 -> 3558 (2).
 // ---------------------------------------------------------------------------------
 constexpr int TS_NT = 512;             // threads of the panel kernel
 constexpr int TS_NW = TS_NT / 32;
@@ -615,6 +624,45 @@ k_tcs_panel(int N, int NC, int k0, float* __restrict__ A, int ld, long long stri
     }
 }
 
+constexpr int TS_PART = TC_TM * TC_NB * 2;   // one part of an operand: 8 KB
+// byte offset of element (row m, k) in a [rows x 32] BF16 tile, K-major, no swizzle: core matrix (m / 8, k / 8)
+// at (m / 8) * 512 + (k / 8) * 128, rows of a core matrix 16 B apart
+__device__ inline int ts_off(int m, int k) { return (m >> 3) * 512 + (k >> 3) * 128 + (m & 7) * 16 + (k & 7) * 2; }
+// shared-memory matrix descriptor as op_desc, 8-row groups 512 B apart
+__device__ inline uint64_t ts_desc(uint32_t saddr) {
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) |
+           ((uint64_t)1 << 46);
+}
+// instruction descriptor of kind::f16 with A and B BF16 (bits 7-9, 10-12 = 1), else as idesc_tf32
+__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+__device__ inline void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc));
+}
+// two values rounded to BF16 (x in the low half)
+__device__ inline uint32_t bf16x2(float x, float y) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(y), "f"(x));
+    return r;
+}
+// four values of one operand row (m, k..k+3) as three BF16 parts whose sum is the value
+__device__ inline void put_split3(unsigned char* sm, int m, int k, float a, float b, float c, float d) {
+    const int o = ts_off(m, k);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        const uint32_t u = bf16x2(a, b), v = bf16x2(c, d);
+        *reinterpret_cast<uint2*>(sm + p * TS_PART + o) = make_uint2(u, v);
+        a -= __uint_as_float(u << 16);
+        b -= __uint_as_float(u & 0xffff0000u);
+        c -= __uint_as_float(v << 16);
+        d -= __uint_as_float(v & 0xffff0000u);
+    }
+}
+
 // one 128 x 128 tile of A22 -= L21 U12 (kb = 16 or 32 panel columns at k0)
 __global__ void __launch_bounds__(256, 3)
 k_tcs_update(int N, int NC, int k0, int kb, int nct, int nrt, float* __restrict__ A, int ld, long long stride,
@@ -653,7 +701,7 @@ k_tcs_update(int N, int NC, int k0, int kb, int nct, int nrt, float* __restrict_
             if (vec4) v = *reinterpret_cast<const float4*>(src);
             else v = make_float4(src[0], src[1], src[2], src[3]);
         }
-        put_split4(sm + SM_B_HI, r, k, v.x, v.y, v.z, v.w);
+        put_split3(sm + 3 * TS_PART, r, k, v.x, v.y, v.z, v.w);
     }
     for (int e = tid; e < TC_TM * k4; e += 256) {
         const int m = e & (TC_TM - 1), k = (e >> 7) * 4;
@@ -661,22 +709,21 @@ k_tcs_update(int N, int NC, int k0, int kb, int nct, int nrt, float* __restrict_
         if (m < ncols)
 #pragma unroll
             for (int q = 0; q < 4; ++q) v[q] = a[piv[k + q] + c0 + m];
-        put_split4(sm + SM_A_HI, m, k, v[0], v[1], v[2], v[3]);
+        put_split3(sm, m, k, v[0], v[1], v[2], v[3]);
     }
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
     if (tid == 0) {
         tc_fence_after();
-        const uint32_t ahi = smem_u32(sm + SM_A_HI), alo = smem_u32(sm + SM_A_LO);
-        const uint32_t bhi = smem_u32(sm + SM_B_HI), blo = bhi + TC_TILE_BYTES;
-        constexpr uint32_t idesc = idesc_tf32(TC_TM, TC_TR);
-        for (int ks = 0; ks < kb / 8; ++ks) {
-            const uint32_t o = ks * 256;
-            mma_tf32(tbase, op_desc(alo + o), op_desc(bhi + o), idesc, ks > 0 ? 1u : 0u);
-            mma_tf32(tbase, op_desc(ahi + o), op_desc(blo + o), idesc, 1u);
-            mma_tf32(tbase, op_desc(ahi + o), op_desc(bhi + o), idesc, 1u);
-        }
+        constexpr int pa[6] = {1, 0, 2, 0, 1, 0}, pb[6] = {1, 2, 0, 1, 0, 0};  // parts, the smallest products first
+        const uint32_t as = smem_u32(sm), bs = as + 3 * TS_PART;
+        constexpr uint32_t idesc = idesc_bf16(TC_TM, TC_TR);
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+            for (int ks = 0; ks < kb / 16; ++ks)
+                mma_bf16(tbase, ts_desc(as + pa[p] * TS_PART + ks * 256), ts_desc(bs + pb[p] * TS_PART + ks * 256), idesc,
+                         p + ks > 0 ? 1u : 0u);
         mma_commit(mb);
     }
     // the tile's first values while the products run: warp w reads TMEM lanes 32 (w % 4) .. (columns)
@@ -753,7 +800,7 @@ cudaError_t bte_lu_factor_tcs(int P, int N, int NC, float* A, int ld, long long 
     if (N < 1 || N > 4 * TS_NT || NC < N || NC > N + 1 || ld < NC) return cudaErrorInvalidValue;
     if ((long long)N * ld >= (1ll << 31)) return cudaErrorInvalidValue;  // row offsets are 32-bit
     const int vec4 = (ld % 4 == 0 && stride % 4 == 0 && ((uintptr_t)A & 15) == 0) ? 1 : 0;
-    const size_t usm = (size_t)4 * TC_TILE_BYTES + 1024;
+    const size_t usm = (size_t)6 * TS_PART + 1024;
     cudaError_t e = bte_raise_smem_limit((const void*)k_tcs_update, usm);
     if (e != cudaSuccess) return e;
     for (int k0 = 0; k0 < N;) {

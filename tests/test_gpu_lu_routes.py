@@ -175,3 +175,35 @@ def test_block_substitution_is_as_accurate_as_row_by_row(N, dtype):
                 res = b.cpu().numpy().astype(np.longdouble) - exact @ y.cpu().numpy().astype(np.longdouble)
                 err[k] += float(np.sqrt((res * res).sum()))
         assert err[0] <= 1.1 * err[1], (part, err[0] / err[1])
+
+
+@pytest.mark.parametrize("graded", [False, True], ids=["normal", "graded"])
+@pytest.mark.parametrize("N", [513, 769, 1025])
+def test_fp32_products_above_512_are_as_accurate_as_multiply_adds(N, graded):
+    """The factors of the split FP32 factorization (tensor cores) against those of the right-looking kernel
+    (FP32 multiply-adds): the Frobenius norm of P A - L U over that of |L| |U|, the mean of 8 matrices, is no
+    larger; 1.05 allows for the sample."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    P, ld = 8, (N + 3) & ~3
+    g = torch.Generator(device="cuda").manual_seed(N)
+    A0 = torch.randn((P, N, ld), device="cuda", generator=g, dtype=torch.float64)
+    if graded:
+        A0 *= torch.exp(3 * torch.randn((P, N, 1), device="cuda", generator=g, dtype=torch.float64))
+        A0 *= torch.exp(3 * torch.randn((P, 1, ld), device="cuda", generator=g, dtype=torch.float64))
+        A0 /= A0.abs().amax(dim=2, keepdim=True)
+    A0 = A0.float()
+    err = []
+    for kernel in (0, 1):
+        A = A0.clone()
+        piv, info = torch.empty((P, N), dtype=torch.int32, device="cuda"), torch.empty(P, dtype=torch.int32, device="cuda")
+        _lib.check(lib.bte_lu_factor_ex(1, P, N, _ptr(A), ld, N * ld, _ptr(piv), _ptr(info), kernel, _stream()), "lu_factor")
+        torch.cuda.synchronize()
+        assert int(info.abs().max()) == 0
+        rows = piv.long()[:, :, None].expand(P, N, N)
+        LU = torch.gather(A[:, :, :N], 1, rows).double()
+        L, U = torch.tril(LU, -1) + torch.eye(N, device="cuda", dtype=torch.float64), torch.triu(LU)
+        R = torch.gather(A0[:, :, :N].double(), 1, rows) - L @ U
+        err.append(float((R.norm(dim=(1, 2)) / (L.abs() @ U.abs()).norm(dim=(1, 2))).mean()))
+    assert err[0] <= 1.05 * err[1], err
