@@ -644,8 +644,9 @@ cudaError_t factor_split(int P, int N, int NC, T* A, int ld, long long stride, i
 //  * products stay as 8 partial sums per lane, added over the lanes when their rows' own diagonal
 //    block comes up (a transposing reduction, 7 shuffles for 32 rows). Eight lanes' sums over
 //    all columns grow larger, and their rounding errors with them, than the 32 of a form with a warp
-//    per row (N = 769 in FP32: 1.7 times the error). So FP32 adds the products of a block first, and
-//    FP64, for whose pipe an addition costs what a product does, adds over the lanes every 128 columns;
+//    per row (N = 769: 1.6 times the error). So FP32 adds the products of a block first and adds over the
+//    lanes every 256 columns (every 512 above N = 512, where twice as often cost 12% of the time),
+//    and FP64, for whose pipe an addition costs what a product does, adds over the lanes every 128;
 //  * the owner of a diagonal block only arrives at the barrier that publishes its x, and can be all
 //    the blocks of its row group ahead of the other warps (lu_solve_form.h: the barriers in turn).
 // Measured (us, the row-oriented kernel with dependent loads and a division per column before ->
@@ -789,7 +790,8 @@ k_lu_solve(int N, const T* __restrict__ A, int ld, long long stride, const int32
            T* __restrict__ b, int mode, const int32_t* __restrict__ mats) {
     using V = typename SolveT<T, VEC>::V;
     constexpr int BW = 8 * VEC;
-    constexpr int FOLD = 128 / BW;  // blocks after which the partial sums enter the right-hand side
+    // blocks after which the partial sums enter the right-hand side
+    constexpr int FOLD = (VEC < 4 ? 128 : NTMAX * ROWS > 512 ? 512 : 256) / BW;
     static_assert(32 / BW < SOLVE_BARRIERS, "an owner's barriers must not repeat before it waits");
     extern __shared__ __align__(16) unsigned char smraw[];
     const int np = (N + 31) & ~31;
@@ -964,7 +966,7 @@ k_lu_solve(int N, const T* __restrict__ A, int ld, long long stride, const int32
                     if (!PREF) load(i, bk, seg[0]);
                     update(i, bk, seg[PREF ? i : 0]);
                     if (PREF) load(i, bn, seg[PREF ? i : 0]);
-                    if (VEC < 4 && (t + 1) % FOLD == 0) {
+                    if ((t + 1) % FOLD == 0) {
                         y[i] -= transpose_reduce8(part[i], lane);
 #pragma unroll
                         for (int k = 0; k < 8; ++k) part[i][k] = T(0);
