@@ -170,19 +170,6 @@ __host__ __device__ inline double interp_clamped(const double* xs, const double*
     return slope * (x - x0) + y0;
 }
 
-// 1 / d for a pivot: the hardware's 20-bit approximation y and one third-order step
-// y (1 + e + e^2), e = 1 - d y, whose error e^3 is below rounding (Householder's method for the
-// reciprocal): three FP64 instructions in the chain of every column instead of a division's
-// eight, 64 cycles each on GB300. Tiny, huge and non-finite values take the division.
-__device__ inline double bte_recip(double d) {
-    const int ex = (__double2hiint(d) >> 20) & 0x7ff;
-    if (ex < 64 || ex > 1983) return 1.0 / d;
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = fma(-d, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-
 template <typename T>
 __device__ inline T warp_sum(T v) {
 #pragma unroll

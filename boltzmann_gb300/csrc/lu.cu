@@ -103,7 +103,7 @@ __device__ inline void warp_argmax(double& best, int& bi) {
     }
 }
 __device__ inline float recip(float d) { return __frcp_rn(d); }
-__device__ inline double recip(double d) { return bte_recip(d); }
+__device__ inline double recip(double d) { return 1.0 / d; }
 
 // Unblocked partial-pivoting factorization of a panel in shared memory, column-major
 // P[c * ldp + r], rows 0..mrows-1 (pivot positions base..base+mrows-1), pivots on the

@@ -137,7 +137,7 @@ __device__ inline void cl_panel(ClShared& sh, double* P, int ldr, int N, int NC,
                 const double d = v[i][j];
 #pragma unroll
                 for (int c = j + 1; c < CL_NB; ++c) prow[c] = v[i][c];
-                sh.inv[j & 1] = (d != 0.0) ? bte_recip(d) : 0.0;
+                sh.inv[j & 1] = (d != 0.0) ? 1.0 / d : 0.0;
                 if (!(d != 0.0) && sh.info == 0) sh.info = q + 1;
             } else if (pos[i] == q) {
                 pos[i] = at_p;

@@ -152,8 +152,8 @@ __device__ inline void put_split4(unsigned char* sm, int m, int k, float a, floa
     *reinterpret_cast<float4*>(sm + lo_off + o) = lo;
 }
 
-// Predicated stores and a reciprocal without branches, for the panels' chain of columns: a branch that
-// may diverge costs about 50 cycles there, whether taken or not.
+// Predicated stores, for the panels' chain of columns: a branch that may diverge costs about 50 cycles
+// there, whether taken or not.
 __device__ inline void put_if(bool on, uint32_t addr, float x, float y, float z, float w) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %0, 0;\n\t@p st.shared.v4.f32 [%1], {%2, %3, %4, %5};\n\t}\n" ::"r"(
                      (uint32_t)on),
@@ -165,14 +165,6 @@ __device__ inline void put_if(bool on, uint32_t addr, uint32_t x, uint32_t y) {
                  "r"(addr), "r"(x), "r"(y)
                  : "memory");
 }
-// 1 / d to within an ulp, 0 for d = 0: the hardware's approximation and one Newton step where that is finite
-__device__ inline float recip_or_0(float d) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;\n" : "=f"(r) : "f"(d));
-    const float c = fmaf(r, fmaf(-d, r, 1.f), r);
-    return (d != 0.f) ? (fabsf(c) <= 3.402823466e38f ? c : r) : 0.f;
-}
-
 template <int ROWS, int OCC, int NT>
 __global__ void __launch_bounds__(NT, OCC)
 k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t* __restrict__ perm_out,
@@ -275,7 +267,7 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
             }
             const float d = pv[j];
             inf = (!(d != 0.f) && inf == 0) ? k0 + j + 1 : inf;
-            const float inv = recip_or_0(d);
+            const float inv = (d != 0.f) ? __frcp_rn(d) : 0.f;
 #pragma unroll
             for (int i = 0; i < ROWS; ++i) {
                 pos[i] = pos[i] == (int)S ? j : (pos[i] == j ? (int)S : pos[i]);

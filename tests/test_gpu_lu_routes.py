@@ -206,3 +206,29 @@ def test_fp32_products_above_512_are_as_accurate_as_multiply_adds(N, graded):
         R = torch.gather(A0[:, :, :N].double(), 1, rows) - L @ U
         err.append(float((R.norm(dim=(1, 2)) / (L.abs() @ U.abs()).norm(dim=(1, 2))).mean()))
     assert err[0] <= 1.05 * err[1], err
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("kernel", [0, 1])
+def test_multipliers_are_products_with_the_rounded_reciprocal(dtype, kernel):
+    """The multiplier of a row whose entry is 1 is the pivot's reciprocal, correctly rounded, at any exponent: the
+    second row of [[d, 0], [1, 1]], |d| >= 1 (2 x 2 and as the first columns of 40 x 40)."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    tdt = torch.float64 if dtype == "f64" else torch.float32
+    g = torch.Generator(device="cuda").manual_seed(1)
+    P = 20000
+    top = 1000 if dtype == "f64" else 120
+    d = (1.0 + torch.rand(P, device="cuda", generator=g, dtype=torch.float64)).to(tdt)
+    d = torch.ldexp(d, torch.randint(0, top, (P,), device="cuda", generator=g)).to(tdt)
+    for N in (2, 40):
+        n = P if N == 2 else 2000
+        A = torch.eye(N, device="cuda", dtype=tdt).repeat(n, 1, 1).contiguous()
+        A[:, 0, 0], A[:, 1, 0] = d[:n], 1.0
+        piv, info = torch.empty((n, N), dtype=torch.int32, device="cuda"), torch.empty(n, dtype=torch.int32, device="cuda")
+        _lib.check(lib.bte_lu_factor_ex(0 if dtype == "f64" else 1, n, N, _ptr(A), N, N * N, _ptr(piv), _ptr(info), kernel,
+                                        _stream()), "lu_factor")
+        torch.cuda.synchronize()
+        assert int(info.abs().max()) == 0 and torch.equal(piv[:, :2].long(), torch.arange(2, device="cuda").expand(n, 2))
+        assert torch.equal(A[:, 1, 0], 1.0 / d[:n])
