@@ -165,6 +165,13 @@ __device__ inline void put_if(bool on, uint32_t addr, uint32_t x, uint32_t y) {
                  "r"(addr), "r"(x), "r"(y)
                  : "memory");
 }
+// x -= l u under a predicate
+__device__ inline void sub_if(bool on, float& x, float l, float u) {
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t@p fma.rn.f32 %0, %1, %2, %0;\n\t}\n"
+        : "+f"(x)
+        : "f"(-l), "f"(u), "r"((uint32_t)on));
+}
+
 template <int ROWS, int OCC, int NT>
 __global__ void __launch_bounds__(NT, OCC)
 k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t* __restrict__ perm_out,
@@ -271,10 +278,12 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
 #pragma unroll
             for (int i = 0; i < ROWS; ++i) {
                 pos[i] = pos[i] == (int)S ? j : (pos[i] == j ? (int)S : pos[i]);
-                const float l = pos[i] > j ? pr[i][j] * inv : 0.f;
-                pr[i][j] = pos[i] > j ? l : pr[i][j];
+                // rows that are done keep their values, also where the pivot row holds an infinity
+                const bool on = pos[i] > j;
+                const float l = pr[i][j] * inv;
+                pr[i][j] = on ? l : pr[i][j];
 #pragma unroll
-                for (int c = j + 1; c < TC_NB; ++c) pr[i][c] -= l * pv[c];
+                for (int c = j + 1; c < TC_NB; ++c) sub_if(on, pr[i][c], l, pv[c]);
             }
         }
         // write the panel back (each position's data returns to its own stored row), the positions

@@ -232,3 +232,23 @@ def test_multipliers_are_products_with_the_rounded_reciprocal(dtype, kernel):
         torch.cuda.synchronize()
         assert int(info.abs().max()) == 0 and torch.equal(piv[:, :2].long(), torch.arange(2, device="cuda").expand(n, 2))
         assert torch.equal(A[:, 1, 0], 1.0 / d[:n])
+
+
+@pytest.mark.parametrize("kernel,dtype", [(0, "f64"), (1, "f64"), (6, "f64"), (0, "f32"), (1, "f32"), (2, "f32"), (3, "f32"),
+                                          (4, "f32"), (5, "f32")])
+@pytest.mark.parametrize("N", [40, 300])
+def test_rows_above_an_infinity_keep_their_values(N, kernel, dtype):
+    """An infinite entry right of its row's pivot: the rows that were factored before it stay as they are."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    tdt = torch.float64 if dtype == "f64" else torch.float32
+    A = torch.eye(N, device="cuda", dtype=tdt)
+    A[:, -1] = 2.0
+    A[5, 20], A[35, 37] = float("inf"), float("-inf")
+    F = A.clone()
+    piv, info = torch.empty(N, dtype=torch.int32, device="cuda"), torch.empty(1, dtype=torch.int32, device="cuda")
+    _lib.check(lib.bte_lu_factor_ex(0 if dtype == "f64" else 1, 1, N, _ptr(F), N, N * N, _ptr(piv), _ptr(info), kernel,
+                                    _stream()), "lu_factor")
+    torch.cuda.synchronize()
+    assert torch.equal(F[:6], A[:6])
