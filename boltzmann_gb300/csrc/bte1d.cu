@@ -401,7 +401,7 @@ struct Bte1d {
     // (allocated on first use)
     double *AxT = nullptr, *DT = nullptr;
     double *Fk = nullptr, *Fr = nullptr, *Fw = nullptr, *Fz = nullptr, *Fx = nullptr, *Fb = nullptr, *Ft = nullptr,
-           *Fg = nullptr;
+           *Fg = nullptr, *Fh = nullptr, *Fl = nullptr;
     double *Fpart = nullptr;
     int fcap = 0;
     std::vector<void*> allocs;
@@ -759,12 +759,14 @@ static int fim_matvec(Bte1d* h, double dt, const double* E, const double* V, dou
     const int Nr = h->Nr, Nvt = h->Nvt, Nx = h->Nx, M = Nr * Nvt;
     if (!h->Ft && alloc1d(h, (void**)&h->Ft, (size_t)M * Nx * 8) != BTE_OK) return BTE_ERR_ALLOC;
     if (!h->Fg && alloc1d(h, (void**)&h->Fg, (size_t)M * Nx * 8) != BTE_OK) return BTE_ERR_ALLOC;
+    if (!h->Fh && alloc1d(h, (void**)&h->Fh, (size_t)h->n * Nx * 8) != BTE_OK) return BTE_ERR_ALLOC;
+    if (!h->Fl && alloc1d(h, (void**)&h->Fl, (size_t)h->n * Nx * 8) != BTE_OK) return BTE_ERR_ALLOC;
     const int n = h->n, R = dgw_rows(M, Nx);
     const size_t N = (size_t)M * Nx;
-    // h->R and h->W hold the harmonics and their operator (the v-step's vectors, free here)
-    k_ords_to_lm<<<nb((size_t)n * Nx, 256), 256, 0, s>>>(Nr, Nvt, h->nsh, Nx, h->Ps, V, h->R, nullptr);
+    // the harmonics and their operator; not the v-step's vectors, which another stream may be using
+    k_ords_to_lm<<<nb((size_t)n * Nx, 256), 256, 0, s>>>(Nr, Nvt, h->nsh, Nx, h->Ps, V, h->Fh, nullptr);
     CK1(cudaGetLastError());
-    launch_lmat<false>(n, Nx, dt, h->CvT, h->AvT, E, h->R, h->W, s);
+    launch_lmat<false>(n, Nx, dt, h->CvT, h->AvT, E, h->Fh, h->Fl, s);
     CK1(cudaGetLastError());
     dgw_dispatch(R, [&](auto rc) {
         k_fim_dx<decltype(rc)::value><<<dgw_grid(M, Nx, R), DGW_WARPS * 32, 0, s>>>(M, Nvt, Nx, h->DT, h->right, V, h->Ft);
@@ -772,7 +774,7 @@ static int fim_matvec(Bte1d* h, double dt, const double* E, const double* V, dou
     CK1(cudaGetLastError());
     launch_radial_mix<true>(Nr, Nvt * Nx, h->AxT, h->Ft, h->Fg, s);
     CK1(cudaGetLastError());
-    k_fim_combine<<<nb(N, 256), 256, 0, s>>>(Nr, Nvt, h->nsh, Nx, dt, h->Po, h->cth, h->right, h->W, h->Fg, V, Y);
+    k_fim_combine<<<nb(N, 256), 256, 0, s>>>(Nr, Nvt, h->nsh, Nx, dt, h->Po, h->cth, h->right, h->Fl, h->Fg, V, Y);
     CK1(cudaGetLastError());
     h->launches += 5;
     return BTE_OK;
