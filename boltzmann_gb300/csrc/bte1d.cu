@@ -397,6 +397,7 @@ struct Bte1d {
     double* hp = nullptr;  // pinned: what the reductions gave
     double* Vt = nullptr;  // ordinates scratch
     double* Vt2 = nullptr;
+    double* Xc = nullptr;  // the input of an operator that overwrites it
     // fully implicit step: adv_x transposed, D transposed, and the ordinates-space GMRES buffers
     // (allocated on first use)
     double *AxT = nullptr, *DT = nullptr;
@@ -485,6 +486,7 @@ int bte1d_create(int device, int Nr, int nsh, int Nvt, int Nx, const double* Q, 
     }
     A((void**)&h->Vt, nv * 8);
     A((void**)&h->Vt2, nv * 8);
+    A((void**)&h->Xc, nu * 8);
     A((void**)&h->AxT, (size_t)Nr * Nr * 8); A((void**)&h->DT, (size_t)Nx * Nx * 8);
     if (rc != BTE_OK) { free1d(h); delete h; return rc; }
     // adv_x = Q diag(d) Q^-1 (transposed), and D transposed, for the fully implicit step
@@ -580,6 +582,10 @@ int bte1d_step_x(Bte1d* h, double hstep, double* V, void* stream) {
 int bte1d_lmat(Bte1d* h, double dt, const double* E, const double* X, double* Y, void* stream) {
     if (!h || !E || !X || !Y) { g_err1d = "null argument"; return BTE_ERR_ARG; }
     cudaSetDevice(h->device);
+    if (X == Y) {  // the warps of a point read what others of it write
+        CK1(cudaMemcpyAsync(h->Xc, X, (size_t)h->n * h->Nx * 8, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
+        X = h->Xc;
+    }
     launch_lmat<true>(h->n, h->Nx, dt, h->CvT, h->AvT, E, X, Y, (cudaStream_t)stream);
     CK1(cudaGetLastError());
     h->launches += 1;

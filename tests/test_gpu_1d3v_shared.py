@@ -36,3 +36,22 @@ def test_implicit_operator_beside_the_v_step(synthetic_xs):
         torch.cuda.synchronize()
         assert all(torch.equal(y, alone_m) for y in got)
         assert torch.equal(v, alone_v)
+
+
+@pytest.mark.parametrize("Np,Nr,lmax", [(9, 7, 1), (65, 15, 2), (201, 31, 1)])
+def test_operators_in_place(synthetic_xs, Np, Nr, lmax):
+    """bte1d_lmat and bte1d_fim_matvec with the output on their input: the same bits as into another buffer."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    b, E, V = _solver(synthetic_xs, Np=Np, Nr=Nr, lmax=lmax)
+    Ed, st = torch.as_tensor(E, device="cuda"), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    X = torch.randn((Np, b.dof_v), device="cuda", dtype=torch.float64, generator=torch.Generator(device="cuda").manual_seed(Np))
+    for f, x in ((lib.bte1d_lmat, X), (lib.bte1d_fim_matvec, torch.as_tensor(V, device="cuda").contiguous())):
+        y, z = torch.empty_like(x), x.clone()
+        assert f(b._h, 1e-3, _lib.ptr(Ed), _lib.ptr(x), _lib.ptr(y), st) == 0
+        for _ in range(20):
+            z.copy_(x)
+            assert f(b._h, 1e-3, _lib.ptr(Ed), _lib.ptr(z), _lib.ptr(z), st) == 0
+            torch.cuda.synchronize()
+            assert torch.equal(z, y)
