@@ -296,7 +296,7 @@ k_fvm_sweep_coef(FvmView v, const double* __restrict__ aE, const double* __restr
     __shared__ double tile[SW_NDMAX - 1][32][33];
     const int nlines = v.Nr * v.Nvt;
     const size_t n = (size_t)nlines * v.Nx;
-    const int l0 = blockIdx.y * 32, x0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int l0 = blockIdx.x * 32, x0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     double* tr = tab;
     double* tt = tr + (size_t)v.ndr * n;
     double* xr = tt + (size_t)v.ndt * n;
@@ -581,7 +581,8 @@ bool natural_sweeps(const bte_fvm* h) {
 // the sweep coefficients for step h at the coefficients in h->aE, h->axvr
 int fvm_sweep_coef(bte_fvm* h, double hstep, cudaStream_t s) {
     if (!natural_sweeps(h)) return BTE_OK;
-    const dim3 grid((unsigned)((h->Nx + 31) / 32), (unsigned)((h->Nr * h->Nvt + 31) / 32));
+    // x rows that fit in shared memory are short; the lines can be more than a grid's 65535 x 32 rows
+    const dim3 grid((unsigned)((h->Nr * h->Nvt + 31) / 32), (unsigned)((h->Nx + 31) / 32));
     k_fvm_sweep_coef<<<grid, 256, 0, s>>>(view_of(h), h->aE, h->axvr, hstep, h->swc);
     ++h->launches;
     return launched("k_fvm_sweep_coef");
