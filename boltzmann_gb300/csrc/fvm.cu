@@ -47,7 +47,7 @@ struct bte_fvm {
     double* gval = nullptr;
     uint32_t* hmask = nullptr;   // per 8-row tile of H: which chunks of HC columns hold a non-zero
     int32_t* bad = nullptr;      // per x: a non-finite ordinate moment (it reaches every row of G m and H m)
-    double* swc = nullptr;       // sweep coefficients (k_fvm_sweep_coef), allocated with the collision inverse
+    double* swc = nullptr;       // sweep coefficients (k_fvm_sweep_coef), allocated with the collision inverse if there is room
     double *B = nullptr, *X = nullptr, *R = nullptr, *W = nullptr, *Z = nullptr, *Tv = nullptr;
     double* Kr = nullptr;
     int kcap = 0;
@@ -578,9 +578,23 @@ bool natural_sweeps(const bte_fvm* h) {
     return h->ndr <= SW_NDMAX && h->ndt <= SW_NDMAX && h->ndx <= SW_NDMAX && sweep_x_rows(h) > 0;
 }
 
+// The sweep coefficients (5 N to 12 N values) only make the sweeps faster, so they never take the room of
+// something that has to be there: they are allocated when the longest Krylov basis (501 N) would still fit
+// beside them, and without them the sweeps run on permuted copies.
+void fvm_alloc_sweep_coef(bte_fvm* h) {
+    if (h->swc || !natural_sweeps(h)) return;
+    const size_t bytes = (size_t)(h->ndr + h->ndt + h->ndx) * h->N * sizeof(double);
+    size_t room = 0, all = 0;
+    if (cudaMemGetInfo(&room, &all) != cudaSuccess || room < bytes + (size_t)501 * h->N * sizeof(double) ||
+        fvm_alloc(h, (void**)&h->swc, bytes) != BTE_OK) {
+        h->swc = nullptr;
+        cudaGetLastError();
+    }
+}
+
 // the sweep coefficients for step h at the coefficients in h->aE, h->axvr
 int fvm_sweep_coef(bte_fvm* h, double hstep, cudaStream_t s) {
-    if (!natural_sweeps(h)) return BTE_OK;
+    if (!h->swc) return BTE_OK;
     // x rows that fit in shared memory are short; the lines can be more than a grid's 65535 x 32 rows
     const dim3 grid((unsigned)((h->Nr * h->Nvt + 31) / 32), (unsigned)((h->Nx + 31) / 32));
     k_fvm_sweep_coef<<<grid, 256, 0, s>>>(view_of(h), h->aE, h->axvr, hstep, h->swc);
@@ -594,9 +608,9 @@ int fvm_precond(bte_fvm* h, double hstep, const double* X, double* Y, cudaStream
     const FvmView v = view_of(h);
     const int Nr = h->Nr, Nvt = h->Nvt, Nx = h->Nx;
     if (int rc = fvm_hmul(h, X, s)) return rc;
-    if (!natural_sweeps(h)) {
-        // stencils wider than the register recurrence or x lines longer than the staged rows:
-        // the drop-in sweeps on permuted copies
+    if (!h->swc) {
+        // stencils wider than the register recurrence, x lines longer than the staged rows or no room for
+        // the coefficients: the drop-in sweeps on permuted copies
         k_fvm_coll_permute<<<fblocks(h->N), FT, 0, s>>>(v, h->dinv, h->T, X, h->A, h->bad);   // (Nx, Nvt, Nr)
         if (int rc = launched("k_fvm_coll_permute")) return rc;
         int rc = sweep_rc(bte_adv_be_sweep(0, h->vrL, h->vrR, h->aE, h->cos_t, hstep, h->A, h->Bf, h->ndr, Nr, Nvt, Nx, s),
@@ -861,8 +875,7 @@ long long bte_fvm_launches(const bte_fvm* h) { return h ? h->launches : 0; }
 int bte_fvm_set_collision_inverse(bte_fvm* h, const double* dinv, const double* H) {
     if (!h || !dinv || !H) return fvm_fail(BTE_ERR_ARG, "bte_fvm_set_collision_inverse: null argument");
     cudaSetDevice(h->device);
-    if (!h->swc && natural_sweeps(h))
-        if (int rc = fvm_alloc(h, (void**)&h->swc, (size_t)(h->ndr + h->ndt + h->ndx) * h->N * sizeof(double))) return rc;
+    fvm_alloc_sweep_coef(h);
     const int Nr = h->Nr, words = ((Nr + HC - 1) / HC + 31) / 32;
     std::vector<uint32_t> mask((size_t)((Nr + HR - 1) / HR) * words, 0u);
     for (int r = 0; r < Nr; ++r)

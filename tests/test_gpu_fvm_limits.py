@@ -60,3 +60,31 @@ def test_more_lines_than_a_grid_has_rows():
     want[:, north, 0] = 0.0
     want[:, ~north, Nx - 1] = 0.0
     assert np.max(np.abs(got - want)) <= Nvt * 2.3e-16 * np.max(np.abs(want))
+
+
+def test_no_room_for_the_sweep_coefficients():
+    """A device with less free memory than the sweeps' coefficients take: the handle works all the same, with the
+    values of one that has them to 1e-12 of the largest (another order of the same operations)."""
+    import torch
+    Nr, Nvt, Nx = 64, 16, 4000
+    g = torch.Generator(device="cuda").manual_seed(2)
+    X = torch.rand((Nr, Nvt, Nx), device="cuda", dtype=torch.float64, generator=g)
+    E = torch.randn(Nx, device="cuda", dtype=torch.float64, generator=g)
+    a = _Handle(Nr, Nvt, Nx)
+    a.set_inverse()
+    want = a.precond(0.7, 0.4, 1e-2, E, X)
+    a.close()
+    b = _Handle(Nr, Nvt, Nx)
+    spare = torch.empty(Nr * Nvt * Nx * 8, device="cuda", dtype=torch.uint8)   # the output's, and a little more
+    torch.cuda.synchronize()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (128 << 20), device="cuda", dtype=torch.uint8)
+    assert torch.cuda.mem_get_info()[0] < 6 * X.numel() * 8
+    del spare
+    try:
+        b.set_inverse()
+        got = b.precond(0.7, 0.4, 1e-2, E, X)
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    b.close()
+    assert float((got - want).abs().max()) <= 1e-12 * float(want.abs().max())
