@@ -1032,7 +1032,7 @@ cudaError_t bte_lu_factor_tcs(int P, int N, int NC, float* A, int ld, long long 
                               cudaStream_t s);
 int bte_lu_cluster_size(int P, int N, int NC);
 cudaError_t bte_lu_factor_cluster(int P, int N, int NC, double* A, int ld, long long stride, int32_t* piv, int32_t* info,
-                                  cudaStream_t s, int C);
+                                  cudaStream_t s, int C, bool* ran);
 cudaError_t bte_lu_factor_tc(int P, int N, int NC, float* A, int ld, long long stride, int32_t* piv, int32_t* info,
                              cudaStream_t s, int variant);
 
@@ -1056,8 +1056,11 @@ cudaError_t bte_lu_factor_t(int P, int N, int NC, T* A, int ld, long long stride
     if (sizeof(T) == 8 && kernel == 0) kernel = 6;
     if (kernel == 6) {
         if constexpr (sizeof(T) == 8) {
-            if (const int C = bte_lu_cluster_size(P, N, NC))
-                return bte_lu_factor_cluster(P, N, NC, A, ld, stride, piv, info, s, C);
+            if (const int C = bte_lu_cluster_size(P, N, NC)) {
+                bool ran;
+                const cudaError_t e = bte_lu_factor_cluster(P, N, NC, A, ld, stride, piv, info, s, C, &ran);
+                if (ran || e != cudaSuccess) return e;
+            }
             return factor_split<T>(P, N, NC, A, ld, stride, piv, info, s);
         } else {
             return cudaErrorInvalidValue;

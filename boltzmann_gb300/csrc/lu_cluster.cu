@@ -314,9 +314,11 @@ k_lu_cluster(int N, int NC, double* __restrict__ A, int ld, long long stride, in
     cluster.sync();  // no CTA leaves while its shared memory is read
 }
 
+// Sets *ran when the device can hold a cluster of this shape, and launches; a device or a partition of one with
+// fewer SMs behind one another than the clusters need leaves the work to the split launches
 template <int RPL, int OCC>
 cudaError_t launch_cluster(int P, int N, int NC, int C, double* A, int ld, long long stride, int32_t* piv, int32_t* info,
-                           cudaStream_t s) {
+                           cudaStream_t s, bool* ran) {
     const size_t sm = cl_smem(N, NC, C, sizeof(double));
     cudaError_t e = bte_raise_smem_limit((const void*)k_lu_cluster<RPL, OCC>, sm);
     if (e != cudaSuccess) return e;
@@ -336,6 +338,12 @@ cudaError_t launch_cluster(int P, int N, int NC, int C, double* A, int ld, long 
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    int held = 0;
+    if (cudaOccupancyMaxActiveClusters(&held, k_lu_cluster<RPL, OCC>, &cfg) != cudaSuccess || held < 1) {
+        cudaGetLastError();
+        return cudaSuccess;
+    }
+    *ran = true;
     return cudaLaunchKernelEx(&cfg, k_lu_cluster<RPL, OCC>, N, NC, A, ld, stride, piv, info);
 }
 
@@ -376,13 +384,14 @@ int bte_lu_cluster_size(int P, int N, int NC) {
     return size;
 }
 
+// One cluster of C CTAs per matrix. *ran stays false, and nothing is done, where no such cluster fits the device.
 cudaError_t bte_lu_factor_cluster(int P, int N, int NC, double* A, int ld, long long stride, int32_t* piv, int32_t* info,
-                                  cudaStream_t s, int C) {
-    if (P <= 0) return cudaSuccess;
+                                  cudaStream_t s, int C, bool* ran) {
+    *ran = false;
     constexpr int PT = 32 * CL_PW;
-    if (N <= PT) return launch_cluster<1, 2>(P, N, NC, C, A, ld, stride, piv, info, s);
-    if (N <= 2 * PT) return launch_cluster<2, 2>(P, N, NC, C, A, ld, stride, piv, info, s);
-    if (N <= 4 * PT) return launch_cluster<4, 2>(P, N, NC, C, A, ld, stride, piv, info, s);
-    if (N <= 8 * PT) return launch_cluster<8, 1>(P, N, NC, C, A, ld, stride, piv, info, s);
+    if (N <= PT) return launch_cluster<1, 2>(P, N, NC, C, A, ld, stride, piv, info, s, ran);
+    if (N <= 2 * PT) return launch_cluster<2, 2>(P, N, NC, C, A, ld, stride, piv, info, s, ran);
+    if (N <= 4 * PT) return launch_cluster<4, 2>(P, N, NC, C, A, ld, stride, piv, info, s, ran);
+    if (N <= 8 * PT) return launch_cluster<8, 1>(P, N, NC, C, A, ld, stride, piv, info, s, ran);
     return cudaErrorInvalidValue;
 }
