@@ -6,11 +6,13 @@ For a bordered system size N the library has several FP32 LU kernels (`bte_lu_fa
      matrices stay in L2);
   5  the same kernel with 128 threads per CTA (4 warps share the per-column pivot search);
   3  the left-looking SIMT kernel (blocks held in registers);
-  1  the right-looking SIMT kernel (any N; the only choice above N = 512).
+  1  the right-looking SIMT kernel (any N).
+Above N = 512 the solver takes the library's own choice (0: panels and trailing tiles on the tensor cores),
+and nothing is timed; `tune_lu` knows only kernel 1 there.
 `tune_lu(N)` times every candidate on seeded synthetic systems of that size (diagonally shifted
 normal matrices, the solver's 16-byte aligned row layout), one matrix per CTA in waves like
 the solve's, and keeps the fastest; the choice is cached in memory and on disk per (GPU name,
-N), in `$BOLTZMANN_GB300_CACHE` or `~/.cache/boltzmann_gb300/lu_autotune.json`. The solver
+N, revision of the kernels), in `$BOLTZMANN_GB300_CACHE` or `~/.cache/boltzmann_gb300/lu_autotune.json`. The solver
 passes it as `bte_solve_opts.lu_kernel`. The reference has no counterpart: it calls one
 library inverse (xp.linalg.inv, bte_0d3v_batched.py:856-880).
 """
@@ -25,6 +27,7 @@ from . import _lib
 
 CANDIDATES_SMALL = (2, 4, 5, 3, 1)
 CANDIDATES_LARGE = (1,)
+REVISION = 2  # of the kernels that are timed: a choice made with others is not read
 _mem: dict = {}
 _lock = threading.Lock()
 
@@ -58,7 +61,7 @@ def _store_disk(key, rec) -> None:
 
 def _key(N, device):
     import torch
-    return "%s|N=%d" % (torch.cuda.get_device_name(device), int(N))
+    return "%s|N=%d|r%d" % (torch.cuda.get_device_name(device), int(N), REVISION)
 
 
 def time_lu(N, kernel, P=1024, reps=3, device=0, seed=17):
@@ -111,7 +114,9 @@ def tune_lu(N, P=1024, device=0, force=False):
 
 
 def lu_kernel_for(N, device=0) -> int:
-    """bte_solve_opts.lu_kernel for bordered size N (tuned on first use)."""
+    """bte_solve_opts.lu_kernel for bordered size N: tuned on first use, 0 (the library's choice) above N = 512."""
+    if N > 512:
+        return 0
     return int(tune_lu(N, device=device)["kernel"])
 
 

@@ -529,11 +529,8 @@ class bte_0d3v_batched:
         k = int(getattr(self._args, "lu_kernel", 0) or 0)
         if k or self._precision() != _lib.PREC_MIXED or not int(getattr(self._args, "autotune", 1)):
             return k
-        N = self._grid_info[grid_idx]["n"] + 1
-        if N > 512:  # above the tuner's candidates the library has one choice
-            return 0
         from . import autotune
-        return autotune.lu_kernel_for(N, device=self._dev_id)
+        return autotune.lu_kernel_for(self._grid_info[grid_idx]["n"] + 1, device=self._dev_id)
 
     def _precision(self):
         p = str(getattr(self._args, "precision", "fp64")).lower()

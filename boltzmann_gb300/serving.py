@@ -213,11 +213,10 @@ class BteServer:
                                   refine=int(refine), krylov=int(krylov))
             for i, k in enumerate(keys):
                 o = opts
-                N = s._grid_info[i]["n"] + 1
-                if precision == "mixed" and autotune and N <= 512:  # above, the library has one choice
+                if precision == "mixed" and autotune:
                     from . import autotune as at
                     o = _lib.SolveOpts.from_buffer_copy(opts)
-                    o.lu_kernel = at.lu_kernel_for(N, device=device)
+                    o.lu_kernel = at.lu_kernel_for(s._grid_info[i]["n"] + 1, device=device)
                 be = EngineBackend(s._grid[i], s._grid_info[i], capacity, fp64_capacity, o, device)
                 self._workers[k] = _Worker(k, be)
         else:
