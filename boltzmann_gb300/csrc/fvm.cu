@@ -2,7 +2,7 @@
 // solver_type "fully_implicit" (bte_1d3v_solver.py:1890-2009), preconditioned by its op-split
 // step (:1745-1870, type XVTVRC).
 //
-// Operator: one fused kernel (k_fvm_mvec, the arithmetic of fvm_core.h's fvm_mvec_at on tabulated
+// Operator: one fused kernel (k_fvm_mvec, fvm_core.h's fvm_mvec_tab_at on the step's tabulated
 // coefficients) reads each value's upwind stencils along x, v_r and v_theta and writes one
 // output, after the ordinate moments m = w^T v (k_fvm_moment) and the gain product G m over
 // the few non-zeros of G's rows (k_fvm_gain). The reference
@@ -104,12 +104,11 @@ __global__ void k_fvm_mvec_coef(FvmView v, FvmCoef c, const double* __restrict__
                                 double* __restrict__ arc, double* __restrict__ lr, int8_t* __restrict__ eflag) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < v.Nx) {
-        const double e = E[i];
-        bx[i] = c.dt * c.tau * (e * c.cA);
-        eflag[i] = (int8_t)((e >= 0.0 ? 1 : 0) | (e < 0.0 ? 2 : 0));
+        bx[i] = fvm_coef_field(c, E[i]);
+        eflag[i] = (int8_t)fvm_field_sign(E[i]);
     }
-    if (i < v.Nr) lr[i] = c.dt * c.tau * (c.kappa * v.loss[i]);
-    if (i < v.Nr * v.Nvt) arc[i] = c.dtx * c.ax * v.vr[i / v.Nvt] * v.cos_t[i % v.Nvt];
+    if (i < v.Nr) lr[i] = fvm_coef_loss(v, c, i);
+    if (i < v.Nr * v.Nvt) arc[i] = fvm_coef_drift(v, c, i / v.Nvt, i % v.Nvt);
 }
 
 // T = kt (G m) over the non-zeros of G's rows: at most two per process and row
@@ -124,7 +123,7 @@ __global__ void k_fvm_gain(int Nr, int Nx, double kt, const int32_t* __restrict_
     T[i] = bad[x] ? __longlong_as_double(0x7ff8000000000000ll) : kt * s;
 }
 
-// Y = rhs_mvec(X) (fvm_mvec_at) with the tabulated coefficients, one thread per value, x fastest:
+// Y = rhs_mvec(X) (fvm_mvec_tab_at) with the tabulated coefficients, one thread per value, x fastest:
 // three stencils and seven more FP64 instructions per value; the form that computes them all per
 // value took 33 with a division (976,000 values, 200 x 305 x 16: 61 us -> 29 us; 16 FP64
 // instructions take 26 us). T = dt tau kappa G m.
@@ -140,23 +139,7 @@ __global__ void k_fvm_mvec(FvmView v, const double* __restrict__ bx, const doubl
     const int rj = (int)(i / v.Nx);
     const int j = rj % v.Nvt, r = rj / v.Nvt;
     if (rj == 0) bad[x] = 0;  // the moments of the next product start clean
-    const double* line = X + (size_t)rj * v.Nx;
-    const double z = line[x];
-    const bool nx = v.north[j] != 0;
-    const double yx = z + arc[rj] * fvm_band_row(nx ? v.xL : v.xR, v.ndx, v.Nx, x, nx, line, 1);
-    if (fvm_inflow(v, j, x)) {
-        Y[i] = yx;
-        return;
-    }
-    const int e = eflag[x];
-    const bool up_r = ((e & 1) != 0) == (cpos[j] != 0);
-    const double dr = fvm_band_row(up_r ? v.vrR : v.vrL, v.ndr, v.Nr, r, !up_r, X + (size_t)j * v.Nx + x,
-                                   (long long)v.Nvt * v.Nx);
-    const bool lo_t = (e & 2) != 0;
-    const double dth = fvm_band_row(lo_t ? v.vtL : v.vtR, v.ndt, v.Nvt, j, lo_t, X + (size_t)r * v.Nvt * v.Nx + x,
-                                    (long long)v.Nx);
-    const double adv = v.cos_t[j] * dr - vinv[r] * dth;
-    Y[i] = (yx - T[(size_t)r * v.Nx + x]) + lr[r] * z - bx[x] * adv;
+    Y[i] = fvm_mvec_tab_at(v, bx[x], arc[rj], lr[r], vinv[r], eflag[x], cpos[j] != 0, T[(size_t)r * v.Nx + x], X, r, j, x);
 }
 
 // T = H M (Nr x Nr by Nr x Nx) for the collision inverse. One warp per 8 rows x 32 columns and a

@@ -69,25 +69,38 @@ FVM_HD double fvm_moment_at(const FvmView& v, const double* X, int r, int x) {
     return s;
 }
 
+// What rhs_mvec takes besides the vector, per x, per (r, j) and per r: the GPU tabulates these once per step
+FVM_HD double fvm_coef_field(const FvmCoef& c, double e) { return c.dt * c.tau * (e * c.cA); }
+FVM_HD double fvm_coef_drift(const FvmView& v, const FvmCoef& c, int r, int j) {
+    return c.dtx * c.ax * v.vr[r] * v.cos_t[j];
+}
+FVM_HD double fvm_coef_loss(const FvmView& v, const FvmCoef& c, int r) { return c.dt * c.tau * (c.kappa * v.loss[r]); }
+FVM_HD int fvm_field_sign(double e) { return (e >= 0.0 ? 1 : 0) | (e < 0.0 ? 2 : 0); }  // neither bit for a NaN
+
+// rhs_mvec at (r, j, x) with the coefficients above: arc the drift's, lr the loss's, bx the field's, vinv = 1 / v_r,
+// esign of fvm_field_sign, T = dt tau kappa times the gain applied to the moments of X, at (r, x)
+FVM_HD double fvm_mvec_tab_at(const FvmView& v, double bx, double arc, double lr, double vinv, int esign, bool cos_positive,
+                              double T, const double* X, int r, int j, int x) {
+    const double* line = X + ((size_t)r * v.Nvt + j) * v.Nx;
+    const double z = line[x];
+    const bool nx = v.north[j] != 0;
+    const double yx = z + arc * fvm_band_row(nx ? v.xL : v.xR, v.ndx, v.Nx, x, nx, line, 1);
+    if (fvm_inflow(v, j, x)) return yx;
+    const bool up_r = ((esign & 1) != 0) == cos_positive;
+    const double dr = fvm_band_row(up_r ? v.vrR : v.vrL, v.ndr, v.Nr, r, !up_r, X + (size_t)j * v.Nx + x,
+                                   (long long)v.Nvt * v.Nx);
+    const bool lo_t = (esign & 2) != 0;
+    const double dth = fvm_band_row(lo_t ? v.vtL : v.vtR, v.ndt, v.Nvt, j, lo_t, X + (size_t)r * v.Nvt * v.Nx + x,
+                                    (long long)v.Nx);
+    const double adv = v.cos_t[j] * dr - vinv * dth;
+    return (yx - T) + lr * z - bx * adv;
+}
+
 // rhs_mvec at (r, j, x); G = gain (Nr x Nr) applied to the moments of X, (Nr, Nx)
 FVM_HD double fvm_mvec_at(const FvmView& v, const FvmCoef& c, const double* E, const double* G, const double* X, int r,
                           int j, int x) {
-    const size_t line = ((size_t)r * v.Nvt + j) * v.Nx;
-    const double z = X[line + x];
-    const bool nx = v.north[j] != 0;
-    const double dx = fvm_band_row(nx ? v.xL : v.xR, v.ndx, v.Nx, x, nx, X + line, 1);
-    const double yx = z + c.dtx * c.ax * v.vr[r] * v.cos_t[j] * dx;
-    if (fvm_inflow(v, j, x)) return yx;
-    const double e = E[x];
-    const bool up_r = (e >= 0.0) == (v.cos_t[j] > 0.0);
-    const double dr = fvm_band_row(up_r ? v.vrR : v.vrL, v.ndr, v.Nr, r, !up_r, X + (size_t)j * v.Nx + x,
-                                   (long long)v.Nvt * v.Nx);
-    const bool lo_t = e < 0.0;
-    const double dth = fvm_band_row(lo_t ? v.vtL : v.vtR, v.ndt, v.Nvt, j, lo_t, X + (size_t)r * v.Nvt * v.Nx + x,
-                                    (long long)v.Nx);
-    const double adv = v.cos_t[j] * dr - dth / v.vr[r];
-    const double col = G[(size_t)r * v.Nx + x] - v.loss[r] * z;
-    return yx - c.dt * c.tau * (c.kappa * col + e * c.cA * adv);
+    return fvm_mvec_tab_at(v, fvm_coef_field(c, E[x]), fvm_coef_drift(v, c, r, j), fvm_coef_loss(v, c, r), 1.0 / v.vr[r],
+                           fvm_field_sign(E[x]), v.cos_t[j] > 0.0, c.dt * c.tau * c.kappa * G[(size_t)r * v.Nx + x], X, r, j, x);
 }
 
 // The collision inverse (I - c C)^-1 = D^-1 (x) I + (H (x) 1 w^T) at (r, j, x): T = H m, m the
