@@ -252,3 +252,45 @@ def test_rows_above_an_infinity_keep_their_values(N, kernel, dtype):
                                     _stream()), "lu_factor")
     torch.cuda.synchronize()
     assert torch.equal(F[:6], A[:6])
+
+
+@pytest.mark.parametrize("kernel,N,P", [(1, 100, 2), (1, 700, 2), (6, 33, 4096), (6, 193, 1024), (6, 513, 24), (6, 769, 2),
+                                        (6, 100, 2), (6, 385, 2)],
+                         ids=["one-cta", "one-cta-large", "split-33", "split-193", "split-513", "split-769", "cluster-100", "cluster-385"])
+def test_zero_pivot_in_every_fp64_kernel(kernel, N, P):
+    """The first zero pivot (1-based) of one matrix among others, in the first, a middle and the last panel and twice in
+    one matrix, from the one-CTA kernel, the split launches (the size rule's choice at these P) and a cluster."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    for zeros in ((3,), (N // 2,), (N - 1,), (N // 3, N - 2)):
+        A = torch.eye(N, device="cuda", dtype=torch.float64).repeat(P, 1, 1).contiguous()
+        for z in zeros:
+            A[P - 1, z, z] = 0.0
+        piv, info = torch.empty((P, N), dtype=torch.int32, device="cuda"), torch.empty(P, dtype=torch.int32, device="cuda")
+        _lib.check(lib.bte_lu_factor_ex(0, P, N, _ptr(A), N, N * N, _ptr(piv), _ptr(info), kernel, _stream()), "lu_factor")
+        torch.cuda.synchronize()
+        assert int(info[P - 1]) == zeros[0] + 1 and int(info[:P - 1].abs().max()) == 0
+        assert torch.equal(piv[P - 1].sort().values.long(), torch.arange(N, device="cuda"))
+
+
+@pytest.mark.parametrize("N,P", [(1, 4098), (8, 4098), (9, 4098), (32, 4098), (64, 8193), (128, 8193), (129, 8193), (193, 1026), (256, 402)])
+def test_fp64_small_factors_are_the_same_from_a_cluster_and_split(N, P):
+    """Sizes that the size rule gives to split launches only in large batches: the same bits as from a cluster in a batch
+    of three, with ties, a negative zero and rows that must be exchanged."""
+    import torch
+    from boltzmann_gb300 import _lib
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(N)
+    M = torch.randn((3, N, N), device="cuda", generator=g, dtype=torch.float64)
+    M[1] = torch.round(M[1] * 2) + 5 * torch.eye(N, dtype=torch.float64, device="cuda").flip(0)
+    if N > 2:
+        M[2, 0, 0] = -0.0
+    got = []
+    for n in (3, P):
+        A = M.repeat(n // 3, 1, 1).contiguous()
+        piv, info = torch.empty((n, N), dtype=torch.int32, device="cuda"), torch.empty(n, dtype=torch.int32, device="cuda")
+        _lib.check(lib.bte_lu_factor_ex(0, n, N, _ptr(A), N, N * N, _ptr(piv), _ptr(info), 6, _stream()), "lu_factor")
+        torch.cuda.synchronize()
+        got.append((A[-3:].clone(), piv[-3:].clone(), info[-3:].clone()))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
