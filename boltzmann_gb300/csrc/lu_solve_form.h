@@ -17,7 +17,8 @@ constexpr int SOLVE_MAX_N = 2048;
 // matrices: 43 us in FP32 against 55 with two groups per warp and loads when used). More
 // matrices than that hide one another's loads, and more resident CTAs pay: two groups per warp
 // without the prefetch registers (N = 385, 4096 matrices: 705 us against 984 in FP32, 2822
-// against 4161 in FP64). Up to N = 256 the prefetching form has one group per warp and two
+// against 4161 in FP64). The third CTA per SM is worth the registers that it makes spill (with two 828 us in
+// FP32, 3131 in FP64). Up to N = 256 the prefetching form has one group per warp and two
 // CTAs per SM and is the faster one for any P (N = 129, 4096 matrices: 146 us against 163). Above
 // N = 1400 the diagonal blocks of 16-byte loads no longer fit in shared memory.
 constexpr int solve_form(int P, int N) {
