@@ -452,10 +452,11 @@ k_lu_tc(int N, int NC, float* __restrict__ A, int ld, long long stride, int32_t*
         __syncthreads();
     }
     if (s_fault) {
-        // an MMA commit never arrived: wait once more (bounded) before giving TMEM back
+        // an MMA commit never arrived: wait once more (bounded) for its phase, the one before `phase`, before
+        // giving TMEM back
         if (tid == 0) {
             uint32_t it = 0;
-            while (!mbar_try_wait(mb, phase) && ++it < TC_WAIT_LIMIT) {}
+            while (!mbar_try_wait(mb, phase ^ 1u) && ++it < TC_WAIT_LIMIT) {}
         }
         __syncthreads();
     }
@@ -824,7 +825,7 @@ cudaError_t bte_lu_factor_tcs(int P, int N, int NC, float* A, int ld, long long 
 // largest N the tensor-core kernel takes (its panel is two 32-column rows per thread)
 int bte_lu_tc_max_n() { return 2 * TC_NT; }
 
-// variant 0: 256 threads, two CTAs per SM (the registers of two, 2 x 128 tensor-memory
+// variant 0: 256 threads, two CTAs per SM (the registers of two, 2 x 256 tensor-memory
 // columns); 1: 256 threads, one CTA per SM (half the matrices in flight, so that their
 // trailing updates stay in L2); 2: 128 threads (4 warps: half the per-column pivot-search work
 // per matrix, up to four panel rows per thread), two CTAs per SM
