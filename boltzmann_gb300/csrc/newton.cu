@@ -1441,6 +1441,10 @@ constexpr double STALL_RTOL = 1e-6;
 // 3.8e-9 (no point above 1e-8, 63 before) and FP64's own spread between two starting points
 // from 9.3e-8 to 3.0e-8, for 18% of the mixed form's throughput (7,505 against 9,155 solves/s;
 // switching every point at the floor cost 30%, a 1e-11 gate 23%).
+// A step above it at such an exit in double-double is not the floor's either: there the merit resolves
+// the step, and one that barely contracts it is inexact (FP32 factors whose refinement did not finish). The
+// point ends with stall_status: the mixed form hands it to FP64, whose step is taken in one or two
+// iterations. Points of the c2 batch had ended 1e-7 and 5e-9 from the fixed point so.
 constexpr double DD_STEP_RTOL = 1e-10;
 __global__ void k_armijo(int nact, const int* __restrict__ act, int* searching, double* alpha,
                          const double* __restrict__ r, const double* __restrict__ rt, double c, double rho,
@@ -1456,6 +1460,7 @@ __global__ void k_armijo(int nact, const int* __restrict__ act, int* searching, 
     bool ok = (0.5 * rn * rn <= 0.5 * rr * rr - c * al * rr * rr);
     if (!isfinite(rn)) ok = false;
     const bool tiny = srel[pt] <= step_rtol;
+    const int at_floor = (ddm && ddm[pt] && srel[pt] > DD_STEP_RTOL) ? stall_status : BTE_ST_ROUNDOFF;
     if (ok) {
         searching[pt] = 0;
         accepted[pt] = 1;
@@ -1465,7 +1470,7 @@ __global__ void k_armijo(int nact, const int* __restrict__ act, int* searching, 
                 ddm[pt] = 1;
                 ddpend[pt] = 1;
             } else {
-                status[pt] = BTE_ST_ROUNDOFF;
+                status[pt] = at_floor;
             }
         }
         return;
@@ -1483,7 +1488,7 @@ __global__ void k_armijo(int nact, const int* __restrict__ act, int* searching, 
         // fixture by their rounding floor, 1e-9, in either direction: no gain.)
         searching[pt] = 0;
         accepted[pt] = 0;
-        status[pt] = BTE_ST_ROUNDOFF;
+        status[pt] = at_floor;
         return;
     }
     al *= rho;
