@@ -585,7 +585,7 @@ def bench_1d(a, peaks):
             "value": 1e3 / ms, "unit": "steps/s", "ms_per_step": ms, "setup_s": t_setup,
             "gmres_iterations": {"mean": float(np.mean(its)), "max": int(np.max(its)), "min": int(np.min(its))},
             "gpu_launches_per_step": launches, "matvec_ms": mv_ms,
-            "roofline_matvec": {"kernel": "k_fim_dx + k_fim_combine", "bound": "fp64",
+            "roofline_matvec": {"kernel": "k_ords_to_lm + k_lmat + k_fim_dx + k_radial_mix + k_fim_combine", "bound": "fp64",
                                 "achieved": mv_flops / (mv_ms * 1e-3) / 1e12, "peak": fp64, "unit": "TFLOP/s",
                                 "frac": mv_flops / (mv_ms * 1e-3) / 1e12 / fp64,
                                 "peak_source": "nominal GB300 FP64 (no measured FP64 peak)",
@@ -681,7 +681,7 @@ def bench_fvm(a, peaks):
             "value": 1e3 / ms, "unit": "steps/s", "ms_per_step": ms, "setup_s": t_setup,
             "gmres_iterations": {"mean": float(np.mean(its)), "max": int(np.max(its))},
             "gpu_launches_per_step": launches, "matvec_ms": timing["matvec"], "precond_ms": timing["precond"],
-            "roofline_matvec": {"kernel": "k_fvm_moment + gain GEMM + k_fvm_mvec", "bound": "hbm",
+            "roofline_matvec": {"kernel": "k_fvm_moment + k_fvm_gain + k_fvm_mvec", "bound": "hbm",
                                 "achieved": mv_bytes / (timing["matvec"] * 1e-3) / 1e9, "peak": hbm, "unit": "GB/s",
                                 "frac": mv_bytes / (timing["matvec"] * 1e-3) / 1e9 / hbm, "alg_bytes": mv_bytes},
             "roofline_precond": {"kernel": "collision solve + coalesced v_r, v_theta, x sweeps", "bound": "hbm",

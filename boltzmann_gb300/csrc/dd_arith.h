@@ -1,7 +1,7 @@
 // Double-double accumulation of products: (hi, lo) += a * b with the product split exactly by
 // an fma (TwoProduct) and the sum by Knuth's TwoSum, the low parts gathered in lo and the pair
 // left unnormalised (hi + lo is the value). Used by the residual of a point at its FP64
-// rounding floor (newton.cu, residual_row_dd); compiled for the host by the CPU tests
+// rounding floor (newton.cu, k_residual); compiled for the host by the CPU tests
 // (tests/host/dd_harness.cpp), hence no CUDA-only constructs.
 #pragma once
 #include <cmath>

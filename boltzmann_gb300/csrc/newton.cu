@@ -1834,8 +1834,15 @@ extern "C" int bte_stats(double* out, int count) {
 // Coulomb product does not count towards the Jacobian's FP64 work; bytes moved to and from HBM)
 static double res_flops_pt(const BteGrid* g, int ee) {
     double n = g->n, nsp = g->nsp, tri = g->ntri;
-    double f = 2.0 * (nsp * nsp * g->nspecies + n * 7 * 4 + n * nsp);  // collisions, bands, M^-1 F
+    double f = 2.0 * (nsp * nsp * g->nspecies + n * 7 * 4);  // collisions, bands
     if (ee) f += 2.0 * (2 * n * nsp) + 2.0 * 2.0 * nsp * tri * BTE_PAIRS;   // potentials, trilinear form
+    return f;
+}
+// the refinement's FP64 product J x: the residual's terms with the e-e part through the stored coefficients
+static double ref_flops_pt(const BteGrid* g, int ee) {
+    double n = g->n, nsp = g->nsp, nsh = g->nsh;
+    double f = 2.0 * (nsp * nsp * g->nspecies + n * 7 * 4);
+    if (ee) f += 2.0 * (2 * n * nsp) + 2.0 * 3.0 * BTE_NB * nsh * n;
     return f;
 }
 static double res_bytes_pt(const BteGrid* g, bool trial) {
@@ -2052,8 +2059,11 @@ static int newton_iteration(SolveCtx& c, Lane& L, int nact, int prec) {
             for (int rf = 0; rf < nrefine; ++rf) {
                 double* cprev = (rf & 1) ? w->corr0 : w->corr1;
                 double* ccur = (rf & 1) ? w->corr1 : w->corr0;
-                CKR(pf.run(PF_REFINE, s, nact * (res_flops_pt(g, ee) + 2.0 * (double)N * N),
-                           nact * (res_bytes_pt(g, true) + 0.5 * N * (N + 1) * wsz), 3, [&] {
+                // counted: FP64 work (the substitution is FP32's), and of the first pass, which every point takes;
+                // how many take the later ones stays on the device. Their substitutions read every point's factors
+                const double fresh = rf == 0 ? nact : 0;
+                CKR(pf.run(PF_REFINE, s, fresh * ref_flops_pt(g, ee),
+                           fresh * res_bytes_pt(g, true) + nact * (double)N * (N + 1) * wsz, 3, [&] {
                     run_refine_residual(gv, nact, s, pp, ee, L.act, nact, w->h, w->F, w->aux,
                                                                   w->scal, w->dh, ldd, beta_scale, L.rowscale, xs,
                                                                   L.sigma, w->refdone, L.kc, nullptr, 0, nullptr, 0,
