@@ -46,7 +46,7 @@ int bte1d_step_v(bte1d* h, double dt, const double* E, double* V, double rtol, d
                  double* info4, void* stream);
 
 /* Y = X - dt (Cv X + E (Av X)) per point, x-major v-space layout (Lmat_mvec,
- * bte_1d3v_solver.py:1051-1055). */
+ * bte_1d3v_solver.py:1051-1055). Y may be X. */
 int bte1d_lmat(bte1d* h, double dt, const double* E, const double* X, double* Y, void* stream);
 
 /* Block preconditioner of the v-step: Y = B_x^-1 X per point, B_x = I - dt (Cv + E_x Av)

@@ -38,7 +38,10 @@ int bte_fvm_destroy(bte_fvm* h);
 
 /* The collision solve of the preconditioner, (I - c C)^-1 = diag(dinv) (x) I + H (x) 1 w^T
  * with c = gmres_pc_cv dt tau kappa: dinv [Nr] = 1 / (1 + c loss), H [Nr x Nr] row-major =
- * c D^-1 gain (D - c |w| gain)^-1, D = diag(1 + c loss). Replaces PmatC (:1346-1375). */
+ * c D^-1 gain (D - c |w| gain)^-1, D = diag(1 + c loss). Replaces PmatC (:1346-1375).
+ * Also allocates the table of the sweeps' coefficients, where the device has room for it beside the
+ * longest Krylov basis (501 vectors); without it the sweeps run on permuted copies, with results that
+ * differ by rounding. */
 int bte_fvm_set_collision_inverse(bte_fvm* h, const double* dinv, const double* H);
 
 /* Y = rhs_mvec(X) (:1915-1955): X v - dt tau (kappa C v + E (x) cA A_sign(E) v), the second

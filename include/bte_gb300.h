@@ -224,7 +224,8 @@ int bte_lu_factor_ex(int dtype, int P, int N, void* A, int ld, long long stride,
                      int kernel, void* stream);
 
 /* Solve A x = b for one right-hand side per matrix using bte_lu_factor's output;
- * b [P x N] (contiguous per point) is overwritten by x. Same dtype as the factors. */
+ * b [P x N] (contiguous per point) is overwritten by x. Same dtype as the factors. Factors of the
+ * caller's own may be larger than bte_lu_factor takes: N values fit in 227 KB. */
 int bte_lu_solve(int dtype, int P, int N, const void* A, int ld, long long stride,
                  const int32_t* piv, void* b, void* stream);
 
