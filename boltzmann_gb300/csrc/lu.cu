@@ -645,13 +645,13 @@ cudaError_t factor_split(int P, int N, int NC, T* A, int ld, long long stride, i
 //    block comes up (a transposing reduction, 7 shuffles for 32 rows). Eight lanes' sums over
 //    all columns grow larger, and their rounding errors with them, than the 32 of a form with a warp
 //    per row (N = 769: 1.6 times the error). So FP32 adds the products of a block first and adds over the
-//    lanes every 256 columns (every 512 above N = 512, where twice as often cost 12% of the time),
-//    and FP64, for whose pipe an addition costs what a product does, adds over the lanes every 128;
+//    lanes every 256 columns (every 512 above N = 512, which is enough there), and FP64, for whose pipe an
+//    addition costs what a product does, adds over the lanes every 128: at most 1.09 times;
 //  * the owner of a diagonal block only arrives at the barrier that publishes its x, and can be all
 //    the blocks of its row group ahead of the other warps (lu_solve_form.h: the barriers in turn).
 // Measured (us, the row-oriented kernel with dependent loads and a division per column before ->
-// now): N = 385: FP32 160 -> 43 (137 matrices) and 1235 -> 705 (4096), FP64 333 -> 158
-// (16) and 3469 -> 2822 (4096); N = 769, 75 matrices: FP32 1137 -> 124; N = 129, 24 matrices: FP64
+// now): N = 385: FP32 160 -> 44 (137 matrices) and 1235 -> 715 (4096), FP64 333 -> 162
+// (16) and 3469 -> 2814 (4096); N = 769, 75 matrices: FP32 1137 -> 131; N = 129, 24 matrices: FP64
 // 106 -> 58.
 // ---------------------------------------------------------------------------------
 // VEC elements per load: a block of 8 VEC columns

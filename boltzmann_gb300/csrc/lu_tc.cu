@@ -26,7 +26,7 @@
 // Bound by latency: the panel's chain of columns and the tiles' reads, writes and barriers; two CTAs
 // share an SM. Reading A22 only after the product, in groups of 16 rows, with tiles of 128 x 128 and
 // rows exchanged between threads under branches, one matrix of N = 385 took 708 us and 4096 took
-// 14.4 ms; now 352 us and 7.0 ms.
+// 14.4 ms; now 358 us and 7.0 ms.
 // Above N = 512 (k_tcs_*) the same steps are separate launches over many CTAs per matrix, with the operands
 // split into three BF16 parts.
 // The split: hi = tf32(x) (round to nearest), lo = x - hi (exact in FP32); hi*hi is exact
